@@ -13,7 +13,7 @@
 //                 the reference's 2x2x2 mean, AMR.h:961-996, is second order)
 //   RK4           four stages over every active domain (covered parents included: a same-depth
 //                 neighbour of a covered parent takes its ghost values from it at every stage):
-//                 derivative pass, then pointwise right-hand side and stage update; the ghost cells
+//                 derivatives, pointwise right-hand side and stage update; the ghost cells
 //                 of each stage's state and of the final state are filled from the neighbours
 //                 (three passes, x then y then z, so that edges and corners are filled too)
 //   ghost values  same-depth neighbour: its state at the same stage; coarser neighbour active at
@@ -61,9 +61,10 @@ enum WaveField : int { W_U = 0, W_V = 1, WAVE_NF = 2 };
 
 constexpr int kMaxFields = 24;
 
-// Derivative scratch written by the derivative pass, one float per inner cell each (slot * N^3 +
+// Derivative scratch written by the derivative pass (for the wave's RK stages and the BSSN
+// constraints; the BSSN stages keep no derivatives in memory), one float per inner cell each (slot * N^3 +
 // cell).  Symmetric second derivatives in the order xx, yy, zz, xy, xz, yz; first derivatives
-// x, y, z.  Where the right-hand side only uses a contraction with the inverse conformal metric,
+// x, y, z.  Where only a contraction with the inverse conformal metric is used,
 // the pass stores the contraction: GLAP[ij] = gt^lm d_l d_m gt_ij, BELAP[i] = gt^jk d_j d_k beta^i,
 // and DDIVB[j] = d_j d_k beta^k.  EXTRA[f] is the advection term beta^k d_k u_f plus the
 // Kreiss-Oliger term of field f.
@@ -120,6 +121,7 @@ struct EvoArgs {
     const uint32_t* positions;
     const uint32_t* items;        // active evolved slots
     uint32_t n_items;
+    uint32_t n_batch;             // domains of the whole substep (n_items, or more where each is launched alone)
     uint32_t n, p, t;             // size_domain, padding_domain, n + 2p
     float dt0;                    // dt at depth 0
     int stage;                    // 1..4

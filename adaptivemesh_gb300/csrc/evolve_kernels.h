@@ -95,7 +95,11 @@ cudaError_t launch_evo_init(const EvoInitArgs& a, cudaStream_t st);
 cudaError_t launch_evo_derivs(const EvoArgs& a, cudaStream_t st);
 // The derivative pass's compiled slab depths for size_domain n (written to out, at most 4); their count.
 uint32_t evo_deriv_zs_candidates(uint32_t n, uint32_t* out);
-cudaError_t launch_evo_rhs(const EvoArgs& a, cudaStream_t st);
+// One RK stage of the BSSN evolution (derivatives, right-hand side and stage update;
+// kernels_evolve_stage.cu), and the kernel's shared-memory limit, to be set outside a stream capture.
+cudaError_t prepare_evo_stage_bssn(uint32_t n);
+cudaError_t launch_evo_stage_bssn(const EvoArgs& a, cudaStream_t st);
+cudaError_t launch_evo_rhs_wave(const EvoArgs& a, cudaStream_t st);
 cudaError_t launch_evo_ghost(const EvoGhostArgs& g, cudaStream_t st);
 cudaError_t launch_evo_constraints(const EvoArgs& a, const ConsPtrs& cons, cudaStream_t st);
 // FP64 norms of the constraints over the composite grid of the listed slots (interior cells no child

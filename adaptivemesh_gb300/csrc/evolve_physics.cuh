@@ -1,6 +1,6 @@
-// evolve_physics.cuh -- pointwise physics of the evolution kernels: analytic initial data, the BSSN
-// right-hand side (moving-puncture form: 1+log or harmonic slicing, Gamma-driver shift) and the
-// Hamiltonian and momentum constraints.  The reference has none of these (its BSSN module stops at
+// evolve_physics.cuh -- pointwise physics of the evolution kernels: analytic initial data and the
+// Hamiltonian and momentum constraints; and the BSSN equations (moving-puncture form: 1+log or harmonic
+// slicing, Gamma-driver shift) that the RK stage kernel (kernels_evolve_stage.cu) evaluates.  The reference has none of these (its BSSN module stops at
 // metric derivatives and Christoffel symbols, BSSN.h:38-102); the equations follow the standard
 // conformal formulation (Baumgarte & Shapiro; Campanelli et al. and Baker et al. 2006 for the
 // puncture gauge), with chi = det(gamma)^(-1/3):
@@ -22,7 +22,7 @@
 //   H   = chi gt^ij R_ij + 2/3 K^2 - At_ij At^ij
 //   M_i = d_j At^j_i - 3/2 At^j_i d_j chi / chi - 1/2 At^jm d_i gt_jm - 2/3 d_i K
 //         (d_j At^j_i = gt^jk d_j At_ki - gt^ja gt^kb d_j gt_ab At_ki: the physical momentum constraint)
-// The advection terms beta.d u and the Kreiss-Oliger dissipation come from the derivative pass.
+// Every d_t u also has the Kreiss-Oliger dissipation of u.
 #pragma once
 
 #include <cmath>
@@ -103,8 +103,7 @@ __device__ __forceinline__ void evo_initial_values(const InitData& id, int physi
     }
 }
 
-// ------------------------------------------------------------------ the pieces both the right-hand
-// side and the constraints use
+// ------------------------------------------------------------------ the geometry the constraints use
 struct Geometry {
     float chi, ichi;              // chi, 1 / max(chi, floor)
     float g[6], gi[3][3];         // conformal metric and its inverse
@@ -189,102 +188,6 @@ __device__ __forceinline__ void geometry(const float* u, const DV& dv, const Evo
                  .25f * G.ichi * G.ichi * (G.dchi[i] * G.dchi[j] + 3.f * G.g[ij] * dchi2);
             G.R[ij] = r;
         }
-}
-
-// ------------------------------------------------------------------ BSSN right-hand side (without the
-// advection and dissipation terms, which the derivative pass supplies)
-template <class DV>
-__device__ __forceinline__ void bssn_rhs(const float* u, const DV& dv, const EvoParams& prm, float* rhs) {
-    Geometry G;
-    geometry(u, dv, prm, G);
-    const float K = u[F_K], alpha = u[F_ALPHA];
-    float A[6];
-    for (int c = 0; c < 6; c++) A[c] = u[F_AXX + c];
-    float dal[3], dK[3], db[3][3];
-    for (int k = 0; k < 3; k++) { dal[k] = dv(D_AL1 + k); dK[k] = dv(D_K1 + k); }
-    for (int i = 0; i < 3; i++)
-        for (int j = 0; j < 3; j++) db[i][j] = dv(D_BE1 + 3 * i + j);   // d_j beta^i
-    const float divb = db[0][0] + db[1][1] + db[2][2];
-    // At^i_j and At^ij
-    float Aud[3][3], Auu[3][3], AA = 0.f;
-    for (int i = 0; i < 3; i++)
-        for (int j = 0; j < 3; j++)
-            Aud[i][j] = G.gi[i][0] * A[sidx(0, j)] + G.gi[i][1] * A[sidx(1, j)] + G.gi[i][2] * A[sidx(2, j)];
-    for (int i = 0; i < 3; i++)
-        for (int j = 0; j < 3; j++) Auu[i][j] = Aud[i][0] * G.gi[0][j] + Aud[i][1] * G.gi[1][j] + Aud[i][2] * G.gi[2][j];
-    for (int i = 0; i < 3; i++)
-        for (int j = 0; j < 3; j++) AA += A[sidx(i, j)] * Auu[i][j];
-    // D_i D_j alpha (physical) and its trace
-    float dda[6], lap_a = 0.f;
-    float dchi_dal = 0.f;
-    for (int k = 0; k < 3; k++)
-        for (int l = 0; l < 3; l++) dchi_dal += G.gi[k][l] * G.dchi[k] * dal[l];
-    for (int i = 0; i < 3; i++)
-        for (int j = i; j < 3; j++) {
-            float v = dv(D_AL2 + didx(i, j));
-            for (int k = 0; k < 3; k++) v -= G.cu[k][sidx(i, j)] * dal[k];
-            v += .5f * G.ichi * (G.dchi[i] * dal[j] + G.dchi[j] * dal[i] - G.g[sidx(i, j)] * dchi_dal);
-            dda[sidx(i, j)] = v;
-        }
-    for (int i = 0; i < 3; i++)
-        for (int j = 0; j < 3; j++) lap_a += G.gi[i][j] * dda[sidx(i, j)];
-    lap_a *= G.chi;
-    // chi
-    rhs[F_CHI] = (2.f / 3.f) * G.chi * (alpha * K - divb);
-    // conformal metric
-    for (int i = 0; i < 3; i++)
-        for (int j = i; j < 3; j++) {
-            float v = -2.f * alpha * A[sidx(i, j)] - (2.f / 3.f) * G.g[sidx(i, j)] * divb;
-            for (int k = 0; k < 3; k++) v += G.g[sidx(i, k)] * db[k][j] + G.g[sidx(j, k)] * db[k][i];
-            rhs[F_GXX + sidx(i, j)] = v;
-        }
-    // K
-    rhs[F_K] = -lap_a + alpha * (AA + K * K * (1.f / 3.f));
-    // trace-free part of -D_i D_j alpha + alpha R_ij
-    float X[6], trX = 0.f;
-    for (int c = 0; c < 6; c++) X[c] = -dda[c] + alpha * G.R[c];
-    for (int i = 0; i < 3; i++)
-        for (int j = 0; j < 3; j++) trX += G.gi[i][j] * X[sidx(i, j)];
-    for (int i = 0; i < 3; i++)
-        for (int j = i; j < 3; j++) {
-            const int ij = sidx(i, j);
-            float v = G.chi * (X[ij] - G.g[ij] * trX * (1.f / 3.f));
-            v += alpha * (K * A[ij] - 2.f * (A[sidx(i, 0)] * Aud[0][j] + A[sidx(i, 1)] * Aud[1][j] + A[sidx(i, 2)] * Aud[2][j]));
-            v -= (2.f / 3.f) * A[ij] * divb;
-            for (int k = 0; k < 3; k++) v += A[sidx(i, k)] * db[k][j] + A[sidx(j, k)] * db[k][i];
-            rhs[F_AXX + ij] = v;
-        }
-    // conformal connection functions (core: without advection)
-    float ddivb[3];   // d_j (d_k beta^k)
-    for (int j = 0; j < 3; j++) ddivb[j] = dv(D_DDIVB + j);
-    float gcore[3];
-    for (int i = 0; i < 3; i++) {
-        float v = (2.f / 3.f) * u[F_GAMX + i] * divb;
-        for (int k = 0; k < 3; k++) v -= u[F_GAMX + k] * db[i][k];
-        v += dv(D_BELAP + i);   // gt^jk d_j d_k beta^i
-        float s1 = 0.f, s2 = 0.f, s3 = 0.f;
-        for (int j = 0; j < 3; j++) {
-            v += (1.f / 3.f) * G.gi[i][j] * ddivb[j] - 2.f * Auu[i][j] * dal[j];
-            s2 += Auu[i][j] * G.dchi[j];
-            s3 += G.gi[i][j] * dK[j];
-            for (int k = 0; k < 3; k++) s1 += G.cu[i][sidx(j, k)] * Auu[j][k];
-        }
-        v += 2.f * alpha * (s1 - 1.5f * s2 * G.ichi - (2.f / 3.f) * s3);
-        gcore[i] = v;
-        rhs[F_GAMX + i] = v;
-    }
-    // lapse
-    rhs[F_ALPHA] = prm.slicing == AMR_SLICING_HARMONIC ? -alpha * alpha * K : -2.f * alpha * K;
-    // shift and its driver
-    for (int i = 0; i < 3; i++) {
-        if (prm.shift) {
-            rhs[F_BETAX + i] = .75f * u[F_BX + i];
-            rhs[F_BX + i] = gcore[i] - prm.eta * u[F_BX + i];
-        } else {
-            rhs[F_BETAX + i] = 0.f;
-            rhs[F_BX + i] = 0.f;
-        }
-    }
 }
 
 // Hamiltonian constraint and the three components of the momentum constraint.

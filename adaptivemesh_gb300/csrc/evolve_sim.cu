@@ -7,8 +7,9 @@
 //                 AMR.h:961-996, averages the 2x2x2 cells: second order)
 //   modify_nodes  nothing (regridding is driven from outside between timesteps: amr_sim_regrid, or
 //                 amr_sim_add_nodes / remove_nodes; new domains are interpolated tricubically)
-//   predictor     the four RK4 stages over the active evolved domains, each a derivative pass and a
-//                 pointwise update, with the ghost cells of stages 2-4 filled in between
+//   predictor     the four RK4 stages over the active evolved domains (BSSN: one kernel each; wave: a
+//                 derivative pass and a pointwise update), with the ghost cells of stages 2-4 filled
+//                 in between
 //   copy_bounds   ghost fill of the final state (so that the next restriction copies valid ghosts)
 //   corrector     nothing (RK4 has no separate corrector stage)
 // Modes: PLAIN launches every kernel once per domain (the plain per-domain form), BATCHED once per
@@ -63,11 +64,12 @@ public:
         if (e == cudaSuccess) e = dev_alloc(&d_lists, s * 2u * ((size_t)1u << kDepthLimit) + 2u * s);
         if (e == cudaSuccess) e = dev_alloc(&d_part, s * 5u);
         if (e == cudaSuccess) e = dev_alloc(&d_norms, 8);
-        if (e == cudaSuccess) {   // the derivative pass's shared-memory limit, outside any stream capture
+        if (e == cudaSuccess) {   // the stage kernels' shared-memory limits, outside any stream capture
             EvoArgs none;
             std::memset(&none, 0, sizeof(none));
             none.n = dims.n;
             e = launch_evo_derivs(none, stream);
+            if (e == cudaSuccess && kind == AMR_SIM_BSSN_EVOLVE) e = prepare_evo_stage_bssn(dims.n);
         }
         return cuda_status(e);
     }
@@ -230,17 +232,16 @@ public:
         for (int stage = 1; stage <= 4; stage++) {
             EvoArgs a = args(s, in[stage - 1], out[stage - 1], stage, 0);
             if (mode == AMR_MODE_PLAIN) {
-                // the plain per-domain form: each domain's derivative pass and update launched alone
+                // the plain per-domain form: each domain's stage launched alone
                 const uint32_t* base = a.items;
                 for (uint32_t i = 0; i < evo_cnt[s]; i++) {
                     a.items = base + i;
                     a.n_items = 1;
-                    if ((st = check(launch_evo_derivs(a, stream))) || (st = check(launch_evo_rhs(a, stream)))) return st;
+                    if ((st = stage_update(a))) return st;
                 }
             } else {
-                if ((st = check(launch_evo_derivs(a, stream)))) return st;
                 time_begin();
-                if ((st = check(launch_evo_rhs(a, stream)))) return st;
+                if ((st = stage_update(a))) return st;
                 time_end();
             }
             if (stage < 4 && (st = fill(s, out[stage - 1], c_next[stage - 1]))) return st;
@@ -332,8 +333,8 @@ public:
     }
     // Launch-shape tuning of the derivative pass (amr_sim_autotune): its slab depth (interior
     // z-planes per CTA) timed at every compiled depth over all evolved domains, reps launches each
-    // with CUDA events; the fastest is kept.  The pass writes only its derivative scratch, which
-    // every RK stage rewrites, so the state is unchanged.
+    // with CUDA events; the fastest is kept.  The pass writes only its derivative scratch, which its
+    // users (the wave's RK stages, the constraints) rewrite, so the state is unchanged.
     int autotune(uint32_t reps, uint32_t* n_tuned) override {
         if (n_tuned) *n_tuned = 0;
         if (capturing || reps == 0u || reps > 100u) return AMR_ERR_INVALID;
@@ -547,7 +548,7 @@ private:
         a.deriv_stride = (uint64_t)tree.max_slots() * dims.n * dims.n * dims.n;
         a.positions = d_positions;
         a.items = d_lists + (evo_off.empty() ? 0u : evo_off[s]);
-        a.n_items = evo_cnt.empty() ? 0u : evo_cnt[s];
+        a.n_items = a.n_batch = evo_cnt.empty() ? 0u : evo_cnt[s];
         a.n = dims.n;
         a.p = dims.p;
         a.t = dims.t;
@@ -558,6 +559,12 @@ private:
         a.prm = prm;
         a.err = err_flag;
         return a;
+    }
+    // one RK stage: the BSSN evolution in one kernel, the wave's derivative pass and update
+    int stage_update(const EvoArgs& a) {
+        if (kind == AMR_SIM_BSSN_EVOLVE) return check(launch_evo_stage_bssn(a, stream));
+        const int st = check(launch_evo_derivs(a, stream));
+        return st ? st : check(launch_evo_rhs_wave(a, stream));
     }
     // ghost fill of `x` (the state at c_stage of the active domains' step), three axis passes
     int fill(uint32_t s, float* const* x, float c_stage) {

@@ -7,9 +7,10 @@
 //   k_evo_init      analytic initial data on every cell (ghosts included) of every live slot
 //   k_evo_derivs    derivative pass: a CTA per (domain, z-slab); each field's padded slab moves into
 //                   shared memory with one 1-D bulk copy (two buffers, the next field in flight),
-//                   then first / second / mixed derivatives, advection and Kreiss-Oliger terms
-//   k_evo_rhs_*     pointwise right-hand side and RK4 stage update (BSSN: every input staged in
-//                   shared memory by bulk copies and cp.async first)
+//                   then first / second / mixed derivatives, advection and Kreiss-Oliger terms (the
+//                   wave's RK stages and the BSSN constraints; the BSSN stages are one kernel,
+//                   kernels_evolve_stage.cu)
+//   k_evo_rhs_wave  the wave's pointwise right-hand side and RK4 stage update
 //   k_evo_ghost     ghost fill of a stage's state, one face-normal axis per launch (copies from
 //                   same-depth neighbours, separable tricubic interpolation from coarser ones)
 //   k_evo_restrict  restriction of children into parents (leaves: 16-byte copies)
@@ -290,10 +291,8 @@ __global__ void __launch_bounds__(DerivShape<N, ZS_>::THREADS, DerivShape<N, ZS_
 // ------------------------------------------------------------------ right-hand sides and stage update
 // RK4: stage 1: acc = old + dt/6 k1, out = old + dt/2 k1; stage 2: acc += dt/3 k2, out = old + dt/2 k2;
 // stage 3: acc += dt/3 k3, out = old + dt k3; stage 4: out = acc + dt/6 k4.
-// `lo`: the stage outputs' lower bound (the conformal factor's floor; -inf for the other fields).
-// A NaN stays a NaN.
 __device__ __forceinline__ void rk_update(const EvoArgs& a, int f, uint64_t pi, uint64_t ii, float u_old, float r,
-                                          float dt, float lo = -INFINITY) {
+                                          float dt) {
     float v;
     switch (a.stage) {
         case 1:
@@ -312,109 +311,7 @@ __device__ __forceinline__ void rk_update(const EvoArgs& a, int f, uint64_t pi, 
             v = fmaf(dt * (1.f / 6.f), r, a.acc[f][ii]);
             break;
     }
-    a.out[f][pi] = v < lo ? lo : v;
-}
-
-// BSSN right-hand side and RK stage update: a CTA per kRhsCells consecutive interior cells of one
-// domain, every input in shared memory before the arithmetic starts.  Thread 0 issues one bulk
-// copy per derivative plane (and, after the first stage, per RK-accumulator plane): kRhsCells * 4
-// contiguous bytes of the inner layout each, counted on one mbarrier.  Every thread meanwhile
-// issues 4-byte asynchronous copies (cp.async) of its cell's fields and their step-start values
-// from the padded layout, and waits for its own.  Consecutive threads read consecutive words.
-// Stage 1 stages the derivatives and fields, stages 2 and 3 also the step-start values and the
-// accumulator, stage 4 the accumulator only (it updates from it): 30, 42 and 36 KB per CTA, so
-// 6, 5 and 6 CTAs per SM (128 cells at stages 2-3: 2 CTAs per SM, 539 against 480 us).
-constexpr int kRhsCells = 64;
-__host__ __device__ constexpr int rhs_planes(int stage) {   // derivatives, fields, [step-start values], [accumulator]
-    return BSSN_ND + BSSN_NF + (stage == 2 || stage == 3 ? 2 * BSSN_NF : (stage == 4 ? BSSN_NF : 0));
-}
-constexpr size_t rhs_smem(int stage) { return (size_t)rhs_planes(stage) * kRhsCells * 4u + 16u; }
-constexpr size_t kRhsSmem = rhs_smem(2);   // the largest
-
-__device__ __forceinline__ void cp_async4(float* dst_smem, const float* src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_addr(dst_smem)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_wait_all() {
-    asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
-}
-
-template <int N>
-__global__ void __launch_bounds__(kRhsCells) k_evo_rhs_bssn(const __grid_constant__ EvoArgs a) {
-    constexpr int P = 3, T = N + 2 * P, C = kRhsCells;
-    constexpr uint32_t CHUNKS = (uint32_t)(N * N * N / kRhsCells);
-    static_assert((N * N * N) % kRhsCells == 0 && (kRhsCells * 4) % 16 == 0, "whole, aligned chunks per domain");
-    extern __shared__ __align__(128) unsigned char smem_raw[];
-    const bool later = a.stage != 1;                        // stages 2-4 read the accumulator
-    const bool start = a.stage == 2 || a.stage == 3;        // stages 2-3 the step-start state
-    float* sd = reinterpret_cast<float*>(smem_raw);   // [BSSN_ND][C] derivatives
-    float* su = sd + (size_t)BSSN_ND * C;              // [BSSN_NF][C] fields (stored form)
-    float* so = su + (size_t)BSSN_NF * C;              // [BSSN_NF][C] step-start values (stages 2-3)
-    float* sa = so + (start ? (size_t)BSSN_NF * C : 0u);   // [BSSN_NF][C] RK accumulator (stages 2-4)
-    uint64_t* bar = reinterpret_cast<uint64_t*>(sa + (later ? (size_t)BSSN_NF * C : 0u));
-    const uint32_t tid = threadIdx.x;
-    const uint32_t item = blockIdx.x / CHUNKS, chunk = blockIdx.x % CHUNKS;
-    if (item >= a.n_items) return;   // the whole CTA
-    const uint32_t slot = a.items[item];
-    const uint32_t cell = chunk * (uint32_t)kRhsCells + tid;
-    const uint64_t ii0 = (uint64_t)slot * N * N * N + chunk * (uint32_t)kRhsCells;
-    if (tid == 0) {
-        mbar_init(bar, 1);
-        mbar_fence_init();
-    }
-    __syncthreads();
-    if (tid == 0) {
-        mbar_arrive_expect_tx(bar, (uint32_t)((BSSN_ND + (later ? BSSN_NF : 0)) * C * 4));
-        for (int k = 0; k < BSSN_ND; k++)
-            bulk_g2s(sd + k * C, a.deriv + (uint64_t)k * a.deriv_stride + ii0, C * 4u, bar);
-        if (later)
-            for (int f = 0; f < BSSN_NF; f++) bulk_g2s(sa + f * C, a.acc[f] + ii0, C * 4u, bar);
-    }
-    const uint32_t x = cell % N, y = (cell / N) % N, z = cell / (N * N);
-    const uint64_t pi = (uint64_t)slot * T * T * T + ((uint64_t)(z + P) * T + (y + P)) * T + (x + P);
-    const uint64_t ii = ii0 + tid;
-#pragma unroll
-    for (int f = 0; f < BSSN_NF; f++) {
-        cp_async4(su + f * C + tid, a.fields[f] + pi);
-        if (start) cp_async4(so + f * C + tid, a.old_f[f] + pi);
-    }
-    const int depth = pos_depth(a.positions[slot]);
-    const float dt = a.dt0 / (float)(1u << depth);
-    cp_async_wait_all();   // this thread's own copies (only it reads them)
-    // every bulk copy lands before any thread reads them or leaves (bounded waits)
-    const bool ok = __syncthreads_and(mbar_wait(bar, 0));
-    if (!ok) {
-        if (tid == 0) {
-            atomicExch(a.err, 1);
-            mbar_wait(bar, 0);
-        }
-        __syncthreads();
-        return;
-    }
-    float u[BSSN_NF];
-#pragma unroll
-    for (int f = 0; f < BSSN_NF; f++) u[f] = su[f * C + tid] + bssn_offset(f);
-    auto dv = [&](int k) { return sd[k * C + tid]; };
-    float rhs[BSSN_NF];
-    bssn_rhs(u, dv, a.prm, rhs);
-    // RK4 (rk_update): stage 1: acc = old + dt/6 k1, out = old + dt/2 k1; stage 2: acc += dt/3 k2,
-    // out = old + dt/2 k2; stage 3: acc += dt/3 k3, out = old + dt k3; stage 4: out = acc + dt/6 k4
-    const float c_acc = a.stage == 1 ? dt * (1.f / 6.f) : dt * (1.f / 3.f);
-    const float c_out = a.stage == 3 ? dt : (a.stage == 4 ? dt * (1.f / 6.f) : dt * .5f);
-#pragma unroll
-    for (int f = 0; f < BSSN_NF; f++) {
-        const float r = rhs[f] + dv(D_EXTRA + f);
-        float v;
-        if (a.stage == 4) {
-            v = fmaf(c_out, r, sa[f * C + tid]);
-        } else {
-            const float uo = start ? so[f * C + tid] : su[f * C + tid];   // the stored form
-            a.acc[f][ii] = fmaf(c_acc, r, later ? sa[f * C + tid] : uo);
-            v = fmaf(c_out, r, uo);
-        }
-        // chi (stored less 1) is kept at or above its floor, as the geometry divides by it
-        const float lo = f == F_CHI ? a.prm.chi_floor - 1.f : -INFINITY;
-        a.out[f][pi] = v < lo ? lo : v;
-    }
+    a.out[f][pi] = v;
 }
 
 template <int N>
@@ -976,18 +873,10 @@ template <int N>
 static cudaError_t rhs_t(const EvoArgs& a, cudaStream_t st) {
     const uint64_t total = (uint64_t)a.n_items * N * N * N;
     if (total == 0) return cudaSuccess;
-    if (a.prm.physics == 0) {
-        static std::atomic<uint64_t> configured{0};
-        const cudaError_t e = ensure_smem_limit(k_evo_rhs_bssn<N>, kRhsSmem, configured);
-        if (e != cudaSuccess) return e;
-        if (a.stage < 1 || a.stage > 4) return cudaErrorInvalidValue;
-        k_evo_rhs_bssn<N><<<(unsigned)(total / kRhsCells), kRhsCells, rhs_smem(a.stage), st>>>(a);
-    } else {
-        k_evo_rhs_wave<N><<<(unsigned)((total + 255) / 256), 256, 0, st>>>(a);
-    }
+    k_evo_rhs_wave<N><<<(unsigned)((total + 255) / 256), 256, 0, st>>>(a);
     return cudaGetLastError();
 }
-cudaError_t launch_evo_rhs(const EvoArgs& a, cudaStream_t st) {
+cudaError_t launch_evo_rhs_wave(const EvoArgs& a, cudaStream_t st) {
     switch (a.n) {
         case 8: return rhs_t<8>(a, st);
         case 16: return rhs_t<16>(a, st);
