@@ -9,23 +9,26 @@
 //   conv2  16 -> 16 channels, 3x3x3, padding 1, stride 2, ReLU     -> 16 x 4^3 = 1024
 //   fc1    1024 -> 32, ReLU
 //   fc2    32 -> 1 (the predicted log10 truncation error of the tile)
-// The convolutions and fc1 run as GEMMs on the fifth-generation tensor cores (tcgen05.mma kind::f16,
-// BF16 operands in shared memory, FP32 accumulation in Tensor Memory) over im2col matrices; the
-// backward pass uses the same GEMM for the weight and input gradients.  Master weights, gradients and the Adam moments are FP32; the GEMM operands
-// (weights, activations, back-propagated gradients) are rounded to BF16.
+// The convolutions and the weight gradients run as GEMMs on the fifth-generation tensor cores
+// (tcgen05.mma kind::f16, BF16 operands in shared memory, FP32 accumulation in Tensor Memory) whose
+// operands are gathered from the activations.
+// Master weights, gradients and the Adam moments are FP32; the products' operands (weights,
+// activations, back-propagated gradients) are rounded to BF16.
 //
-// Layouts: activations are position-major, channel-last ([tile][position][channel]); im2col column
-// j = channel * 27 + (dz * 9 + dy * 3 + dx) for the tap at offset (dx, dy, dz) - 1; conv1's 81
-// columns are padded to 96 with zeros.  The flat parameter vector is W1[96][16], b1[16],
+// Layouts: activations are position-major, channel-last ([tile][position][channel]); receptive-field
+// index j = channel * 27 + (dz * 9 + dy * 3 + dx) for the tap at offset (dx, dy, dz) - 1; conv1's 81
+// are padded to 96 with zeros.  The flat parameter vector is W1[96][16], b1[16],
 // W2[432][16], b2[16], W3[1024][32], b3[32], W4[32], b4[1] (row-major, K rows by N columns).
 #include <cuda_bf16.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <new>
 #include <vector>
 
 #include "capi_internal.h"
+#include "kernels.h"
 #include "tcgen05.cuh"
 
 namespace amr {
@@ -42,31 +45,33 @@ constexpr size_t kOffW1 = 0, kOffB1 = kOffW1 + kK1 * kC1, kOffW2 = kOffB1 + kC1,
                  kOffB4 = kOffW4 + kF, kParams = kOffB4 + 1;
 
 // ------------------------------------------------------------------ BF16 GEMM on the tensor cores
-// C[m][n] (+)= sum_k A(m, k) B(k, n); A(m, k) = A[m * sam + k * sak], B(k, n) = B[k * sbk + n * sbn],
-// C[m * scm + n * scn] (FP32).  A CTA of 4 warps computes a 128 x NT tile (NT = 16 or 32) with the
-// fifth-generation tensor cores: per K block of 64 the threads stage A (128 x 64) and B (NT x 64)
-// into shared memory as K-major core matrices (zero past the edges), one thread issues four
-// tcgen05.mma of K = 16 into a TMEM accumulator and commits them to an mbarrier, and after the last
-// block each warp reads its 32 rows of the accumulator back with tcgen05.ld.  Every wait is bounded;
-// a wait that runs out raises *err, waits once more for the MMAs in flight and frees the TMEM.
-struct GemmArgs {
-    const bf16* A;
-    int64_t sam, sak;
-    const bf16* B;
-    int64_t sbk, sbn;
-    float* C;
-    int64_t scm, scn;
-    int M, N, K;
-    int accumulate;   // 1: C += A B, 0: C = A B
-    int* err;         // device flag raised when a wait gives up
-};
-
+// C = A B for one 128 x NT tile (NT = 16 or 32) and one range of K per CTA of 4 warps, on the
+// fifth-generation tensor cores: per K block of 64 the threads stage A (128 x 64) and B (NT x 64) into
+// shared memory as K-major core matrices, one thread issues four tcgen05.mma of K = 16 into a TMEM
+// accumulator and commits them to an mbarrier, and after the last block each warp reads its 32 rows of
+// the accumulator back with tcgen05.ld and hands each row to the epilogue.  Every wait is bounded; a
+// wait that runs out raises *err, waits once more for the MMAs in flight and frees the TMEM.
+//
+// The operands are functors: thread t stages row t of A, eight K values (16 bytes) at a time, so that
+// the convolutions gather their receptive fields straight from the activations (no im2col matrix in
+// memory, 98 KB a tile for conv1 before) and a row's geometry is computed once; a block's values are
+// loaded while the block before it is multiplied.  The epilogue takes the bias, the ReLU and its
+// backward form, which were passes of their own.
 constexpr int kGemmM = 128, kGemmK = 64;
 
-template <int NT>
-__global__ void __launch_bounds__(128) k_gemm_bf16(const GemmArgs g) {
+struct __align__(16) Chunk {   // eight consecutive K values of one row
+    bf16 v[8];
+};
+__device__ __forceinline__ Chunk zero_chunk() {
+    Chunk c;
+    *reinterpret_cast<uint4*>(&c) = make_uint4(0u, 0u, 0u, 0u);
+    return c;
+}
+
+template <int NT, class A, class B, class Epilogue>
+__global__ void __launch_bounds__(128) k_gemm_bf16(const A fa, const B fb, const Epilogue epi, int K, int* err) {
     static_assert(NT == 16 || NT == 32, "M = 128 tiles take N in multiples of 16; 32 TMEM columns");
-    constexpr int MT = kGemmM, KT = kGemmK;
+    constexpr int MT = kGemmM, KT = kGemmK, BC = NT * KT / 8 / 128;   // chunks of B per thread
     constexpr uint32_t LBO = 128u, SBO = (KT / 8) * 128u;   // bytes between core matrices along K / M
     __shared__ __align__(1024) bf16 As[MT * KT];
     __shared__ __align__(1024) bf16 Bs[NT * KT];
@@ -74,7 +79,7 @@ __global__ void __launch_bounds__(128) k_gemm_bf16(const GemmArgs g) {
     __shared__ uint32_t s_tmem;
     __shared__ int s_fail;
     const int tid = threadIdx.x, warp = tid / 32;
-    const int m0 = blockIdx.y * MT, n0 = blockIdx.x * NT;
+    const int m = blockIdx.x * MT + tid, n0 = blockIdx.y * NT;
     if (warp == 0) tmem_alloc(&s_tmem, 32u);   // the 128 x NT FP32 accumulator
     if (tid == 0) {
         mbar_init(&bar, 1);
@@ -87,21 +92,29 @@ __global__ void __launch_bounds__(128) k_gemm_bf16(const GemmArgs g) {
     if (warp == 0) tmem_relinquish();
     const uint32_t tmem = s_tmem;
     constexpr uint32_t idesc = umma_idesc_bf16_f32(MT, NT);
-    const bf16 zero = __float2bfloat16_rn(0.f);
-    // element (row r, k) of a K-major operand: core matrix (r / 8, k / 8) of 64 elements, row r % 8
-    auto at = [](int r, int k) { return ((r >> 3) * (KT / 8) + (k >> 3)) * 64 + (r & 7) * 8 + (k & 7); };
+    // chunk k of row r: core matrix (r / 8, k) of eight 16-byte rows, row r % 8
+    auto at = [](int r, int k) { return (r >> 3) * (KT / 8) * 8 + k * 8 + (r & 7); };
+    Chunk* const a16 = reinterpret_cast<Chunk*>(As);
+    Chunk* const b16 = reinterpret_cast<Chunk*>(Bs);
     uint32_t phase = 0;
-    const int nkb = (g.K + KT - 1) / KT;
+    const int nkb = (K + KT - 1) / KT;
+    const auto row = fa.row(m);
+    Chunk ca[KT / 8], cb[BC];
+    auto load = [&](int k0) {
+#pragma unroll
+        for (int k = 0; k < KT / 8; k++) ca[k] = fa(row, k0 + 8 * k);
+#pragma unroll
+        for (int i = 0; i < BC; i++) {
+            const int e = tid + 128 * i;
+            cb[i] = fb(n0 + e % NT, k0 + 8 * (e / NT));
+        }
+    };
+    load(0);
     for (int kb = 0; kb < nkb; kb++) {
-        const int k0 = kb * KT;
-        for (int e = tid; e < MT * KT; e += 128) {
-            const int r = e / KT, c = e % KT, m = m0 + r, k = k0 + c;
-            As[at(r, c)] = (m < g.M && k < g.K) ? g.A[(int64_t)m * g.sam + (int64_t)k * g.sak] : zero;
-        }
-        for (int e = tid; e < NT * KT; e += 128) {
-            const int r = e / KT, c = e % KT, n = n0 + r, k = k0 + c;
-            Bs[at(r, c)] = (n < g.N && k < g.K) ? g.B[(int64_t)k * g.sbk + (int64_t)n * g.sbn] : zero;
-        }
+#pragma unroll
+        for (int k = 0; k < KT / 8; k++) a16[at(tid, k)] = ca[k];
+#pragma unroll
+        for (int i = 0; i < BC; i++) b16[at((tid + 128 * i) % NT, (tid + 128 * i) / NT)] = cb[i];
         fence_proxy_async_smem();   // these writes, visible to the tensor core
         __syncthreads();
         if (tid == 0) {
@@ -113,6 +126,7 @@ __global__ void __launch_bounds__(128) k_gemm_bf16(const GemmArgs g) {
                           idesc, kb > 0 || kk > 0);
             umma_commit(&bar);
         }
+        if (kb + 1 < nkb) load((kb + 1) * KT);
         // the block's MMAs have read As and Bs once the barrier's phase completes
         const bool ok = mbar_wait(&bar, phase);
         phase ^= 1u;
@@ -126,17 +140,9 @@ __global__ void __launch_bounds__(128) k_gemm_bf16(const GemmArgs g) {
         const uint32_t row_addr = tmem + ((uint32_t)(warp * 32) << 16);   // lanes 32 w .. 32 w + 31
         tmem_ld16(row_addr, v);
         if constexpr (NT == 32) tmem_ld16(row_addr + 16u, v + 16);
-        const int m = m0 + warp * 32 + (tid & 31);
-        if (m < g.M) {
-#pragma unroll
-            for (int n = 0; n < NT; n++)
-                if (n0 + n < g.N) {
-                    float* c = g.C + (int64_t)m * g.scm + (int64_t)(n0 + n) * g.scn;
-                    *c = g.accumulate ? *c + v[n] : v[n];
-                }
-        }
+        epi(m, n0, v);
     } else if (tid == 0) {
-        atomicExch(g.err, 1);
+        atomicExch(err, 1);
         mbar_wait(&bar, phase ^ 1u);   // the MMAs of the block whose wait gave up
     }
     tc_fence_before_sync();
@@ -147,49 +153,372 @@ __global__ void __launch_bounds__(128) k_gemm_bf16(const GemmArgs g) {
     }
 }
 
-cudaError_t gemm(GemmArgs g, cudaStream_t st) {
-    if (g.M <= 0 || g.N <= 0) return cudaSuccess;
-    if (!g.err) g.err = device_error_flag();
-    if (!g.err) return cudaErrorMemoryAllocation;
-    const int nt = g.N <= 16 ? 16 : 32;
-    const dim3 grid((unsigned)((g.N + nt - 1) / nt), (unsigned)((g.M + kGemmM - 1) / kGemmM));
-    if (nt == 16) k_gemm_bf16<16><<<grid, 128, 0, st>>>(g);
-    else k_gemm_bf16<32><<<grid, 128, 0, st>>>(g);
+// C (rows x cols) over all of K
+template <int NT, class A, class B, class Epilogue>
+cudaError_t gemm(const A& fa, const B& fb, const Epilogue& epi, int rows, int cols, int K, cudaStream_t st) {
+    if (rows <= 0 || K <= 0) return cudaSuccess;
+    int* err = device_error_flag();
+    if (!err) return cudaErrorMemoryAllocation;
+    k_gemm_bf16<NT><<<dim3((unsigned)((rows + kGemmM - 1) / kGemmM), (unsigned)((cols + NT - 1) / NT)), 128, 0, st>>>(fa, fb, epi,
+                                                                                                                 K, err);
     return cudaGetLastError();
 }
 
-// ------------------------------------------------------------------ elementwise and layout kernels
-__global__ void k_im2col1(const float* __restrict__ x, int B, bf16* __restrict__ a) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (int64_t)B * kP1 * kK1) return;
-    const int j = (int)(i % kK1);
-    const int64_t row = i / kK1;
-    const int b = (int)(row / kP1), pos = (int)(row % kP1);
-    float v = 0.f;
-    if (j < kK1Real) {
-        const int c = j / 27, tap = j % 27;
-        const int x0 = pos % 8 + tap % 3 - 1, y0 = (pos / 8) % 8 + (tap / 3) % 3 - 1, z0 = pos / 64 + tap / 9 - 1;
-        if (x0 >= 0 && x0 < 8 && y0 >= 0 && y0 < 8 && z0 >= 0 && z0 < 8)
-            v = x[((int64_t)b * kIn + c) * kP1 + (z0 * 8 + y0) * 8 + x0];
+// ------------------------------------------------------------------ weight gradients of the convolutions
+// dW = A^T dY contracts over every position of the batch (K = 32 768 for conv1 with 64 tiles) into 96 or 432
+// rows of 16.  One CTA per 128 rows staged and multiplied all of K block after block: 2 529 us for
+// conv1's.  The sums stay in that one order (K ascending, 16 at a time), so that a training run's
+// losses do not change; instead k_pack lays both operands out in parallel, as the core matrices the
+// tensor core reads, and k_stream_gemm, one CTA per 8 rows, streams its slabs through a ring of bulk
+// copies with nothing between the MMAs.  The chain of dependent MMAs is what is left: 2 048 of them for
+// conv1's 64 tiles, 50 ns each, 102 us, whatever few of a 128 x 16 x 16 MMA's rows are used (ranges of K
+// summed afterwards took 12 us and changed the last bits of the gradients).
+//
+// One Adam step of 64 tiles, GB300: 2 730 -> 260 us, 27 -> 13 launches, every bit as before; forward
+// pass of 256 tiles 330 -> 80 us.
+constexpr int kSlabRows = 8;
+constexpr int kSlabA = kSlabRows * kGemmK * 2, kSlabB = 16 * kGemmK * 2;   // bytes per K block
+
+// A^T's slabs [row / 8][K block][k chunk][row % 8] and dY's [K block][n / 8][k chunk][n % 8], chunks of
+// eight K values; `rows` a multiple of 8, K a multiple of 64.
+template <class A, class B>
+__device__ __forceinline__ void pack_chunk(const A& fa, const B& fb, int rows, int K, int i, Chunk* pa, Chunk* pb) {
+    const int nkb = K / kGemmK, na = rows * nkb * 8;
+    if (i < na) {
+        const int r = i % 8, kc = (i / 8) % 8, kb = (i / 64) % nkb, g = i / 64 / nkb;
+        pa[i] = fa(fa.row(8 * g + r), kb * kGemmK + 8 * kc);
+    } else if (i < na + 16 * nkb * 8) {
+        const int e = i - na, r = e % 8, kc = (e / 8) % 8, g = (e / 64) % 2, kb = e / 128;
+        pb[e] = fb(8 * g + r, kb * kGemmK + 8 * kc);
     }
-    a[i] = __float2bfloat16_rn(v);
 }
-// conv2's im2col: stride 2, padding 1, from H1 [tile][512][16]
-__global__ void k_im2col2(const bf16* __restrict__ h1, int B, bf16* __restrict__ a) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (int64_t)B * kP2 * kK2) return;
-    const int j = (int)(i % kK2);
-    const int64_t row = i / kK2;
-    const int b = (int)(row / kP2), o = (int)(row % kP2);
-    const int c = j / 27, tap = j % 27;
-    const int x0 = 2 * (o % 4) + tap % 3 - 1, y0 = 2 * ((o / 4) % 4) + (tap / 3) % 3 - 1, z0 = 2 * (o / 16) + tap / 9 - 1;
-    bf16 v = __float2bfloat16_rn(0.f);
-    if (x0 >= 0 && x0 < 8 && y0 >= 0 && y0 < 8 && z0 >= 0 && z0 < 8) v = h1[((int64_t)b * kP1 + (z0 * 8 + y0) * 8 + x0) * kC1 + c];
-    a[i] = v;
+template <class A1, class B1, class A2, class B2>
+__global__ void __launch_bounds__(256) k_pack(const A1 a1, const B1 b1, int rows1, int K1, Chunk* pa1, Chunk* pb1, const A2 a2,
+                                              const B2 b2, int rows2, int K2, Chunk* pa2, Chunk* pb2) {
+    const int n1 = (rows1 + 16) * (K1 / kGemmK) * 8, i = blockIdx.x * 256 + threadIdx.x;
+    if (i < n1) pack_chunk(a1, b1, rows1, K1, i, pa1, pb1);
+    else pack_chunk(a2, b2, rows2, K2, i - n1, pa2, pb2);
 }
-// conv2's col2im (backward): dH1[tile][pos][c] = sum of dA2 over the (output, tap) pairs reading it,
-// gathered (a fixed order: no atomics)
-__global__ void k_col2im2(const float* __restrict__ da, int B, float* __restrict__ dh1) {
+struct StreamGemm {
+    const Chunk* a;
+    const Chunk* b;
+    float* out;   // [rows][16]
+    int rows, nkb;
+};
+// K blocks per ring stage, stages; the MMAs' rows past a slab's 8 read what lies behind it in shared
+// memory (their results are not used): 16 KB more than the ring.
+constexpr int kStageBlocks = 4, kStages = 6;
+constexpr size_t kStreamSmem = (size_t)kStages * kStageBlocks * (kSlabA + kSlabB) + 16384u;
+__global__ void __launch_bounds__(64) k_stream_gemm(const StreamGemm g1, const StreamGemm g2, int* err) {
+    extern __shared__ __align__(1024) unsigned char smem[];
+    __shared__ __align__(8) uint64_t full[kStages], empty[kStages], done;
+    __shared__ uint32_t s_tmem;
+    const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+    const bool first = (int)blockIdx.x < g1.rows / kSlabRows;
+    const StreamGemm& g = first ? g1 : g2;
+    const int slab = first ? (int)blockIdx.x : (int)blockIdx.x - g1.rows / kSlabRows;
+    if (warp == 0) tmem_alloc(&s_tmem, 32u);
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < kStages; s++) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
+        mbar_init(&done, 1);
+        mbar_fence_init();
+    }
+    tc_fence_before_sync();
+    __syncthreads();
+    tc_fence_after_sync();
+    if (warp == 0) tmem_relinquish();
+    const uint32_t tmem = s_tmem;
+    constexpr uint32_t idesc = umma_idesc_bf16_f32(kGemmM, 16), LBO = 128u, SBO = (kGemmK / 8) * 128u;
+    constexpr int kStageA = kStageBlocks * kSlabA;
+    const int ns = (g.nkb + kStageBlocks - 1) / kStageBlocks;
+    bool ok = true;
+    if (warp == 0 && lane == 0) {   // producer
+        for (int i = 0; i < ns && ok; i++) {
+            const int s = i % kStages, n = min(kStageBlocks, g.nkb - i * kStageBlocks);
+            if (i >= kStages) ok = mbar_wait(&empty[s], (uint32_t)(i / kStages - 1) & 1u);
+            if (!ok) break;
+            unsigned char* dst = smem + (size_t)s * kStageBlocks * (kSlabA + kSlabB);
+            mbar_arrive_expect_tx(&full[s], (uint32_t)(n * (kSlabA + kSlabB)));
+            bulk_g2s(dst, g.a + ((size_t)slab * g.nkb + (size_t)i * kStageBlocks) * (kSlabA / 16), (uint32_t)(n * kSlabA), &full[s]);
+            bulk_g2s(dst + kStageA, g.b + (size_t)i * kStageBlocks * (kSlabB / 16), (uint32_t)(n * kSlabB), &full[s]);
+        }
+    } else if (warp == 1 && lane == 0) {   // the MMAs, in the order of K
+        for (int i = 0; i < ns && ok; i++) {
+            const int s = i % kStages, n = min(kStageBlocks, g.nkb - i * kStageBlocks);
+            ok = mbar_wait(&full[s], (uint32_t)(i / kStages) & 1u);
+            if (!ok) break;
+            tc_fence_after_sync();
+            const uint32_t a0 = smem_addr(smem + (size_t)s * kStageBlocks * (kSlabA + kSlabB)), b0 = a0 + kStageA;
+            for (int k = 0; k < n; k++)
+#pragma unroll
+                for (int kk = 0; kk < kGemmK / 16; kk++)
+                    umma_bf16(tmem, umma_desc_kmajor(a0 + k * kSlabA + kk * 2 * LBO, LBO, SBO),
+                              umma_desc_kmajor(b0 + k * kSlabB + kk * 2 * LBO, LBO, SBO), idesc, i > 0 || k > 0 || kk > 0);
+            umma_commit(&empty[s]);
+        }
+        umma_commit(&done);   // also after a wait gave up: the MMAs in flight
+    }
+    __syncwarp();
+    const bool fin = mbar_wait(&done, 0u) && ok;
+    // every copy issued lands before the CTA leaves: in a normal run the MMAs consumed them all
+    const bool good = __syncthreads_and(fin);
+    if (!good) {
+        if (threadIdx.x == 0) {
+            atomicExch(err, 1);
+            for (int s = 0; s < kStages; s++)   // both parities: one of them is the stage's last request (bounded waits)
+                for (uint32_t q = 0; q < 2; q++) mbar_wait(&full[s], q, 4096u);
+        }
+        __syncthreads();
+    } else if (warp == 0) {
+        tc_fence_after_sync();
+        float v[16];
+        tmem_ld16(tmem, v);   // lanes 0 .. 31: the slab's rows are the first 8
+        if (lane < kSlabRows) {
+            float4* o = reinterpret_cast<float4*>(g.out + (size_t)(slab * kSlabRows + lane) * 16);
+#pragma unroll
+            for (int n = 0; n < 4; n++) o[n] = make_float4(v[4 * n], v[4 * n + 1], v[4 * n + 2], v[4 * n + 3]);
+        }
+    }
+    tc_fence_before_sync();
+    __syncthreads();
+    if (warp == 0) {
+        tc_fence_after_sync();
+        tmem_dealloc(tmem, 32u);
+    }
+}
+
+// ------------------------------------------------------------------ the GEMMs' operands
+// conv1's receptive fields: row = (tile, position), K = channel * 27 + tap, from the features
+struct Conv1A {
+    const float* x;
+    int rows;
+    struct Row { const float* p; uint32_t taps; };   // the position's cell in channel 0, the taps inside the tile
+    __device__ Row row(int m) const {
+        Row r{x, 0u};
+        if (m >= rows) return r;
+        const int pos = m % kP1, px = pos % 8, py = (pos / 8) % 8, pz = pos / 64;
+        r.p = x + (int64_t)(m / kP1) * kIn * kP1 + pos;
+#pragma unroll
+        for (int t = 0; t < 27; t++) {
+            const int x0 = px + t % 3 - 1, y0 = py + (t / 3) % 3 - 1, z0 = pz + t / 9 - 1;
+            if (x0 >= 0 && x0 < 8 && y0 >= 0 && y0 < 8 && z0 >= 0 && z0 < 8) r.taps |= 1u << t;
+        }
+        return r;
+    }
+    __device__ Chunk operator()(const Row& r, int k) const {
+        Chunk c;
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            const int j = k + i, ch = j / 27, t = j - 27 * ch;
+            float v = 0.f;
+            if (j < kK1Real && (r.taps >> t & 1u)) v = r.p[ch * kP1 + (t % 3 - 1) + ((t / 3) % 3 - 1) * 8 + (t / 9 - 1) * 64];
+            c.v[i] = __float2bfloat16_rn(v);
+        }
+        return c;
+    }
+};
+// A weight matrix [K][cols] as the B operand: row n of its transpose
+template <int COLS, int KREAL>
+struct WeightB {
+    const bf16* w;
+    __device__ Chunk operator()(int n, int k) const {
+        Chunk c;
+#pragma unroll
+        for (int i = 0; i < 8; i++) c.v[i] = k + i < KREAL ? w[(k + i) * COLS + n] : __float2bfloat16_rn(0.f);
+        return c;
+    }
+};
+struct Conv2A {
+    const bf16* h1;   // [tile][512][16]
+    int rows;
+    struct Row { const bf16* p; uint32_t taps; };
+    __device__ Row row(int m) const {
+        Row r{h1, 0u};
+        if (m >= rows) return r;
+        const int o = m % kP2, px = 2 * (o % 4), py = 2 * ((o / 4) % 4), pz = 2 * (o / 16);   // stride 2
+        r.p = h1 + ((int64_t)(m / kP2) * kP1 + (pz * 8 + py) * 8 + px) * kC1;
+#pragma unroll
+        for (int t = 0; t < 27; t++) {
+            const int x0 = px + t % 3 - 1, y0 = py + (t / 3) % 3 - 1, z0 = pz + t / 9 - 1;
+            if (x0 >= 0 && x0 < 8 && y0 >= 0 && y0 < 8 && z0 >= 0 && z0 < 8) r.taps |= 1u << t;
+        }
+        return r;
+    }
+    __device__ Chunk operator()(const Row& r, int k) const {
+        Chunk c;
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            const int j = k + i, ch = j / 27, t = j - 27 * ch;
+            c.v[i] = j < kK2 && (r.taps >> t & 1u) ? r.p[((t % 3 - 1) + ((t / 3) % 3 - 1) * 8 + (t / 9 - 1) * 64) * kC1 + ch]
+                                                   : __float2bfloat16_rn(0.f);
+        }
+        return c;
+    }
+};
+// Rows of a matrix whose K = KREAL values are contiguous: [row][KREAL]
+template <int KREAL>
+struct RowsA {
+    const bf16* p;
+    int rows;
+    struct Row { const bf16* p; };
+    __device__ Row row(int m) const { return Row{m < rows ? p + (int64_t)m * KREAL : nullptr}; }
+    __device__ Chunk operator()(const Row& r, int k) const {
+        return r.p && k < KREAL ? *reinterpret_cast<const Chunk*>(r.p + k) : zero_chunk();
+    }
+    __device__ Chunk operator()(int n, int k) const { return (*this)(row(n), k); }
+};
+// The transposed receptive fields for the weight gradients: row = K index of the forward pass,
+// K = (tile, position)
+struct Conv1At {
+    const float* x;
+    struct Row { int ch, dx, dy, dz; };   // ch = -1: a padding row
+    __device__ Row row(int j) const {
+        const int t = j % 27;
+        return Row{j < kK1Real ? j / 27 : -1, t % 3 - 1, (t / 3) % 3 - 1, t / 9 - 1};
+    }
+    __device__ Chunk operator()(const Row& r, int k) const {   // eight positions: one row of x
+        const int pos = k % kP1, y = (pos / 8) % 8 + r.dy, z = pos / 64 + r.dz;
+        if (r.ch < 0 || y < 0 || y >= 8 || z < 0 || z >= 8) return zero_chunk();
+        const float* p = x + ((int64_t)(k / kP1) * kIn + r.ch) * kP1 + (z * 8 + y) * 8 + r.dx;
+        Chunk c;
+#pragma unroll
+        for (int i = 0; i < 8; i++) c.v[i] = __float2bfloat16_rn(i + r.dx >= 0 && i + r.dx < 8 ? p[i] : 0.f);
+        return c;
+    }
+};
+struct Conv2At {
+    const bf16* h1;
+    struct Row { int ch, dx, dy, dz; };
+    __device__ Row row(int j) const {
+        const int t = j % 27;
+        return Row{j < kK2 ? j / 27 : -1, t % 3 - 1, (t / 3) % 3 - 1, t / 9 - 1};
+    }
+    __device__ Chunk operator()(const Row& r, int k) const {   // eight outputs: two rows of four
+        const int o = k % kP2, z = 2 * (o / 16) + r.dz;
+        if (r.ch < 0 || z < 0 || z >= 8) return zero_chunk();
+        const bf16* p = h1 + ((int64_t)(k / kP2) * kP1 + z * 64) * kC1 + r.ch;
+        Chunk c;
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            const int x = 2 * (i % 4) + r.dx, y = 2 * ((o / 4) % 4 + i / 4) + r.dy;
+            c.v[i] = x >= 0 && x < 8 && y >= 0 && y < 8 ? p[(y * 8 + x) * kC1] : __float2bfloat16_rn(0.f);
+        }
+        return c;
+    }
+};
+// Rows of a [K][cols] matrix read down its columns (H2 and the back-propagated gradients)
+template <int COLS>
+struct ColumnsT {
+    const bf16* p;
+    int K;
+    struct Row { const bf16* p; };
+    __device__ Row row(int m) const { return Row{p + (m < COLS ? m : 0)}; }
+    __device__ Chunk operator()(const Row& r, int k) const {
+        Chunk c;
+#pragma unroll
+        for (int i = 0; i < 8; i++) c.v[i] = k + i < K ? r.p[(int64_t)(k + i) * COLS] : __float2bfloat16_rn(0.f);
+        return c;
+    }
+    __device__ Chunk operator()(int n, int k) const { return (*this)(row(n), k); }
+};
+
+// ------------------------------------------------------------------ the GEMMs' epilogues
+// z = y + bias (kept for the backward pass where z is set), h = bf16(relu(z)); NT columns
+template <int NT>
+struct BiasRelu {
+    const float* bias;
+    float* z;
+    bf16* h;
+    int rows;
+    __device__ void operator()(int m, int, float* v) const {
+        if (m >= rows) return;
+#pragma unroll
+        for (int n = 0; n < NT; n += 8) {
+            Chunk c;
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                v[n + i] = v[n + i] + bias[n + i];
+                c.v[i] = __float2bfloat16_rn(fmaxf(v[n + i], 0.f));
+            }
+            *reinterpret_cast<Chunk*>(h + (int64_t)m * NT + n) = c;
+        }
+        if (z)
+#pragma unroll
+            for (int n = 0; n < NT; n += 4)
+                *reinterpret_cast<float4*>(z + (int64_t)m * NT + n) = make_float4(v[n], v[n + 1], v[n + 2], v[n + 3]);
+    }
+};
+// the tile of a rows x COLS matrix
+template <int NT, int COLS>
+struct Store {
+    float* out;
+    int rows;
+    __device__ void operator()(int m, int n0, const float* v) const {
+        if (m >= rows) return;
+#pragma unroll
+        for (int n = 0; n < NT; n += 4)
+            if (n0 + n < COLS)
+                *reinterpret_cast<float4*>(out + (int64_t)m * COLS + n0 + n) = make_float4(v[n], v[n + 1], v[n + 2], v[n + 3]);
+    }
+};
+// gradient through the ReLU: dz = dh * (z > 0), FP32 (for the bias gradient) and BF16 (an operand)
+template <int NT, int COLS>
+struct ReluBack {
+    const float* z;
+    float* dz;
+    bf16* dzb;
+    int rows;
+    __device__ void operator()(int m, int n0, float* v) const {
+        if (m >= rows) return;
+        const int64_t o = (int64_t)m * COLS + n0;
+#pragma unroll
+        for (int n = 0; n < NT; n += 8) {
+            Chunk c;
+#pragma unroll
+            for (int i = 0; i < 8; i += 4) {
+                const float4 zz = *reinterpret_cast<const float4*>(z + o + n + i);
+                const float zv[4] = {zz.x, zz.y, zz.z, zz.w};
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    v[n + i + q] = zv[q] > 0.f ? v[n + i + q] : 0.f;
+                    c.v[i + q] = __float2bfloat16_rn(v[n + i + q]);
+                }
+                *reinterpret_cast<float4*>(dz + o + n + i) = make_float4(v[n + i], v[n + i + 1], v[n + i + 2], v[n + i + 3]);
+            }
+            *reinterpret_cast<Chunk*>(dzb + o + n) = c;
+        }
+    }
+};
+
+// ------------------------------------------------------------------ the last layer, sums and Adam
+// fc2 and the loss, a warp per tile: out[b] = h3[b] . w4 + b4 (in the order of k); with targets, dout = 2 (out - t) / B,
+// the loss terms, and dZ3 = (dout w4) through fc1's ReLU (FP32 and BF16)
+__global__ void __launch_bounds__(128) k_fc2(const bf16* __restrict__ h3, const float* __restrict__ w4, const float* __restrict__ b4,
+                                             int B, float* __restrict__ out, const float* __restrict__ target,
+                                             float* __restrict__ dout, float* __restrict__ sq, const float* __restrict__ z3,
+                                             float* __restrict__ dz3, bf16* __restrict__ dz3b) {
+    const int b = blockIdx.x * 4 + threadIdx.x / 32, k = threadIdx.x % 32;
+    if (b >= B) return;
+    const float h = __bfloat162float(h3[(int64_t)b * kF + k]), w = __bfloat162float(__float2bfloat16_rn(w4[k]));
+    float s = b4[0];
+#pragma unroll
+    for (int i = 0; i < kF; i++) s = fmaf(__shfl_sync(0xffffffffu, h, i), __shfl_sync(0xffffffffu, w, i), s);
+    if (k == 0) out[b] = s;
+    if (!target) return;
+    const float d = s - target[b], g = 2.f * d / (float)B;
+    if (k == 0) {
+        dout[b] = g;
+        sq[b] = d * d;
+    }
+    const int64_t i = (int64_t)b * kF + k;
+    const float v = z3[i] > 0.f ? g * w : 0.f;
+    dz3[i] = v;
+    dz3b[i] = __float2bfloat16_rn(v);
+}
+// conv2's col2im through conv1's ReLU: dH1[tile][pos][c] = sum of dA2 over the (output, tap) pairs reading
+// it, gathered in a fixed order (no atomics); dZ1 in FP32 and BF16
+__global__ void __launch_bounds__(256) k_col2im2(const float* __restrict__ da, const float* __restrict__ z1, int B,
+                                                 float* __restrict__ dz1, bf16* __restrict__ dz1b) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (int64_t)B * kP1 * kC1) return;
     const int c = (int)(i % kC1);
@@ -197,92 +526,80 @@ __global__ void k_col2im2(const float* __restrict__ da, int B, float* __restrict
     const int b = (int)(row / kP1), pos = (int)(row % kP1);
     const int px = pos % 8, py = (pos / 8) % 8, pz = pos / 64;
     float s = 0.f;
-    for (int dz = 0; dz < 3; dz++) {
-        const int tz = pz + 1 - dz;
-        if (tz < 0 || (tz & 1) || tz / 2 >= 4) continue;
-        for (int dy = 0; dy < 3; dy++) {
-            const int ty = py + 1 - dy;
-            if (ty < 0 || (ty & 1) || ty / 2 >= 4) continue;
-            for (int dx = 0; dx < 3; dx++) {
-                const int tx = px + 1 - dx;
-                if (tx < 0 || (tx & 1) || tx / 2 >= 4) continue;
-                const int o = (tz / 2 * 4 + ty / 2) * 4 + tx / 2;
-                s += da[((int64_t)b * kP2 + o) * kK2 + c * 27 + dz * 9 + dy * 3 + dx];
+    if (z1[i] > 0.f) {
+        for (int dz = (pz + 1) & 1; dz < 3; dz += 2) {   // the stride of 2: taps of the position's parity
+            const int tz = pz + 1 - dz;
+            if (tz >= 8) continue;
+            for (int dy = (py + 1) & 1; dy < 3; dy += 2) {
+                const int ty = py + 1 - dy;
+                if (ty >= 8) continue;
+                for (int dx = (px + 1) & 1; dx < 3; dx += 2) {
+                    const int tx = px + 1 - dx;
+                    if (tx >= 8) continue;
+                    const int o = (tz / 2 * 4 + ty / 2) * 4 + tx / 2;
+                    s += da[((int64_t)b * kP2 + o) * kK2 + c * 27 + dz * 9 + dy * 3 + dx];
+                }
             }
         }
     }
-    dh1[i] = s;
+    dz1[i] = s;
+    dz1b[i] = __float2bfloat16_rn(s);
 }
-// z = y + bias (kept for the backward pass), h = bf16(relu(z))
-__global__ void k_bias_relu(const float* __restrict__ y, const float* __restrict__ bias, int64_t rows, int cols,
-                            float* __restrict__ z, bf16* __restrict__ h) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= rows * cols) return;
-    const float v = y[i] + bias[i % cols];
-    z[i] = v;
-    h[i] = __float2bfloat16_rn(fmaxf(v, 0.f));
-}
-// gradient through the ReLU: dz = dh * (z > 0), as FP32 (for the bias gradient) and BF16 (GEMM operand)
-__global__ void k_relu_back(const float* __restrict__ dh, const float* __restrict__ z, int64_t n, float* __restrict__ dz,
-                            bf16* __restrict__ dzb) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float v = z[i] > 0.f ? dh[i] : 0.f;
-    dz[i] = v;
-    dzb[i] = __float2bfloat16_rn(v);
-}
-// column sums (bias gradients), one block per column, fixed reduction order
-__global__ void k_colsum(const float* __restrict__ x, int64_t rows, int cols, float* __restrict__ out) {
-    const int c = blockIdx.x;
+// The first half of db1's column sums: part[t][c] = sum of rows t, t + 256, ... of column c, in that order.
+// 16 lanes read a row's 16 columns.
+__global__ void __launch_bounds__(256) k_colsum1(const float* __restrict__ x, int64_t rows, float* __restrict__ part) {
+    const int t = blockIdx.x * 16 + threadIdx.x / kC1, c = threadIdx.x % kC1;
     float s = 0.f;
-    for (int64_t r = threadIdx.x; r < rows; r += blockDim.x) s += x[r * cols + c];
+#pragma unroll 16
+    for (int64_t r = t; r < rows; r += 256) s += x[r * kC1 + c];
+    part[t * kC1 + c] = s;
+}
+// The small gradients and the loss, one block each, in a fixed order.  Block 0: the sum of the squared
+// errors; 1: db4; 2 .. 33: dW4; then db3 (32), db2 (16) and db1 (16, from k_colsum1's sums).
+constexpr int kSmallBlocks = 2 + 2 * kF + kC2 + kC1;
+__global__ void __launch_bounds__(256) k_small_grads(const float* __restrict__ sq, const float* __restrict__ dout,
+                                                     const bf16* __restrict__ h3, const float* __restrict__ dz3,
+                                                     const float* __restrict__ dz2, const float* __restrict__ part1, int B,
+                                                     float* __restrict__ grads, float* __restrict__ loss) {
+    const int k = blockIdx.x;
+    float s = 0.f;
+    if (k >= 1 && k < 2 + kF) {   // one chain over the tiles
+        __shared__ float v[2][256];
+        for (int b0 = 0; b0 < B; b0 += 256) {
+            const int b = b0 + threadIdx.x;
+            if (b < B) {
+                v[0][threadIdx.x] = dout[b];
+                v[1][threadIdx.x] = k == 1 ? 1.f : __bfloat162float(h3[(int64_t)b * kF + (k - 2)]);
+            }
+            __syncthreads();
+            if (threadIdx.x == 0)
+                for (int i = 0; i < min(256, B - b0); i++) s = k == 1 ? s + v[0][i] : fmaf(v[1][i], v[0][i], s);
+            __syncthreads();
+        }
+        if (threadIdx.x == 0) grads[k == 1 ? kOffB4 : kOffW4 + (k - 2)] = s;
+        return;
+    }
+    float* dst;
+    auto sum = [&](const float* x, int64_t rows, int cols, int c) {
+#pragma unroll 8
+        for (int64_t r = threadIdx.x; r < rows; r += 256) s += x[r * cols + c];
+    };
+    if (k == 0) { dst = loss; sum(sq, B, 1, 0); }
+    else if (k < 2 + 2 * kF) { dst = grads + kOffB3 + (k - 2 - kF); sum(dz3, B, kF, k - 2 - kF); }
+    else if (k < 2 + 2 * kF + kC2) { dst = grads + kOffB2 + (k - 2 - 2 * kF); sum(dz2, (int64_t)B * kP2, kC2, k - 2 - 2 * kF); }
+    else { dst = grads + kOffB1 + (k - 2 - 2 * kF - kC2); s = part1[threadIdx.x * kC1 + (k - 2 - 2 * kF - kC2)]; }
     __shared__ float red[256];
     red[threadIdx.x] = s;
     __syncthreads();
-    for (int w = blockDim.x / 2; w > 0; w >>= 1) {
+    for (int w = 128; w > 0; w >>= 1) {
         if ((int)threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
         __syncthreads();
     }
-    if (threadIdx.x == 0) out[c] = red[0];
+    if (threadIdx.x == 0) *dst = red[0];
 }
-// fc2 and the loss: out[b] = h3[b] . w4 + b4; with targets, dout = 2 (out - t) / B and the loss terms
-__global__ void k_fc2(const bf16* __restrict__ h3, const float* __restrict__ w4, const float* __restrict__ b4, int B,
-                      float* __restrict__ out, const float* __restrict__ target, float* __restrict__ dout,
-                      float* __restrict__ sq) {
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= B) return;
-    float s = b4[0];
-    for (int k = 0; k < kF; k++) s = fmaf(__bfloat162float(h3[(int64_t)b * kF + k]), __bfloat162float(__float2bfloat16_rn(w4[k])), s);
-    out[b] = s;
-    if (target) {
-        const float d = s - target[b];
-        dout[b] = 2.f * d / (float)B;
-        sq[b] = d * d;
-    }
-}
-// fc2 backward: dW4[k] = sum_b h3[b][k] dout[b], db4 = sum dout, dH3[b][k] = dout[b] w4[k]
-__global__ void k_fc2_back(const bf16* __restrict__ h3, const float* __restrict__ w4, const float* __restrict__ dout, int B,
-                           float* __restrict__ dw4, float* __restrict__ db4, float* __restrict__ dh3) {
-    const int t = threadIdx.x;
-    if (t < kF) {
-        float s = 0.f;
-        for (int b = 0; b < B; b++) s = fmaf(__bfloat162float(h3[(int64_t)b * kF + t]), dout[b], s);
-        dw4[t] = s;
-    } else if (t == kF) {
-        float s = 0.f;
-        for (int b = 0; b < B; b++) s += dout[b];
-        db4[0] = s;
-    }
-    for (int64_t i = t; i < (int64_t)B * kF; i += blockDim.x)
-        dh3[i] = dout[i / kF] * __bfloat162float(__float2bfloat16_rn(w4[i % kF]));
-}
-__global__ void k_to_bf16(const float* __restrict__ x, int64_t n, bf16* __restrict__ y) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) y[i] = __float2bfloat16_rn(x[i]);
-}
-// Adam on the FP32 master parameters
+// Adam on the FP32 master parameters, and the BF16 copies of W1, W2, W3
 __global__ void k_adam(float* __restrict__ w, const float* __restrict__ g, float* __restrict__ m, float* __restrict__ v,
-                       int64_t n, float lr, float b1, float b2, float eps, float c1, float c2) {
+                       int64_t n, float lr, float b1, float b2, float eps, float c1, float c2, bf16* __restrict__ wb) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float gi = g[i];
@@ -290,19 +607,15 @@ __global__ void k_adam(float* __restrict__ w, const float* __restrict__ g, float
     m[i] = mi;
     v[i] = vi;
     w[i] -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+    constexpr int N1 = kK1 * kC1, N2 = kK2 * kC2;
+    const bf16 r = __float2bfloat16_rn(w[i]);
+    if (i < N1) wb[i] = r;
+    else if (i >= (int)kOffW2 && i < (int)kOffB2) wb[N1 + (i - (int)kOffW2)] = r;
+    else if (i >= (int)kOffW3 && i < (int)kOffB3) wb[N1 + N2 + (i - (int)kOffW3)] = r;
 }
-// sum of the squared errors (the loss), fixed order
-__global__ void k_sum(const float* __restrict__ x, int n, float* __restrict__ out) {
-    __shared__ float red[256];
-    float s = 0.f;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) s += x[i];
-    red[threadIdx.x] = s;
-    __syncthreads();
-    for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-        if ((int)threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) out[0] = red[0];
+__global__ void k_to_bf16(const float* __restrict__ x, int64_t n, bf16* __restrict__ y) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) y[i] = __float2bfloat16_rn(x[i]);
 }
 
 inline unsigned blocks(int64_t n, int t = 256) { return (unsigned)((n + t - 1) / t); }
@@ -318,21 +631,21 @@ struct Estimator {
     float* adam_v = nullptr;
     bf16* wb = nullptr;          // BF16 copies of W1, W2, W3 (GEMM operands)
     // activations and their gradients for max_batch tiles
-    bf16 *a1 = nullptr, *h1 = nullptr, *a2 = nullptr, *h2 = nullptr, *h3 = nullptr;
-    float *y1 = nullptr, *z1 = nullptr, *y2 = nullptr, *z2 = nullptr, *y3 = nullptr, *z3 = nullptr, *out = nullptr;
-    float *dout = nullptr, *sq = nullptr, *dh3 = nullptr, *dz3 = nullptr, *dh2 = nullptr, *dz2 = nullptr,
-          *da2 = nullptr, *dh1 = nullptr, *dz1 = nullptr, *loss = nullptr;
+    bf16 *h1 = nullptr, *h2 = nullptr, *h3 = nullptr;
+    float *z1 = nullptr, *z2 = nullptr, *z3 = nullptr, *out = nullptr;
+    float *dout = nullptr, *sq = nullptr, *dz3 = nullptr, *dz2 = nullptr, *dz1 = nullptr, *da2 = nullptr, *loss = nullptr;
     bf16 *dz3b = nullptr, *dz2b = nullptr, *dz1b = nullptr;
+    Chunk *pa1 = nullptr, *pb1 = nullptr, *pa2 = nullptr, *pb2 = nullptr;   // packed operands of dW1 and dW2
+    float* part1 = nullptr;                                                 // db1's column sums, first half
     int step = 0;
     cudaStream_t stream = nullptr;
 
     ~Estimator() {
         if (stream) cudaStreamSynchronize(stream);
-        for (void* p : {(void*)params, (void*)grads, (void*)adam_m, (void*)adam_v, (void*)wb, (void*)a1, (void*)h1,
-                        (void*)a2, (void*)h2, (void*)h3, (void*)y1, (void*)z1, (void*)y2, (void*)z2, (void*)y3,
-                        (void*)z3, (void*)out, (void*)dout, (void*)sq, (void*)dh3, (void*)dz3, (void*)dh2,
-                        (void*)dz2, (void*)da2, (void*)dh1, (void*)dz1, (void*)loss, (void*)dz3b, (void*)dz2b,
-                        (void*)dz1b})
+        for (void* p : {(void*)params, (void*)grads, (void*)adam_m, (void*)adam_v, (void*)wb, (void*)h1, (void*)h2,
+                        (void*)h3, (void*)z1, (void*)z2, (void*)z3, (void*)out, (void*)dout, (void*)sq, (void*)dz3,
+                        (void*)dz2, (void*)dz1, (void*)da2, (void*)loss, (void*)dz3b, (void*)dz2b, (void*)dz1b,
+                        (void*)pa1, (void*)pb1, (void*)pa2, (void*)pb2, (void*)part1})
             cudaFree(p);
         if (stream) cudaStreamDestroy(stream);
     }
@@ -348,31 +661,28 @@ struct Estimator {
         if (e == cudaSuccess) e = alloc(&adam_m, kParams);
         if (e == cudaSuccess) e = alloc(&adam_v, kParams);
         if (e == cudaSuccess) e = alloc(&wb, (size_t)kK1 * kC1 + (size_t)kK2 * kC2 + (size_t)kK3 * kF);
-        if (e == cudaSuccess) e = alloc(&a1, B * kP1 * kK1);
         if (e == cudaSuccess) e = alloc(&h1, B * kP1 * kC1);
-        if (e == cudaSuccess) e = alloc(&a2, B * kP2 * kK2);
         if (e == cudaSuccess) e = alloc(&h2, B * kK3);
         if (e == cudaSuccess) e = alloc(&h3, B * kF);
-        if (e == cudaSuccess) e = alloc(&y1, B * kP1 * kC1);
         if (e == cudaSuccess) e = alloc(&z1, B * kP1 * kC1);
-        if (e == cudaSuccess) e = alloc(&y2, B * kP2 * kC2);
         if (e == cudaSuccess) e = alloc(&z2, B * kP2 * kC2);
-        if (e == cudaSuccess) e = alloc(&y3, B * kF);
         if (e == cudaSuccess) e = alloc(&z3, B * kF);
         if (e == cudaSuccess) e = alloc(&out, B);
         if (e == cudaSuccess) e = alloc(&dout, B);
         if (e == cudaSuccess) e = alloc(&sq, B);
-        if (e == cudaSuccess) e = alloc(&dh3, B * kF);
         if (e == cudaSuccess) e = alloc(&dz3, B * kF);
-        if (e == cudaSuccess) e = alloc(&dh2, B * kK3);
         if (e == cudaSuccess) e = alloc(&dz2, B * kK3);
-        if (e == cudaSuccess) e = alloc(&da2, B * kP2 * kK2);
-        if (e == cudaSuccess) e = alloc(&dh1, B * kP1 * kC1);
-        if (e == cudaSuccess) e = alloc(&dz1, B * kP1 * kC1);
         if (e == cudaSuccess) e = alloc(&loss, 1);
         if (e == cudaSuccess) e = alloc(&dz3b, B * kF);
         if (e == cudaSuccess) e = alloc(&dz2b, B * kK3);
         if (e == cudaSuccess) e = alloc(&dz1b, B * kP1 * kC1);
+        if (e == cudaSuccess) e = alloc(&dz1, B * kP1 * kC1);
+        if (e == cudaSuccess) e = alloc(&da2, B * kP2 * kK2);
+        if (e == cudaSuccess) e = alloc(&pa1, B * kP1 * kK1 / 8);
+        if (e == cudaSuccess) e = alloc(&pb1, B * kP1 * kC1 / 8);
+        if (e == cudaSuccess) e = alloc(&pa2, B * kP2 * kK2 / 8);
+        if (e == cudaSuccess) e = alloc(&pb2, B * kP2 * kC2 / 8);
+        if (e == cudaSuccess) e = alloc(&part1, 256u * kC1);
         if (e != cudaSuccess) return e;
         // He-uniform initial weights from a seeded 64-bit LCG, zero biases
         std::vector<float> h(kParams, 0.f);
@@ -411,47 +721,51 @@ struct Estimator {
         return e;
     }
 
-    // forward pass of B tiles (x: device [B][3][512] FP32); predictions in `out`
-    cudaError_t forward(const float* x, int B, const float* target) {
+    // forward pass of B tiles (x: device [B][3][512] FP32); predictions in `pred`; with targets, also
+    // what backward() needs
+    cudaError_t forward(const float* x, int B, const float* target, float* pred) {
         const bf16* W1 = wb;
         const bf16* W2 = wb + kK1 * kC1;
         const bf16* W3 = wb + kK1 * kC1 + kK2 * kC2;
-        k_im2col1<<<blocks((int64_t)B * kP1 * kK1), 256, 0, stream>>>(x, B, a1);
-        cudaError_t e = gemm({a1, kK1, 1, W1, kC1, 1, y1, kC1, 1, B * kP1, kC1, kK1, 0}, stream);
+        const int r1 = B * kP1, r2 = B * kP2;
+        cudaError_t e = gemm<16>(Conv1A{x, r1}, WeightB<kC1, kK1>{W1}, BiasRelu<16>{params + kOffB1, target ? z1 : nullptr, h1, r1},
+                                 r1, kC1, kK1, stream);
+        if (e == cudaSuccess)
+            e = gemm<16>(Conv2A{h1, r2}, WeightB<kC2, kK2>{W2}, BiasRelu<16>{params + kOffB2, target ? z2 : nullptr, h2, r2}, r2, kC2,
+                         kK2, stream);
+        if (e == cudaSuccess)
+            e = gemm<32>(RowsA<kK3>{h2, B}, WeightB<kF, kK3>{W3}, BiasRelu<32>{params + kOffB3, z3, h3, B}, B, kF, kK3, stream);
         if (e != cudaSuccess) return e;
-        k_bias_relu<<<blocks((int64_t)B * kP1 * kC1), 256, 0, stream>>>(y1, params + kOffB1, (int64_t)B * kP1, kC1, z1, h1);
-        k_im2col2<<<blocks((int64_t)B * kP2 * kK2), 256, 0, stream>>>(h1, B, a2);
-        if ((e = gemm({a2, kK2, 1, W2, kC2, 1, y2, kC2, 1, B * kP2, kC2, kK2, 0}, stream)) != cudaSuccess) return e;
-        k_bias_relu<<<blocks((int64_t)B * kK3), 256, 0, stream>>>(y2, params + kOffB2, (int64_t)B * kP2, kC2, z2, h2);
-        if ((e = gemm({h2, kK3, 1, W3, kF, 1, y3, kF, 1, B, kF, kK3, 0}, stream)) != cudaSuccess) return e;
-        k_bias_relu<<<blocks((int64_t)B * kF), 256, 0, stream>>>(y3, params + kOffB3, B, kF, z3, h3);
-        k_fc2<<<blocks(B), 256, 0, stream>>>(h3, params + kOffW4, params + kOffB4, B, out, target, dout, sq);
+        k_fc2<<<(unsigned)((B + 3) / 4), 128, 0, stream>>>(h3, params + kOffW4, params + kOffB4, B, pred, target, dout, sq, z3, dz3,
+                                                           dz3b);
         return cudaGetLastError();
     }
-    // gradients of the mean squared error of the last forward pass (with targets) into `grads`
-    cudaError_t backward(int B) {
+    // gradients of the mean squared error of the last forward pass (of x, with targets) into `grads`
+    cudaError_t backward(const float* x, int B) {
         const bf16* W2 = wb + kK1 * kC1;
         const bf16* W3 = wb + kK1 * kC1 + kK2 * kC2;
-        k_fc2_back<<<1, 256, 0, stream>>>(h3, params + kOffW4, dout, B, grads + kOffW4, grads + kOffB4, dh3);
-        k_relu_back<<<blocks((int64_t)B * kF), 256, 0, stream>>>(dh3, z3, (int64_t)B * kF, dz3, dz3b);
-        k_colsum<<<kF, 256, 0, stream>>>(dz3, B, kF, grads + kOffB3);
-        // dW3 = H2^T dZ3, dH2 = dZ3 W3^T
-        cudaError_t e = gemm({h2, 1, kK3, dz3b, kF, 1, grads + kOffW3, kF, 1, kK3, kF, B, 0}, stream);
-        if (e == cudaSuccess) e = gemm({dz3b, kF, 1, W3, 1, kF, dh2, kK3, 1, B, kK3, kF, 0}, stream);
+        const int k1 = B * kP1, k2 = B * kP2;
+        // dW3 = H2^T dZ3, dH2 = dZ3 W3^T through conv2's ReLU
+        cudaError_t e = gemm<32>(ColumnsT<kK3>{h2, B}, ColumnsT<kF>{dz3b, B}, Store<32, kF>{grads + kOffW3, kK3}, kK3, kF, B, stream);
+        if (e == cudaSuccess)
+            e = gemm<32>(RowsA<kF>{dz3b, B}, RowsA<kF>{W3, kK3}, ReluBack<32, kK3>{z2, dz2, dz2b, B}, B, kK3, kF, stream);
+        // dA2 = dY2 W2^T, then col2im through conv1's ReLU
+        if (e == cudaSuccess)
+            e = gemm<32>(RowsA<kC2>{dz2b, k2}, RowsA<kC2>{W2, kK2}, Store<32, kK2>{da2, k2}, k2, kK2, kC2, stream);
         if (e != cudaSuccess) return e;
-        k_relu_back<<<blocks((int64_t)B * kK3), 256, 0, stream>>>(dh2, z2, (int64_t)B * kK3, dz2, dz2b);
-        k_colsum<<<kC2, 256, 0, stream>>>(dz2, (int64_t)B * kP2, kC2, grads + kOffB2);
-        // dW2 = A2^T dY2, dA2 = dY2 W2^T, then col2im
-        e = gemm({a2, 1, kK2, dz2b, kC2, 1, grads + kOffW2, kC2, 1, kK2, kC2, B * kP2, 0}, stream);
-        if (e == cudaSuccess) e = gemm({dz2b, kC2, 1, W2, 1, kC2, da2, kK2, 1, B * kP2, kK2, kC2, 0}, stream);
-        if (e != cudaSuccess) return e;
-        k_col2im2<<<blocks((int64_t)B * kP1 * kC1), 256, 0, stream>>>(da2, B, dh1);
-        k_relu_back<<<blocks((int64_t)B * kP1 * kC1), 256, 0, stream>>>(dh1, z1, (int64_t)B * kP1 * kC1, dz1, dz1b);
-        k_colsum<<<kC1, 256, 0, stream>>>(dz1, (int64_t)B * kP1, kC1, grads + kOffB1);
-        // dW1 = A1^T dY1 (rows 81..95 of A1 are zero, so their gradient is too)
-        e = gemm({a1, 1, kK1, dz1b, kC1, 1, grads + kOffW1, kC1, 1, kK1, kC1, B * kP1, 0}, stream);
-        if (e != cudaSuccess) return e;
-        k_sum<<<1, 256, 0, stream>>>(sq, B, loss);
+        k_col2im2<<<blocks((int64_t)B * kP1 * kC1), 256, 0, stream>>>(da2, z1, B, dz1, dz1b);
+        // dW1 = A1^T dY1 (rows 81..95 of A1 are zero, so their gradient is too) and dW2 = A2^T dY2
+        const int64_t chunks = (int64_t)(kK1 + 16) * (k1 / kGemmK) * 8 + (int64_t)(kK2 + 16) * (k2 / kGemmK) * 8;
+        k_pack<<<blocks(chunks), 256, 0, stream>>>(Conv1At{x}, ColumnsT<kC1>{dz1b, k1}, kK1, k1, pa1, pb1, Conv2At{h1},
+                                                   ColumnsT<kC2>{dz2b, k2}, kK2, k2, pa2, pb2);
+        int* err = device_error_flag();
+        if (!err) return cudaErrorMemoryAllocation;
+        static std::atomic<uint64_t> configured{0};
+        if ((e = ensure_smem_limit(k_stream_gemm, kStreamSmem, configured)) != cudaSuccess) return e;
+        k_stream_gemm<<<(kK1 + kK2) / kSlabRows, 64, kStreamSmem, stream>>>(
+            StreamGemm{pa1, pb1, grads + kOffW1, kK1, k1 / kGemmK}, StreamGemm{pa2, pb2, grads + kOffW2, kK2, k2 / kGemmK}, err);
+        k_colsum1<<<16, 256, 0, stream>>>(dz1, k1, part1);
+        k_small_grads<<<kSmallBlocks, 256, 0, stream>>>(sq, dout, h3, dz3, dz2, part1, B, grads, loss);
         return cudaGetLastError();
     }
     cudaError_t adam(float lr) {
@@ -459,9 +773,8 @@ struct Estimator {
         const float b1 = .9f, b2 = .999f;
         k_adam<<<blocks((int64_t)kParams), 256, 0, stream>>>(params, grads, adam_m, adam_v, (int64_t)kParams, lr, b1, b2,
                                                             1e-8f, 1.f - std::pow(b1, (float)step),
-                                                            1.f - std::pow(b2, (float)step));
-        cudaError_t e = cudaGetLastError();
-        return e == cudaSuccess ? refresh_bf16() : e;
+                                                            1.f - std::pow(b2, (float)step), wb);
+        return cudaGetLastError();
     }
 };
 
@@ -508,8 +821,7 @@ AMR_API int amr_estimator_forward(amr_estimator* e, const float* features, uint3
     if (!e || (n && (!features || !out))) return AMR_ERR_INVALID;
     for (uint32_t b0 = 0; b0 < n; b0 += e->net.max_batch) {
         const int B = (int)std::min<uint32_t>(e->net.max_batch, n - b0);
-        cudaError_t st = e->net.forward(features + (size_t)b0 * kIn * kP1, B, nullptr);
-        if (st == cudaSuccess) st = cudaMemcpyAsync(out + b0, e->net.out, (size_t)B * 4, cudaMemcpyDeviceToDevice, e->net.stream);
+        const cudaError_t st = e->net.forward(features + (size_t)b0 * kIn * kP1, B, nullptr, out + b0);
         if (st != cudaSuccess) return cuda_status(st);
     }
     const int st = cuda_status(cudaStreamSynchronize(e->net.stream));
@@ -518,8 +830,8 @@ AMR_API int amr_estimator_forward(amr_estimator* e, const float* features, uint3
 AMR_API int amr_estimator_gradients(amr_estimator* e, const float* features, const float* targets, uint32_t n,
                                     float* grads_host, float* loss) {
     if (!e || !features || !targets || n == 0 || n > e->net.max_batch) return AMR_ERR_INVALID;
-    cudaError_t st = e->net.forward(features, (int)n, targets);
-    if (st == cudaSuccess) st = e->net.backward((int)n);
+    cudaError_t st = e->net.forward(features, (int)n, targets, e->net.out);
+    if (st == cudaSuccess) st = e->net.backward(features, (int)n);
     float l = 0.f;
     if (st == cudaSuccess && grads_host)
         st = cudaMemcpyAsync(grads_host, e->net.grads, kParams * 4, cudaMemcpyDeviceToHost, e->net.stream);
@@ -532,8 +844,8 @@ AMR_API int amr_estimator_gradients(amr_estimator* e, const float* features, con
 AMR_API int amr_estimator_train_step(amr_estimator* e, const float* features, const float* targets, uint32_t n,
                                      float lr, float* loss) {
     if (!e || !features || !targets || n == 0 || n > e->net.max_batch || !(lr > 0.f)) return AMR_ERR_INVALID;
-    cudaError_t st = e->net.forward(features, (int)n, targets);
-    if (st == cudaSuccess) st = e->net.backward((int)n);
+    cudaError_t st = e->net.forward(features, (int)n, targets, e->net.out);
+    if (st == cudaSuccess) st = e->net.backward(features, (int)n);
     if (st == cudaSuccess) st = e->net.adam(lr);
     float l = 0.f;
     if (st == cudaSuccess && loss) st = cudaMemcpyAsync(&l, e->net.loss, 4, cudaMemcpyDeviceToHost, e->net.stream);

@@ -403,14 +403,18 @@ public:
     }
 
     // ---- refinement (the learned estimator with the plain criterion as fallback and judge)
-    // Features and plain-criterion indicators of every leaf, in leaf order (device buffers kept).
-    int tile_features(std::vector<uint32_t>& leaf_slots) {
+    // The leaves, in leaf order.
+    int leaf_slots(std::vector<uint32_t>& out) {
         if (kind != AMR_SIM_BSSN_EVOLVE) return AMR_ERR_INVALID;
-        int st = prepare();
-        if (st) return st;
-        leaf_slots = leaves;
+        const int st = prepare();
+        if (!st) out = leaves;
+        return st;
+    }
+    // Features and plain-criterion indicators of every leaf, in leaf order, into the caller's device
+    // buffers or, where one is null, into buffers kept here.
+    int tile_features(float* features, float* indicators) {
         const size_t need = leaves.size();
-        if (need > feat_cap) {
+        if (need > feat_cap && (!features || !indicators)) {
             cudaStreamSynchronize(stream);
             cudaFree(d_feat); cudaFree(d_ind); cudaFree(d_pred);
             d_feat = d_ind = d_pred = nullptr;
@@ -429,13 +433,14 @@ public:
         g.n_items = (uint32_t)leaves.size();
         g.n = dims.n; g.p = dims.p; g.t = dims.t;
         g.outer_size = cfg.outer_size;
-        g.features = d_feat;
-        g.indicator = d_ind;
+        g.features = features ? features : d_feat;
+        g.indicator = indicators ? indicators : d_ind;
         return check(launch_evo_features(g, stream));
     }
     int regrid(amr_estimator* est, const amr_regrid& r, uint32_t* stats) {
         std::vector<uint32_t> leaf;
-        int st = tile_features(leaf);
+        int st = leaf_slots(leaf);
+        if (!st) st = tile_features(nullptr, nullptr);
         if (st) return st;
         const size_t nl = leaf.size();
         std::vector<float> ind(nl), pred(nl, 0.f);
@@ -526,8 +531,6 @@ public:
         }
         return AMR_OK;
     }
-    float* features_ptr() const { return d_feat; }
-    float* indicator_ptr() const { return d_ind; }
 
 private:
     float* d_feat = nullptr;
@@ -656,18 +659,14 @@ AMR_API int amr_sim_tile_features(amr_sim* s, float* features, float* indicators
     if (!v) return AMR_ERR_INVALID;
     int st = s->impl->wait_side(-1, 0);
     std::vector<uint32_t> leaf;
-    if (!st) st = v->tile_features(leaf);
+    if (!st) st = v->leaf_slots(leaf);
     if (st) return st;
     *n_leaves = (uint32_t)leaf.size();
-    if (leaf.size() > capacity) return AMR_ERR_CAPACITY;
-    cudaStream_t stream = s->impl->stream;
-    cudaError_t e = cudaSuccess;
-    if (features && !leaf.empty())
-        e = cudaMemcpyAsync(features, v->features_ptr(), leaf.size() * 1536u * 4u, cudaMemcpyDeviceToDevice, stream);
-    if (e == cudaSuccess && indicators && !leaf.empty())
-        e = cudaMemcpyAsync(indicators, v->indicator_ptr(), leaf.size() * 4u, cudaMemcpyDeviceToDevice, stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
-    if (e != cudaSuccess) return cuda_status(e);
+    if (leaf.size() > capacity) return AMR_ERR_CAPACITY;   // the count alone: nothing is launched
+    if (!leaf.empty() && (features || indicators)) {
+        if ((st = v->tile_features(features, indicators))) return st;
+        if ((st = cuda_status(cudaStreamSynchronize(s->impl->stream)))) return st;
+    }
     if (leaf_slots) std::memcpy(leaf_slots, leaf.data(), leaf.size() * 4u);
     return AMR_OK;
 }
