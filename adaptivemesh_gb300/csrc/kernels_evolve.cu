@@ -758,66 +758,50 @@ __global__ void __launch_bounds__(256) k_evo_prolong(const __grid_constant__ Evo
 }
 
 // ------------------------------------------------------------------ tile features and the plain criterion
-// One CTA of 512 threads per leaf.  A feature cell of the 8^3 grid covers (N/8)^3 domain cells.  Per
-// domain cell: the undivided gradients |d chi| and |d alpha| (second-order centred differences, i.e. the
-// gradient times the cell size) and |d gt| (the norm over the conformal metric's components and axes).
-// Features of a feature cell: the mean conformal factor, log10(max (|d chi| + |d alpha|) + 1e-10) / 5 + 1
-// and log10(rms |d gt| + 1e-10) / 5 + 1.  The plain criterion's indicator of the tile is the largest
-// |d chi| + |d alpha| over its cells.
-// A thread takes one x of a feature cell and its (N/8)^2 rows, so that a warp reads runs of consecutive
-// cells, and the N/8 lanes of a feature cell combine by shuffles (a thread per feature cell read every
-// second cell, twice the L1 wavefronts).
+// One CTA of 512 threads per leaf; thread = cell of the 8^3 feature grid, which covers (N/8)^3
+// domain cells.  Per domain cell: the undivided gradients |d chi| and |d alpha| (second-order centred
+// differences, i.e. the gradient times the cell size) and |d gt| (the norm over the conformal
+// metric's components and axes).  Features of a feature cell: the mean conformal factor,
+// log10(max (|d chi| + |d alpha|) + 1e-10) / 5 + 1 and log10(rms |d gt| + 1e-10) / 5 + 1.  The plain
+// criterion's indicator of the tile is the largest |d chi| + |d alpha| over its cells.
 __global__ void __launch_bounds__(512) k_evo_features(const EvoFeatureArgs g) {
     const uint32_t b = blockIdx.x;
     if (b >= g.n_items) return;
     const uint32_t slot = g.items[b], n = g.n, t = g.t, p = g.p, r = n / 8u;
+    const uint32_t c = threadIdx.x, cx = c % 8, cy = (c / 8) % 8, cz = c / 64;
     const uint64_t base = (uint64_t)slot * t * t * t;
-    const uint32_t st[3] = {1, t, t * t};
+    const uint64_t st[3] = {1, t, (uint64_t)t * t};
+    float chi = 0.f, g2 = 0.f, ind = 0.f;
+    for (uint32_t k = 0; k < r * r * r; k++) {
+        const uint32_t x = cx * r + k % r + p, y = cy * r + (k / r) % r + p, z = cz * r + k / (r * r) + p;
+        const uint64_t o = base + ((uint64_t)z * t + y) * t + x;
+        chi += g.state[F_CHI][o] + bssn_offset(F_CHI);
+        float dchi = 0.f, dal = 0.f;
+        for (int a = 0; a < 3; a++) {
+            const float dc = .5f * (g.state[F_CHI][o + st[a]] - g.state[F_CHI][o - st[a]]);
+            const float da = .5f * (g.state[F_ALPHA][o + st[a]] - g.state[F_ALPHA][o - st[a]]);
+            dchi += dc * dc;
+            dal += da * da;
+            for (int q = 0; q < 6; q++) {
+                const float dg = .5f * (g.state[F_GXX + q][o + st[a]] - g.state[F_GXX + q][o - st[a]]);
+                g2 += dg * dg;
+            }
+        }
+        ind = fmaxf(ind, sqrtf(dchi) + sqrtf(dal));   // per-cell differences are already times dx
+    }
     const float inv = 1.f / (float)(r * r * r);
     float* f = g.features + (uint64_t)b * 3u * 512u;
-    float top = 0.f;
-    for (uint32_t w = threadIdx.x; w < n * 64u; w += 512u) {   // n = 8, 16 or 32: whole rounds
-        const uint32_t x = w % n, fy = (w / n) % 8u, fz = w / (n * 8u);
-        float chi = 0.f, g2 = 0.f, ind = 0.f;
-        for (uint32_t k = 0; k < r * r; k++) {
-            const uint64_t o = base + ((uint64_t)(fz * r + k / r + p) * t + fy * r + k % r + p) * t + x + p;
-            chi += g.state[F_CHI][o] + bssn_offset(F_CHI);
-            float dchi = 0.f, dal = 0.f;
-#pragma unroll
-            for (int a = 0; a < 3; a++) {
-                const float dc = .5f * (g.state[F_CHI][o + st[a]] - g.state[F_CHI][o - st[a]]);
-                const float da = .5f * (g.state[F_ALPHA][o + st[a]] - g.state[F_ALPHA][o - st[a]]);
-                dchi += dc * dc;
-                dal += da * da;
-#pragma unroll
-                for (int q = 0; q < 6; q++) {
-                    const float dg = .5f * (g.state[F_GXX + q][o + st[a]] - g.state[F_GXX + q][o - st[a]]);
-                    g2 += dg * dg;
-                }
-            }
-            ind = fmaxf(ind, sqrtf(dchi) + sqrtf(dal));   // per-cell differences are already times dx
-        }
-        for (uint32_t q = 1; q < r; q <<= 1) {
-            chi += __shfl_xor_sync(0xffffffffu, chi, q);
-            g2 += __shfl_xor_sync(0xffffffffu, g2, q);
-            ind = fmaxf(ind, __shfl_xor_sync(0xffffffffu, ind, q));
-        }
-        top = fmaxf(top, ind);
-        if (x % r == 0u) {
-            const uint32_t c = (fz * 8u + fy) * 8u + x / r;
-            f[c] = chi * inv;
-            f[512 + c] = log10f(ind + 1e-10f) * .2f + 1.f;
-            f[1024 + c] = log10f(sqrtf(g2 * inv) + 1e-10f) * .2f + 1.f;
-        }
-    }
-    __shared__ float red[16];
-    for (uint32_t q = 16; q > 0; q >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, q));
-    if (threadIdx.x % 32u == 0u) red[threadIdx.x / 32u] = top;
+    f[c] = chi * inv;
+    f[512 + c] = log10f(ind + 1e-10f) * .2f + 1.f;
+    f[1024 + c] = log10f(sqrtf(g2 * inv) + 1e-10f) * .2f + 1.f;
+    __shared__ float red[512];
+    red[c] = ind;
     __syncthreads();
-    if (threadIdx.x == 0u) {
-        for (int q = 1; q < 16; q++) top = fmaxf(top, red[q]);
-        g.indicator[b] = top;
+    for (uint32_t w = 256; w > 0; w >>= 1) {
+        if (c < w) red[c] = fmaxf(red[c], red[c + w]);
+        __syncthreads();
     }
+    if (c == 0) g.indicator[b] = red[0];
 }
 
 }  // namespace
