@@ -21,22 +21,23 @@ struct EvoInitArgs {
     InitData id;
 };
 
-// Ghost fill of X (the state being filled) for the faces normal to `axis` of the listed slots.
+// Ghost fill of X (the state being filled) for listed faces normal to `axis`: n_interp faces with a
+// coarser source, then n_copy with a same-depth one.
 struct EvoGhostArgs {
     float* X[kMaxFields];
     const float* old_f[kMaxFields];
     const float* new_f[kMaxFields];
     const uint64_t* boundaries;
     const uint8_t* evolved;       // per slot: 1 if the slot is evolved (not covered by eight children)
-    const uint32_t* items;
-    uint32_t n_items;
-    uint32_t n, p, t;
+    const uint32_t* faces;        // slot << 1 | side (0: the + face); nullptr: the words in `face`
+    uint32_t face[2];
+    uint32_t n_interp, n_copy;
+    uint32_t n;
     uint32_t substep, max_depth;
     int axis;
     int nf;
     float c_stage;                // time of the state being filled, as a fraction of the target's step
-    uint32_t interp_floats;       // shared memory of the interpolating faces (set by the launcher)
-    int* err;                     // raised when a face needs more than that
+    int* err;                     // raised when a face needs more shared memory than its launch provides
 };
 
 // Device addresses of the four constraint buffers (H, M_x, M_y, M_z; inner layout).
@@ -101,6 +102,7 @@ cudaError_t prepare_evo_stage_bssn(uint32_t n);
 cudaError_t launch_evo_stage_bssn(const EvoArgs& a, cudaStream_t st);
 cudaError_t launch_evo_rhs_wave(const EvoArgs& a, cudaStream_t st);
 cudaError_t launch_evo_ghost(const EvoGhostArgs& g, cudaStream_t st);
+cudaError_t prepare_evo_ghost(uint32_t n);   // its shared-memory limits, outside a stream capture
 cudaError_t launch_evo_constraints(const EvoArgs& a, const ConsPtrs& cons, cudaStream_t st);
 // FP64 norms of the constraints over the composite grid of the listed slots (interior cells no child
 // covers), leaving out cells within the excision radius of a puncture: out[0] rms H, [1] max |H|,

@@ -43,7 +43,7 @@ public:
         if (graph_exec) cudaGraphExecDestroy(graph_exec);
         for (int f = 0; f < kMaxFields; f++) { cudaFree(old_f[f]); cudaFree(new_f[f]); cudaFree(stage_f[f]); cudaFree(acc[f]); }
         for (float* c : cons.c) cudaFree(c);
-        cudaFree(deriv); cudaFree(d_evolved); cudaFree(d_lists); cudaFree(d_part); cudaFree(d_norms);
+        cudaFree(deriv); cudaFree(d_evolved); cudaFree(d_faces); cudaFree(d_lists); cudaFree(d_part); cudaFree(d_norms);
         cudaFree(d_feat); cudaFree(d_ind); cudaFree(d_pred);
     }
     int init() override {
@@ -69,6 +69,7 @@ public:
             std::memset(&none, 0, sizeof(none));
             none.n = dims.n;
             e = launch_evo_derivs(none, stream);
+            if (e == cudaSuccess) e = prepare_evo_ghost(dims.n);
             if (e == cudaSuccess && kind == AMR_SIM_BSSN_EVOLVE) e = prepare_evo_stage_bssn(dims.n);
         }
         return cuda_status(e);
@@ -169,10 +170,37 @@ public:
         all_evolved_cnt = (uint32_t)all.size() - all_evolved_off;
         leaves_off = (uint32_t)all.size();
         all.insert(all.end(), leaves.begin(), leaves.end());
+        // the ghost fill's faces per substep and axis: interpolating ones first, then copies
+        std::vector<uint32_t> faces, copies;
+        for (int a = 0; a < 3; a++) { face_off[a].assign(nsub, 0); face_interp[a].assign(nsub, 0); face_copy[a].assign(nsub, 0); }
+        for (uint32_t s = 0; s < nsub; s++)
+            for (int a = 0; a < 3; a++) {
+                copies.clear();
+                face_off[a][s] = (uint32_t)faces.size();
+                for (uint32_t k = evo_off[s]; k < evo_off[s] + evo_cnt[s]; k++)
+                    for (uint32_t side = 0; side < 2; side++) {
+                        const int c = face_class(all[k], a, side);
+                        if (c) (c == 2 ? faces : copies).push_back(all[k] << 1 | side);
+                    }
+                face_interp[a][s] = (uint32_t)faces.size() - face_off[a][s];
+                face_copy[a][s] = (uint32_t)copies.size();
+                faces.insert(faces.end(), copies.begin(), copies.end());
+            }
+        if (faces.size() > faces_cap) {
+            cudaError_t e = cudaStreamSynchronize(stream);
+            cudaFree(d_faces);
+            d_faces = nullptr;
+            faces_cap = 0;
+            if (e == cudaSuccess) e = dev_alloc(&d_faces, faces.size());
+            if (e != cudaSuccess) return cuda_status(e);
+            faces_cap = faces.size();
+        }
         const size_t cap = (size_t)tree.max_slots() * 2u * ((size_t)1u << kDepthLimit) + 2u * tree.max_slots();
         if (all.size() > cap) return AMR_ERR_CAPACITY;
         cudaError_t e = cudaMemcpyAsync(d_lists, all.data(), all.size() * 4u, cudaMemcpyHostToDevice, stream);
         if (e == cudaSuccess) e = cudaMemcpyAsync(d_evolved, evolved.data(), evolved.size(), cudaMemcpyHostToDevice, stream);
+        if (e == cudaSuccess && !faces.empty())
+            e = cudaMemcpyAsync(d_faces, faces.data(), faces.size() * 4u, cudaMemcpyHostToDevice, stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
         if (e != cudaSuccess) return cuda_status(e);
         lists_valid = true;
@@ -577,9 +605,7 @@ private:
         for (int f = 0; f < nf; f++) { g.X[f] = x[f]; g.old_f[f] = old_f[f]; g.new_f[f] = new_f[f]; }
         g.boundaries = d_boundaries;
         g.evolved = d_evolved;
-        g.items = d_lists + evo_off[s];
-        g.n_items = evo_cnt[s];
-        g.n = dims.n; g.p = dims.p; g.t = dims.t;
+        g.n = dims.n;
         g.substep = s;
         g.max_depth = (uint32_t)tree.read_max_depth();
         g.nf = nf;
@@ -588,19 +614,47 @@ private:
         for (int axis = 0; axis < 3; axis++) {   // every domain's pass along an axis before the next axis
             g.axis = axis;
             if (mode == AMR_MODE_PLAIN) {   // one launch per domain
-                const uint32_t* base = d_lists + evo_off[s];
-                for (uint32_t i = 0; i < evo_cnt[s]; i++) {
-                    g.items = base + i;
-                    g.n_items = 1;
+                for (uint32_t i : sub_evolved(s)) {
+                    g.faces = nullptr;
+                    g.n_interp = g.n_copy = 0;
+                    for (int c = 2; c >= 1; c--)
+                        for (uint32_t side = 0; side < 2; side++)
+                            if (face_class(i, axis, side) == c) {
+                                g.face[g.n_interp + g.n_copy] = i << 1 | side;
+                                (c == 2 ? g.n_interp : g.n_copy)++;
+                            }
+                    if (g.n_interp + g.n_copy == 0u) continue;
                     const int st = check(launch_evo_ghost(g, stream));
                     if (st) return st;
                 }
                 continue;
             }
+            g.faces = d_faces + face_off[axis][s];
+            g.n_interp = face_interp[axis][s];
+            g.n_copy = face_copy[axis][s];
+            if (g.n_interp + g.n_copy == 0u) continue;
             const int st = check(launch_evo_ghost(g, stream));
             if (st) return st;
         }
         return AMR_OK;
+    }
+    // how the ghost fill treats a face: 0 not at all (no source, or the root's), 1 copy, 2 interpolate
+    int face_class(uint32_t slot, int axis, uint32_t side) const {
+        const uint32_t nd = (uint32_t)tree.boundaries()[(size_t)slot * 6u + (size_t)axis + 3u * side];
+        const bool none = (nd & 0xFFFFFFu) == 0xFFFFFFu;                // target -1
+        const uint32_t depth = nd >> 28, diff = (nd >> 24) & 15u;
+        if (none || depth == 15u || depth == 0u) return 0;
+        return diff == 0u ? 1 : 2;
+    }
+    // the substep's active evolved domains in slot order
+    std::vector<uint32_t> sub_evolved(uint32_t s) const {
+        const uint32_t md = (uint32_t)tree.read_max_depth();
+        std::vector<uint32_t> v;
+        for (uint32_t i = 0; i < tree.curr_used_slots(); i++) {
+            const int d = pos_depth_host(tree.positions()[i]);
+            if (d != -1 && (s & ((1u << (md - (uint32_t)d)) - 1u)) == 0u) v.push_back(i);
+        }
+        return v;
     }
 
     int kind, nf, nd;
@@ -617,6 +671,9 @@ private:
     double* d_part = nullptr;
     double* d_norms = nullptr;
     bool lists_valid = false;
+    uint32_t* d_faces = nullptr;   // the ghost fill's face lists
+    size_t faces_cap = 0;
+    std::vector<uint32_t> face_off[3], face_interp[3], face_copy[3];   // per axis and substep
     std::vector<uint32_t> act_off, act_cnt, act_leaves, evo_off, evo_cnt, leaves;
     uint32_t all_evolved_off = 0, all_evolved_cnt = 0, leaves_off = 0;
     uint32_t deriv_zs = 0;   // the derivative pass's slab depth (0: the default; amr_sim_autotune)

@@ -336,126 +336,149 @@ __global__ void __launch_bounds__(256) k_evo_rhs_wave(const __grid_constant__ Ev
 }
 
 // ------------------------------------------------------------------ ghost fill
-// A CTA per (slot, side, group of kGhostFields fields).  A same-depth face is a copy: the geometry of
-// a ghost cell is computed once per group and every load of a cell's group is issued before its
-// stores.  A face with a coarser source is interpolated separably through shared memory (below).
-// Within one launch (one face-normal axis) no cell is both read and written: the fill writes the
-// cells whose index along the axis lies in a ghost layer and reads sources inside the interior
-// along it.
-constexpr int kGhostFields = 4;
-constexpr uint32_t kGhostMaxT = 38;   // the largest padded edge (32 + 2 * 3)
-// Shared memory of the interpolating faces, in floats, for padded edge t, size n, padding p: the
-// per-axis tables, then the largest source box (E_a <= ext_a / 2 + 5 cells along each axis, the
-// source being at least twice as coarse) and the two intermediate stages, over the three passes.
-inline uint32_t ghost_interp_floats(uint32_t n, uint32_t p, uint32_t t) {
-    uint32_t best = 0;
-    for (uint32_t d = 0; d < 3; d++) {
-        uint32_t ext[3], E[3];
-        for (uint32_t a = 0; a < 3; a++) {
-            ext[a] = a == d ? p : (a < d ? t : n);
-            E[a] = ext[a] / 2u + 5u;
-        }
-        const uint32_t need = E[0] * E[1] * E[2] + E[2] * E[1] * ext[0] + E[2] * ext[1] * ext[0];
-        best = need > best ? need : best;
-    }
-    return best;
-}
+// Per launch the faces normal to one axis: the host lists those that have a source, the interpolating
+// ones (a coarser source) first, as they take longest, then the same-depth copies (evolve_sim.cu).  The
+// axis and the domain size are compile-time, so that every division of an index is by a constant.
+// Within a launch no cell is both read and written: the fill writes the cells whose index along the axis
+// lies in a ghost layer and reads sources inside the interior along it.
+//
+// Copies: a CTA per (face, kGhostCopyFields fields); a same-depth source is this domain shifted by a whole
+// domain, so that rows and planes are moved as 8- and 16-byte vectors (a y face is three whole rows a plane, a z
+// face three whole planes; an x face three cells a row), kGhostInFlight loads per thread before their
+// stores.
+// Interpolations: a CTA per (face, 2 fields), the two fields as the lanes of packed pairs, so that one
+// index computation, one shared-memory read and one instruction serve both; the fields of a face in CTAs
+// of their own instead of one after another in one CTA, whose twelve synchronised passes were the
+// latency of the launch.
+// GB300, per launch, before -> now: 585 domains of 16^3, all copies, x 168 -> 124 us (12-byte runs: 1.25
+// sectors read and 1.25 written for each, 860 MB of them, 129 us at the copy bandwidth), y 78 -> 54, z 76 -> 47 (326 MB, 49 us);
+// nested tree of 201 domains 39 -> 23 on average; two fields beside a coarser domain 13.2 -> 8.3 (latency).
+constexpr int kGhostCopyFields = 8, kGhostInFlight = 8;
+template <int N, int AXIS>
+struct GhostShape {
+    static constexpr int P = 3, T = N + 2 * P;
+    // extents of the fill: axes before the normal over the whole padded range (their ghosts are
+    // filled), axes after it over the interior
+    static constexpr int ext(int a) { return a == AXIS ? P : (a < AXIS ? T : N); }
+    static constexpr int E0 = ext(0), E1 = ext(1), E2 = ext(2);
+    static constexpr int VEC = AXIS == 0 ? 1 : (AXIS == 1 ? 2 : 4);       // floats per copied vector
+    static constexpr int COUNT = E0 * E1 * E2 / VEC;                      // vectors per face and field
+    static_assert(AXIS != 2 || (T * T) % 4 == 0, "whole planes are 16-byte vectors");
+    static_assert(AXIS == 0 || (P * T) % 2 == 0, "whole rows are 8-byte vectors");
+    // Interpolation: the largest source box (the source is at least twice as coarse) and the two
+    // intermediate stages; the second takes the box's place.
+    static constexpr int box(int a) { return ext(a) / 2 + 5; }
+    static constexpr int even(int v) { return (v + 1) / 2 * 2; }   // the weights behind them are 16-byte vectors
+    static constexpr int BOX = box(0) * box(1) * box(2), ST1 = even(box(2) * box(1) * E0), ST2 = box(2) * E1 * E0;
+    static constexpr int FIRST = even(BOX > ST2 ? BOX : ST2);
+    static constexpr size_t SMEM = (size_t)(FIRST + ST1) * 8u + (size_t)(E0 + E1 + E2) * 5u * 4u;
+};
 
-__global__ void __launch_bounds__(256, 4) k_evo_ghost(const __grid_constant__ EvoGhostArgs g) {
-    const uint32_t item = blockIdx.x >> 1, side = blockIdx.x & 1u;   // side 0: + face, 1: - face
-    const int f0 = (int)blockIdx.y * kGhostFields;
-    if (item >= g.n_items || f0 >= g.nf) return;
-    const uint32_t slot = g.items[item];
-    const uint32_t n = g.n, p = g.p, t = g.t, d = (uint32_t)g.axis;
-    const uint32_t face = d + 3u * side;
-    const uint64_t bd = g.boundaries[(size_t)slot * 6u + face];
+template <int N, int AXIS>
+__global__ void __launch_bounds__(256) k_evo_ghost(const __grid_constant__ EvoGhostArgs g) {
+    using S = GhostShape<N, AXIS>;
+    constexpr int P = S::P, T = S::T;
+    constexpr int64_t CELLS = (int64_t)T * T * T;
+    const uint32_t gi = (uint32_t)(g.nf + 1) / 2u, gc = (uint32_t)(g.nf + kGhostCopyFields - 1) / kGhostCopyFields;
+    const bool interp = blockIdx.x < g.n_interp * gi;
+    const uint32_t b = interp ? blockIdx.x : blockIdx.x - g.n_interp * gi;
+    const uint32_t k = interp ? b / gi : g.n_interp + b / gc;
+    const uint32_t word = g.faces ? g.faces[k] : g.face[k];   // slot << 1 | side; side 0: + face, 1: - face
+    const uint32_t slot = word >> 1, side = word & 1u;
+    const uint64_t bd = g.boundaries[(size_t)slot * 6u + AXIS + 3u * side];
     const int32_t src = bd_target(bd);
     const int cd = bd_curr_depth(bd);
-    if (src == -1 || cd <= 0) return;
     const uint32_t dd = bd_depth_diff(bd);
-    const int sd = cd - (int)dd;
-    const bool root_src = src == 0;
     const bool src_evolved = g.evolved[src] != 0;
-    const bool src_active = active_depth(g.substep, (uint32_t)sd, g.max_depth);
+    const float3 relp = cf3_decode((uint32_t)(bd >> 32));
+    constexpr int lo_other[3] = {AXIS > 0 ? 0 : P, AXIS > 1 ? 0 : P, P};   // the fill's first index along the other axes
+    const int lo_d = side == 0u ? P + N : 0;
+    const int lo0 = AXIS == 0 ? lo_d : lo_other[0], lo1 = AXIS == 1 ? lo_d : lo_other[1], lo2 = AXIS == 2 ? lo_d : lo_other[2];
+
+    if (!interp) {   // ---- a same-depth source: active whenever this domain is; its state at the same stage
+        const int f0 = (int)(b % gc) * kGhostCopyFields, nfg = min(kGhostCopyFields, g.nf - f0);
+        const int r0 = __float2int_rn(relp.x * (float)N), r1 = __float2int_rn(relp.y * (float)N),
+                  r2 = __float2int_rn(relp.z * (float)N);
+        const int64_t shift = ((int64_t)src - (int64_t)slot) * CELLS + ((int64_t)r2 * T + r1) * T + r0;
+        const int64_t dst = (int64_t)slot * CELLS;
+        auto move = [&](auto vec, int count, auto cell) {   // count vectors a field, cell(k) their first cell
+            using V = decltype(vec);
+            const int total = nfg * count;
+            for (int e0 = (int)threadIdx.x; e0 < total; e0 += 256 * kGhostInFlight) {
+                V v[kGhostInFlight];
+#pragma unroll
+                for (int i = 0; i < kGhostInFlight; i++) {
+                    const int e = e0 + 256 * i;
+                    if (e >= total) break;
+                    const float* s = src_evolved ? g.X[f0 + e / count] : g.old_f[f0 + e / count];
+                    v[i] = *reinterpret_cast<const V*>(s + (dst + shift + cell(e % count)));
+                }
+#pragma unroll
+                for (int i = 0; i < kGhostInFlight; i++) {
+                    const int e = e0 + 256 * i;
+                    if (e >= total) break;
+                    *reinterpret_cast<V*>(g.X[f0 + e / count] + (dst + cell(e % count))) = v[i];
+                }
+            }
+        };
+        if constexpr (AXIS == 0) {
+            move(0.f, S::COUNT, [&](int q) { return ((q / (P * N) + P) * T + (q / P) % N + P) * T + lo0 + q % P; });
+        } else if (shift % S::VEC == 0) {
+            if constexpr (AXIS == 1)
+                move(float2{}, S::COUNT, [&](int q) { return ((q / (P * T / 2) + P) * T + lo1) * T + 2 * (q % (P * T / 2)); });
+            else
+                move(float4{}, S::COUNT, [&](int q) { return lo2 * T * T + 4 * q; });
+        } else {   // a caller's own boundary record with another offset: cell by cell
+            move(0.f, S::COUNT * S::VEC, [&](int q) {
+                return ((lo2 + q / (S::E0 * S::E1)) * T + lo1 + (q / S::E0) % S::E1) * T + lo0 + q % S::E0;
+            });
+        }
+        return;
+    }
+    // ---- A coarser source: separable tricubic interpolation through shared memory.  Along each axis a
+    // the ghost cell's coordinate w_a alone gives the base cell b_a of its four-point stencil
+    // b_a - 1 .. b_a + 2 and the four Lagrange weights; b_a is kept inside the cells that are
+    // valid (the interior along the normal axis and the later axes, the whole padded range along
+    // the earlier axes, which earlier passes filled, and everywhere in the root, whose frozen
+    // ghost layer is the outer boundary).  b_a grows with w_a, so the source cells read form a
+    // box.  The box, with the time interpolation applied to each source cell (frac X + (1 - frac) old, or
+    // old alone), then the interpolation along x, along y and along z, each stage through shared memory.
+    extern __shared__ __align__(16) unsigned char ghost_smem[];
+    float2* const box = reinterpret_cast<float2*>(ghost_smem);   // the source box, then the second stage
+    float2* const t1 = box + S::FIRST;                           // [E2][E1][ext0]
+    float2* const t2 = box;                                      // [E2][ext1][ext0]
+    float* const W = reinterpret_cast<float*>(t1 + S::ST1);      // [ext0 + ext1 + ext2][4] weights
+    int* const B = reinterpret_cast<int*>(W + (S::E0 + S::E1 + S::E2) * 4);   // base cells
+    const int f0 = (int)(b % gi) * 2, f1 = min(f0 + 1, g.nf - 1);
+    const bool root_src = src == 0;
+    const bool src_active = active_depth(g.substep, (uint32_t)(cd - (int)dd), g.max_depth);
     // the source's state at the time of the value being filled (evolve.h)
-    int mode;      // 0: old only, 1: X only, 2: old..X, 3: old..new
+    int mode;      // 0: old only, 2: old..X, 3: old..new
     float frac = 0.f;
     if (!src_evolved) mode = 0;
     else if (src_active) {
-        mode = dd == 0u ? 1 : 2;
+        mode = 2;
         frac = 1.f / (float)(1u << dd);
     } else {
         mode = 3;
         const uint32_t kp = (g.substep >> (g.max_depth - (uint32_t)cd)) & ((1u << dd) - 1u);
         frac = ((float)kp + g.c_stage) / (float)(1u << dd);
     }
-    const float3 relp = cf3_decode((uint32_t)(bd >> 32));
     const float rel_scale = 1.f / (float)(1u << dd);
-    // extents of the fill: axes before d over the whole padded range (their ghosts are filled),
-    // axes after d over the interior
-    auto lo_of = [&](uint32_t a2) { return a2 == d ? (side == 0 ? p + n : 0u) : (a2 < d ? 0u : p); };
-    auto ext_of = [&](uint32_t a2) { return a2 == d ? p : (a2 < d ? t : n); };
-    const uint32_t lo0 = lo_of(0), lo1 = lo_of(1), lo2 = lo_of(2);
-    const uint32_t ext0 = ext_of(0), ext1 = ext_of(1), ext2 = ext_of(2);
-    const int nfg = min(kGhostFields, g.nf - f0);
-    // field of group member q (members past the last field repeat it; they are never stored)
-    auto fld = [&](int q) { return f0 + min(q, nfg - 1); };
-    auto A0 = [&](int q) { return g.old_f[fld(q)]; };
-    auto A1 = [&](int q) { return mode == 3 ? g.new_f[fld(q)] : (const float*)g.X[fld(q)]; };
-    const uint32_t count = ext0 * ext1 * ext2;
-    const uint64_t cells = (uint64_t)t * t * t;
-    const bool exact = dd == 0u;
-    // k -> (w0, w1, w2) by multiplication: floor(k * ceil(2^21 / e) / 2^21) = floor(k / e) for
-    // k < 2^21 / 38^2 and e <= 38 (the error k * (ceil - exact) / 2^21 stays below 1 / e)
-    const uint32_t m0 = ((1u << 21) + ext0 - 1u) / ext0, m1 = ((1u << 21) + ext1 - 1u) / ext1;
-    // a same-depth source is this domain shifted by rel * n cells (rel = 0 or +-1 per axis, exact)
-    const int r0 = __float2int_rn(relp.x * (float)n), r1 = __float2int_rn(relp.y * (float)n),
-              r2 = __float2int_rn(relp.z * (float)n);
-    if (exact) {
-        for (uint32_t k = threadIdx.x; k < count; k += blockDim.x) {
-            const uint32_t q = (uint32_t)(((uint64_t)k * m0) >> 21), q2 = (uint32_t)(((uint64_t)q * m1) >> 21);
-            const uint32_t w0 = lo0 + (k - q * ext0), w1 = lo1 + (q - q2 * ext1), w2 = lo2 + q2;
-            const uint64_t dst = (uint64_t)slot * cells + ((uint64_t)w2 * t + w1) * t + w0;
-            // a copy: every load of the group, then the stores
-            const int64_t si = (int64_t)src * (int64_t)cells + ((int64_t)((int)w2 + r2) * t + ((int)w1 + r1)) * t +
-                               ((int)w0 + r0);
-            float v[kGhostFields];
-#pragma unroll
-            for (int q4 = 0; q4 < kGhostFields; q4++)
-                v[q4] = mode == 0 ? A0(q4)[si] : (mode == 1 ? A1(q4)[si] : fmaf(frac, A1(q4)[si], (1.f - frac) * A0(q4)[si]));
-#pragma unroll
-            for (int q4 = 0; q4 < kGhostFields; q4++)
-                if (q4 < nfg) g.X[f0 + q4][dst] = v[q4];
-        }
-        return;
-    }
-    // A coarser source: separable tricubic interpolation through shared memory.  Along each axis a
-    // the ghost cell's coordinate w_a alone gives the base cell b_a of its four-point stencil
-    // b_a - 1 .. b_a + 2 and the four Lagrange weights; b_a is kept inside the cells that are
-    // valid (the interior along the normal axis and the later axes, the whole padded range along
-    // the earlier axes, which earlier passes filled, and everywhere in the root, whose frozen
-    // ghost layer is the outer boundary).  b_a grows with w_a, so the source cells read form a
-    // box.  Per field: the box, with the time interpolation applied to each source cell
-    // (frac X + (1 - frac) old, or old alone), then the interpolation along x, along y and along z,
-    // each stage through shared memory.
-    extern __shared__ __align__(16) float gsm[];
-    float* W = gsm;                                                  // [3][kGhostMaxT][4] weights
-    int* B = reinterpret_cast<int*>(W + 3 * kGhostMaxT * 4);         // [3][kGhostMaxT] base cells
-    float* S = reinterpret_cast<float*>(B + 3 * kGhostMaxT);         // source box (time-interpolated)
-    for (uint32_t e = threadIdx.x; e < ext0 + ext1 + ext2; e += blockDim.x) {
-        const uint32_t a2 = e < ext0 ? 0u : (e < ext0 + ext1 ? 1u : 2u);
-        const uint32_t j = e - (a2 == 0u ? 0u : (a2 == 1u ? ext0 : ext0 + ext1));
-        const uint32_t wa = (a2 == 0u ? lo0 : (a2 == 1u ? lo1 : lo2)) + j;
-        float rp = ((float)wa - (float)p + .5f) / (float)n - .5f;
-        rp = rp * rel_scale + (a2 == 0u ? relp.x : (a2 == 1u ? relp.y : relp.z));
-        const float ri = (rp + .5f) * (float)n + (float)p - .5f;
-        const int lo_c = root_src || a2 < d ? 1 : (int)p + 1;
-        const int hi_c = root_src || a2 < d ? (int)t - 3 : (int)(t - p) - 3;
-        int b = __float2int_rd(ri);
-        b = b < lo_c ? lo_c : (b > hi_c ? hi_c : b);
-        const float x = ri - (float)b;
-        B[a2 * kGhostMaxT + j] = b;
-        float* w = W + (a2 * kGhostMaxT + j) * 4;
+    for (int e = (int)threadIdx.x; e < S::E0 + S::E1 + S::E2; e += 256) {
+        const int a2 = e < S::E0 ? 0 : (e < S::E0 + S::E1 ? 1 : 2);
+        const int j = e - (a2 == 0 ? 0 : (a2 == 1 ? S::E0 : S::E0 + S::E1));
+        const int wa = (a2 == 0 ? lo0 : (a2 == 1 ? lo1 : lo2)) + j;
+        float rp = ((float)wa - (float)P + .5f) / (float)N - .5f;
+        rp = rp * rel_scale + (a2 == 0 ? relp.x : (a2 == 1 ? relp.y : relp.z));
+        const float ri = (rp + .5f) * (float)N + (float)P - .5f;
+        const int lo_c = root_src || a2 < AXIS ? 1 : P + 1;
+        const int hi_c = root_src || a2 < AXIS ? T - 3 : (T - P) - 3;
+        int c = __float2int_rd(ri);
+        c = c < lo_c ? lo_c : (c > hi_c ? hi_c : c);
+        const float x = ri - (float)c;
+        B[e] = c;
+        float* w = W + e * 4;
         w[0] = -x * (x - 1.f) * (x - 2.f) * (1.f / 6.f);
         w[1] = (x + 1.f) * (x - 1.f) * (x - 2.f) * .5f;
         w[2] = -(x + 1.f) * x * (x - 2.f) * .5f;
@@ -463,59 +486,54 @@ __global__ void __launch_bounds__(256, 4) k_evo_ghost(const __grid_constant__ Ev
     }
     __syncthreads();
     // the box: from b_min - 1 to b_max + 2 along each axis (the first and the last w_a)
-    const int bmin[3] = {B[0], B[kGhostMaxT], B[2 * kGhostMaxT]};
-    const int E[3] = {B[ext0 - 1] - bmin[0] + 4, B[kGhostMaxT + ext1 - 1] - bmin[1] + 4,
-                      B[2 * kGhostMaxT + ext2 - 1] - bmin[2] + 4};
-    const uint32_t nS = (uint32_t)(E[0] * E[1] * E[2]), nT1 = (uint32_t)(E[2] * E[1]) * ext0,
-                   nT2 = (uint32_t)E[2] * ext1 * ext0;
-    if (nS + nT1 + nT2 > g.interp_floats) {   // larger than the launch provided: report, skip the face
+    const int* const B1 = B + S::E0;
+    const int* const B2 = B1 + S::E1;
+    const int m0 = B[0], m1 = B1[0], m2 = B2[0];
+    const int n0 = B[S::E0 - 1] - m0 + 4, n1 = B1[S::E1 - 1] - m1 + 4, n2 = B2[S::E2 - 1] - m2 + 4;
+    const int nS = n0 * n1 * n2, nT1 = n2 * n1 * S::E0, nT2 = n2 * S::E1 * S::E0;
+    if (nS > S::FIRST || nT1 > S::ST1 || nT2 > S::FIRST) {   // larger than the launch provides: report, skip the face
         if (threadIdx.x == 0) atomicExch(g.err, 1);
         return;
     }
-    float* T1 = S + nS;    // [E2][E1][ext0]
-    float* T2 = T1 + nT1;  // [E2][ext1][ext0]
-    const int64_t sbase = (int64_t)src * (int64_t)cells;
-    for (int q4 = 0; q4 < nfg; q4++) {
-        const float* a0 = A0(q4);
-        const float* a1 = A1(q4);
-        for (uint32_t e = threadIdx.x; e < nS; e += blockDim.x) {
-            const uint32_t i0 = e % (uint32_t)E[0], r = e / (uint32_t)E[0];
-            const uint32_t i1 = r % (uint32_t)E[1], i2 = r / (uint32_t)E[1];
-            const int64_t si = sbase + ((int64_t)(bmin[2] - 1 + (int)i2) * t + (bmin[1] - 1 + (int)i1)) * t +
-                               (bmin[0] - 1 + (int)i0);
-            S[e] = mode == 0 ? a0[si] : fmaf(frac, a1[si], (1.f - frac) * a0[si]);
-        }
-        __syncthreads();
-        for (uint32_t e = threadIdx.x; e < nT1; e += blockDim.x) {   // along x
-            const uint32_t j0 = e % ext0, r = e / ext0;              // r = i2 * E1 + i1
-            const float* w = W + j0 * 4;
-            const float* src_row = S + r * (uint32_t)E[0] + (B[j0] - bmin[0]);
-            float v = 0.f;
-#pragma unroll
-            for (int k = 0; k < 4; k++) v = fmaf(w[k], src_row[k], v);
-            T1[e] = v;
-        }
-        __syncthreads();
-        for (uint32_t e = threadIdx.x; e < nT2; e += blockDim.x) {   // along y
-            const uint32_t j0 = e % ext0, r = e / ext0, j1 = r % ext1, i2 = r / ext1;
-            const float* w = W + (kGhostMaxT + j1) * 4;
-            const float* col = T1 + ((size_t)i2 * E[1] + (B[kGhostMaxT + j1] - bmin[1])) * ext0 + j0;
-            float v = 0.f;
-#pragma unroll
-            for (int k = 0; k < 4; k++) v = fmaf(w[k], col[(size_t)k * ext0], v);
-            T2[e] = v;
-        }
-        __syncthreads();
-        for (uint32_t e = threadIdx.x; e < count; e += blockDim.x) {   // along z, into the ghost cells
-            const uint32_t j0 = e % ext0, r = e / ext0, j1 = r % ext1, j2 = r / ext1;
-            const float* w = W + (2 * kGhostMaxT + j2) * 4;
-            const float* col = T2 + ((size_t)(B[2 * kGhostMaxT + j2] - bmin[2]) * ext1 + j1) * ext0 + j0;
-            float v = 0.f;
-#pragma unroll
-            for (int k = 0; k < 4; k++) v = fmaf(w[k], col[(size_t)k * ext1 * ext0], v);
-            g.X[f0 + q4][(uint64_t)slot * cells + ((uint64_t)(lo2 + j2) * t + lo1 + j1) * t + lo0 + j0] = v;
-        }
-        __syncthreads();   // S, T1, T2 are reused by the next field
+    // e -> (i0, i1, i2) by multiplication: floor(e * ceil(2^21 / n) / 2^21) = floor(e / n) for e < 4332 and
+    // n <= 38 (a box has at most 3456 cells)
+    const uint32_t q0 = ((1u << 21) + n0 - 1u) / n0, q1 = ((1u << 21) + n1 - 1u) / n1;
+    const float* const a00 = g.old_f[f0];
+    const float* const a01 = g.old_f[f1];
+    const float* const a10 = mode == 3 ? g.new_f[f0] : (const float*)g.X[f0];
+    const float* const a11 = mode == 3 ? g.new_f[f1] : (const float*)g.X[f1];
+    const int64_t corner = (int64_t)src * CELLS + ((int64_t)(m2 - 1) * T + (m1 - 1)) * T + (m0 - 1);
+    const float2 fr = splat2(frac), om = splat2(1.f - frac);
+#pragma unroll 4
+    for (int e = (int)threadIdx.x; e < nS; e += 256) {
+        const uint32_t r = (uint32_t)(((uint64_t)e * q0) >> 21), i2 = (uint32_t)(((uint64_t)r * q1) >> 21);
+        const int64_t s = corner + ((int)i2 * T + (int)(r - i2 * n1)) * T + (int)(e - r * n0);
+        const float2 o = make_float2(a00[s], a01[s]);
+        box[e] = mode == 0 ? o : fma2(fr, make_float2(a10[s], a11[s]), mul2(om, o));
+    }
+    __syncthreads();
+    auto cubic = [&](const float* w, const float2* p, int stride) {
+        const float4 c = *reinterpret_cast<const float4*>(w);
+        return fma2(splat2(c.w), p[3 * stride], fma2(splat2(c.z), p[2 * stride], fma2(splat2(c.y), p[stride], mul2(splat2(c.x), p[0]))));
+    };
+    for (int e = (int)threadIdx.x; e < nT1; e += 256) {   // along x
+        const int j0 = e % S::E0, r = e / S::E0;          // r = i2 * n1 + i1
+        t1[e] = cubic(W + j0 * 4, box + r * n0 + (B[j0] - m0), 1);
+    }
+    __syncthreads();
+    for (int e = (int)threadIdx.x; e < nT2; e += 256) {   // along y
+        const int j0 = e % S::E0, r = e / S::E0, j1 = r % S::E1, i2 = r / S::E1;
+        t2[e] = cubic(W + (S::E0 + j1) * 4, t1 + (i2 * n1 + (B1[j1] - m1)) * S::E0 + j0, S::E0);
+    }
+    __syncthreads();
+    float* const x0 = g.X[f0] + (int64_t)slot * CELLS;
+    float* const x1 = g.X[f1] + (int64_t)slot * CELLS;
+    for (int e = (int)threadIdx.x; e < S::E0 * S::E1 * S::E2; e += 256) {   // along z, into the ghost cells
+        const int j0 = e % S::E0, r = e / S::E0, j1 = r % S::E1, j2 = r / S::E1;
+        const float2 v = cubic(W + (S::E0 + S::E1 + j2) * 4, t2 + ((B2[j2] - m2) * S::E1 + j1) * S::E0 + j0, S::E1 * S::E0);
+        const int o = ((lo2 + j2) * T + lo1 + j1) * T + lo0 + j0;
+        x0[o] = v.x;
+        if (f1 != f0) x1[o] = v.y;
     }
 }
 
@@ -892,19 +910,48 @@ cudaError_t launch_evo_restrict(const EvoRestrictArgs& g, cudaStream_t st) {
     return cudaGetLastError();
 }
 
-cudaError_t launch_evo_ghost(const EvoGhostArgs& g, cudaStream_t st) {
-    if (g.n_items == 0) return cudaSuccess;
-    if (g.t > kGhostMaxT) return cudaErrorInvalidValue;   // the kernel's index arithmetic and tables cover edges up to 38
-    EvoGhostArgs a = g;
-    a.interp_floats = ghost_interp_floats(g.n, g.p, g.t);
-    const size_t smem = (size_t)(3u * kGhostMaxT * 5u + a.interp_floats) * 4u;
-    static std::atomic<uint64_t> configured{0};   // the limit for the largest edge, once per device
-    const cudaError_t e = ensure_smem_limit(k_evo_ghost, (size_t)(3u * kGhostMaxT * 5u + ghost_interp_floats(32u, 3u, 38u)) * 4u,
-                                            configured);
+template <int N, int AXIS>
+static cudaError_t ghost_limit() {
+    static std::atomic<uint64_t> configured{0};
+    return ensure_smem_limit(k_evo_ghost<N, AXIS>, GhostShape<N, AXIS>::SMEM, configured);
+}
+template <int N, int AXIS>
+static cudaError_t ghost_t(const EvoGhostArgs& g, cudaStream_t st) {
+    const cudaError_t e = ghost_limit<N, AXIS>();
     if (e != cudaSuccess) return e;
-    const dim3 grid(g.n_items * 2u, (unsigned)((g.nf + kGhostFields - 1) / kGhostFields));
-    k_evo_ghost<<<grid, 256, smem, st>>>(a);
+    const uint32_t blocks = g.n_interp * (uint32_t)((g.nf + 1) / 2) +
+                            g.n_copy * (uint32_t)((g.nf + kGhostCopyFields - 1) / kGhostCopyFields);
+    // launches without an interpolating face need none of its shared memory
+    k_evo_ghost<N, AXIS><<<blocks, 256, g.n_interp ? GhostShape<N, AXIS>::SMEM : 0u, st>>>(g);
     return cudaGetLastError();
+}
+template <int N>
+static cudaError_t ghost_n(const EvoGhostArgs& g, cudaStream_t st) {
+    return g.axis == 0 ? ghost_t<N, 0>(g, st) : (g.axis == 1 ? ghost_t<N, 1>(g, st) : ghost_t<N, 2>(g, st));
+}
+template <int N>
+static cudaError_t ghost_limits() {
+    cudaError_t e = ghost_limit<N, 0>();
+    if (e == cudaSuccess) e = ghost_limit<N, 1>();
+    return e == cudaSuccess ? ghost_limit<N, 2>() : e;
+}
+cudaError_t launch_evo_ghost(const EvoGhostArgs& g, cudaStream_t st) {
+    if (g.n_interp + g.n_copy == 0u) return cudaSuccess;
+    if (g.axis < 0 || g.axis > 2 || g.nf < 1 || g.nf > kMaxFields) return cudaErrorInvalidValue;
+    switch (g.n) {
+        case 8: return ghost_n<8>(g, st);
+        case 16: return ghost_n<16>(g, st);
+        case 32: return ghost_n<32>(g, st);
+        default: return cudaErrorInvalidValue;
+    }
+}
+cudaError_t prepare_evo_ghost(uint32_t n) {
+    switch (n) {
+        case 8: return ghost_limits<8>();
+        case 16: return ghost_limits<16>();
+        case 32: return ghost_limits<32>();
+        default: return cudaErrorInvalidValue;
+    }
 }
 
 template <int N>
