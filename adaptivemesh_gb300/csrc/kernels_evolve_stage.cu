@@ -711,7 +711,6 @@ cudaError_t stage_t(const EvoArgs& a, int sms, cudaStream_t st) {
 cudaError_t launch_evo_stage_bssn(const EvoArgs& a, cudaStream_t st) {
     if (a.n_items == 0u) return cudaSuccess;
     if (a.stage < 1 || a.stage > 4) return cudaErrorInvalidValue;
-    if (getenv("PF")) const_cast<EvoArgs&>(a).deriv_zs = 100 + atoi(getenv("PF"));
     // The tile: 512 cells of whole planes at 16^3 and 8^3 (one copy a field; 8 rows of two planes at 32^3,
     // where whole planes would be 1024 threads), except where the domains are too few to give every SM
     // such a tile.  Then smaller tiles of one cell a thread, with more CTAs: at 8^3, 9 domains, a root
