@@ -125,7 +125,6 @@ struct EvoArgs {
     uint32_t n, p, t;             // size_domain, padding_domain, n + 2p
     float dt0;                    // dt at depth 0
     int stage;                    // 1..4
-    int constraints;              // derivative pass: also store d_k A_ij
     uint32_t deriv_zs;            // derivative pass: interior z-planes per slab (0: the default)
     EvoParams prm;
     int* err;

@@ -103,10 +103,13 @@ cudaError_t launch_evo_stage_bssn(const EvoArgs& a, cudaStream_t st);
 cudaError_t launch_evo_rhs_wave(const EvoArgs& a, cudaStream_t st);
 cudaError_t launch_evo_ghost(const EvoGhostArgs& g, cudaStream_t st);
 cudaError_t prepare_evo_ghost(uint32_t n);   // its shared-memory limits, outside a stream capture
+// Hamiltonian and momentum constraints of a.fields in the listed domains' interior cells; a.deriv_zs is
+// the depth of a CTA's tile, one of evo_deriv_zs_candidates or 0 (kernels_evolve_constraints.cu).
 cudaError_t launch_evo_constraints(const EvoArgs& a, const ConsPtrs& cons, cudaStream_t st);
 // FP64 norms of the constraints over the composite grid of the listed slots (interior cells no child
 // covers), leaving out cells within the excision radius of a puncture: out[0] rms H, [1] max |H|,
-// [2] rms |M|, [3] max |M|, [4] cells.  `part` holds 5 doubles per slot.
+// [2] rms |M|, [3] max |M|, [4] cells.  `part` holds 5 doubles per part and slot.
+constexpr uint32_t kEvoNormParts = 4;   // CTAs a domain
 struct EvoNormArgs {
     ConsPtrs cons;
     const uint32_t* items;

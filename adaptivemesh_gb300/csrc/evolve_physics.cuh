@@ -57,6 +57,16 @@ __device__ __forceinline__ void inverse_sym(const float* g, float gi[3][3]) {
     gi[2][2] = (g[0] * g[3] - g[1] * g[1]) * id;
 }
 
+// Centre of a slot's domain in units of the root edge (the root spans [-1/2, 1/2]).
+__device__ __forceinline__ void slot_centre(uint32_t pos, float c[3]) {
+    const int depth = pos_depth(pos);
+    c[0] = c[1] = c[2] = 0.f;
+    uint32_t path = pos & kPathMask;
+    float step = .25f;
+    for (int i = 0; i < depth; i++, path >>= 3, step *= .5f)
+        for (int a = 0; a < 3; a++) c[a] += (path & (1u << a)) ? step : -step;
+}
+
 // ------------------------------------------------------------------ initial data at a point
 // In double precision (a one-off cost): the stored deviations from flat space (evolve.h) are then
 // rounded once, instead of carrying the float rounding of the values near 1.
@@ -118,8 +128,10 @@ template <class DV>
 __device__ __forceinline__ void geometry(const float* u, const DV& dv, const EvoParams& prm, Geometry& G) {
     G.chi = u[F_CHI];
     G.ichi = 1.f / fmaxf(G.chi, prm.chi_floor);
+#pragma unroll
     for (int c = 0; c < 6; c++) G.g[c] = u[F_GXX + c];
     inverse_sym(G.g, G.gi);
+#pragma unroll
     for (int k = 0; k < 3; k++) G.dchi[k] = dv(D_CHI1 + k);
     // lowered Christoffels: Gt_ijk = (d_j gt_ik + d_k gt_ij - d_i gt_jk) / 2
     auto dg = [&](int a, int b, int k) { return dv(D_G1 + 3 * sidx(a, b) + k); };
@@ -170,14 +182,19 @@ __device__ __forceinline__ void geometry(const float* u, const DV& dv, const Evo
             // -1/2 gt^lm d_l d_m gt_ij (contracted by the derivative pass)
             r -= .5f * dv(D_GLAP + ij);
             // gt_k(i d_j) Gt^k
+#pragma unroll
             for (int k = 0; k < 3; k++)
                 r += .5f * (G.g[sidx(k, i)] * dv(D_GAM1 + 3 * k + j) + G.g[sidx(k, j)] * dv(D_GAM1 + 3 * k + i));
             // Gt_d^k Gt_(ij)k
+#pragma unroll
             for (int k = 0; k < 3; k++) r += .5f * G.gd[k] * (G.cl[i][sidx(j, k)] + G.cl[j][sidx(i, k)]);
             // gt^lm (Gt^k_li Gt_jkm + Gt^k_lj Gt_ikm + Gt^k_im Gt_klj)
+#pragma unroll
             for (int l = 0; l < 3; l++)
+#pragma unroll
                 for (int m = 0; m < 3; m++) {
                     float s = 0.f;
+#pragma unroll
                     for (int k = 0; k < 3; k++)
                         s += G.cu[k][sidx(l, i)] * G.cl[j][sidx(k, m)] + G.cu[k][sidx(l, j)] * G.cl[i][sidx(k, m)] +
                              G.cu[k][sidx(i, m)] * G.cl[k][sidx(l, j)];
@@ -197,30 +214,43 @@ __device__ __forceinline__ void bssn_constraints(const float* u, const DV& dv, c
     geometry(u, dv, prm, G);
     const float K = u[F_K];
     float A[6];
+#pragma unroll
     for (int c = 0; c < 6; c++) A[c] = u[F_AXX + c];
     float Aud[3][3], Auu[3][3], AA = 0.f, trR = 0.f;
+#pragma unroll
     for (int i = 0; i < 3; i++)
+#pragma unroll
         for (int j = 0; j < 3; j++)
             Aud[i][j] = G.gi[i][0] * A[sidx(0, j)] + G.gi[i][1] * A[sidx(1, j)] + G.gi[i][2] * A[sidx(2, j)];
+#pragma unroll
     for (int i = 0; i < 3; i++)
+#pragma unroll
         for (int j = 0; j < 3; j++) Auu[i][j] = Aud[i][0] * G.gi[0][j] + Aud[i][1] * G.gi[1][j] + Aud[i][2] * G.gi[2][j];
+#pragma unroll
     for (int i = 0; i < 3; i++)
+#pragma unroll
         for (int j = 0; j < 3; j++) {
             AA += A[sidx(i, j)] * Auu[i][j];
             trR += G.gi[i][j] * G.R[sidx(i, j)];
         }
     hm[0] = G.chi * trR + (2.f / 3.f) * K * K - AA;
+#pragma unroll
     for (int i = 0; i < 3; i++) {
         float v = -(2.f / 3.f) * dv(D_K1 + i);
+#pragma unroll
         for (int j = 0; j < 3; j++)
+#pragma unroll
             for (int k = 0; k < 3; k++) {
                 v += G.gi[j][k] * dv(D_AT1 + 3 * sidx(k, i) + j);
                 float s = 0.f;
+#pragma unroll
                 for (int a = 0; a < 3; a++)
+#pragma unroll
                     for (int b = 0; b < 3; b++) s += G.gi[j][a] * G.gi[k][b] * dv(D_G1 + 3 * sidx(a, b) + j);
                 v -= s * A[sidx(k, i)];
                 v -= .5f * Auu[j][k] * dv(D_G1 + 3 * sidx(j, k) + i);
             }
+#pragma unroll
         for (int l = 0; l < 3; l++) v -= 1.5f * Aud[l][i] * G.dchi[l] * G.ichi;
         hm[1 + i] = v;
     }

@@ -62,7 +62,7 @@ public:
         for (int k = 0; k < 4 && e == cudaSuccess && kind == AMR_SIM_BSSN_EVOLVE; k++) e = dev_alloc(&cons.c[k], inner);
         if (e == cudaSuccess) e = dev_alloc(&d_evolved, s);
         if (e == cudaSuccess) e = dev_alloc(&d_lists, s * 2u * ((size_t)1u << kDepthLimit) + 2u * s);
-        if (e == cudaSuccess) e = dev_alloc(&d_part, s * 5u);
+        if (e == cudaSuccess) e = dev_alloc(&d_part, s * 5u * kEvoNormParts);
         if (e == cudaSuccess) e = dev_alloc(&d_norms, 8);
         if (e == cudaSuccess) {   // the stage kernels' shared-memory limits, outside any stream capture
             EvoArgs none;
@@ -258,7 +258,7 @@ public:
         float* const* out[4] = {stage_f, new_f, stage_f, new_f};
         const float c_next[3] = {.5f, .5f, 1.f};
         for (int stage = 1; stage <= 4; stage++) {
-            EvoArgs a = args(s, in[stage - 1], out[stage - 1], stage, 0);
+            EvoArgs a = args(s, in[stage - 1], out[stage - 1], stage);
             if (mode == AMR_MODE_PLAIN) {
                 // the plain per-domain form: each domain's stage launched alone
                 const uint32_t* base = a.items;
@@ -359,10 +359,10 @@ public:
         tree.set_timer(0u);
         return check(launch_evo_init(a, stream));
     }
-    // Launch-shape tuning of the derivative pass (amr_sim_autotune): its slab depth (interior
-    // z-planes per CTA) timed at every compiled depth over all evolved domains, reps launches each
-    // with CUDA events; the fastest is kept.  The pass writes only its derivative scratch, which its
-    // users (the wave's RK stages, the constraints) rewrite, so the state is unchanged.
+    // Launch-shape tuning (amr_sim_autotune): the depth (interior z-planes per CTA) of the wave's derivative
+    // pass, or of the BSSN constraints' tiles, timed at every compiled depth over all evolved domains, reps
+    // launches each with CUDA events; the fastest is kept.  Only the derivative scratch is written, so
+    // the state is unchanged.
     int autotune(uint32_t reps, uint32_t* n_tuned) override {
         if (n_tuned) *n_tuned = 0;
         if (capturing || reps == 0u || reps > 100u) return AMR_ERR_INVALID;
@@ -372,7 +372,11 @@ public:
         if (all_evolved_cnt == 0u) return AMR_OK;
         uint32_t cand[4];
         const uint32_t nc = evo_deriv_zs_candidates(dims.n, cand);
-        EvoArgs a = args(0, new_f, new_f, 1, 0);
+        EvoArgs a = args(0, new_f, new_f, 1);
+        ConsPtrs scratch;   // planes of the derivative scratch
+        for (size_t k = 0; k < 4; k++) scratch.c[k] = deriv + (k < (size_t)nd ? k : 0u) * (size_t)a.deriv_stride;
+        const bool bssn = kind == AMR_SIM_BSSN_EVOLVE;
+        auto launch = [&]() { return bssn ? launch_evo_constraints(a, scratch, stream) : launch_evo_derivs(a, stream); };
         a.items = d_lists + all_evolved_off;
         a.n_items = all_evolved_cnt;
         cudaEvent_t ev[2] = {nullptr, nullptr};
@@ -382,9 +386,9 @@ public:
         float best_ms = 0.f;
         for (uint32_t i = 0; i < nc && e == cudaSuccess; i++) {
             a.deriv_zs = cand[i];
-            e = launch_evo_derivs(a, stream);   // warm-up
+            e = launch();   // warm-up
             if (e == cudaSuccess) e = cudaEventRecord(ev[0], stream);
-            for (uint32_t r = 0; r < reps && e == cudaSuccess; r++) e = launch_evo_derivs(a, stream);
+            for (uint32_t r = 0; r < reps && e == cudaSuccess; r++) e = launch();
             if (e == cudaSuccess) e = cudaEventRecord(ev[1], stream);
             if (e == cudaSuccess) e = cudaEventSynchronize(ev[1]);
             float ms = 0.f;
@@ -405,11 +409,9 @@ public:
         if (kind != AMR_SIM_BSSN_EVOLVE) return AMR_ERR_INVALID;
         int st = prepare();
         if (st) return st;
-        // derivatives of the current state (new) on every evolved domain, then the constraints
-        EvoArgs a = args(0, new_f, new_f, 0, 1);
+        EvoArgs a = args(0, new_f, new_f, 0);   // the current state, on every evolved domain
         a.items = d_lists + all_evolved_off;
         a.n_items = all_evolved_cnt;
-        if ((st = check(launch_evo_derivs(a, stream)))) return st;
         if ((st = check(launch_evo_constraints(a, cons, stream)))) return st;
         EvoNormArgs g;
         std::memset(&g, 0, sizeof(g));
@@ -566,7 +568,7 @@ private:
     float* d_pred = nullptr;
     size_t feat_cap = 0;
 
-    EvoArgs args(uint32_t s, float* const* in, float* const* out, int stage, int constraints) {
+    EvoArgs args(uint32_t s, float* const* in, float* const* out, int stage) {
         EvoArgs a;
         std::memset(&a, 0, sizeof(a));
         for (int f = 0; f < nf; f++) {
@@ -585,7 +587,6 @@ private:
         a.t = dims.t;
         a.dt0 = prm.cfl * cfg.outer_size / (float)dims.n;
         a.stage = stage;
-        a.constraints = constraints;
         a.deriv_zs = deriv_zs;
         a.prm = prm;
         a.err = err_flag;

@@ -15,7 +15,6 @@
 //                   same-depth neighbours, separable tricubic interpolation from coarser ones)
 //   k_evo_restrict  restriction of children into parents (leaves: 16-byte copies)
 //   k_evo_prolong   tricubic prolongation of new domains
-//   k_evo_constraints, k_evo_norms_*   Hamiltonian and momentum constraints, FP64 norms
 #include <cmath>
 #include <type_traits>
 
@@ -29,16 +28,6 @@
 namespace amr {
 
 namespace {
-
-// Centre of a slot's domain in units of the root edge (the root spans [-1/2, 1/2]).
-__device__ __forceinline__ void slot_centre(uint32_t pos, float c[3]) {
-    const int depth = pos_depth(pos);
-    c[0] = c[1] = c[2] = 0.f;
-    uint32_t path = pos & kPathMask;
-    float step = .25f;
-    for (int i = 0; i < depth; i++, path >>= 3, step *= .5f)
-        for (int a = 0; a < 3; a++) c[a] += (path & (1u << a)) ? step : -step;
-}
 
 // ------------------------------------------------------------------ initial data
 __global__ void k_evo_init(EvoInitArgs a) {
@@ -179,7 +168,6 @@ __global__ void __launch_bounds__(DerivShape<N, ZS_>::THREADS, DerivShape<N, ZS_
             if (f == F_CHI) { kind = 2; first = D_CHI1; second = D_CHI2; }
             else if (f >= F_GXX && f <= F_GZZ) { kind = 3; first = D_G1 + 3 * (f - F_GXX); second = D_GLAP + (f - F_GXX); }
             else if (f == F_K) { kind = 1; first = D_K1; }
-            else if (f >= F_AXX && f <= F_AZZ) { if (a.constraints) { kind = 1; first = D_AT1 + 3 * (f - F_AXX); } }
             else if (f >= F_GAMX && f <= F_GAMZ) { kind = 1; first = D_GAM1 + 3 * (f - F_GAMX); }
             else if (f == F_ALPHA) { kind = 2; first = D_AL1; second = D_AL2; }
             else if (f >= F_BETAX && f <= F_BETAZ) { kind = 4; first = D_BE1 + 3 * (f - F_BETAX); second = D_BELAP + (f - F_BETAX); }
@@ -622,102 +610,6 @@ __global__ void __launch_bounds__(256) k_evo_restrict(const __grid_constant__ Ev
     }
 }
 
-// ------------------------------------------------------------------ constraints and FP64 norms
-template <int N>
-__global__ void __launch_bounds__(128) k_evo_constraints(const __grid_constant__ EvoArgs a, const ConsPtrs cons) {
-    constexpr int P = 3, T = N + 2 * P;
-    const uint64_t gid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (gid >= (uint64_t)a.n_items * N * N * N) return;
-    const uint32_t item = (uint32_t)(gid / (N * N * N)), cell = (uint32_t)(gid % (N * N * N));
-    const uint32_t slot = a.items[item];
-    const uint32_t x = cell % N, y = (cell / N) % N, z = cell / (N * N);
-    const uint64_t pi = (uint64_t)slot * T * T * T + ((uint64_t)(z + P) * T + (y + P)) * T + (x + P);
-    const uint64_t ii = (uint64_t)slot * N * N * N + cell;
-    float u[BSSN_NF], uo[BSSN_NF];
-#pragma unroll
-    for (int f = 0; f < BSSN_NF; f++) {
-        const float s = a.fields[f][pi];   // the stored form
-        u[f] = s + bssn_offset(f);
-        uo[f] = a.stage == 1 ? s : a.old_f[f][pi];
-    }
-    const float* D = a.deriv;
-    const uint64_t ds = a.deriv_stride;
-    auto dv = [&](int k) { return D[(uint64_t)k * ds + ii]; };
-    float hm[4];
-    bssn_constraints(u, dv, a.prm, hm);
-    for (int k = 0; k < 4; k++) cons.c[k][ii] = hm[k];
-}
-
-// One CTA per live slot: sum of H^2, max |H|, sum of |M|^2, max |M| and the cell count over its
-// interior cells that no child covers and that lie outside the excision radius of every puncture, in
-// double, with a fixed reduction order.
-__device__ __forceinline__ double nan_max(double a, double b) { return (a != a || b != b) ? (a + b) : fmax(a, b); }
-__global__ void __launch_bounds__(256) k_evo_norms_domain(const EvoNormArgs g, double* part) {
-    const uint32_t b = blockIdx.x;
-    if (b >= g.n_items) return;
-    const uint32_t slot = g.items[b], n = g.n, hn = n / 2;
-    const uint32_t cells = n * n * n;
-    const uint32_t pos = g.positions[slot];
-    const int depth = pos_depth(pos);
-    float ctr[3];
-    slot_centre(pos, ctr);
-    const float h = g.outer_size / ((float)n * (float)(1u << depth));
-    double s[5] = {0, 0, 0, 0, 0};
-    for (uint32_t c = threadIdx.x; c < cells; c += blockDim.x) {
-        const uint32_t x = c % n, y = (c / n) % n, z = c / (n * n);
-        const uint32_t oct = (x / hn) | ((y / hn) << 1) | ((z / hn) << 2);
-        if (g.children[slot * 8u + oct] != -1) continue;
-        bool excised = false;
-        for (int a = 0; a < g.n_punctures; a++) {
-            const float dx = ctr[0] * g.outer_size + ((float)x + .5f - .5f * (float)n) * h - g.pos[a][0];
-            const float dy = ctr[1] * g.outer_size + ((float)y + .5f - .5f * (float)n) * h - g.pos[a][1];
-            const float dz = ctr[2] * g.outer_size + ((float)z + .5f - .5f * (float)n) * h - g.pos[a][2];
-            excised |= dx * dx + dy * dy + dz * dz < g.excision2;
-        }
-        if (excised) continue;
-        const uint64_t i = (uint64_t)slot * cells + c;
-        const double hv = g.cons.c[0][i];
-        const double m2 = (double)g.cons.c[1][i] * g.cons.c[1][i] + (double)g.cons.c[2][i] * g.cons.c[2][i] +
-                          (double)g.cons.c[3][i] * g.cons.c[3][i];
-        s[0] += hv * hv;
-        s[1] = nan_max(s[1], fabs(hv));
-        s[2] += m2;
-        s[3] = nan_max(s[3], sqrt(m2));
-        s[4] += 1.0;
-    }
-    __shared__ double red[5][256];
-    for (int k = 0; k < 5; k++) red[k][threadIdx.x] = s[k];
-    __syncthreads();
-    for (uint32_t w = blockDim.x / 2; w > 0; w >>= 1) {
-        if (threadIdx.x < w) {
-            red[0][threadIdx.x] += red[0][threadIdx.x + w];
-            red[1][threadIdx.x] = nan_max(red[1][threadIdx.x], red[1][threadIdx.x + w]);
-            red[2][threadIdx.x] += red[2][threadIdx.x + w];
-            red[3][threadIdx.x] = nan_max(red[3][threadIdx.x], red[3][threadIdx.x + w]);
-            red[4][threadIdx.x] += red[4][threadIdx.x + w];
-        }
-        __syncthreads();
-    }
-    if (threadIdx.x == 0)
-        for (int k = 0; k < 5; k++) part[(size_t)b * 5 + k] = red[k][0];
-}
-__global__ void k_evo_norms_total(const double* part, uint32_t n_items, double* out) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    double s[5] = {0, 0, 0, 0, 0};
-    for (uint32_t b = 0; b < n_items; b++) {
-        s[0] += part[(size_t)b * 5];
-        s[1] = nan_max(s[1], part[(size_t)b * 5 + 1]);
-        s[2] += part[(size_t)b * 5 + 2];
-        s[3] = nan_max(s[3], part[(size_t)b * 5 + 3]);
-        s[4] += part[(size_t)b * 5 + 4];
-    }
-    out[0] = s[4] > 0 ? sqrt(s[0] / s[4]) : 0.;
-    out[1] = s[1];
-    out[2] = s[4] > 0 ? sqrt(s[2] / s[4]) : 0.;
-    out[3] = s[3];
-    out[4] = s[4];
-}
-
 // ------------------------------------------------------------------ prolongation of new domains
 // One CTA per (child, buffer).  Child cell w (padded index) lies at parent index coordinate
 // o * n/2 + p + (w - p + 1/2) / 2 - 1/2 along each axis (o: the child's octant bit), which stays in
@@ -952,27 +844,6 @@ cudaError_t prepare_evo_ghost(uint32_t n) {
         case 32: return ghost_limits<32>();
         default: return cudaErrorInvalidValue;
     }
-}
-
-template <int N>
-static cudaError_t cons_t(const EvoArgs& a, const ConsPtrs& cons, cudaStream_t st) {
-    const uint64_t total = (uint64_t)a.n_items * N * N * N;
-    if (total == 0) return cudaSuccess;
-    k_evo_constraints<N><<<(unsigned)((total + 127) / 128), 128, 0, st>>>(a, cons);
-    return cudaGetLastError();
-}
-cudaError_t launch_evo_constraints(const EvoArgs& a, const ConsPtrs& cons, cudaStream_t st) {
-    switch (a.n) {
-        case 8: return cons_t<8>(a, cons, st);
-        case 16: return cons_t<16>(a, cons, st);
-        case 32: return cons_t<32>(a, cons, st);
-        default: return cudaErrorInvalidValue;
-    }
-}
-cudaError_t launch_evo_norms(const EvoNormArgs& g, double* part, double* out, cudaStream_t st) {
-    if (g.n_items) k_evo_norms_domain<<<g.n_items, 256, 0, st>>>(g, part);
-    k_evo_norms_total<<<1, 32, 0, st>>>(part, g.n_items, out);
-    return cudaGetLastError();
 }
 
 }  // namespace amr
