@@ -61,13 +61,9 @@ enum WaveField : int { W_U = 0, W_V = 1, WAVE_NF = 2 };
 
 constexpr int kMaxFields = 24;
 
-// Derivative scratch written by the derivative pass (for the wave's RK stages and the BSSN
-// constraints; the BSSN stages keep no derivatives in memory), one float per inner cell each (slot * N^3 +
-// cell).  Symmetric second derivatives in the order xx, yy, zz, xy, xz, yz; first derivatives
-// x, y, z.  Where only a contraction with the inverse conformal metric is used,
-// the pass stores the contraction: GLAP[ij] = gt^lm d_l d_m gt_ij, BELAP[i] = gt^jk d_j d_k beta^i,
-// and DDIVB[j] = d_j d_k beta^k.  EXTRA[f] is the advection term beta^k d_k u_f plus the
-// Kreiss-Oliger term of field f.
+// Derivatives the BSSN constraints use, in the thread's column of shared memory (kernels_evolve_constraints.cu).
+// Symmetric second derivatives in the order xx, yy, zz, xy, xz, yz; first derivatives x, y, z.  GLAP[ij] =
+// gt^lm d_l d_m gt_ij.
 enum BssnDeriv : int {
     D_CHI1 = 0,                   // 3
     D_CHI2 = 3,                   // 6
@@ -75,17 +71,11 @@ enum BssnDeriv : int {
     D_GLAP = 27,                  // 6
     D_K1 = 33,                    // 3
     D_GAM1 = 36,                  // 3 components x 3: d_j Gamma^i at D_GAM1 + 3 i + j
-    D_AL1 = 45,                   // 3
-    D_AL2 = 48,                   // 6
-    D_BE1 = 54,                   // 3 components x 3: d_j beta^i at D_BE1 + 3 i + j
-    D_BELAP = 63,                 // 3
-    D_DDIVB = 66,                 // 3
-    D_EXTRA = 69,                 // 24
-    BSSN_ND = 93,
-    D_AT1 = 93,                   // constraint mode only: d_k A_ij at D_AT1 + 3 c + k (6 components)
-    BSSN_ND_CONSTRAINTS = 111
+    D_AT1 = 45,                   // d_k A_ij at D_AT1 + 3 c + k (6 components)
+    BSSN_ND = 63
 };
-enum WaveDeriv : int { WD_LAP = 0, WD_EXTRA = 1, WAVE_ND = 3 };
+// Planes of the derivative scratch (amr_sim_buffer 5), which the tuning call writes.
+constexpr int kBssnScratch = 111, kWaveScratch = 3;
 
 // Physics and gauge choices (the C ABI's amr_evolution, resolved).
 struct EvoParams {
@@ -116,8 +106,6 @@ struct EvoArgs {
     float* out[kMaxFields];       // stage output (padded interior written)
     float* old_f[kMaxFields];     // state at the start of the step (padded)
     float* acc[kMaxFields];       // RK accumulator (inner layout)
-    float* deriv;                 // derivative scratch: nd planes of slots * N^3 floats
-    uint64_t deriv_stride;        // floats per derivative plane (slots * N^3)
     const uint32_t* positions;
     const uint32_t* items;        // active evolved slots
     uint32_t n_items;
@@ -125,7 +113,7 @@ struct EvoArgs {
     uint32_t n, p, t;             // size_domain, padding_domain, n + 2p
     float dt0;                    // dt at depth 0
     int stage;                    // 1..4
-    uint32_t deriv_zs;            // derivative pass: interior z-planes per slab (0: the default)
+    uint32_t deriv_zs;            // interior z-planes per CTA of the wave's stage and the constraints (0: the default)
     EvoParams prm;
     int* err;
 };

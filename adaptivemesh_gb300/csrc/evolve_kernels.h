@@ -93,14 +93,13 @@ cudaError_t launch_evo_prolong(const EvoProlongArgs& g, cudaStream_t st);
 bool evo_config_supported(uint32_t n, uint32_t p);
 cudaError_t launch_evo_restrict(const EvoRestrictArgs& g, cudaStream_t st);
 cudaError_t launch_evo_init(const EvoInitArgs& a, cudaStream_t st);
-cudaError_t launch_evo_derivs(const EvoArgs& a, cudaStream_t st);
 // The derivative pass's compiled slab depths for size_domain n (written to out, at most 4); their count.
 uint32_t evo_deriv_zs_candidates(uint32_t n, uint32_t* out);
 // One RK stage of the BSSN evolution (derivatives, right-hand side and stage update;
 // kernels_evolve_stage.cu), and the kernel's shared-memory limit, to be set outside a stream capture.
 cudaError_t prepare_evo_stage_bssn(uint32_t n);
 cudaError_t launch_evo_stage_bssn(const EvoArgs& a, cudaStream_t st);
-cudaError_t launch_evo_rhs_wave(const EvoArgs& a, cudaStream_t st);
+cudaError_t launch_evo_stage_wave(const EvoArgs& a, cudaStream_t st);   // one RK stage of the wave
 cudaError_t launch_evo_ghost(const EvoGhostArgs& g, cudaStream_t st);
 cudaError_t prepare_evo_ghost(uint32_t n);   // its shared-memory limits, outside a stream capture
 // Hamiltonian and momentum constraints of a.fields in the listed domains' interior cells; a.deriv_zs is

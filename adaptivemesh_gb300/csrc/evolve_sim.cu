@@ -27,7 +27,7 @@ class EvolveSim : public SimBase {
 public:
     EvolveSim(const amr_config& c, int kind, uint32_t slots, int mode) : SimBase(c, slots, mode), kind(kind) {
         nf = kind == AMR_SIM_BSSN_EVOLVE ? BSSN_NF : WAVE_NF;
-        nd = kind == AMR_SIM_BSSN_EVOLVE ? BSSN_ND_CONSTRAINTS : WAVE_ND;
+        nd = kind == AMR_SIM_BSSN_EVOLVE ? kBssnScratch : kWaveScratch;
         kind_id = kind;
         prm.physics = kind == AMR_SIM_BSSN_EVOLVE ? 0 : 1;
         prm.slicing = AMR_SLICING_1PLUSLOG;
@@ -58,7 +58,8 @@ public:
             if (e == cudaSuccess) e = dev_alloc(&stage_f[f], padded);
             if (e == cudaSuccess) e = dev_alloc(&acc[f], inner);
         }
-        if (e == cudaSuccess) e = dev_alloc(&deriv, inner * (size_t)nd);
+        // the wave's tuning call writes its two fields, padded, to the scratch
+        if (e == cudaSuccess) e = dev_alloc(&deriv, std::max(inner * (size_t)nd, kind == AMR_SIM_BSSN_EVOLVE ? 0u : padded * WAVE_NF));
         for (int k = 0; k < 4 && e == cudaSuccess && kind == AMR_SIM_BSSN_EVOLVE; k++) e = dev_alloc(&cons.c[k], inner);
         if (e == cudaSuccess) e = dev_alloc(&d_evolved, s);
         if (e == cudaSuccess) e = dev_alloc(&d_lists, s * 2u * ((size_t)1u << kDepthLimit) + 2u * s);
@@ -68,8 +69,8 @@ public:
             EvoArgs none;
             std::memset(&none, 0, sizeof(none));
             none.n = dims.n;
-            e = launch_evo_derivs(none, stream);
-            if (e == cudaSuccess) e = prepare_evo_ghost(dims.n);
+            e = prepare_evo_ghost(dims.n);
+            if (e == cudaSuccess && kind != AMR_SIM_BSSN_EVOLVE) e = launch_evo_stage_wave(none, stream);
             if (e == cudaSuccess && kind == AMR_SIM_BSSN_EVOLVE) e = prepare_evo_stage_bssn(dims.n);
         }
         return cuda_status(e);
@@ -359,8 +360,8 @@ public:
         tree.set_timer(0u);
         return check(launch_evo_init(a, stream));
     }
-    // Launch-shape tuning (amr_sim_autotune): the depth (interior z-planes per CTA) of the wave's derivative
-    // pass, or of the BSSN constraints' tiles, timed at every compiled depth over all evolved domains, reps
+    // Launch-shape tuning (amr_sim_autotune): the depth (interior z-planes per CTA) of the wave's stage
+    // kernel, or of the BSSN constraints' tiles, timed at every compiled depth over all evolved domains, reps
     // launches each with CUDA events; the fastest is kept.  Only the derivative scratch is written, so
     // the state is unchanged.
     int autotune(uint32_t reps, uint32_t* n_tuned) override {
@@ -372,11 +373,17 @@ public:
         if (all_evolved_cnt == 0u) return AMR_OK;
         uint32_t cand[4];
         const uint32_t nc = evo_deriv_zs_candidates(dims.n, cand);
-        EvoArgs a = args(0, new_f, new_f, 1);
-        ConsPtrs scratch;   // planes of the derivative scratch
-        for (size_t k = 0; k < 4; k++) scratch.c[k] = deriv + (k < (size_t)nd ? k : 0u) * (size_t)a.deriv_stride;
+        const size_t inner = (size_t)tree.max_slots() * dims.n * dims.n * dims.n;
+        const size_t padded = (size_t)tree.max_slots() * dims.t * dims.t * dims.t;
         const bool bssn = kind == AMR_SIM_BSSN_EVOLVE;
-        auto launch = [&]() { return bssn ? launch_evo_constraints(a, scratch, stream) : launch_evo_derivs(a, stream); };
+        // the results go to the derivative scratch: the constraints' four planes, or the wave's two
+        // fields (stage 4, which writes nothing else)
+        float* to[kMaxFields] = {};
+        ConsPtrs cons_to = {};
+        for (size_t k = 0; k < 4 && bssn; k++) cons_to.c[k] = deriv + k * inner;
+        for (size_t k = 0; k < WAVE_NF && !bssn; k++) to[k] = deriv + k * padded;
+        EvoArgs a = args(0, new_f, to, 4);
+        auto launch = [&]() { return bssn ? launch_evo_constraints(a, cons_to, stream) : launch_evo_stage_wave(a, stream); };
         a.items = d_lists + all_evolved_off;
         a.n_items = all_evolved_cnt;
         cudaEvent_t ev[2] = {nullptr, nullptr};
@@ -577,8 +584,6 @@ private:
             a.old_f[f] = old_f[f];
             a.acc[f] = acc[f];
         }
-        a.deriv = deriv;
-        a.deriv_stride = (uint64_t)tree.max_slots() * dims.n * dims.n * dims.n;
         a.positions = d_positions;
         a.items = d_lists + (evo_off.empty() ? 0u : evo_off[s]);
         a.n_items = a.n_batch = evo_cnt.empty() ? 0u : evo_cnt[s];
@@ -592,11 +597,8 @@ private:
         a.err = err_flag;
         return a;
     }
-    // one RK stage: the BSSN evolution in one kernel, the wave's derivative pass and update
-    int stage_update(const EvoArgs& a) {
-        if (kind == AMR_SIM_BSSN_EVOLVE) return check(launch_evo_stage_bssn(a, stream));
-        const int st = check(launch_evo_derivs(a, stream));
-        return st ? st : check(launch_evo_rhs_wave(a, stream));
+    int stage_update(const EvoArgs& a) {   // one RK stage
+        return check(kind == AMR_SIM_BSSN_EVOLVE ? launch_evo_stage_bssn(a, stream) : launch_evo_stage_wave(a, stream));
     }
     // ghost fill of `x` (the state at c_stage of the active domains' step), three axis passes
     int fill(uint32_t s, float* const* x, float c_stage) {

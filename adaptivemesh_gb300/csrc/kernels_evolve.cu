@@ -5,12 +5,7 @@
 // (oracle/bssn_evolve.c) within stated tolerances.
 //
 //   k_evo_init      analytic initial data on every cell (ghosts included) of every live slot
-//   k_evo_derivs    derivative pass: a CTA per (domain, z-slab); each field's padded slab moves into
-//                   shared memory with one 1-D bulk copy (two buffers, the next field in flight),
-//                   then first / second / mixed derivatives, advection and Kreiss-Oliger terms (the
-//                   wave's RK stages and the BSSN constraints; the BSSN stages are one kernel,
-//                   kernels_evolve_stage.cu)
-//   k_evo_rhs_wave  the wave's pointwise right-hand side and RK4 stage update
+//   k_evo_stage_wave  one RK4 stage of the wave: derivatives, right-hand side and stage update
 //   k_evo_ghost     ghost fill of a stage's state, one face-normal axis per launch (copies from
 //                   same-depth neighbours, separable tricubic interpolation from coarser ones)
 //   k_evo_restrict  restriction of children into parents (leaves: 16-byte copies)
@@ -54,25 +49,18 @@ __global__ void k_evo_init(EvoInitArgs a) {
     }
 }
 
-// ------------------------------------------------------------------ derivative pass
-// A CTA per (domain, slab of ZS interior z-planes): the slab's padded planes (ZS + 6) of one field
-// fit twice in shared memory.  ZS is a launch-shape choice (amr_sim_autotune times the compiled
-// ones, DerivZs below); the default takes two cells per thread at 16^3 (one at 8^3 and 32^3): a
-// thread keeps, per cell, the shift through the whole pass.
-constexpr int deriv_default_zs(int n) { return n == 8 ? 4 : (n == 16 ? 2 : 1); }
-template <int N, int ZS_ = deriv_default_zs(N)>
-struct DerivShape {
-    static constexpr int P = 3, T = N + 2 * P;
-    static constexpr int ZS = ZS_;
-    static constexpr int THREADS = 256;
-    static constexpr int CELLS = N * N * ZS;
-    static constexpr int CPT = CELLS / THREADS;          // cells per thread
+// ------------------------------------------------------------------ one RK4 stage of the wave
+// A CTA per (domain, slab of ZS interior z-planes): the padded planes (ZS + 6) of u and v, one bulk copy
+// each, then per cell the Laplacian, the Kreiss-Oliger terms, the right-hand side and the stage update.
+// A derivative pass and an update kernel took 9 us a stage on 15 domains of 16^3, most of it their two
+// launches.  ZS is a launch-shape choice (amr_sim_autotune times the compiled ones); the default takes
+// two cells per thread at 16^3, one at 8^3, four at 32^3.
+constexpr int wave_default_zs(int n) { return n == 8 ? 4 : (n == 16 ? 2 : 1); }
+template <int N, int ZS>
+struct WaveShape {
+    static constexpr int T = N + 6, THREADS = 256, CELLS = N * N * ZS, CPT = CELLS / THREADS;
     static constexpr uint32_t SLAB = (uint32_t)((ZS + 6) * T * T);   // floats
-    static constexpr uint32_t SLAB_BYTES = SLAB * 4u;
-    // two field slabs, then per cell the inverse conformal metric (6) and the running sums of
-    // d_j d_k beta^k (3), which the BSSN pass keeps across its visits
-    static constexpr size_t SMEM = 2u * SLAB_BYTES + 9u * CELLS * 4u + 64u;
-    static_assert(CELLS % THREADS == 0 && N % ZS == 0, "whole cells per thread and planes per slab");
+    static constexpr size_t SMEM = 2u * SLAB * 4u;
     // The row of a cell.  At N = 16 a warp would cover rows y and y + 1 of the 22-float padded
     // rows, whose shared-memory banks overlap for 6 lanes; rows y and y + 8 (176 floats = 16 banks
     // apart) make every tap of the warp conflict-free.
@@ -80,203 +68,10 @@ struct DerivShape {
         const uint32_t r = (cell / N) % N;
         return N == 16 ? (r >> 1) | ((r & 1u) << 3) : r;
     }
-    static_assert(SLAB_BYTES % 16u == 0u && (T * T * 4) % 16 == 0, "slabs are aligned bulk copies");
+    static_assert(CELLS % THREADS == 0 && N % ZS == 0, "whole cells per thread and planes per slab");
+    static_assert(SLAB * 4u % 16u == 0u && (T * T * 4) % 16 == 0, "slabs are aligned bulk copies");
 };
 
-// The order in which the derivative pass visits the fields: the shift first, so that the advection
-// terms of the others can use it.
-__device__ __forceinline__ int deriv_field_order(int physics, int i) {
-    if (physics != 0) return i;
-    return i < 3 ? F_BETAX + i : (i < 21 ? i - 3 : i);
-}
-
-template <int N, int ZS_>
-__global__ void __launch_bounds__(DerivShape<N, ZS_>::THREADS, DerivShape<N, ZS_>::CPT <= 2 ? 3 : 2)
-    k_evo_derivs(const __grid_constant__ EvoArgs a) {
-    using S = DerivShape<N, ZS_>;
-    constexpr int T = S::T, ZS = S::ZS, CPT = S::CPT;
-    extern __shared__ __align__(128) unsigned char smem_raw[];
-    float* buf = reinterpret_cast<float*>(smem_raw);
-    float* s_gi = reinterpret_cast<float*>(smem_raw + 2u * S::SLAB_BYTES);   // [6][CELLS]
-    float* s_ddb = s_gi + 6 * S::CELLS;                                         // [3][CELLS]
-    uint64_t* bar = reinterpret_cast<uint64_t*>(s_ddb + 3 * S::CELLS);
-    __shared__ int s_abort;
-
-    const uint32_t tid = threadIdx.x;
-    const uint32_t slabs = N / ZS;
-    const uint32_t item = blockIdx.x / slabs, slab = blockIdx.x % slabs;
-    if (item >= a.n_items) return;
-    const uint32_t slot = a.items[item];
-    const int depth = pos_depth(a.positions[slot]);
-    const int nf = a.prm.physics == 0 ? BSSN_NF : WAVE_NF;
-    if (tid == 0) {
-        mbar_init(&bar[0], 1);
-        mbar_init(&bar[1], 1);
-        mbar_fence_init();
-        s_abort = 0;
-    }
-    __syncthreads();
-    const size_t src_off = (size_t)slot * T * T * T + (size_t)slab * ZS * T * T;   // padded plane slab*ZS (p = 3)
-    auto issue = [&](int i) {   // field of visit i into buffer i % 2
-        const int f = deriv_field_order(a.prm.physics, i);
-        mbar_arrive_expect_tx(&bar[i & 1], S::SLAB_BYTES);
-        bulk_g2s(buf + (size_t)(i & 1) * S::SLAB, a.fields[f] + src_off, S::SLAB_BYTES, &bar[i & 1]);
-    };
-    if (tid == 0) {
-        issue(0);
-        if (nf > 1) issue(1);
-    }
-    const float h = a.prm.outer_size / ((float)N * (float)(1u << depth));
-    const float i12h = 1.f / (12.f * h), i12h2 = 1.f / (12.f * h * h), i144h2 = 1.f / (144.f * h * h);
-    const float ko = a.prm.ko_sigma / (64.f * h);
-    const bool bssn = a.prm.physics == 0;
-    const bool shift_on = bssn && a.prm.shift != 0;
-    // the shift at each of this thread's cells, for the advection terms of every field, and the
-    // inverse conformal metric, for the contracted second derivatives (evolve.h)
-    float beta[CPT][3];
-#pragma unroll
-    for (int c = 0; c < CPT; c++) {
-        const uint32_t cell = tid + (uint32_t)c * S::THREADS;
-        const uint32_t x = cell % N, y = S::row(cell), z = slab * ZS + cell / (N * N);
-        const size_t pi = (size_t)slot * T * T * T + ((size_t)(z + 3) * T + (y + 3)) * T + (x + 3);
-#pragma unroll
-        for (int k = 0; k < 3; k++) { beta[c][k] = bssn ? a.fields[F_BETAX + k][pi] : 0.f; s_ddb[k * S::CELLS + cell] = 0.f; }
-        float g[6], m[3][3];
-#pragma unroll
-        for (int k = 0; k < 6; k++) g[k] = bssn ? a.fields[F_GXX + k][pi] + bssn_offset(F_GXX + k) : (k == 0 || k == 3 || k == 5 ? 1.f : 0.f);
-        inverse_sym(g, m);
-        const float gi6[6] = {m[0][0], m[1][1], m[2][2], m[0][1], m[0][2], m[1][2]};   // xx yy zz xy xz yz
-#pragma unroll
-        for (int k = 0; k < 6; k++) s_gi[k * S::CELLS + cell] = gi6[k];
-    }
-    float* D = a.deriv;
-    const uint64_t ds = a.deriv_stride;
-
-    int stopped = nf;   // the visit at which a wait gave up
-    for (int i = 0; i < nf; i++) {
-        const int f = deriv_field_order(a.prm.physics, i);
-        const bool ok = mbar_wait(&bar[i & 1], (uint32_t)(i >> 1) & 1u);
-        if (!ok) s_abort = 1;
-        __syncthreads();
-        if (s_abort) { stopped = i; break; }
-        const float* tile = buf + (size_t)(i & 1) * S::SLAB;
-        // what this field keeps (evolve.h), decided once per visit: 0 nothing but its extra term,
-        // 1 first derivatives, 2 first and all six second (chi, alpha), 3 first and the metric
-        // contraction of the second (gt_ij), 4 as 3 plus d_j d_k beta^k (beta^i), 5 the Laplacian (u)
-        int kind = 0, first = -1, second = -1;
-        if (bssn) {
-            if (f == F_CHI) { kind = 2; first = D_CHI1; second = D_CHI2; }
-            else if (f >= F_GXX && f <= F_GZZ) { kind = 3; first = D_G1 + 3 * (f - F_GXX); second = D_GLAP + (f - F_GXX); }
-            else if (f == F_K) { kind = 1; first = D_K1; }
-            else if (f >= F_GAMX && f <= F_GAMZ) { kind = 1; first = D_GAM1 + 3 * (f - F_GAMX); }
-            else if (f == F_ALPHA) { kind = 2; first = D_AL1; second = D_AL2; }
-            else if (f >= F_BETAX && f <= F_BETAZ) { kind = 4; first = D_BE1 + 3 * (f - F_BETAX); second = D_BELAP + (f - F_BETAX); }
-        } else if (f == W_U) {
-            kind = 5;
-        }
-        const int bk = f - F_BETAX;   // kind 4: the shift component
-        const bool zero_extra = bssn && !shift_on && f >= F_BETAX;   // a frozen shift and its driver
-        float* const Dx = D + (uint64_t)((bssn ? D_EXTRA : WD_EXTRA) + f) * ds;
-        float* const D1 = D + (uint64_t)(first < 0 ? 0 : first) * ds;
-        float* const D2 = D + (uint64_t)(second < 0 ? 0 : second) * ds;
-        auto cells = [&](auto KIND) {
-            constexpr int K = decltype(KIND)::value;
-#pragma unroll
-            for (int c = 0; c < CPT; c++) {
-                const uint32_t cell = tid + (uint32_t)c * S::THREADS;
-                const uint32_t x = cell % N, y = S::row(cell), zl = cell / (N * N);
-                const uint32_t z = slab * ZS + zl;
-                const float* q = tile + ((zl + 3) * T + (y + 3)) * T + (x + 3);
-                const uint64_t o = ((uint64_t)slot * N + z) * N * N + (uint64_t)y * N + x;
-                constexpr int st[3] = {1, T, T * T};
-                float d1[3], ko_sum = 0.f;
-#pragma unroll
-                for (int ax = 0; ax < 3; ax++) {
-                    const int s = st[ax];
-                    d1[ax] = ((q[-2 * s] - q[2 * s]) + 8.f * (q[s] - q[-s])) * i12h;
-                    ko_sum += (q[-3 * s] + q[3 * s]) - 6.f * (q[-2 * s] + q[2 * s]) + 15.f * (q[-s] + q[s]) - 20.f * q[0];
-                }
-                if constexpr (K >= 1 && K <= 4)
-#pragma unroll
-                    for (int ax = 0; ax < 3; ax++) D1[(uint64_t)ax * ds + o] = d1[ax];
-                if constexpr (K >= 2) {
-                    float dd[3];
-#pragma unroll
-                    for (int ax = 0; ax < 3; ax++) {
-                        const int s = st[ax];
-                        dd[ax] = (16.f * (q[-s] + q[s]) - (q[-2 * s] + q[2 * s]) - 30.f * q[0]) * i12h2;
-                    }
-                    if constexpr (K == 5) {
-                        D[(uint64_t)WD_LAP * ds + o] = dd[0] + dd[1] + dd[2];
-                    } else {
-                        constexpr int pa[3] = {0, 0, 1}, pb[3] = {1, 2, 2};
-                        constexpr float w[4] = {1.f, -8.f, 8.f, -1.f};
-                        constexpr int off[4] = {-2, -1, 1, 2};
-                        float d2[6] = {dd[0], dd[1], dd[2], 0.f, 0.f, 0.f};   // xx yy zz xy xz yz
-#pragma unroll
-                        for (int m = 0; m < 3; m++) {
-                            const int sa = st[pa[m]], sb = st[pb[m]];
-                            float acc = 0.f;
-#pragma unroll
-                            for (int u = 0; u < 4; u++) {
-                                float row = 0.f;
-#pragma unroll
-                                for (int v = 0; v < 4; v++) row = fmaf(w[v], q[off[u] * sa + off[v] * sb], row);
-                                acc = fmaf(w[u], row, acc);
-                            }
-                            d2[3 + m] = acc * i144h2;
-                        }
-                        if constexpr (K == 2) {   // all six
-#pragma unroll
-                            for (int k = 0; k < 6; k++) D2[(uint64_t)k * ds + o] = d2[k];
-                        } else {
-                            // gt^lm d_l d_m of the field (the metric's and the shift's components)
-                            const float* G = s_gi + cell;   // G[k * CELLS]: this cell's inverse metric
-                            constexpr int C = S::CELLS;
-                            D2[o] = G[0] * d2[0] + G[C] * d2[1] + G[2 * C] * d2[2] +
-                                    2.f * (G[3 * C] * d2[3] + G[4 * C] * d2[4] + G[5 * C] * d2[5]);
-                            if constexpr (K == 4) {   // d_j d_k beta^k, k = this component
-                                float* B = s_ddb + cell;
-                                B[0] += bk == 0 ? d2[0] : (bk == 1 ? d2[3] : d2[4]);
-                                B[C] += bk == 0 ? d2[3] : (bk == 1 ? d2[1] : d2[5]);
-                                B[2 * C] += bk == 0 ? d2[4] : (bk == 1 ? d2[5] : d2[2]);
-                                if (bk == 2)
-#pragma unroll
-                                    for (int j = 0; j < 3; j++) D[(uint64_t)(D_DDIVB + j) * ds + o] = B[j * C];
-                            }
-                        }
-                    }
-                }
-                // advection along the shift and dissipation
-                float extra = ko * ko_sum;
-                if (bssn) {
-                    extra = fmaf(beta[c][0], d1[0], fmaf(beta[c][1], d1[1], fmaf(beta[c][2], d1[2], extra)));
-                    if (zero_extra) extra = 0.f;
-                }
-                Dx[o] = extra;
-            }
-        };
-        switch (kind) {
-            case 1: cells(std::integral_constant<int, 1>{}); break;
-            case 2: cells(std::integral_constant<int, 2>{}); break;
-            case 3: cells(std::integral_constant<int, 3>{}); break;
-            case 4: cells(std::integral_constant<int, 4>{}); break;
-            case 5: cells(std::integral_constant<int, 5>{}); break;
-            default: cells(std::integral_constant<int, 0>{}); break;
-        }
-        __syncthreads();   // every thread is done with buffer i % 2
-        if (tid == 0 && i + 2 < nf) issue(i + 2);
-    }
-    // Every copy issued was waited for, except after a wait gave up at visit `stopped`: the copies
-    // of visits stopped and stopped + 1 may still be in flight, and the CTA's shared memory must
-    // outlive them (bounded waits).
-    if (stopped < nf && tid == 0) {
-        atomicExch(a.err, 1);
-        for (int i = stopped; i < nf && i <= stopped + 1; i++) mbar_wait(&bar[i & 1], (uint32_t)(i >> 1) & 1u);
-    }
-}
-
-// ------------------------------------------------------------------ right-hand sides and stage update
 // RK4: stage 1: acc = old + dt/6 k1, out = old + dt/2 k1; stage 2: acc += dt/3 k2, out = old + dt/2 k2;
 // stage 3: acc += dt/3 k3, out = old + dt k3; stage 4: out = acc + dt/6 k4.
 __device__ __forceinline__ void rk_update(const EvoArgs& a, int f, uint64_t pi, uint64_t ii, float u_old, float r,
@@ -302,25 +97,61 @@ __device__ __forceinline__ void rk_update(const EvoArgs& a, int f, uint64_t pi, 
     a.out[f][pi] = v;
 }
 
-template <int N>
-__global__ void __launch_bounds__(256) k_evo_rhs_wave(const __grid_constant__ EvoArgs a) {
-    constexpr int P = 3, T = N + 2 * P;
-    const uint64_t gid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (gid >= (uint64_t)a.n_items * N * N * N) return;
-    const uint32_t item = (uint32_t)(gid / (N * N * N)), cell = (uint32_t)(gid % (N * N * N));
+template <int N, int ZS>
+__global__ void __launch_bounds__(256) k_evo_stage_wave(const __grid_constant__ EvoArgs a) {
+    using S = WaveShape<N, ZS>;
+    constexpr int T = S::T;
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    float* buf = reinterpret_cast<float*>(smem_raw);   // u, v
+    __shared__ uint64_t bar;
+    const uint32_t tid = threadIdx.x;
+    const uint32_t item = blockIdx.x / (N / ZS), slab = blockIdx.x % (N / ZS);
+    if (item >= a.n_items) return;
     const uint32_t slot = a.items[item];
-    const uint32_t x = cell % N, y = (cell / N) % N, z = cell / (N * N);
+    if (tid == 0) {
+        mbar_init(&bar, 1);
+        mbar_fence_init();
+        mbar_arrive_expect_tx(&bar, 2u * S::SLAB * 4u);
+        const size_t src = (size_t)slot * T * T * T + (size_t)slab * ZS * T * T;   // padded plane slab * ZS (p = 3)
+        for (int f = 0; f < WAVE_NF; f++) bulk_g2s(buf + (size_t)f * S::SLAB, a.fields[f] + src, S::SLAB * 4u, &bar);
+    }
     const int depth = pos_depth(a.positions[slot]);
+    const float h = a.prm.outer_size / ((float)N * (float)(1u << depth));
+    const float i12h2 = 1.f / (12.f * h * h), ko = a.prm.ko_sigma / (64.f * h);
     const float dt = a.dt0 / (float)(1u << depth);
-    const uint64_t pi = (uint64_t)slot * T * T * T + ((uint64_t)(z + P) * T + (y + P)) * T + (x + P);
-    const uint64_t ii = (uint64_t)slot * N * N * N + cell;
-    const float* D = a.deriv;
-    const uint64_t ds = a.deriv_stride;
-    const float uu = a.fields[W_U][pi], vv = a.fields[W_V][pi];
-    const float r_u = vv + D[(uint64_t)(WD_EXTRA + W_U) * ds + ii];
-    const float r_v = D[(uint64_t)WD_LAP * ds + ii] + D[(uint64_t)(WD_EXTRA + W_V) * ds + ii];
-    rk_update(a, W_U, pi, ii, a.stage == 1 ? uu : a.old_f[W_U][pi], r_u, dt);
-    rk_update(a, W_V, pi, ii, a.stage == 1 ? vv : a.old_f[W_V][pi], r_v, dt);
+    __syncthreads();
+    const bool ok = mbar_wait(&bar, 0);   // a wait that gave up is reported and its cells are left alone
+    if (!ok) atomicExch(a.err, 1);
+#pragma unroll
+    for (int c = 0; c < S::CPT && ok; c++) {
+        const uint32_t cell = tid + (uint32_t)c * S::THREADS;
+        const uint32_t x = cell % N, y = S::row(cell), zl = cell / (N * N), z = slab * ZS + zl;
+        const uint64_t pi = (uint64_t)slot * T * T * T + ((uint64_t)(z + 3) * T + (y + 3)) * T + (x + 3);
+        const uint64_t ii = ((uint64_t)slot * N + z) * N * N + (uint64_t)y * N + x;
+        constexpr int st[3] = {1, T, T * T};
+        float extra[WAVE_NF], lap = 0.f;
+#pragma unroll
+        for (int f = 0; f < WAVE_NF; f++) {
+            const float* q = buf + (size_t)f * S::SLAB + ((zl + 3) * T + (y + 3)) * T + (x + 3);
+            float ko_sum = 0.f, dd[3];
+#pragma unroll
+            for (int ax = 0; ax < 3; ax++) {
+                const int s = st[ax];
+                ko_sum += (q[-3 * s] + q[3 * s]) - 6.f * (q[-2 * s] + q[2 * s]) + 15.f * (q[-s] + q[s]) - 20.f * q[0];
+                dd[ax] = (16.f * (q[-s] + q[s]) - (q[-2 * s] + q[2 * s]) - 30.f * q[0]) * i12h2;
+            }
+            if (f == W_U) lap = dd[0] + dd[1] + dd[2];
+            extra[f] = __fmul_rn(ko, ko_sum);   // rounded by itself
+        }
+        const float* q = buf + ((zl + 3) * T + (y + 3)) * T + (x + 3);
+        const float uu = q[0], vv = q[S::SLAB];
+        const float r_u = vv + extra[W_U], r_v = lap + extra[W_V];
+        rk_update(a, W_U, pi, ii, a.stage == 1 ? uu : a.old_f[W_U][pi], r_u, dt);
+        rk_update(a, W_V, pi, ii, a.stage == 1 ? vv : a.old_f[W_V][pi], r_v, dt);
+    }
+    __syncthreads();
+    // the CTA's shared memory must outlive its copies: after a wait that gave up, wait once more
+    if (!ok && tid == 0) mbar_wait(&bar, 0);
 }
 
 // ------------------------------------------------------------------ ghost fill
@@ -739,35 +570,40 @@ cudaError_t launch_evo_init(const EvoInitArgs& a, cudaStream_t st) {
 }
 
 template <int N, int ZS>
-static cudaError_t derivs_zs(const EvoArgs& a, cudaStream_t st) {
-    using S = DerivShape<N, ZS>;
+static cudaError_t wave_limit() {
     static std::atomic<uint64_t> configured{0};
-    cudaError_t e = ensure_smem_limit(k_evo_derivs<N, ZS>, S::SMEM, configured);
+    return ensure_smem_limit(k_evo_stage_wave<N, ZS>, WaveShape<N, ZS>::SMEM, configured);
+}
+template <int N, int ZS>
+static cudaError_t wave_zs(const EvoArgs& a, cudaStream_t st) {
+    using S = WaveShape<N, ZS>;
+    const cudaError_t e = wave_limit<N, ZS>();
     if (e != cudaSuccess || a.n_items == 0) return e;
-    k_evo_derivs<N, ZS><<<a.n_items * (N / ZS), S::THREADS, S::SMEM, st>>>(a);
+    k_evo_stage_wave<N, ZS><<<a.n_items * (N / ZS), S::THREADS, S::SMEM, st>>>(a);
     return cudaGetLastError();
 }
 // The compiled slab depths (a.deriv_zs; 0 = the default): whole cells per thread of 256.
 template <int N>
-static cudaError_t derivs_t(const EvoArgs& a, cudaStream_t st) {
-    const uint32_t zs = a.deriv_zs ? a.deriv_zs : (uint32_t)deriv_default_zs(N);
+static cudaError_t wave_t(const EvoArgs& a, cudaStream_t st) {
+    const uint32_t zs = a.deriv_zs ? a.deriv_zs : (uint32_t)wave_default_zs(N);
     if constexpr (N == 8) {
-        if (zs == 4) return derivs_zs<8, 4>(a, st);
-        if (zs == 8) return derivs_zs<8, 8>(a, st);
+        if (zs == 4) return wave_zs<8, 4>(a, st);
+        if (zs == 8) return wave_zs<8, 8>(a, st);
     } else if constexpr (N == 16) {
-        if (zs == 1) return derivs_zs<16, 1>(a, st);
-        if (zs == 2) return derivs_zs<16, 2>(a, st);
-        if (zs == 4) return derivs_zs<16, 4>(a, st);
+        if (zs == 1) return wave_zs<16, 1>(a, st);
+        if (zs == 2) return wave_zs<16, 2>(a, st);
+        if (zs == 4) return wave_zs<16, 4>(a, st);
     } else {
-        if (zs == 1) return derivs_zs<32, 1>(a, st);   // deeper slabs would spill registers
+        if (zs == 1) return wave_zs<32, 1>(a, st);
     }
     return cudaErrorInvalidValue;
 }
-cudaError_t launch_evo_derivs(const EvoArgs& a, cudaStream_t st) {
+cudaError_t launch_evo_stage_wave(const EvoArgs& a, cudaStream_t st) {
+    if (a.n_items != 0 && (a.stage < 1 || a.stage > 4)) return cudaErrorInvalidValue;
     switch (a.n) {
-        case 8: return derivs_t<8>(a, st);
-        case 16: return derivs_t<16>(a, st);
-        case 32: return derivs_t<32>(a, st);
+        case 8: return wave_t<8>(a, st);
+        case 16: return wave_t<16>(a, st);
+        case 32: return wave_t<32>(a, st);
         default: return cudaErrorInvalidValue;
     }
 }
@@ -777,22 +613,6 @@ uint32_t evo_deriv_zs_candidates(uint32_t n, uint32_t* out) {
     const uint32_t k = n == 16 ? 3u : (n == 8 ? 2u : 1u);
     for (uint32_t i = 0; i < k; i++) out[i] = c[i];
     return n == 8 || n == 16 || n == 32 ? k : 0u;
-}
-
-template <int N>
-static cudaError_t rhs_t(const EvoArgs& a, cudaStream_t st) {
-    const uint64_t total = (uint64_t)a.n_items * N * N * N;
-    if (total == 0) return cudaSuccess;
-    k_evo_rhs_wave<N><<<(unsigned)((total + 255) / 256), 256, 0, st>>>(a);
-    return cudaGetLastError();
-}
-cudaError_t launch_evo_rhs_wave(const EvoArgs& a, cudaStream_t st) {
-    switch (a.n) {
-        case 8: return rhs_t<8>(a, st);
-        case 16: return rhs_t<16>(a, st);
-        case 32: return rhs_t<32>(a, st);
-        default: return cudaErrorInvalidValue;
-    }
 }
 
 cudaError_t launch_evo_restrict(const EvoRestrictArgs& g, cudaStream_t st) {

@@ -26,9 +26,6 @@ namespace amr {
 namespace {
 
 constexpr int kConsFields = F_GAMZ + 1;   // chi, gt_ij, K, At_ij, Gt^i: the first 17, in the state's order
-constexpr int kConsColumns = 63;
-// the column of a derivative (evolve.h): the constraints' are D_CHI1 .. D_GAM1 + 8 and D_AT1 on
-__device__ constexpr int cons_column(int k) { return k < D_AL1 ? k : k - (D_AT1 - D_AL1); }
 
 // A tile of N x TY x TZ interior cells of one domain, a cell a thread.
 template <int N, int TY, int TZ, int R_, int MINB>
@@ -49,7 +46,7 @@ struct ConsShape {
     static constexpr int COPIES = WHOLE ? 1 : PLANES;
     static constexpr uint32_t COPY_BYTES = 4u * (WHOLE ? SLOT : CHUNK);
     static constexpr int TILES = (N / TY) * (N / TZ);
-    static constexpr size_t SMEM = ((size_t)R * SLOT + (size_t)kConsColumns * CT) * 4u + 2u * R * 8u;
+    static constexpr size_t SMEM = ((size_t)R * SLOT + (size_t)BSSN_ND * CT) * 4u + 2u * R * 8u;
     static_assert(CT % 32 == 0 && N % TY == 0 && N % TZ == 0 && COPIES <= 32 && AHEAD >= 1, "whole warps and tiles");
     static_assert((CHUNK * 4) % 16 == 0 && (TY * T * 4) % 16 == 0 && (T * T * 4) % 16 == 0 && PP % 4 == 0 &&
                   (SLOT * 4) % 16 == 0, "every copy is aligned");
@@ -64,7 +61,7 @@ __global__ void __launch_bounds__(ConsShape<N, TY, TZ, R_, MINB>::CT, MINB)
     extern __shared__ __align__(128) unsigned char smem_raw[];
     float* ring = reinterpret_cast<float*>(smem_raw);
     float* const my = ring + (size_t)R * S::SLOT + threadIdx.x;   // this thread's column
-    uint64_t* full = reinterpret_cast<uint64_t*>(ring + (size_t)R * S::SLOT + (size_t)kConsColumns * CT);
+    uint64_t* full = reinterpret_cast<uint64_t*>(ring + (size_t)R * S::SLOT + (size_t)BSSN_ND * CT);
     uint64_t* empty = full + R;
     __shared__ volatile int s_abort;
     __shared__ uint32_t s_asked;   // visits requested
@@ -195,14 +192,14 @@ __global__ void __launch_bounds__(ConsShape<N, TY, TZ, R_, MINB>::CT, MINB)
         for (int f = 0; f <= F_GZZ; f++) {
             const float* q = visit(f);
             float d2[6];
-            gradient(q, f == F_CHI ? cons_column(D_CHI1) : cons_column(D_G1) + 3 * (f - F_GXX));
+            gradient(q, f == F_CHI ? D_CHI1 : D_G1 + 3 * (f - F_GXX));
             hessian(q, d2);
             release();
             if (f == F_CHI) {
 #pragma unroll
-                for (int c = 0; c < 6; c++) my[(cons_column(D_CHI2) + c) * CT] = d2[c];
+                for (int c = 0; c < 6; c++) my[(D_CHI2 + c) * CT] = d2[c];
             } else {   // gt^lm d_l d_m gt_ij
-                my[(cons_column(D_GLAP) + f - F_GXX) * CT] = gi[0] * d2[0] + gi[1] * d2[1] + gi[2] * d2[2] +
+                my[(D_GLAP + f - F_GXX) * CT] = gi[0] * d2[0] + gi[1] * d2[1] + gi[2] * d2[2] +
                                                               2.f * (gi[3] * d2[3] + gi[4] * d2[4] + gi[5] * d2[5]);
             }
         }
@@ -213,8 +210,8 @@ __global__ void __launch_bounds__(ConsShape<N, TY, TZ, R_, MINB>::CT, MINB)
 #pragma unroll 1
         for (int f = F_K; f < kConsFields; f++) {
             const float* q = visit(f);
-            gradient(q, f == F_K ? cons_column(D_K1)
-                                 : (f <= F_AZZ ? cons_column(D_AT1) + 3 * (f - F_AXX) : cons_column(D_GAM1) + 3 * (f - F_GAMX)));
+            gradient(q, f == F_K ? D_K1
+                                 : (f <= F_AZZ ? D_AT1 + 3 * (f - F_AXX) : D_GAM1 + 3 * (f - F_GAMX)));
             release();
         }
         if (!ok) {   // a wait gave up: report it; the tile's results are dropped
@@ -222,7 +219,7 @@ __global__ void __launch_bounds__(ConsShape<N, TY, TZ, R_, MINB>::CT, MINB)
             atomicExch(a.err, 1);
         }
         if (__any_sync(0xffffffffu, s_abort)) break;
-        auto dv = [&](int d) { return my[cons_column(d) * CT]; };
+        auto dv = [&](int d) { return my[d * CT]; };
         float hm[4];
         bssn_constraints(u, dv, a.prm, hm);
 #pragma unroll
