@@ -396,4 +396,38 @@ __device__ __forceinline__ float interp10(const float* __restrict__ d, float rx,
     return interp10_strided(d, T, T * T, rx, ry, rz);
 }
 
+// Christoffel symbols of one cell from the six compressed metric gradients (BSSN.h:72-90).
+// `M` multiplies the lowered symbols: the metric itself (reference) or its inverse.
+// `noise` holds the encodes' noise pairs in draw order (noise_pairs1 per symbol pair).
+__device__ __forceinline__ void christoffel_cell(const uint32_t* G, const Sym& M, const float2* noise, uint32_t* out) {
+    float3 d[6];
+#pragma unroll
+    for (int k = 0; k < 6; k++) d[k] = cf3_decode(G[k]);
+    // rows of float3x3_sym(float3, float3, float3), tensors.h:138: S_l(j,k) = (d_j g_lk + d_k g_lj)/2
+    const Sym Sx{d[0].x, __fmul_rn(__fadd_rn(d[0].y, d[1].x), .5f), __fmul_rn(__fadd_rn(d[0].z, d[2].x), .5f),
+                 d[1].y, __fmul_rn(__fadd_rn(d[2].y, d[1].z), .5f), d[2].z};
+    const Sym Sy{d[1].x, __fmul_rn(__fadd_rn(d[1].y, d[3].x), .5f), __fmul_rn(__fadd_rn(d[1].z, d[4].x), .5f),
+                 d[3].y, __fmul_rn(__fadd_rn(d[4].y, d[3].z), .5f), d[4].z};
+    const Sym Sz{d[2].x, __fmul_rn(__fadd_rn(d[2].y, d[4].x), .5f), __fmul_rn(__fadd_rn(d[2].z, d[5].x), .5f),
+                 d[4].y, __fmul_rn(__fadd_rn(d[5].y, d[4].z), .5f), d[5].z};
+    const float sx[6] = {Sx.xx, Sx.xy, Sx.xz, Sx.yy, Sx.yz, Sx.zz};
+    const float sy[6] = {Sy.xx, Sy.xy, Sy.xz, Sy.yy, Sy.yz, Sy.zz};
+    const float sz[6] = {Sz.xx, Sz.xy, Sz.xz, Sz.yy, Sz.yz, Sz.zz};
+    // symbols jk and jk+1 as the two lanes of a pair; fma(-d, .5, s) = fma(d, -.5, s) exactly
+#pragma unroll
+    for (int jk = 0; jk < 6; jk += 2) {
+        const float2 vx = fma2(make_float2(d[jk].x, d[jk + 1].x), splat2(-.5f), make_float2(sx[jk], sx[jk + 1]));
+        const float2 vy = fma2(make_float2(d[jk].y, d[jk + 1].y), splat2(-.5f), make_float2(sy[jk], sy[jk + 1]));
+        const float2 vz = fma2(make_float2(d[jk].z, d[jk + 1].z), splat2(-.5f), make_float2(sz[jk], sz[jk + 1]));
+        // M * v (sym_times)
+        const float2 rx = fma2(vz, splat2(M.xz), fma2(vx, splat2(M.xx), mul2(vy, splat2(M.xy))));
+        const float2 ry = fma2(vz, splat2(M.yz), fma2(vx, splat2(M.xy), mul2(vy, splat2(M.yy))));
+        const float2 rz = fma2(vz, splat2(M.zz), fma2(vx, splat2(M.xz), mul2(vy, splat2(M.yz))));
+        const Cf3Pair w = cf3_encode2<false>(rx, ry, rz, noise[3 * (jk / 2)], noise[3 * (jk / 2) + 1],
+                                             noise[3 * (jk / 2) + 2]);
+        out[jk] = w.w0;
+        out[jk + 1] = w.w1;
+    }
+}
+
 }  // namespace amr

@@ -67,13 +67,15 @@ uint32_t stencil_grid(const amr_config& c, int kind, uint32_t n_items) {
 #undef AMR_SMEM
     const uint32_t threads = c.size_domain * c.size_domain;
     uint32_t per_sm = (uint32_t)(220u * 1024u / (smem ? smem : 1));
-    per_sm = per_sm < 2048u / threads ? per_sm : 2048u / threads;
+    // the registers of the single operators (up to 64 a thread) hold 1024 threads an SM
+    const uint32_t resident = (kind == SK_BSSN ? 2048u : 1024u) / threads;
+    per_sm = per_sm < resident ? per_sm : resident;
     if (per_sm < 1) per_sm = 1;
     const uint32_t cap = per_sm * (uint32_t)sms;
     // few items: wider grids than one CTA per item.  The fused kind splits its planes evenly over
     // the CTAs: at least 4 interior planes each (each CTA also streams 2p halo planes), unless
-    // that leaves SMs idle, then one CTA per SM down to one plane each.  The others cut items
-    // into z-ranges.
+    // that leaves SMs idle, then one CTA per SM down to one plane each.  The others split them evenly
+    // too, at least two planes each.
     const uint64_t planes = (uint64_t)n_items * c.size_domain;
     const uint64_t one_per_sm = planes < (uint64_t)sms ? planes : (uint64_t)sms;
     const uint64_t want = kind == SK_BSSN ? std::max((planes + 3u) / 4u, one_per_sm)

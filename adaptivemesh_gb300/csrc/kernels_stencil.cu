@@ -29,9 +29,9 @@ template <int N, int P, int KIND>
 struct StencilShape {
     static constexpr int T = N + 2 * P;
     static constexpr int NC = KIND == SK_BSSN ? 6 : 1;
-    // ring slots: 2P+1 in use and 2 in flight; the fused kind keeps one in flight so that two
+    // ring slots: 2P+2 in use (two planes' windows) and 2 in flight; the fused kind keeps one in flight so that two
     // CTAs (with their generator and gradient tables) fit in one SM's shared memory
-    static constexpr int R = KIND == SK_BSSN ? 2 * P + 2 : 2 * P + 3;
+    static constexpr int R = KIND == SK_BSSN ? 2 * P + 2 : 2 * P + 4;
     static constexpr uint32_t PLANE = (uint32_t)(T * T);         // floats per plane
     static constexpr uint32_t PLANE_BYTES = PLANE * 4u;
     // SK_BSSN works on y-tiles of TY interior rows: the whole plane, or half of it where six
@@ -207,40 +207,6 @@ __device__ __forceinline__ void mixed_partials2(const PL& pl, int c0, uint32_t x
     }
 }
 
-// Christoffel symbols of one cell from the six compressed metric gradients (BSSN.h:72-90).
-// `M` multiplies the lowered symbols: the metric itself (reference) or its inverse.
-// `noise` holds the encodes' noise pairs in draw order (noise_pairs1 per symbol pair).
-__device__ __forceinline__ void christoffel_cell(const uint32_t* G, const Sym& M, const float2* noise, uint32_t* out) {
-    float3 d[6];
-#pragma unroll
-    for (int k = 0; k < 6; k++) d[k] = cf3_decode(G[k]);
-    // rows of float3x3_sym(float3, float3, float3), tensors.h:138: S_l(j,k) = (d_j g_lk + d_k g_lj)/2
-    const Sym Sx{d[0].x, __fmul_rn(__fadd_rn(d[0].y, d[1].x), .5f), __fmul_rn(__fadd_rn(d[0].z, d[2].x), .5f),
-                 d[1].y, __fmul_rn(__fadd_rn(d[2].y, d[1].z), .5f), d[2].z};
-    const Sym Sy{d[1].x, __fmul_rn(__fadd_rn(d[1].y, d[3].x), .5f), __fmul_rn(__fadd_rn(d[1].z, d[4].x), .5f),
-                 d[3].y, __fmul_rn(__fadd_rn(d[4].y, d[3].z), .5f), d[4].z};
-    const Sym Sz{d[2].x, __fmul_rn(__fadd_rn(d[2].y, d[4].x), .5f), __fmul_rn(__fadd_rn(d[2].z, d[5].x), .5f),
-                 d[4].y, __fmul_rn(__fadd_rn(d[5].y, d[4].z), .5f), d[5].z};
-    const float sx[6] = {Sx.xx, Sx.xy, Sx.xz, Sx.yy, Sx.yz, Sx.zz};
-    const float sy[6] = {Sy.xx, Sy.xy, Sy.xz, Sy.yy, Sy.yz, Sy.zz};
-    const float sz[6] = {Sz.xx, Sz.xy, Sz.xz, Sz.yy, Sz.yz, Sz.zz};
-    // symbols jk and jk+1 as the two lanes of a pair; fma(-d, .5, s) = fma(d, -.5, s) exactly
-#pragma unroll
-    for (int jk = 0; jk < 6; jk += 2) {
-        const float2 vx = fma2(make_float2(d[jk].x, d[jk + 1].x), splat2(-.5f), make_float2(sx[jk], sx[jk + 1]));
-        const float2 vy = fma2(make_float2(d[jk].y, d[jk + 1].y), splat2(-.5f), make_float2(sy[jk], sy[jk + 1]));
-        const float2 vz = fma2(make_float2(d[jk].z, d[jk + 1].z), splat2(-.5f), make_float2(sz[jk], sz[jk + 1]));
-        // M * v (sym_times)
-        const float2 rx = fma2(vz, splat2(M.xz), fma2(vx, splat2(M.xx), mul2(vy, splat2(M.xy))));
-        const float2 ry = fma2(vz, splat2(M.yz), fma2(vx, splat2(M.xy), mul2(vy, splat2(M.yy))));
-        const float2 rz = fma2(vz, splat2(M.zz), fma2(vx, splat2(M.xz), mul2(vy, splat2(M.yz))));
-        const Cf3Pair w = cf3_encode2<false>(rx, ry, rz, noise[3 * (jk / 2)], noise[3 * (jk / 2) + 1],
-                                             noise[3 * (jk / 2) + 2]);
-        out[jk] = w.w0;
-        out[jk + 1] = w.w1;
-    }
-}
-
 // ---------------------------------------------------------------- the streaming kernel
 template <int N, int P, int KIND>
 __global__ void __launch_bounds__(N * N, N * N <= 256 ? 2 : 1) k_stencil(const __grid_constant__ StencilArgs a) {
@@ -290,16 +256,25 @@ __global__ void __launch_bounds__(N * N, N * N <= 256 ? 2 : 1) k_stencil(const _
     // cut into Q z-ranges of N/Q interior planes so that it spreads over every CTA.  A unit streams
     // its nz + 2P padded planes through the ring; thread 0 keeps the ring R planes ahead of the
     // plane being computed, across unit boundaries.
-    // With a.zsplit > 1 every item is cut that way instead (few items, launched on a wider grid).
+    // With a.even (fewer items than CTAs) CTA b takes planes [b P / G, (b + 1) P / G) of the P planes of all
+    // items instead: a range of one item, and maybe the first planes of the next.
     const uint32_t G = gridDim.x;
     const uint32_t rem = a.n_items % G;
-    const bool all_split = a.zsplit > 1u;
-    const uint32_t Q = all_split ? a.zsplit : S::Q, NZQ = N / Q;
-    const bool split = all_split || (rem != 0u && Q * rem <= (Q - 1u) * G);
-    const uint32_t n_whole = all_split ? 0u : split ? a.n_items - rem : a.n_items;
-    const uint32_t n_units = n_whole + (all_split ? a.n_items * Q : split ? rem * Q : 0u);
+    const bool even = a.even != 0u;
+    constexpr uint32_t Q = S::Q, NZQ = N / Q;
+    const bool split = rem != 0u && Q * rem <= (Q - 1u) * G;
+    const uint32_t n_whole = split ? a.n_items - rem : a.n_items;
+    const uint32_t n_units = even ? 2u * G : n_whole + (split ? rem * Q : 0u);
+    const uint32_t lo = even ? (uint32_t)((uint64_t)blockIdx.x * a.n_items * N / G) : 0u;
+    const uint32_t hi = even ? (uint32_t)((uint64_t)(blockIdx.x + 1u) * a.n_items * N / G) : 0u;
     auto unit_of = [&](uint32_t u, uint32_t& item, uint32_t& z0, uint32_t& nz) {
-        if (u < n_whole) { item = u; z0 = 0; nz = N; }
+        if (even) {   // u: blockIdx.x, then blockIdx.x + G
+            item = lo / N;
+            z0 = lo % N;
+            nz = min(N - z0, hi - lo);
+            if (u >= G) { item++; z0 = 0; nz = hi - lo - nz; }
+        }
+        else if (u < n_whole) { item = u; z0 = 0; nz = N; }
         else { const uint32_t v = u - n_whole; item = n_whole + v / Q; z0 = (v % Q) * NZQ; nz = NZQ; }
     };
     auto active_node = [&](uint32_t item, uint32_t& node, int& depth) {
@@ -312,7 +287,7 @@ __global__ void __launch_bounds__(N * N, N * N <= 256 ? 2 : 1) k_stencil(const _
             uint32_t item, z0, nz, node;
             int depth;
             unit_of(u, item, z0, nz);
-            if (active_node(item, node, depth)) break;
+            if (nz != 0u && active_node(item, node, depth)) break;
         }
         return u;
     };
@@ -353,17 +328,19 @@ __global__ void __launch_bounds__(N * N, N * N <= 256 ? 2 : 1) k_stencil(const _
         active_node(item, node, depth);
         const float dx1 = a.geo.inv_dx[depth], dx2 = a.geo.inv_dx2[depth];
 #pragma unroll 1
-        for (uint32_t zl = 0; zl < nz; zl++) {
-            const uint32_t g = g_base + zl, z = z0 + zl;   // planes g .. g+2P hold padded z .. z+2P
-            if (tid == 0) issue_upto(g + R);               // every plane below g is finished
-            // a unit's first window needs all its planes, later windows one more
+        for (uint32_t zp = 0; zp < nz; zp += 2) {   // two planes a barrier: 16.6 us a launch with one, 15.0 with two
+            const uint32_t gp = g_base + zp;
+            if (tid == 0) issue_upto(gp + R);               // every plane below gp is finished
             bool ok = true;
-            for (int j = zl == 0 ? 0 : 2 * P; j <= 2 * P; j++) {
-                const uint32_t sq = g + j;
-                ok &= mbar_wait(&bars[sq % R], (sq / R) & 1u);
-            }
-            if (!ok) s_abort = 1;
-            if (ok) {
+#pragma unroll 1
+            for (uint32_t zl = zp; zl < min(zp + 2u, nz); zl++) {
+                const uint32_t g = g_base + zl, z = z0 + zl;   // planes g .. g+2P hold padded z .. z+2P
+                // a unit's first window needs all its planes, later windows one more
+                for (int j = zl == 0 ? 0 : 2 * P; j <= 2 * P; j++) {
+                    const uint32_t sq = g + j;
+                    ok &= mbar_wait(&bars[sq % R], (sq / R) & 1u);
+                }
+                if (!ok) break;
                 const uint32_t base = g % R;
                 uint32_t slot[2 * P + 1];
 #pragma unroll
@@ -376,9 +353,17 @@ __global__ void __launch_bounds__(N * N, N * N <= 256 ? 2 : 1) k_stencil(const _
                     float gx, gy, gz, hx, hy, hz;
                     fd_axes<P, T>(pl, c0, gx, gy, gz, hx, hy, hz);
                     int32_t rng = cell_rng_at(pre_d[0], zg);
-                    if (KIND == SK_GRAD_HESS)
-                        a.hdiag[o] = cf3_encode(__fmul_rn(hx, dx2), __fmul_rn(hy, dx2), __fmul_rn(hz, dx2), rng);
-                    a.grad[0][o] = cf3_encode(__fmul_rn(gx, dx1), __fmul_rn(gy, dx1), __fmul_rn(gz, dx1), rng);
+                    if (KIND == SK_GRAD_HESS) {   // the Hessian's word, then the gradient's, as a pair
+                        float2 nx, ny, nz;
+                        noise_pairs1(rng, nx, ny, nz);
+                        const Cf3Pair w = cf3_encode2<false>(make_float2(__fmul_rn(hx, dx2), __fmul_rn(gx, dx1)),
+                                                             make_float2(__fmul_rn(hy, dx2), __fmul_rn(gy, dx1)),
+                                                             make_float2(__fmul_rn(hz, dx2), __fmul_rn(gz, dx1)), nx, ny, nz);
+                        a.hdiag[o] = w.w0;
+                        a.grad[0][o] = w.w1;
+                    } else {
+                        a.grad[0][o] = cf3_encode(__fmul_rn(gx, dx1), __fmul_rn(gy, dx1), __fmul_rn(gz, dx1), rng);
+                    }
                 } else if (KIND == SK_MIXED) {
                     auto pl = [&](int j) { return (const float*)(ring + (size_t)slot[j] * PLANE); };
                     const float3 m = mixed_partials<N, P, T>(pl, c0, x, y, z);
@@ -386,11 +371,12 @@ __global__ void __launch_bounds__(N * N, N * N <= 256 ? 2 : 1) k_stencil(const _
                     a.hoff[o] = cf3_encode(__fmul_rn(m.x, dx2), __fmul_rn(m.y, dx2), __fmul_rn(m.z, dx2), rng);
                 }
             }
-            __syncthreads();   // every thread is done with plane g: its slot may be refilled
+            if (!ok) s_abort = 1;
+            __syncthreads();   // every thread is done with these planes: their slots may be refilled
             if (s_abort) {
                 if (tid == 0) {
                     atomicExch(a.err, 1);
-                    for (uint32_t sq = g; sq < issued; sq++) mbar_wait(&bars[sq % R], (sq / R) & 1u);   // drain (bounded)
+                    for (uint32_t sq = gp; sq < issued; sq++) mbar_wait(&bars[sq % R], (sq / R) & 1u);   // drain (bounded)
                 }
                 return;
             }
@@ -677,15 +663,13 @@ cudaError_t launch_stencil_t(const StencilArgs& a, uint32_t grid, cudaStream_t s
     if (e != cudaSuccess) return e;
     if (grid == 0) return cudaSuccess;
     if constexpr (KIND != SK_BSSN) {
-        // a grid wider than the items (few domains): cut each into the most z-ranges of at
-        // least two planes that the grid holds
+        // a grid wider than the items (few domains): their planes are split evenly over the CTAs, which
+        // leaves no last wave (z-ranges of a divisor of N planes: 196 CTAs for 49 domains of 28^3 on 152
+        // SMs, 22.2 us; evenly 16.6)
         if (a.n_items > 0u && grid > a.n_items) {
-            uint32_t q = 1;
-            for (uint32_t d = 2; d <= (uint32_t)N / 2u; d++)
-                if (N % d == 0 && (uint64_t)d * a.n_items <= grid) q = d;
             StencilArgs b = a;
-            b.zsplit = q;
-            kernel<<<a.n_items * q, S::THREADS, S::SMEM, st>>>(b);
+            b.even = 1;
+            kernel<<<grid, S::THREADS, S::SMEM, st>>>(b);
             return cudaGetLastError();
         }
     }
