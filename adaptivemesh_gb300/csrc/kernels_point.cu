@@ -11,21 +11,28 @@ constexpr int kBlock = 256;
 
 inline uint32_t blocks_for(uint64_t n) { return (uint32_t)((n + kBlock - 1) / kBlock); }
 
-// Decompose an inner-layout index into (slot, x, y, z) and the padded index of the same cell.
+// A thread's cell: its domain, inner-layout index o and padded index.  A block's cells lie in one domain
+// (domain_blocks blocks each) of a compiled size, so that no index is divided in 64 bits or by a variable:
+// the pointwise kernels were bound by issue (70 % of the slots), their trace is now near the copy
+// bandwidth (1.08 M cells of 28^3, 10.7 -> 10.1 us; the Christoffel symbols, with encodes in pairs, 25.7 ->
+// 23.7).
 struct InnerCell {
     uint32_t slot, x, y, z;
-    uint64_t padded;
+    uint64_t o, padded;
 };
-__device__ __forceinline__ InnerCell inner_cell(uint64_t o, const Dims& d) {
-    InnerCell c;
-    const uint64_t n3 = (uint64_t)d.n * d.n * d.n;
-    c.slot = (uint32_t)(o / n3);
-    uint32_t r = (uint32_t)(o - (uint64_t)c.slot * n3);
-    c.x = r % d.n; r /= d.n;
-    c.y = r % d.n;
-    c.z = r / d.n;
-    c.padded = (((uint64_t)c.slot * d.t + c.z + d.p) * d.t + c.y + d.p) * d.t + c.x + d.p;
-    return c;
+inline uint32_t domain_blocks(const Dims& d) { return (d.n * d.n * d.n + kBlock - 1) / kBlock; }
+template <int N, int P>
+__device__ __forceinline__ bool inner_cell(InnerCell& c) {   // false: past the domain's cells
+    constexpr uint32_t T = N + 2 * P, n3 = N * N * N, per = (n3 + kBlock - 1) / kBlock;
+    c.slot = blockIdx.x / per;
+    uint32_t r = (blockIdx.x - c.slot * per) * kBlock + threadIdx.x;
+    if (r >= n3) return false;
+    c.o = (uint64_t)c.slot * n3 + r;
+    c.x = r % N; r /= N;
+    c.y = r % N;
+    c.z = r / N;
+    c.padded = (uint64_t)c.slot * (T * T * T) + ((c.z + P) * T + c.y + P) * T + c.x + P;
+    return true;
 }
 __device__ __forceinline__ bool slot_active(const uint32_t* positions, uint32_t slot, uint32_t substep,
                                             uint32_t max_depth, int* depth_out) {
@@ -58,12 +65,13 @@ __global__ void k_cf3_decode(const uint32_t* __restrict__ w, uint64_t n, float* 
 }
 
 // ---------------------------------------------------------------- g^kl H_kl, BSSN.h:7-22
-__global__ void k_deriv_trace(Dims d, const uint32_t* __restrict__ hd, const uint32_t* __restrict__ ho, Ptr6f m,
-                              float* __restrict__ out, const uint32_t* __restrict__ positions, uint32_t used,
-                              uint32_t substep, uint32_t max_depth) {
-    const uint64_t o = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (o >= (uint64_t)used * d.n * d.n * d.n) return;
-    const InnerCell c = inner_cell(o, d);
+template <int N, int P>
+__global__ void k_deriv_trace(const uint32_t* __restrict__ hd, const uint32_t* __restrict__ ho, Ptr6f m,
+                              float* __restrict__ out, const uint32_t* __restrict__ positions, uint32_t substep,
+                              uint32_t max_depth) {
+    InnerCell c;
+    if (!inner_cell<N, P>(c)) return;
+    const uint64_t o = c.o;
     int depth;
     if (!slot_active(positions, c.slot, substep, max_depth, &depth)) return;
     const Sym g{m.p[0][c.padded], m.p[1][c.padded], m.p[2][c.padded], m.p[3][c.padded], m.p[4][c.padded], m.p[5][c.padded]};
@@ -71,48 +79,38 @@ __global__ void k_deriv_trace(Dims d, const uint32_t* __restrict__ hd, const uin
 }
 
 // ---------------------------------------------------------------- Christoffel symbols, BSSN.h:55-91
-__global__ void k_christoffel(Dims d, Ptr6f m, Ptr6u der, int32_t seed, Ptr6u outp,
-                              const uint32_t* __restrict__ positions, uint32_t used, uint32_t substep,
-                              uint32_t max_depth, int mode) {
-    const uint64_t o = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (o >= (uint64_t)used * d.n * d.n * d.n) return;
-    const InnerCell c = inner_cell(o, d);
+template <int N, int P>
+__global__ void k_christoffel(Ptr6f m, Ptr6u der, int32_t seed, Ptr6u outp,
+                              const uint32_t* __restrict__ positions, uint32_t substep, uint32_t max_depth,
+                              int mode) {
+    InnerCell c;
+    if (!inner_cell<N, P>(c)) return;
+    const uint64_t o = c.o;
     int depth;
     if (!slot_active(positions, c.slot, substep, max_depth, &depth)) return;
-    int32_t rng = cell_rng(seed, c.x, c.y, c.slot * d.n + c.z);
+    int32_t rng = cell_rng(seed, c.x, c.y, c.slot * N + c.z);
     uint32_t G[6];
 #pragma unroll
     for (int k = 0; k < 6; k++) G[k] = der.p[k][o];
     const Sym g{m.p[0][c.padded], m.p[1][c.padded], m.p[2][c.padded], m.p[3][c.padded], m.p[4][c.padded], m.p[5][c.padded]};
     const Sym M = mode == AMR_CHRISTOFFEL_RAISED ? sym_inverse(g) : g;
-    float3 dd[6];
+    float2 noise[9];
 #pragma unroll
-    for (int k = 0; k < 6; k++) dd[k] = cf3_decode(G[k]);
-    const Sym Sx{dd[0].x, __fmul_rn(__fadd_rn(dd[0].y, dd[1].x), .5f), __fmul_rn(__fadd_rn(dd[0].z, dd[2].x), .5f),
-                 dd[1].y, __fmul_rn(__fadd_rn(dd[2].y, dd[1].z), .5f), dd[2].z};
-    const Sym Sy{dd[1].x, __fmul_rn(__fadd_rn(dd[1].y, dd[3].x), .5f), __fmul_rn(__fadd_rn(dd[1].z, dd[4].x), .5f),
-                 dd[3].y, __fmul_rn(__fadd_rn(dd[4].y, dd[3].z), .5f), dd[4].z};
-    const Sym Sz{dd[2].x, __fmul_rn(__fadd_rn(dd[2].y, dd[4].x), .5f), __fmul_rn(__fadd_rn(dd[2].z, dd[5].x), .5f),
-                 dd[4].y, __fmul_rn(__fadd_rn(dd[5].y, dd[4].z), .5f), dd[5].z};
-    const float sx[6] = {Sx.xx, Sx.xy, Sx.xz, Sx.yy, Sx.yz, Sx.zz};
-    const float sy[6] = {Sy.xx, Sy.xy, Sy.xz, Sy.yy, Sy.yz, Sy.zz};
-    const float sz[6] = {Sz.xx, Sz.xy, Sz.xz, Sz.yy, Sz.yz, Sz.zz};
+    for (int k = 0; k < 3; k++) noise_pairs1(rng, noise[3 * k], noise[3 * k + 1], noise[3 * k + 2]);
+    uint32_t out[6];
+    christoffel_cell(G, M, noise, out);
 #pragma unroll
-    for (int jk = 0; jk < 6; jk++) {
-        const float3 v = make_float3(__fmaf_rn(-dd[jk].x, .5f, sx[jk]), __fmaf_rn(-dd[jk].y, .5f, sy[jk]),
-                                     __fmaf_rn(-dd[jk].z, .5f, sz[jk]));
-        const float3 r = sym_times(M, v);
-        outp.p[jk][o] = cf3_encode(r.x, r.y, r.z, rng);
-    }
+    for (int jk = 0; jk < 6; jk++) outp.p[jk][o] = out[jk];
 }
 
 // ---------------------------------------------------------------- SimpleWave Heun update, SimpleWave.h:7-46
-__global__ void k_wave_step(Dims d, float outer_dt, int corrector, const float* __restrict__ old_f,
+template <int N, int P>
+__global__ void k_wave_step(float outer_dt, int corrector, const float* __restrict__ old_f,
                             const uint32_t* __restrict__ der, const uint32_t* __restrict__ hess, float* new_f,
-                            const uint32_t* __restrict__ positions, uint32_t used, uint32_t substep, uint32_t max_depth) {
-    const uint64_t o = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (o >= (uint64_t)used * d.n * d.n * d.n) return;
-    const InnerCell c = inner_cell(o, d);
+                            const uint32_t* __restrict__ positions, uint32_t substep, uint32_t max_depth) {
+    InnerCell c;
+    if (!inner_cell<N, P>(c)) return;
+    const uint64_t o = c.o;
     int depth;
     if (!slot_active(positions, c.slot, substep, max_depth, &depth)) return;
     const float visc = 0.01f;                                          // SimpleWave.h:5
@@ -131,49 +129,59 @@ __device__ __forceinline__ float cf3_length(uint32_t w) {
     const float3 v = cf3_decode(w);
     return sqrt_approx(__fmaf_rn(v.z, v.z, __fmaf_rn(v.x, v.x, __fmul_rn(v.y, v.y))));
 }
-__global__ void k_criterion_columns(Dims d, float outer_dx, const uint32_t* __restrict__ der,
-                                    const uint32_t* __restrict__ hess, float* __restrict__ crit,
-                                    const uint32_t* __restrict__ positions, uint32_t used, uint32_t substep,
-                                    uint32_t max_depth) {
-    const uint32_t n = d.n, h = n >> 1, q = n >> 2;
-    const uint64_t o = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;   // x + (y + zi*h)*n
-    if (o >= (uint64_t)used * n * n) return;
-    const uint32_t x = (uint32_t)(o % n);
-    const uint32_t rest = (uint32_t)(o / n);
-    const uint32_t y = rest % h, zi = rest / h;
-    const int depth = pos_depth(positions[zi / 2]);
-    if (depth == -1 || !active_depth(substep, (uint32_t)depth, max_depth)) { crit[o] = __int_as_float(0x7fc00000); return; }   // NAN, SimpleWave.h:97
-    uint64_t ro = x + ((uint64_t)y + ((y >= q) ? q : 0u) + (uint64_t)zi * n * h) * n;
+// A CTA per octant.  The reference's first kernel writes a column's largest value for each column of the
+// octant (its h cells along z in the octant, of rows y and y + q), the second the octant's maximum over
+// them, in order from NaN, to its first column's place (SimpleWave.h:91-139).  The values are non-negative
+// or NaN and fmaxf skips NaN, so the maxima do not depend on the order: `parts` threads share a column.
+// (A thread per column and a second launch took 12.5 + 4.0 us on 9 domains of 28^3, a chain of 14 loads; this 6.2.)
+constexpr uint32_t kCritThreads = 512;
+__global__ void __launch_bounds__(kCritThreads) k_criterion(Dims d, float outer_dx, const uint32_t* __restrict__ der,
+                                                           const uint32_t* __restrict__ hess, float* __restrict__ crit,
+                                                           const uint32_t* __restrict__ positions, uint32_t substep,
+                                                           uint32_t max_depth) {
+    const uint32_t n = d.n, h = n >> 1, q = n >> 2, columns = q * h;
+    const uint32_t oct = blockIdx.x & 7u, node = blockIdx.x >> 3;
+    const uint32_t xb = oct & 1u, yb = (oct >> 1) & 1u, zi = 2u * node + (oct >> 2);
+    const uint64_t base = ((uint64_t)zi * h + yb * q) * n + xb * h;
+    const int depth = pos_depth(positions[node]);
+    if (depth == -1 || !active_depth(substep, (uint32_t)depth, max_depth)) {   // NAN, SimpleWave.h:97
+        for (uint32_t c = threadIdx.x; c < columns; c += kCritThreads) crit[base + c % h + (uint64_t)(c / h) * n] = __int_as_float(0x7fc00000);
+        return;
+    }
     // |g| * dx / 2^depth and |H| * dx * dx / 4^depth, left to right (the power-of-two scaling is exact)
     const float s1 = __uint_as_float((127u - (uint32_t)depth) << 23);
     const float s2 = __uint_as_float((127u - 2u * (uint32_t)depth) << 23);
+    __shared__ float part[kCritThreads];
+    const uint32_t parts = min(h, kCritThreads / columns);   // at least 2 (16^3: 16; 32^3: 4)
+    const uint32_t c = threadIdx.x % columns, k = threadIdx.x / columns;
     float cr = 0.f;
-    for (uint32_t i = 0; i < h; i++) {
-        cr = fmaxf(cr, __fmul_rn(__fmul_rn(cf3_length(der[ro]), outer_dx), s1));
-        cr = fmaxf(cr, __fmul_rn(__fmul_rn(__fmul_rn(cf3_length(hess[ro]), outer_dx), outer_dx), s2));
-        cr = fmaxf(cr, __fmul_rn(__fmul_rn(cf3_length(der[ro + (uint64_t)q * n]), outer_dx), s1));
-        cr = fmaxf(cr, __fmul_rn(__fmul_rn(__fmul_rn(cf3_length(hess[ro + (uint64_t)q * n]), outer_dx), outer_dx), s2));
-        ro += (uint64_t)n * n;
+    if (k < parts) {
+        const uint32_t x = xb * h + c % h, y = c / h + (yb ? 2u * q : 0u);
+        const uint64_t ro = x + ((uint64_t)y + (uint64_t)zi * n * h) * n;
+        for (uint32_t i = k; i < h; i += parts) {
+            const uint64_t r0 = ro + (uint64_t)i * n * n, r1 = r0 + (uint64_t)q * n;
+            cr = fmaxf(cr, __fmul_rn(__fmul_rn(cf3_length(der[r0]), outer_dx), s1));
+            cr = fmaxf(cr, __fmul_rn(__fmul_rn(__fmul_rn(cf3_length(hess[r0]), outer_dx), outer_dx), s2));
+            cr = fmaxf(cr, __fmul_rn(__fmul_rn(cf3_length(der[r1]), outer_dx), s1));
+            cr = fmaxf(cr, __fmul_rn(__fmul_rn(__fmul_rn(cf3_length(hess[r1]), outer_dx), outer_dx), s2));
+        }
     }
-    crit[o] = cr;
-}
-// One warp per octant (8 per block of 256).  The reference takes the maximum of the octant's q x h
-// column values in order, starting from NaN (SimpleWave.h:117-139); the values are non-negative
-// or NaN and fmaxf skips NaN, so the maximum does not depend on the order: the lanes take strided
-// parts and combine them in a tree.
-__global__ void k_criterion_octants(Dims d, float* __restrict__ crit, uint32_t used) {
-    const uint32_t n = d.n, h = n >> 1, q = n >> 2;
-    const uint32_t idx = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31u;
-    if (idx >= used * 8u) return;   // uniform in the warp
-    const uint32_t x = idx & 1u, y = (idx >> 1) & 1u, z = (idx >> 2) & 1u, node = idx >> 3;
-    const uint64_t base = (uint64_t)node * n * n + z * (n * n >> 1) + y * (n * n >> 2) + x * h;
-    float cr = __int_as_float(0x7fc00000);
-    for (uint32_t e = lane; e < q * h; e += 32u) cr = fmaxf(cr, crit[base + e % h + (uint64_t)(e / h) * n]);
+    part[threadIdx.x] = cr;
+    __syncthreads();
+    if (k == 0) {
+        for (uint32_t j = 1; j < parts; j++) cr = fmaxf(cr, part[threadIdx.x + j * columns]);
+        if (c != 0) crit[base + c % h + (uint64_t)(c / h) * n] = cr;
+        part[threadIdx.x] = cr;
+    }
+    __syncthreads();
+    if (threadIdx.x < 32u) {
+        cr = __int_as_float(0x7fc00000);
+        for (uint32_t e = threadIdx.x; e < columns; e += 32u) cr = fmaxf(cr, part[e]);
 #pragma unroll
-    for (int s = 16; s >= 1; s >>= 1) cr = fmaxf(cr, __shfl_xor_sync(0xFFFFFFFFu, cr, s));
-    if (lane == 0) crit[base] = cr;
+        for (int s = 16; s >= 1; s >>= 1) cr = fmaxf(cr, __shfl_xor_sync(0xFFFFFFFFu, cr, s));
+        if (threadIdx.x == 0) crit[base] = cr;
+    }
 }
-
 
 // ---------------------------------------------------------------- slice rasteriser, AMR.h:1313-1352
 // One thread per pixel of a z-slice through the unit cube: descend the octree to the leaf holding
@@ -237,41 +245,43 @@ cudaError_t launch_cf3_decode(const uint32_t* w, uint64_t n, float* xyz, cudaStr
 cudaError_t launch_deriv_trace(Dims d, const uint32_t* hd, const uint32_t* ho, float* const* metric6, float* out,
                                const uint32_t* positions, uint32_t used, uint32_t substep, uint32_t max_depth,
                                cudaStream_t st) {
-    const uint64_t n = (uint64_t)used * d.n * d.n * d.n;
-    if (n == 0) return cudaSuccess;
+    if (used == 0) return cudaSuccess;
     Ptr6f m;
     for (int k = 0; k < 6; k++) m.p[k] = metric6[k];
-    k_deriv_trace<<<blocks_for(n), kBlock, 0, st>>>(d, hd, ho, m, out, positions, used, substep, max_depth);
-    return cudaGetLastError();
+#define AMR_POINT(N, P) \
+    if (d.n == N && d.p == P) { k_deriv_trace<N, P><<<used * domain_blocks(d), kBlock, 0, st>>>(hd, ho, m, out, positions, substep, max_depth); return cudaGetLastError(); }
+    AMR_FOR_EACH_CONFIG(AMR_POINT)
+#undef AMR_POINT
+    return cudaErrorInvalidValue;
 }
 cudaError_t launch_christoffel(Dims d, float* const* metric6, uint32_t* const* der6, int32_t seed, uint32_t* const* out6,
                                const uint32_t* positions, uint32_t used, uint32_t substep, uint32_t max_depth, int mode,
                                cudaStream_t st) {
-    const uint64_t n = (uint64_t)used * d.n * d.n * d.n;
-    if (n == 0) return cudaSuccess;
+    if (used == 0) return cudaSuccess;
     Ptr6f m; Ptr6u der, out;
     for (int k = 0; k < 6; k++) { m.p[k] = metric6[k]; der.p[k] = der6[k]; out.p[k] = out6[k]; }
-    k_christoffel<<<blocks_for(n), kBlock, 0, st>>>(d, m, der, seed, out, positions, used, substep, max_depth, mode);
-    return cudaGetLastError();
+#define AMR_POINT(N, P) \
+    if (d.n == N && d.p == P) { k_christoffel<N, P><<<used * domain_blocks(d), kBlock, 0, st>>>(m, der, seed, out, positions, substep, max_depth, mode); return cudaGetLastError(); }
+    AMR_FOR_EACH_CONFIG(AMR_POINT)
+#undef AMR_POINT
+    return cudaErrorInvalidValue;
 }
 cudaError_t launch_wave_step(Dims d, const Geo& g, int corrector, const float* old_f, const uint32_t* der,
                              const uint32_t* hess, float* new_f, const uint32_t* positions, uint32_t used,
                              uint32_t substep, uint32_t max_depth, cudaStream_t st) {
-    const uint64_t n = (uint64_t)used * d.n * d.n * d.n;
-    if (n == 0) return cudaSuccess;
-    k_wave_step<<<blocks_for(n), kBlock, 0, st>>>(d, g.outer_dt, corrector, old_f, der, hess, new_f, positions, used,
-                                                  substep, max_depth);
-    return cudaGetLastError();
+    if (used == 0) return cudaSuccess;
+#define AMR_POINT(N, P) \
+    if (d.n == N && d.p == P) { k_wave_step<N, P><<<used * domain_blocks(d), kBlock, 0, st>>>(g.outer_dt, corrector, old_f, der, hess, new_f, positions, substep, max_depth); return cudaGetLastError(); }
+    AMR_FOR_EACH_CONFIG(AMR_POINT)
+#undef AMR_POINT
+    return cudaErrorInvalidValue;
 }
 cudaError_t launch_criterion(Dims d, const Geo& g, const uint32_t* der, const uint32_t* hess, float* crit,
                              const uint32_t* positions, uint32_t used, uint32_t substep, uint32_t max_depth,
                              cudaStream_t st) {
-    const uint64_t n = (uint64_t)used * d.n * d.n;
-    if (n == 0) return cudaSuccess;
-    k_criterion_columns<<<blocks_for(n), kBlock, 0, st>>>(d, g.outer_dx, der, hess, crit, positions, used, substep, max_depth);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    k_criterion_octants<<<(uint32_t)(((uint64_t)used * 8u + kBlock / 32u - 1u) / (kBlock / 32u)), kBlock, 0, st>>>(d, crit, used);
+    if (used == 0) return cudaSuccess;
+    if (d.n < 4u || (d.n >> 1) * (d.n >> 2) > kCritThreads) return cudaErrorInvalidValue;
+    k_criterion<<<used * 8u, kCritThreads, 0, st>>>(d, g.outer_dx, der, hess, crit, positions, substep, max_depth);
     return cudaGetLastError();
 }
 
