@@ -50,15 +50,11 @@ struct EvoRestrictArgs {
     float* old_f[kMaxFields];
     const float* new_f[kMaxFields];
     const int32_t* children;
-    const uint32_t* items;
-    uint32_t n_items;
-    uint32_t n, p, t;
+    const uint32_t* items;   // n_leaves slots without children, then n_parents with some
+    uint32_t n_leaves, n_parents;
+    uint32_t n;
     int nf;
-    int fgroup;   // fields per CTA: the grid's y extent is ceil(nf / fgroup)
 };
-// Fields per CTA when restricting domains with children: each covered cell costs 64 loads per field,
-// so those CTAs take few fields and many run side by side (the leaves' straight copies take all).
-constexpr int kEvoRestrictGroup = 4;
 
 // Tile features of the learned estimator and the plain criterion's indicator, per listed slot
 // (kernels_evolve.cu, k_evo_features): features [slot][3][8^3], indicator [slot].

@@ -218,36 +218,28 @@ public:
     int copy_back() override {
         int st = prepare();
         if (st) return st;
-        const uint32_t s = tree.timer(), md = (uint32_t)tree.read_max_depth();
+        const uint32_t s = tree.timer();
         if (act_cnt[s] == 0) return AMR_OK;
         EvoRestrictArgs g;
         std::memset(&g, 0, sizeof(g));
         for (int f = 0; f < nf; f++) { g.old_f[f] = old_f[f]; g.new_f[f] = new_f[f]; }
         g.children = d_children;
-        g.items = d_lists + act_off[s];
-        g.n_items = act_cnt[s];
-        g.n = dims.n; g.p = dims.p; g.t = dims.t;
+        g.items = d_lists + act_off[s];   // the leaves, then the domains with children
+        g.n = dims.n;
         g.nf = nf;
-        g.fgroup = nf;
-        (void)md;
         if (mode == AMR_MODE_PLAIN) {   // one launch per domain
             const uint32_t* base = g.items;
             for (uint32_t i = 0; i < act_cnt[s]; i++) {
                 g.items = base + i;
-                g.n_items = 1;
+                g.n_leaves = i < act_leaves[s] ? 1u : 0u;
+                g.n_parents = 1u - g.n_leaves;
                 if ((st = check(launch_evo_restrict(g, stream)))) return st;
             }
             return AMR_OK;
         }
-        // the leaves with every field of a plane per CTA, then the domains with children with
-        // kEvoRestrictGroup fields per CTA
-        g.n_items = act_leaves[s];
-        if (g.n_items && (st = check(launch_evo_restrict(g, stream)))) return st;
-        g.items = d_lists + act_off[s] + act_leaves[s];
-        g.n_items = act_cnt[s] - act_leaves[s];
-        g.fgroup = kEvoRestrictGroup;
-        if (g.n_items && (st = check(launch_evo_restrict(g, stream)))) return st;
-        return AMR_OK;
+        g.n_leaves = act_leaves[s];
+        g.n_parents = act_cnt[s] - act_leaves[s];
+        return check(launch_evo_restrict(g, stream));
     }
     int modify_nodes() override { return AMR_OK; }
     int predictor() override {

@@ -8,7 +8,7 @@
 //   k_evo_stage_wave  one RK4 stage of the wave: derivatives, right-hand side and stage update
 //   k_evo_ghost     ghost fill of a stage's state, one face-normal axis per launch (copies from
 //                   same-depth neighbours, separable tricubic interpolation from coarser ones)
-//   k_evo_restrict  restriction of children into parents (leaves: 16-byte copies)
+//   k_evo_restrict  restriction of children into parents, axis by axis (leaves: 16-byte copies)
 //   k_evo_prolong   tricubic prolongation of new domains
 #include <cmath>
 #include <type_traits>
@@ -361,82 +361,106 @@ __global__ void __launch_bounds__(256) k_evo_ghost(const __grid_constant__ EvoGh
 // centre (the corner shared by 2x2x2 child cells), by the 4-point midpoint rule (-1, 9, 9, -1)/16 along
 // each axis (child cells 2c-1 .. 2c+2, the child's ghost layer at its faces included).  The reference
 // averages the 2x2x2 block (AMR.h:961-996), a second-order rule.
-// A CTA per (slot, plane z, group of g.fgroup fields).
+//
+// One launch, three kinds of CTAs, the longest first: the covered octants' interpolation; the other cells of
+// the domains with children, a CTA per (domain, plane, kRestrictCopyFields fields); the domains without,
+// straight copies of a plane of every field.
+//
+// Interpolation: a CTA per (octant, four planes of it, F fields), axis by axis: along x from the child's rows
+// (each tap a half of an aligned pair) into shared memory, along y from there into registers, ten planes
+// that give four along z.  The sum over 64 taps of every cell was bound by its loads, 64 a cell against 12
+// here (20 instructions): 585 domains of 16^3, 73 of them with children, 151 + 306 -> 341 us (the leaves alone 148), 9 of 8^3 5 + 22 -> 5.7.
+constexpr int kRestrictCopyFields = 8;
+template <int N>
+struct RestrictShape {
+    static constexpr int T = N + 6, H = N / 2;
+    static constexpr int F = N == 8 ? 4 : 256 / (H * H);      // fields per CTA
+    static constexpr int SLABS = H / 4, PLANES = 10, ROWS = N + 2;
+    static constexpr int PITCH = N == 8 ? 6 : (N == 16 ? 12 : 24);   // floats per row: the y taps of a warp meet no bank twice
+    static constexpr int WORDS = F * PLANES * ROWS * PITCH;
+    static_assert(F * H * H <= 256 && PITCH >= H && WORDS * 4 <= 48 * 1024, "a column per thread");
+};
+template <int N>
 __global__ void __launch_bounds__(256) k_evo_restrict(const __grid_constant__ EvoRestrictArgs g) {
-    const uint32_t t = g.t, p = g.p, n = g.n, hn = n / 2;
-    const uint32_t item = blockIdx.x / t, z = blockIdx.x % t;
-    const int fb = (int)blockIdx.y * g.fgroup, fe = min(g.nf, fb + g.fgroup);   // this CTA's fields
-    if (item >= g.n_items || fb >= fe) return;
-    const uint32_t slot = g.items[item];
-    const uint64_t cells = (uint64_t)t * t * t;
-    bool leaf = true;
+    using S = RestrictShape<N>;
+    constexpr int T = S::T, P = 3, H = S::H;
+    constexpr uint64_t CELLS = (uint64_t)T * T * T;
+    const uint32_t tid = threadIdx.x;
+    uint32_t b = blockIdx.x;
+    const uint32_t groups = (uint32_t)(g.nf + S::F - 1) / S::F;
+    const uint32_t units = 8u * S::SLABS * groups;      // interpolating CTAs per domain with children
+    const uint32_t copies = T * (uint32_t)((g.nf + kRestrictCopyFields - 1) / kRestrictCopyFields);
+    if (b < g.n_parents * units) {
+        const uint32_t slot = g.items[g.n_leaves + b / units], u = b % units;
+        const uint32_t oct = u % 8u, slab = u / 8u % S::SLABS;
+        const int f0 = (int)(u / (8u * S::SLABS)) * S::F;
+        const int32_t ch = g.children[slot * 8u + oct];
+        if (ch == -1) return;
+        extern __shared__ float sx[];
+        constexpr float wa = -1.f / 16.f, wb = 9.f / 16.f;
+        auto four = [](float a, float c, float d, float e) { return fmaf(wa, e, fmaf(wb, d, fmaf(wb, c, wa * a))); };
+        // along x: child planes 8 slab - 1 .. 8 slab + 8 and rows -1 .. N of its interior
+        const uint64_t src = (uint64_t)ch * CELLS + (uint64_t)(P - 1 + 8 * slab) * T * T + (P - 1) * T + (P - 1);
+#pragma unroll 4
+        for (int e = (int)tid; e < S::F * S::PLANES * S::ROWS * H; e += 256) {
+            const int i = e % H, row = e / H % S::ROWS, z = e / (H * S::ROWS) % S::PLANES, f = e / (H * S::ROWS * S::PLANES);
+            if (f0 + f >= g.nf) break;
+            const float2* q = reinterpret_cast<const float2*>(g.new_f[f0 + f] + src + (z * T + row) * T + 2 * i);
+            const float2 l = q[0], r = q[1];
+            sx[((f * S::PLANES + z) * S::ROWS + row) * S::PITCH + i] = four(l.x, l.y, r.x, r.y);
+        }
+        __syncthreads();
+        const int x = (int)tid % H, y = (int)tid / H % H, f = (int)tid / (H * H);
+        if (f >= S::F || f0 + f >= g.nf) return;
+        float c[S::PLANES];   // along y
 #pragma unroll
-    for (int c = 0; c < 8; c++) leaf &= g.children[slot * 8u + c] == -1;
-    if (leaf) {
-        // a domain without children: plane z of every field is a straight copy, 16 bytes at a time
-        // (planes are t^2 floats, t^2 * 4 a multiple of 16, every plane 16-byte aligned)
-        const uint32_t q4 = t * t / 4u;
-        const uint64_t base4 = (slot * cells + (uint64_t)z * t * t) / 4u;
-        const uint32_t total = (uint32_t)(fe - fb) * q4;
-        constexpr uint32_t U = 4;   // loads in flight per thread before their stores
-        for (uint32_t e0 = threadIdx.x; e0 < total; e0 += U * blockDim.x) {
-            float4 v[U];
+        for (int z = 0; z < S::PLANES; z++) {
+            const float* q = sx + ((f * S::PLANES + z) * S::ROWS + 2 * y) * S::PITCH + x;
+            c[z] = four(q[0], q[S::PITCH], q[2 * S::PITCH], q[3 * S::PITCH]);
+        }
+        float* dst = g.old_f[f0 + f] + slot * CELLS + (uint64_t)(P + (oct >> 2) * H + 4 * slab) * T * T +
+                     (P + ((oct >> 1) & 1u) * H + y) * T + P + (oct & 1u) * H + x;
 #pragma unroll
-            for (uint32_t u = 0; u < U; u++) {
-                const uint32_t e = e0 + u * blockDim.x;
-                if (e < total) v[u] = reinterpret_cast<const float4*>(g.new_f[fb + (int)(e / q4)])[base4 + e % q4];
-            }
+        for (int z = 0; z < 4; z++) dst[z * T * T] = four(c[2 * z], c[2 * z + 1], c[2 * z + 2], c[2 * z + 3]);
+        return;
+    }
+    b -= g.n_parents * units;
+    if (b < g.n_parents * copies) {
+        const uint32_t slot = g.items[g.n_leaves + b / copies], z = b % copies % T;
+        const int f0 = (int)(b % copies / T) * kRestrictCopyFields;
+        for (int k = (int)tid; k < T * T; k += 256) {
+            const uint32_t x = k % T, y = k / T;
+            const uint32_t tx = (x - P) / H, ty = (y - P) / H, tz = (z - P) / H;   // unsigned wrap for ghosts
+            if (tx < 2u && ty < 2u && tz < 2u && g.children[tx + ty * 2u + tz * 4u + slot * 8u] != -1) continue;
+            const uint64_t o = slot * CELLS + (uint64_t)z * T * T + k;
+            float v[kRestrictCopyFields];   // every load before the stores (old and new are distinct buffers)
 #pragma unroll
-            for (uint32_t u = 0; u < U; u++) {
-                const uint32_t e = e0 + u * blockDim.x;
-                if (e < total) reinterpret_cast<float4*>(g.old_f[fb + (int)(e / q4)])[base4 + e % q4] = v[u];
-            }
+            for (int q = 0; q < kRestrictCopyFields; q++)
+                if (f0 + q < g.nf) v[q] = g.new_f[f0 + q][o];
+#pragma unroll
+            for (int q = 0; q < kRestrictCopyFields; q++)
+                if (f0 + q < g.nf) g.old_f[f0 + q][o] = v[q];
         }
         return;
     }
-    constexpr float w4[4] = {-1.f / 16.f, 9.f / 16.f, 9.f / 16.f, -1.f / 16.f};
-    for (uint32_t k = threadIdx.x; k < t * t; k += blockDim.x) {
-        const uint32_t x = k % t, y = k / t;
-        const uint32_t tx = (x - p) / hn, ty = (y - p) / hn, tz = (z - p) / hn;   // unsigned wrap for ghosts
-        const int32_t ch = (tx < 2u && ty < 2u && tz < 2u) ? g.children[tx + ty * 2u + tz * 4u + slot * 8u] : -1;
-        const uint64_t o = slot * cells + ((uint64_t)z * t + y) * t + x;
-        // fields in groups, every load of a group before its stores (old and new are distinct buffers)
-        constexpr int G = 8;
-        if (ch == -1) {
-            for (int f0 = fb; f0 < fe; f0 += G) {
-                float v[G];
+    b -= g.n_parents * copies;
+    // a plane of every field, 16 bytes at a time (planes are T^2 floats, T^2 * 4 a multiple of 16)
+    const uint32_t slot = g.items[b / T], z = b % T;
+    constexpr uint32_t q4 = T * T / 4;
+    const uint64_t base4 = (slot * CELLS + (uint64_t)z * T * T) / 4u;
+    const uint32_t total = (uint32_t)g.nf * q4;
+    constexpr uint32_t U = 4;   // loads in flight per thread before their stores
+    for (uint32_t e0 = tid; e0 < total; e0 += U * 256u) {
+        float4 v[U];
 #pragma unroll
-                for (int q = 0; q < G; q++)
-                    if (f0 + q < fe) v[q] = g.new_f[f0 + q][o];
-#pragma unroll
-                for (int q = 0; q < G; q++)
-                    if (f0 + q < fe) g.old_f[f0 + q][o] = v[q];
-            }
-            continue;
+        for (uint32_t u = 0; u < U; u++) {
+            const uint32_t e = e0 + u * 256u;
+            if (e < total) v[u] = reinterpret_cast<const float4*>(g.new_f[e / q4])[base4 + e % q4];
         }
-        const uint32_t cx = ((x - p) * 2u) % n + p, cy = ((y - p) * 2u) % n + p, cz = ((z - p) * 2u) % n + p;
-        const uint64_t base = (uint64_t)ch * cells + ((uint64_t)(cz - 1) * t + (cy - 1)) * t + (cx - 1);
-        constexpr int GI = 2;
-        for (int f0 = fb; f0 < fe; f0 += GI) {
-            float acc[GI];
 #pragma unroll
-            for (int q = 0; q < GI; q++) acc[q] = 0.f;
-#pragma unroll
-            for (int k2 = 0; k2 < 4; k2++)
-#pragma unroll
-                for (int k1 = 0; k1 < 4; k1++) {
-#pragma unroll
-                    for (int q = 0; q < GI; q++) {
-                        const float* v = g.new_f[min(f0 + q, fe - 1)];
-                        float row = 0.f;
-#pragma unroll
-                        for (int k0 = 0; k0 < 4; k0++) row = fmaf(w4[k0], v[base + ((uint64_t)k2 * t + k1) * t + k0], row);
-                        acc[q] = fmaf(w4[k1] * w4[k2], row, acc[q]);
-                    }
-                }
-#pragma unroll
-            for (int q = 0; q < GI; q++)
-                if (f0 + q < fe) g.old_f[f0 + q][o] = acc[q];
+        for (uint32_t u = 0; u < U; u++) {
+            const uint32_t e = e0 + u * 256u;
+            if (e < total) reinterpret_cast<float4*>(g.old_f[e / q4])[base4 + e % q4] = v[u];
         }
     }
 }
@@ -615,11 +639,24 @@ uint32_t evo_deriv_zs_candidates(uint32_t n, uint32_t* out) {
     return n == 8 || n == 16 || n == 32 ? k : 0u;
 }
 
-cudaError_t launch_evo_restrict(const EvoRestrictArgs& g, cudaStream_t st) {
-    if (g.n_items == 0) return cudaSuccess;
-    if (g.nf <= 0 || g.nf > kMaxFields || g.fgroup <= 0) return cudaErrorInvalidValue;
-    k_evo_restrict<<<dim3(g.n_items * g.t, (unsigned)((g.nf + g.fgroup - 1) / g.fgroup)), 256, 0, st>>>(g);
+template <int N>
+static cudaError_t restrict_t(const EvoRestrictArgs& g, cudaStream_t st) {
+    using S = RestrictShape<N>;
+    const uint32_t units = 8u * S::SLABS * (uint32_t)((g.nf + S::F - 1) / S::F);
+    const uint32_t copies = S::T * (uint32_t)((g.nf + kRestrictCopyFields - 1) / kRestrictCopyFields);
+    // launches over leaves alone need no shared memory
+    k_evo_restrict<N><<<g.n_parents * (units + copies) + g.n_leaves * (uint32_t)S::T, 256, g.n_parents ? S::WORDS * 4u : 0u, st>>>(g);
     return cudaGetLastError();
+}
+cudaError_t launch_evo_restrict(const EvoRestrictArgs& g, cudaStream_t st) {
+    if (g.n_leaves + g.n_parents == 0) return cudaSuccess;
+    if (g.nf <= 0 || g.nf > kMaxFields) return cudaErrorInvalidValue;
+    switch (g.n) {
+        case 8: return restrict_t<8>(g, st);
+        case 16: return restrict_t<16>(g, st);
+        case 32: return restrict_t<32>(g, st);
+        default: return cudaErrorInvalidValue;
+    }
 }
 
 template <int N, int AXIS>
