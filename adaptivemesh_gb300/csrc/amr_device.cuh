@@ -13,6 +13,14 @@
 
 namespace amr {
 
+// For kernels launched by launch_dependent (kernels.h), by every thread, before any access to global memory:
+// lets the next kernel's CTAs start to take free places, and waits until the kernel before has
+// completed and its writes are visible.
+__device__ __forceinline__ void grid_dependency() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 // ------------------------------------------------------------------ packed pairs (f32x2, sm_100+)
 // One instruction performs the same operation on two independent floats.  Each lane rounds as the
 // scalar operation does and flushes subnormals as the -ftz=true scalar code.  One difference: the

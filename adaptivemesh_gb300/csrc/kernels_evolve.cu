@@ -105,6 +105,7 @@ __global__ void __launch_bounds__(256) k_evo_stage_wave(const __grid_constant__ 
     float* buf = reinterpret_cast<float*>(smem_raw);   // u, v
     __shared__ uint64_t bar;
     const uint32_t tid = threadIdx.x;
+    grid_dependency();
     const uint32_t item = blockIdx.x / (N / ZS), slab = blockIdx.x % (N / ZS);
     if (item >= a.n_items) return;
     const uint32_t slot = a.items[item];
@@ -198,6 +199,7 @@ __global__ void __launch_bounds__(256) k_evo_ghost(const __grid_constant__ EvoGh
     using S = GhostShape<N, AXIS>;
     constexpr int P = S::P, T = S::T;
     constexpr int64_t CELLS = (int64_t)T * T * T;
+    grid_dependency();
     const uint32_t gi = (uint32_t)(g.nf + 1) / 2u, gc = (uint32_t)(g.nf + kGhostCopyFields - 1) / kGhostCopyFields;
     const bool interp = blockIdx.x < g.n_interp * gi;
     const uint32_t b = interp ? blockIdx.x : blockIdx.x - g.n_interp * gi;
@@ -386,6 +388,7 @@ __global__ void __launch_bounds__(256) k_evo_restrict(const __grid_constant__ Ev
     constexpr int T = S::T, P = 3, H = S::H;
     constexpr uint64_t CELLS = (uint64_t)T * T * T;
     const uint32_t tid = threadIdx.x;
+    grid_dependency();
     uint32_t b = blockIdx.x;
     const uint32_t groups = (uint32_t)(g.nf + S::F - 1) / S::F;
     const uint32_t units = 8u * S::SLABS * groups;      // interpolating CTAs per domain with children
@@ -603,8 +606,7 @@ static cudaError_t wave_zs(const EvoArgs& a, cudaStream_t st) {
     using S = WaveShape<N, ZS>;
     const cudaError_t e = wave_limit<N, ZS>();
     if (e != cudaSuccess || a.n_items == 0) return e;
-    k_evo_stage_wave<N, ZS><<<a.n_items * (N / ZS), S::THREADS, S::SMEM, st>>>(a);
-    return cudaGetLastError();
+    return launch_dependent(true, k_evo_stage_wave<N, ZS>, a.n_items * (N / ZS), S::THREADS, S::SMEM, st, a);
 }
 // The compiled slab depths (a.deriv_zs; 0 = the default): whole cells per thread of 256.
 template <int N>
@@ -645,8 +647,8 @@ static cudaError_t restrict_t(const EvoRestrictArgs& g, cudaStream_t st) {
     const uint32_t units = 8u * S::SLABS * (uint32_t)((g.nf + S::F - 1) / S::F);
     const uint32_t copies = S::T * (uint32_t)((g.nf + kRestrictCopyFields - 1) / kRestrictCopyFields);
     // launches over leaves alone need no shared memory
-    k_evo_restrict<N><<<g.n_parents * (units + copies) + g.n_leaves * (uint32_t)S::T, 256, g.n_parents ? S::WORDS * 4u : 0u, st>>>(g);
-    return cudaGetLastError();
+    return launch_dependent(g.nf == WAVE_NF, k_evo_restrict<N>, g.n_parents * (units + copies) + g.n_leaves * (uint32_t)S::T, 256,
+                            g.n_parents ? S::WORDS * 4u : 0u, st, g);
 }
 cudaError_t launch_evo_restrict(const EvoRestrictArgs& g, cudaStream_t st) {
     if (g.n_leaves + g.n_parents == 0) return cudaSuccess;
@@ -671,8 +673,7 @@ static cudaError_t ghost_t(const EvoGhostArgs& g, cudaStream_t st) {
     const uint32_t blocks = g.n_interp * (uint32_t)((g.nf + 1) / 2) +
                             g.n_copy * (uint32_t)((g.nf + kGhostCopyFields - 1) / kGhostCopyFields);
     // launches without an interpolating face need none of its shared memory
-    k_evo_ghost<N, AXIS><<<blocks, 256, g.n_interp ? GhostShape<N, AXIS>::SMEM : 0u, st>>>(g);
-    return cudaGetLastError();
+    return launch_dependent(g.nf == WAVE_NF, k_evo_ghost<N, AXIS>, blocks, 256, g.n_interp ? GhostShape<N, AXIS>::SMEM : 0u, st, g);
 }
 template <int N>
 static cudaError_t ghost_n(const EvoGhostArgs& g, cudaStream_t st) {

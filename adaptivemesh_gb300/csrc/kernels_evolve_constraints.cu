@@ -72,6 +72,7 @@ __global__ void __launch_bounds__(ConsShape<N, TY, TZ, R_, MINB>::CT, MINB)
         s_abort = 0;
         s_asked = 0;
     }
+    grid_dependency();
     __syncthreads();
     const uint32_t tiles = a.n_items * (uint32_t)S::TILES;
     bool ok = true;
@@ -271,6 +272,7 @@ __device__ __forceinline__ void norm_reduce(NormSum& s) {
 }
 __global__ void __launch_bounds__(256) k_evo_norms_domain(const __grid_constant__ EvoNormArgs g, double* part) {
     const uint32_t b = blockIdx.x;
+    grid_dependency();
     if (b >= g.n_items) return;
     const uint32_t slot = g.items[b], n = g.n, hn = n / 2;
     const uint32_t cells = n * n * n, quarter = cells / kEvoNormParts;
@@ -317,6 +319,7 @@ __global__ void __launch_bounds__(256) k_evo_norms_domain(const __grid_constant_
 // The parts' totals and the norms, in one CTA: thread t adds the parts t, t + 256, ... (a serial sum of
 // 264 domains' parts, five loads each, took 107 us).
 __global__ void __launch_bounds__(256) k_evo_norms_total(const double* part, uint32_t parts, double* out) {
+    grid_dependency();
     NormSum s = {};
     for (uint32_t b = threadIdx.x; b < parts; b += blockDim.x) {
         const double* p = part + (size_t)b * 5;
@@ -367,9 +370,11 @@ cudaError_t launch_evo_constraints(const EvoArgs& a, const ConsPtrs& cons, cudaS
     }
 }
 cudaError_t launch_evo_norms(const EvoNormArgs& g, double* part, double* out, cudaStream_t st) {
-    if (g.n_items) k_evo_norms_domain<<<dim3(g.n_items, kEvoNormParts), 256, 0, st>>>(g, part);
-    k_evo_norms_total<<<1, 256, 0, st>>>(part, g.n_items * kEvoNormParts, out);
-    return cudaGetLastError();
+    if (g.n_items) {
+        const cudaError_t e = launch_dependent(true, k_evo_norms_domain, dim3(g.n_items, kEvoNormParts), 256, 0, st, g, part);
+        if (e != cudaSuccess) return e;
+    }
+    return launch_dependent(true, k_evo_norms_total, 1, 256, 0, st, part, g.n_items * kEvoNormParts, out);
 }
 
 }  // namespace amr
