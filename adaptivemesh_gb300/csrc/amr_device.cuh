@@ -438,4 +438,13 @@ __device__ __forceinline__ void christoffel_cell(const uint32_t* G, const Sym& M
     }
 }
 
+// The SimpleWave Heun update's new value from v, the gradient's x component and the diagonal Hessian
+// (SimpleWave.h:7-46): v + (lap - v*gx) * dt / 2^depth; the division by a power of two is exact.
+__device__ __forceinline__ float wave_update(float v, float gx, float3 h, float outer_dt, int depth) {
+    const float visc = 0.01f;                                          // SimpleWave.h:5
+    const float lap = __fmaf_rn(h.z, visc, __fmaf_rn(h.x, visc, __fmul_rn(h.y, visc)));
+    const float upd = __fmul_rn(__fmul_rn(__fmaf_rn(-v, gx, lap), outer_dt), __uint_as_float((127u - (uint32_t)depth) << 23));
+    return __fadd_rn(v, upd);
+}
+
 }  // namespace amr

@@ -35,11 +35,11 @@ cudaError_t ensure_smem_limit(K* kernel, size_t bytes, std::atomic<uint64_t>& ma
 // A launch whose CTAs may take their places while the kernel before it on the stream drains (programmatic
 // dependent launch, also between the kernel nodes of a captured graph).  Such a kernel calls
 // grid_dependency() (amr_device.cuh) before it touches global memory: what it reads and writes is ordered
-// as in a plain launch.  early false: a plain launch, for the kernels of the BSSN evolution.  Its stage kernel
-// needs most of an SM's shared memory, and CTAs of the other kind that take their places early hold the SM's
-// split between cache and shared memory back: 9 domains of 8^3 with every launch early took 657 us a pass
-// against 523, with the last two axes of the ghost fill alone 527.  The wave's small kernels gain: 53.7
-// -> 48.4 us a pass, and the constraints' norms, 204 -> 196.
+// as in a plain launch.  early false: a plain launch, for the kernels of the BSSN evolution, which gain nothing:
+// 9 domains of 8^3 with every launch early took 657 us a pass against 523 (a kernel of fewer CTAs than SMs,
+// placed while the one before still holds most of them, shares the free ones), with the last two axes of the
+// ghost fill alone 527.  The wave's small kernels gain, 53.7 -> 49.5 us a pass, and so do the constraints'
+// norms, 204 -> 197, and the SimpleWave plugin's timestep (99.5 -> 79.9 with the two launches a substep less).
 template <class... P, class... A>
 cudaError_t launch_dependent(bool early, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
     cudaLaunchAttribute at;
@@ -75,6 +75,10 @@ struct StencilArgs {
     uint32_t n_items;
     // single-operator kinds: 1 splits the items' planes evenly over the grid (fewer items than CTAs)
     uint32_t even;
+    uint32_t early;               // launched as launch_dependent's
+    // gradient and Hessian: also the SimpleWave predictor's new value into this padded field (nullptr: no)
+    float* step_out;
+    float outer_dt;
     uint32_t substep, max_depth;
     Geo geo;
     int* err;                     // set to 1 if a bounded wait gave up
@@ -112,7 +116,7 @@ cudaError_t launch_christoffel(Dims d, float* const* metric6, uint32_t* const* d
                                cudaStream_t st);
 cudaError_t launch_wave_step(Dims d, const Geo& g, int corrector, const float* old_f, const uint32_t* der,
                              const uint32_t* hess, float* new_f, const uint32_t* positions, uint32_t used,
-                             uint32_t substep, uint32_t max_depth, cudaStream_t st);
+                             uint32_t substep, uint32_t max_depth, cudaStream_t st, bool early = false);
 cudaError_t launch_rasterise(Dims d, const float* data, const int32_t* children, uint32_t used, uint32_t width,
                              uint32_t height, float z_slice, int boxes, float* raster, cudaStream_t st);
 // Write n words into device memory with kernels that carry them as launch parameters (1 000 per
@@ -134,7 +138,7 @@ struct CopyList {
 cudaError_t launch_copy_many(const CopyList& l, cudaStream_t st);
 cudaError_t launch_criterion(Dims d, const Geo& g, const uint32_t* der, const uint32_t* hess, float* crit,
                              const uint32_t* positions, uint32_t used, uint32_t substep, uint32_t max_depth,
-                             cudaStream_t st);
+                             cudaStream_t st, bool early = false);
 
 // Restriction / prolongation / ghost fill (kernels_amr.cu).  `ncomp` components are processed in
 // one launch (component k at fields_old[k], fields_new[k]).
@@ -145,7 +149,7 @@ struct FieldSet {
 };
 cudaError_t launch_copy_new_to_old(Dims d, const FieldSet& f, const uint32_t* positions, const int32_t* children,
                                    const uint32_t* items, uint32_t n_items, uint32_t substep, uint32_t max_depth,
-                                   cudaStream_t st, bool parents_only = false);
+                                   cudaStream_t st, bool parents_only = false, bool early = false);
 cudaError_t launch_copy_to_child(Dims d, float* buf, uint32_t offset, int32_t child, int32_t parent, cudaStream_t st);
 // Prolongation of n_items new nodes at once into each of nbuf (<= 12) buffers; items holds
 // (child, parent, offset) triples in device memory, none a parent of another.
@@ -165,6 +169,6 @@ size_t ghost_scratch_floats(Dims d, uint32_t used, int ncomp);
 // value in place, in one launch without staging.
 cudaError_t launch_copy_boundaries(Dims d, const FieldSet& f, const uint64_t* boundaries, uint32_t used,
                                    uint32_t substep, uint32_t max_depth, int copy_only_new, float* scratch,
-                                   cudaStream_t st, bool sources_restricted = false);
+                                   cudaStream_t st, bool sources_restricted = false, bool early = false);
 
 }  // namespace amr

@@ -108,20 +108,14 @@ template <int N, int P>
 __global__ void k_wave_step(float outer_dt, int corrector, const float* __restrict__ old_f,
                             const uint32_t* __restrict__ der, const uint32_t* __restrict__ hess, float* new_f,
                             const uint32_t* __restrict__ positions, uint32_t substep, uint32_t max_depth) {
+    grid_dependency();
     InnerCell c;
     if (!inner_cell<N, P>(c)) return;
     const uint64_t o = c.o;
     int depth;
     if (!slot_active(positions, c.slot, substep, max_depth, &depth)) return;
-    const float visc = 0.01f;                                          // SimpleWave.h:5
-    const float gx = cf3_decode(der[o]).x;
-    const float3 h = cf3_decode(hess[o]);
-    const float lap = __fmaf_rn(h.z, visc, __fmaf_rn(h.x, visc, __fmul_rn(h.y, visc)));
-    const float v = old_f[c.padded];
-    // (lap - v*gx) * dt / 2^depth; the division by a power of two is exact
-    const float upd = __fmul_rn(__fmul_rn(__fmaf_rn(-v, gx, lap), outer_dt), __uint_as_float((127u - (uint32_t)depth) << 23));
-    if (!corrector) new_f[c.padded] = __fadd_rn(v, upd);
-    else new_f[c.padded] = __fmul_rn(__fadd_rn(new_f[c.padded], __fadd_rn(v, upd)), .5f);
+    const float w = wave_update(old_f[c.padded], cf3_decode(der[o]).x, cf3_decode(hess[o]), outer_dt, depth);
+    new_f[c.padded] = corrector ? __fmul_rn(__fadd_rn(new_f[c.padded], w), .5f) : w;
 }
 
 // ---------------------------------------------------------------- refinement criterion, SimpleWave.h:91-139
@@ -140,6 +134,7 @@ __global__ void __launch_bounds__(kCritThreads) k_criterion(Dims d, float outer_
                                                            const uint32_t* __restrict__ positions, uint32_t substep,
                                                            uint32_t max_depth) {
     const uint32_t n = d.n, h = n >> 1, q = n >> 2, columns = q * h;
+    grid_dependency();
     const uint32_t oct = blockIdx.x & 7u, node = blockIdx.x >> 3;
     const uint32_t xb = oct & 1u, yb = (oct >> 1) & 1u, zi = 2u * node + (oct >> 2);
     const uint64_t base = ((uint64_t)zi * h + yb * q) * n + xb * h;
@@ -268,21 +263,23 @@ cudaError_t launch_christoffel(Dims d, float* const* metric6, uint32_t* const* d
 }
 cudaError_t launch_wave_step(Dims d, const Geo& g, int corrector, const float* old_f, const uint32_t* der,
                              const uint32_t* hess, float* new_f, const uint32_t* positions, uint32_t used,
-                             uint32_t substep, uint32_t max_depth, cudaStream_t st) {
+                             uint32_t substep, uint32_t max_depth, cudaStream_t st, bool early) {
     if (used == 0) return cudaSuccess;
 #define AMR_POINT(N, P) \
-    if (d.n == N && d.p == P) { k_wave_step<N, P><<<used * domain_blocks(d), kBlock, 0, st>>>(g.outer_dt, corrector, old_f, der, hess, new_f, positions, substep, max_depth); return cudaGetLastError(); }
+    if (d.n == N && d.p == P) { \
+        return launch_dependent(early, k_wave_step<N, P>, used * domain_blocks(d), kBlock, 0, st, g.outer_dt, corrector, old_f, der,    \
+                                hess, new_f, positions, substep, max_depth); }
     AMR_FOR_EACH_CONFIG(AMR_POINT)
 #undef AMR_POINT
     return cudaErrorInvalidValue;
 }
 cudaError_t launch_criterion(Dims d, const Geo& g, const uint32_t* der, const uint32_t* hess, float* crit,
                              const uint32_t* positions, uint32_t used, uint32_t substep, uint32_t max_depth,
-                             cudaStream_t st) {
+                             cudaStream_t st, bool early) {
     if (used == 0) return cudaSuccess;
     if (d.n < 4u || (d.n >> 1) * (d.n >> 2) > kCritThreads) return cudaErrorInvalidValue;
-    k_criterion<<<used * 8u, kCritThreads, 0, st>>>(d, g.outer_dx, der, hess, crit, positions, substep, max_depth);
-    return cudaGetLastError();
+    return launch_dependent(early, k_criterion, used * 8u, kCritThreads, 0, st, d, g.outer_dx, der, hess, crit, positions, substep,
+                            max_depth);
 }
 
 cudaError_t launch_rasterise(Dims d, const float* data, const int32_t* children, uint32_t used, uint32_t width,

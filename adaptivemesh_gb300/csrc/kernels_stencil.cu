@@ -232,6 +232,7 @@ __global__ void __launch_bounds__(N * N, N * N <= 256 ? 2 : 1) k_stencil(const _
         mbar_fence_init();
         s_abort = 0;
     }
+    grid_dependency();
     __syncthreads();
 
     // per-cell generators: the part that depends on (seed, x, y) only, once per thread
@@ -361,6 +362,9 @@ __global__ void __launch_bounds__(N * N, N * N <= 256 ? 2 : 1) k_stencil(const _
                                                              make_float2(__fmul_rn(hz, dx2), __fmul_rn(gz, dx1)), nx, ny, nz);
                         a.hdiag[o] = w.w0;
                         a.grad[0][o] = w.w1;
+                        if (a.step_out)
+                            a.step_out[(size_t)node * T * PLANE + (size_t)(z + P) * PLANE + c0] =
+                                wave_update(pl(P)[c0], cf3_decode(w.w1).x, cf3_decode(w.w0), a.outer_dt, depth);
                     } else {
                         a.grad[0][o] = cf3_encode(__fmul_rn(gx, dx1), __fmul_rn(gy, dx1), __fmul_rn(gz, dx1), rng);
                     }
@@ -656,7 +660,7 @@ template <int N, int P, int KIND>
 cudaError_t launch_stencil_t(const StencilArgs& a, uint32_t grid, cudaStream_t st) {
     using S = StencilShape<N, P, KIND>;
     static std::atomic<uint64_t> configured{0};
-    void (*kernel)(const StencilArgs);
+    void (*kernel)(StencilArgs);
     if constexpr (KIND == SK_BSSN) kernel = k_stencil_bssn<N, P>;
     else kernel = k_stencil<N, P, KIND>;
     const cudaError_t e = ensure_smem_limit(kernel, S::SMEM, configured);
@@ -669,12 +673,10 @@ cudaError_t launch_stencil_t(const StencilArgs& a, uint32_t grid, cudaStream_t s
         if (a.n_items > 0u && grid > a.n_items) {
             StencilArgs b = a;
             b.even = 1;
-            kernel<<<grid, S::THREADS, S::SMEM, st>>>(b);
-            return cudaGetLastError();
+            return launch_dependent(a.early != 0u, kernel, grid, S::THREADS, S::SMEM, st, b);
         }
     }
-    kernel<<<grid, S::THREADS, S::SMEM, st>>>(a);
-    return cudaGetLastError();
+    return launch_dependent(KIND != SK_BSSN && a.early != 0u, kernel, grid, S::THREADS, S::SMEM, st, a);
 }
 
 #define AMR_STENCIL_INSTANCES(N, P)                                                                      \

@@ -385,16 +385,16 @@ public:
         std::memset(&f, 0, sizeof(f));
         f.old_f[0] = old_f; f.new_f[0] = new_f; f.ncomp = 1;
         return check(launch_copy_new_to_old(dims, f, d_positions, d_children, nullptr, tree.curr_used_slots(), tree.timer(),
-                                            (uint32_t)tree.read_max_depth(), stream));
+                                            (uint32_t)tree.read_max_depth(), stream, false, true));
     }
     // amr_criterion (SimpleWave.h:142-187) followed by the triage of modify_nodes (:228-248).
     int modify_nodes() override {
+        grown = false;
         int st = sync_octree();
         if (st) return st;
         const uint32_t used = tree.curr_used_slots(), n = dims.n;
         if ((st = check(launch_criterion(dims, geo, derivs, hess, crit, d_positions, used, tree.timer(),
-                                         (uint32_t)tree.read_max_depth(), stream)))) return st;
-        launches++;
+                                         (uint32_t)tree.read_max_depth(), stream, true)))) return st;
         cudaError_t e = cudaMemcpyAsync(crit_host, crit, sizeof(float) * used * n * n, cudaMemcpyDeviceToHost, stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
         if (e != cudaSuccess) return cuda_status(e);
@@ -436,7 +436,10 @@ public:
         }
         for (uint32_t i = 0, s = used * 8u; i < s; i++) {
             const float weight = ay * 3.f / (1.f - urgency);
-            if (c[i] > weight && tree.children()[i] == -1) tree.add_node((int32_t)(i >> 3u), (int32_t)(i & 7u));
+            if (c[i] > weight && tree.children()[i] == -1) {
+                tree.add_node((int32_t)(i >> 3u), (int32_t)(i & 7u));
+                grown = true;
+            }
         }
         tree.end_batch();
         return take_ctor_status();
@@ -444,9 +447,7 @@ public:
     int predictor() override {                                   // SimpleWave.h:249-255
         int st = sync_octree();
         if (st) return st;
-        if ((st = differentiate(old_f))) return st;
-        return check(launch_wave_step(dims, geo, 0, old_f, derivs, hess, new_f, d_positions, tree.curr_used_slots(),
-                                      tree.timer(), (uint32_t)tree.read_max_depth(), stream));
+        return differentiate(old_f, new_f);   // the stencil writes the predicted values too
     }
     int copy_bounds() override {                                 // SimpleWave.h:256-260
         int st = sync_octree();
@@ -454,17 +455,20 @@ public:
         FieldSet f;
         std::memset(&f, 0, sizeof(f));
         f.old_f[0] = old_f; f.new_f[0] = new_f; f.ncomp = 1;
+        // in place where the substep's restriction still holds: the predictor writes interiors alone, but new
+        // domains' old and new fields are interpolated separately
+        const bool restricted = in_timestep && !grown;
         st = check(launch_copy_boundaries(dims, f, d_boundaries, tree.curr_used_slots(), tree.timer(),
-                                          (uint32_t)tree.read_max_depth(), 1, ghost_stage, stream));
-        if (!st) launches++;
+                                          (uint32_t)tree.read_max_depth(), 1, ghost_stage, stream, restricted, true));
+        if (!st && !restricted) launches++;
         return st;
     }
     int corrector() override {                                   // SimpleWave.h:261-267
         int st = sync_octree();
         if (st) return st;
-        if ((st = differentiate(new_f))) return st;
+        if ((st = differentiate(new_f, nullptr))) return st;   // its planes are read by other CTAs: no update in place
         return check(launch_wave_step(dims, geo, 1, old_f, derivs, hess, new_f, d_positions, tree.curr_used_slots(),
-                                      tree.timer(), (uint32_t)tree.read_max_depth(), stream));
+                                      tree.timer(), (uint32_t)tree.read_max_depth(), stream, true));
     }
     int buffer(int which, int comp, void** ptr, uint64_t* count) override {
         if (comp != 0) return AMR_ERR_INVALID;
@@ -480,7 +484,7 @@ public:
     }
 
 private:
-    int differentiate(const float* field) {
+    int differentiate(const float* field, float* step_out) {
         StencilArgs a;
         std::memset(&a, 0, sizeof(a));
         a.positions = d_positions;
@@ -493,6 +497,9 @@ private:
         a.grad[0] = derivs;
         a.hdiag = hess;
         a.seed_d[0] = next_seed();
+        a.early = 1;
+        a.step_out = step_out;
+        a.outer_dt = geo.outer_dt;
         time_begin();
         const int st = check(launch_stencil(cfg, SK_GRAD_HESS, a, stencil_grid(cfg, SK_GRAD_HESS, a.n_items), stream));
         time_end();
@@ -504,6 +511,7 @@ private:
     uint32_t* hess = nullptr;
     float* crit = nullptr;
     float* crit_host = nullptr;
+    bool grown = false;   // domains were added in this substep
 };
 
 }  // namespace amr
