@@ -54,9 +54,12 @@ constexpr size_t kOffW1 = 0, kOffB1 = kOffW1 + kK1 * kC1, kOffW2 = kOffB1 + kC1,
 //
 // The operands are functors: thread t stages row t of A, eight K values (16 bytes) at a time, so that
 // the convolutions gather their receptive fields straight from the activations (no im2col matrix in
-// memory, 98 KB a tile for conv1 before) and a row's geometry is computed once; a block's values are
-// loaded while the block before it is multiplied.  The epilogue takes the bias, the ReLU and its
-// backward form, which were passes of their own.
+// memory, 98 KB a tile for conv1 before) and a row's geometry is computed once.  G blocks are staged at a
+// time, all their loads in flight together, and the next G are loaded while they are multiplied: a block's
+// load latency, paid 16 times, was most of fc1's time (one or two CTAs; 36 us for 256 tiles, 22 with four).  A
+// convolution's K is a template parameter and its loop unrolled, so that channel, tap and offset of every
+// gathered value are constants (conv2 21.6 -> 17.7 us, conv1 18.2 -> 9.5, 256 tiles).  The epilogue takes the
+// bias, the ReLU and its backward form, which were passes of their own.
 constexpr int kGemmM = 128, kGemmK = 64;
 
 struct __align__(16) Chunk {   // eight consecutive K values of one row
@@ -68,13 +71,12 @@ __device__ __forceinline__ Chunk zero_chunk() {
     return c;
 }
 
-template <int NT, class A, class B, class Epilogue>
-__global__ void __launch_bounds__(128) k_gemm_bf16(const A fa, const B fb, const Epilogue epi, int K, int* err) {
+template <int NT, int KC, int G, class A, class B, class Epilogue>
+__global__ void __launch_bounds__(128) k_gemm_bf16(const A fa, const B fb, const Epilogue epi, int k_runtime, int* err) {
     static_assert(NT == 16 || NT == 32, "M = 128 tiles take N in multiples of 16; 32 TMEM columns");
-    constexpr int MT = kGemmM, KT = kGemmK, BC = NT * KT / 8 / 128;   // chunks of B per thread
+    constexpr int MT = kGemmM, KT = kGemmK, BC = NT * KT / 8 / 128;   // chunks of B per thread and block
     constexpr uint32_t LBO = 128u, SBO = (KT / 8) * 128u;   // bytes between core matrices along K / M
-    __shared__ __align__(1024) bf16 As[MT * KT];
-    __shared__ __align__(1024) bf16 Bs[NT * KT];
+    extern __shared__ __align__(1024) unsigned char smem_raw[];   // G blocks of A, then of B
     __shared__ __align__(8) uint64_t bar;
     __shared__ uint32_t s_tmem;
     __shared__ int s_fail;
@@ -94,45 +96,74 @@ __global__ void __launch_bounds__(128) k_gemm_bf16(const A fa, const B fb, const
     constexpr uint32_t idesc = umma_idesc_bf16_f32(MT, NT);
     // chunk k of row r: core matrix (r / 8, k) of eight 16-byte rows, row r % 8
     auto at = [](int r, int k) { return (r >> 3) * (KT / 8) * 8 + k * 8 + (r & 7); };
-    Chunk* const a16 = reinterpret_cast<Chunk*>(As);
-    Chunk* const b16 = reinterpret_cast<Chunk*>(Bs);
+    Chunk* const a16 = reinterpret_cast<Chunk*>(smem_raw);
+    Chunk* const b16 = a16 + G * MT * KT / 8;
     uint32_t phase = 0;
-    const int nkb = (K + KT - 1) / KT;
-    const auto row = fa.row(m);
-    Chunk ca[KT / 8], cb[BC];
-    auto load = [&](int k0) {
+    const int nkb = ((KC ? KC : k_runtime) + KT - 1) / KT;
+    // Thread t stages row t where a row's geometry costs; where its K values are contiguous, a warp takes eight
+    // rows and four chunks of each, 64 bytes of a line instead of 16 (and no two rows' banks meet).
+    const auto row = fa.row(A::kByRow ? 0 : m);
+    auto row_of = [&](int i) { return A::kByRow ? 8 * ((warp * (KT / 8) + i) / 2) + (tid & 7) : tid; };
+    auto chunk_of = [&](int i) { return A::kByRow ? 4 * (i & 1) + (tid % 32) / 8 : i; };
+    Chunk ca[G][KT / 8], cb[G][BC];
+    auto load = [&](int kb) {   // blocks kb .. kb + G - 1, as far as there are
 #pragma unroll
-        for (int k = 0; k < KT / 8; k++) ca[k] = fa(row, k0 + 8 * k);
+        for (int j = 0; j < G; j++) {
+            if (kb + j >= nkb) break;
+            const int k0 = (kb + j) * KT;
 #pragma unroll
-        for (int i = 0; i < BC; i++) {
-            const int e = tid + 128 * i;
-            cb[i] = fb(n0 + e % NT, k0 + 8 * (e / NT));
+            for (int i = 0; i < KT / 8; i++) {
+                if constexpr (A::kByRow) ca[j][i] = fa(blockIdx.x * MT + row_of(i), k0 + 8 * chunk_of(i));
+                else ca[j][i] = fa(row, k0 + 8 * i);
+            }
+#pragma unroll
+            for (int i = 0; i < BC; i++) {
+                const int e = tid + 128 * i;
+                cb[j][i] = fb(n0 + e % NT, k0 + 8 * (e / NT));
+            }
         }
     };
-    load(0);
-    for (int kb = 0; kb < nkb; kb++) {
+    auto group = [&](int kb) {
 #pragma unroll
-        for (int k = 0; k < KT / 8; k++) a16[at(tid, k)] = ca[k];
+        for (int j = 0; j < G; j++) {
+            if (kb + j >= nkb) break;
 #pragma unroll
-        for (int i = 0; i < BC; i++) b16[at((tid + 128 * i) % NT, (tid + 128 * i) / NT)] = cb[i];
+            for (int i = 0; i < KT / 8; i++) a16[j * MT * KT / 8 + at(row_of(i), chunk_of(i))] = ca[j][i];
+#pragma unroll
+            for (int i = 0; i < BC; i++) b16[j * NT * KT / 8 + at((tid + 128 * i) % NT, (tid + 128 * i) / NT)] = cb[j][i];
+        }
         fence_proxy_async_smem();   // these writes, visible to the tensor core
         __syncthreads();
         if (tid == 0) {
             tc_fence_after_sync();
-            const uint32_t a0 = smem_addr(As), b0 = smem_addr(Bs);
+            const uint32_t a0 = smem_addr(a16), b0 = smem_addr(b16);
 #pragma unroll
-            for (int kk = 0; kk < KT / 16; kk++)   // K = 16 per MMA: two core matrices along K
-                umma_bf16(tmem, umma_desc_kmajor(a0 + kk * 2 * LBO, LBO, SBO), umma_desc_kmajor(b0 + kk * 2 * LBO, LBO, SBO),
-                          idesc, kb > 0 || kk > 0);
+            for (int j = 0; j < G; j++) {
+                if (kb + j >= nkb) break;
+#pragma unroll
+                for (int kk = 0; kk < KT / 16; kk++)   // K = 16 per MMA: two core matrices along K
+                    umma_bf16(tmem, umma_desc_kmajor(a0 + j * MT * KT * 2 + kk * 2 * LBO, LBO, SBO),
+                              umma_desc_kmajor(b0 + j * NT * KT * 2 + kk * 2 * LBO, LBO, SBO), idesc, kb > 0 || j > 0 || kk > 0);
+            }
             umma_commit(&bar);
         }
-        if (kb + 1 < nkb) load((kb + 1) * KT);
-        // the block's MMAs have read As and Bs once the barrier's phase completes
+        load(kb + G);
+        // the group's MMAs have read its operands once the barrier's phase completes
         const bool ok = mbar_wait(&bar, phase);
         phase ^= 1u;
         if (!ok) s_fail = 1;
         __syncthreads();
-        if (s_fail) break;
+        return s_fail == 0;
+    };
+    load(0);
+    if constexpr (KC != 0 && KC <= 8 * KT) {
+#pragma unroll
+        for (int kb = 0; kb < nkb; kb += G)
+            if (!group(kb)) break;
+    } else {
+#pragma unroll 1
+        for (int kb = 0; kb < nkb; kb += G)
+            if (!group(kb)) break;
     }
     if (!s_fail) {
         tc_fence_after_sync();
@@ -143,7 +174,7 @@ __global__ void __launch_bounds__(128) k_gemm_bf16(const A fa, const B fb, const
         epi(m, n0, v);
     } else if (tid == 0) {
         atomicExch(err, 1);
-        mbar_wait(&bar, phase ^ 1u);   // the MMAs of the block whose wait gave up
+        mbar_wait(&bar, phase ^ 1u);   // the MMAs of the group whose wait gave up
     }
     tc_fence_before_sync();
     __syncthreads();
@@ -153,14 +184,18 @@ __global__ void __launch_bounds__(128) k_gemm_bf16(const A fa, const B fb, const
     }
 }
 
-// C (rows x cols) over all of K
-template <int NT, class A, class B, class Epilogue>
+// C (rows x cols) over all of K; KC: K where it is known, G: K blocks staged at a time
+template <int NT, int KC, int G, class A, class B, class Epilogue>
 cudaError_t gemm(const A& fa, const B& fb, const Epilogue& epi, int rows, int cols, int K, cudaStream_t st) {
     if (rows <= 0 || K <= 0) return cudaSuccess;
     int* err = device_error_flag();
     if (!err) return cudaErrorMemoryAllocation;
-    k_gemm_bf16<NT><<<dim3((unsigned)((rows + kGemmM - 1) / kGemmM), (unsigned)((cols + NT - 1) / NT)), 128, 0, st>>>(fa, fb, epi,
-                                                                                                                 K, err);
+    constexpr size_t smem = (size_t)G * (kGemmM + NT) * kGemmK * sizeof(bf16);
+    static std::atomic<uint64_t> configured{0};
+    const cudaError_t e = ensure_smem_limit(k_gemm_bf16<NT, KC, G, A, B, Epilogue>, smem, configured);
+    if (e != cudaSuccess) return e;
+    k_gemm_bf16<NT, KC, G><<<dim3((unsigned)((rows + kGemmM - 1) / kGemmM), (unsigned)((cols + NT - 1) / NT)), 128, smem, st>>>(
+        fa, fb, epi, K, err);
     return cudaGetLastError();
 }
 
@@ -174,8 +209,8 @@ cudaError_t gemm(const A& fa, const B& fb, const Epilogue& epi, int rows, int co
 // conv1's 64 tiles, 50 ns each, 102 us, whatever few of a 128 x 16 x 16 MMA's rows are used (ranges of K
 // summed afterwards took 12 us and changed the last bits of the gradients).
 //
-// One Adam step of 64 tiles, GB300: 2 730 -> 260 us, 27 -> 13 launches, every bit as before; forward
-// pass of 256 tiles 330 -> 80 us.
+// One Adam step of 64 tiles, GB300: 2 730 -> 244 us, 27 -> 13 launches, every bit as before; forward
+// pass of 256 tiles 330 -> 52 us.
 constexpr int kSlabRows = 8;
 constexpr int kSlabA = kSlabRows * kGemmK * 2, kSlabB = 16 * kGemmK * 2;   // bytes per K block
 
@@ -290,6 +325,7 @@ __global__ void __launch_bounds__(64) k_stream_gemm(const StreamGemm g1, const S
 // ------------------------------------------------------------------ the GEMMs' operands
 // conv1's receptive fields: row = (tile, position), K = channel * 27 + tap, from the features
 struct Conv1A {
+    static constexpr bool kByRow = false;
     const float* x;
     int rows;
     struct Row { const float* p; uint32_t taps; };   // the position's cell in channel 0, the taps inside the tile
@@ -324,11 +360,13 @@ struct WeightB {
     __device__ Chunk operator()(int n, int k) const {
         Chunk c;
 #pragma unroll
-        for (int i = 0; i < 8; i++) c.v[i] = k + i < KREAL ? w[(k + i) * COLS + n] : __float2bfloat16_rn(0.f);
+        for (int i = 0; i < 8; i++)   // (whole blocks of K need no test, which would part the loads)
+            c.v[i] = KREAL % kGemmK == 0 || k + i < KREAL ? w[(k + i) * COLS + n] : __float2bfloat16_rn(0.f);
         return c;
     }
 };
 struct Conv2A {
+    static constexpr bool kByRow = false;
     const bf16* h1;   // [tile][512][16]
     int rows;
     struct Row { const bf16* p; uint32_t taps; };
@@ -358,14 +396,19 @@ struct Conv2A {
 // Rows of a matrix whose K = KREAL values are contiguous: [row][KREAL]
 template <int KREAL>
 struct RowsA {
+    static constexpr bool kByRow = true;
     const bf16* p;
     int rows;
-    struct Row { const bf16* p; };
-    __device__ Row row(int m) const { return Row{m < rows ? p + (int64_t)m * KREAL : nullptr}; }
-    __device__ Chunk operator()(const Row& r, int k) const {
-        return r.p && k < KREAL ? *reinterpret_cast<const Chunk*>(r.p + k) : zero_chunk();
+    struct Row { const bf16* p; bool ok; };
+    __device__ Row row(int m) const { return Row{p + (int64_t)(m < rows ? m : 0) * KREAL, m < rows}; }
+    __device__ Chunk operator()(const Row& r, int k) const {   // loaded in any case: a branch would part the loads
+        const uint4 c = *reinterpret_cast<const uint4*>(r.p + (KREAL % kGemmK == 0 || k < KREAL ? k : 0));
+        const bool ok = r.ok && (KREAL % kGemmK == 0 || k < KREAL);
+        Chunk z;
+        *reinterpret_cast<uint4*>(&z) = make_uint4(ok ? c.x : 0u, ok ? c.y : 0u, ok ? c.z : 0u, ok ? c.w : 0u);
+        return z;
     }
-    __device__ Chunk operator()(int n, int k) const { return (*this)(row(n), k); }
+    __device__ Chunk operator()(int n, int k) const { return (*this)(row(n), k); }   // row n: of A by rows, or of B
 };
 // The transposed receptive fields for the weight gradients: row = K index of the forward pass,
 // K = (tile, position)
@@ -409,6 +452,7 @@ struct Conv2At {
 // Rows of a [K][cols] matrix read down its columns (H2 and the back-propagated gradients)
 template <int COLS>
 struct ColumnsT {
+    static constexpr bool kByRow = false;
     const bf16* p;
     int K;
     struct Row { const bf16* p; };
@@ -728,13 +772,13 @@ struct Estimator {
         const bf16* W2 = wb + kK1 * kC1;
         const bf16* W3 = wb + kK1 * kC1 + kK2 * kC2;
         const int r1 = B * kP1, r2 = B * kP2;
-        cudaError_t e = gemm<16>(Conv1A{x, r1}, WeightB<kC1, kK1>{W1}, BiasRelu<16>{params + kOffB1, target ? z1 : nullptr, h1, r1},
+        cudaError_t e = gemm<16, kK1, 2>(Conv1A{x, r1}, WeightB<kC1, kK1>{W1}, BiasRelu<16>{params + kOffB1, target ? z1 : nullptr, h1, r1},
                                  r1, kC1, kK1, stream);
         if (e == cudaSuccess)
-            e = gemm<16>(Conv2A{h1, r2}, WeightB<kC2, kK2>{W2}, BiasRelu<16>{params + kOffB2, target ? z2 : nullptr, h2, r2}, r2, kC2,
+            e = gemm<16, kK2, 4>(Conv2A{h1, r2}, WeightB<kC2, kK2>{W2}, BiasRelu<16>{params + kOffB2, target ? z2 : nullptr, h2, r2}, r2, kC2,
                          kK2, stream);
         if (e == cudaSuccess)
-            e = gemm<32>(RowsA<kK3>{h2, B}, WeightB<kF, kK3>{W3}, BiasRelu<32>{params + kOffB3, z3, h3, B}, B, kF, kK3, stream);
+            e = gemm<32, kK3, 4>(RowsA<kK3>{h2, B}, WeightB<kF, kK3>{W3}, BiasRelu<32>{params + kOffB3, z3, h3, B}, B, kF, kK3, stream);
         if (e != cudaSuccess) return e;
         k_fc2<<<(unsigned)((B + 3) / 4), 128, 0, stream>>>(h3, params + kOffW4, params + kOffB4, B, pred, target, dout, sq, z3, dz3,
                                                            dz3b);
@@ -746,12 +790,12 @@ struct Estimator {
         const bf16* W3 = wb + kK1 * kC1 + kK2 * kC2;
         const int k1 = B * kP1, k2 = B * kP2;
         // dW3 = H2^T dZ3, dH2 = dZ3 W3^T through conv2's ReLU
-        cudaError_t e = gemm<32>(ColumnsT<kK3>{h2, B}, ColumnsT<kF>{dz3b, B}, Store<32, kF>{grads + kOffW3, kK3}, kK3, kF, B, stream);
+        cudaError_t e = gemm<32, 0, 1>(ColumnsT<kK3>{h2, B}, ColumnsT<kF>{dz3b, B}, Store<32, kF>{grads + kOffW3, kK3}, kK3, kF, B, stream);
         if (e == cudaSuccess)
-            e = gemm<32>(RowsA<kF>{dz3b, B}, RowsA<kF>{W3, kK3}, ReluBack<32, kK3>{z2, dz2, dz2b, B}, B, kK3, kF, stream);
+            e = gemm<32, kF, 1>(RowsA<kF>{dz3b, B}, RowsA<kF>{W3, kK3}, ReluBack<32, kK3>{z2, dz2, dz2b, B}, B, kK3, kF, stream);
         // dA2 = dY2 W2^T, then col2im through conv1's ReLU
         if (e == cudaSuccess)
-            e = gemm<32>(RowsA<kC2>{dz2b, k2}, RowsA<kC2>{W2, kK2}, Store<32, kK2>{da2, k2}, k2, kK2, kC2, stream);
+            e = gemm<32, kC2, 1>(RowsA<kC2>{dz2b, k2}, RowsA<kC2>{W2, kK2}, Store<32, kK2>{da2, k2}, k2, kK2, kC2, stream);
         if (e != cudaSuccess) return e;
         k_col2im2<<<blocks((int64_t)B * kP1 * kC1), 256, 0, stream>>>(da2, z1, B, dz1, dz1b);
         // dW1 = A1^T dY1 (rows 81..95 of A1 are zero, so their gradient is too) and dW2 = A2^T dY2

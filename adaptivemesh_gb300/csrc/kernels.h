@@ -146,10 +146,11 @@ struct FieldSet {
     float* old_f[6];
     float* new_f[6];
     int ncomp;
+    int early;   // launched as launch_dependent's
 };
 cudaError_t launch_copy_new_to_old(Dims d, const FieldSet& f, const uint32_t* positions, const int32_t* children,
                                    const uint32_t* items, uint32_t n_items, uint32_t substep, uint32_t max_depth,
-                                   cudaStream_t st, bool parents_only = false, bool early = false);
+                                   cudaStream_t st, bool parents_only = false);
 cudaError_t launch_copy_to_child(Dims d, float* buf, uint32_t offset, int32_t child, int32_t parent, cudaStream_t st);
 // Prolongation of n_items new nodes at once into each of nbuf (<= 12) buffers; items holds
 // (child, parent, offset) triples in device memory, none a parent of another.
@@ -169,6 +170,6 @@ size_t ghost_scratch_floats(Dims d, uint32_t used, int ncomp);
 // value in place, in one launch without staging.
 cudaError_t launch_copy_boundaries(Dims d, const FieldSet& f, const uint64_t* boundaries, uint32_t used,
                                    uint32_t substep, uint32_t max_depth, int copy_only_new, float* scratch,
-                                   cudaStream_t st, bool sources_restricted = false, bool early = false);
+                                   cudaStream_t st, bool sources_restricted = false);
 
 }  // namespace amr

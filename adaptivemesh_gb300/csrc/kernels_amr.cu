@@ -30,7 +30,7 @@ __global__ void __launch_bounds__(kBlock) k_copy_new_to_old(const __grid_constan
                                                         uint32_t max_depth) {
     constexpr uint32_t T = N + 2 * P, CELLS = T * T * T, H = N / 2;
     static_assert(CELLS % 4 == 0, "padded domains are whole 16-byte vectors");
-    grid_dependency();
+    if (f.early) grid_dependency();
     const uint32_t slot = items ? items[blockIdx.x] : blockIdx.x;
     const int depth = pos_depth(positions[slot]);
     if (depth == -1 || !active_depth(substep, (uint32_t)depth, max_depth)) return;
@@ -242,7 +242,7 @@ __global__ void __launch_bounds__(kBlock, GhostBox<N, P>::MIN_CTAS) k_ghost_face
     extern __shared__ float sbox[];
     __shared__ uint32_t s_off[3][T];   // per axis and written coordinate: box-relative source index
     __shared__ float s_r[3][T];        // and offset from it
-    grid_dependency();
+    if (f.early) grid_dependency();
     const uint32_t slot = blockIdx.x / 6u, face = blockIdx.x - slot * 6u;
     const uint64_t bd = bds[(size_t)slot * 6u + face];
     const GhostJob j = ghost_job(bd, substep, max_depth);
@@ -451,7 +451,7 @@ __global__ void __launch_bounds__(256) k_ghost_commit(const __grid_constant__ Fi
 // ---------------------------------------------------------------- launchers
 cudaError_t launch_copy_new_to_old(Dims d, const FieldSet& f, const uint32_t* positions, const int32_t* children,
                                    const uint32_t* items, uint32_t n_items, uint32_t substep, uint32_t max_depth,
-                                   cudaStream_t st, bool parents_only, bool early) {
+                                   cudaStream_t st, bool parents_only) {
     if (n_items == 0 || f.ncomp == 0) return cudaSuccess;
     // few domains: more slabs per domain, up to eight CTAs per SM in all, as many as an SM holds (a domain
     // with children gathers 8 values a cell, 32 cells a thread in 4 slabs: 49 domains of 28^3, 8 of them
@@ -464,7 +464,7 @@ cudaError_t launch_copy_new_to_old(Dims d, const FieldSet& f, const uint32_t* po
     while (slabs < 64u && per_slab * slabs * 2u <= 8u * (uint64_t)(sms > 0 ? sms : 1)) slabs *= 2u;
     const dim3 grid(n_items, (uint32_t)f.ncomp, slabs);
 #define AMR_RESTRICT(N, P) \
-    if (d.n == N && d.p == P) return launch_dependent(early, k_copy_new_to_old<N, P>, grid, kBlock, 0, st, f, positions, children, items, substep, max_depth);
+    if (d.n == N && d.p == P) return launch_dependent(f.early != 0, k_copy_new_to_old<N, P>, grid, kBlock, 0, st, f, positions, children, items, substep, max_depth);
     AMR_FOR_EACH_CONFIG(AMR_RESTRICT)
 #undef AMR_RESTRICT
     return cudaErrorInvalidValue;
@@ -494,7 +494,7 @@ size_t ghost_scratch_floats(Dims d, uint32_t used, int ncomp) {
 }
 cudaError_t launch_copy_boundaries(Dims d, const FieldSet& f, const uint64_t* boundaries, uint32_t used,
                                    uint32_t substep, uint32_t max_depth, int copy_only_new, float* scratch,
-                                   cudaStream_t st, bool sources_restricted, bool early) {
+                                   cudaStream_t st, bool sources_restricted) {
     const int in_place = copy_only_new && sources_restricted ? 1 : 0;
 #define AMR_GHOST(N, P)                                                                                     \
     if (d.n == N && d.p == P) {                                                                             \
@@ -502,7 +502,7 @@ cudaError_t launch_copy_boundaries(Dims d, const FieldSet& f, const uint64_t* bo
         if (const cudaError_t e0 = ensure_smem_limit(k_ghost_face<N, P>, GhostBox<N, P>::SMEM, configured))   \
             return e0;                                                                                      \
         if (used == 0 || f.ncomp == 0) return cudaSuccess;                                                  \
-        cudaError_t e = launch_dependent(early, k_ghost_face<N, P>, used * 6u, kBlock, GhostBox<N, P>::SMEM, st, f, \
+        cudaError_t e = launch_dependent(f.early != 0, k_ghost_face<N, P>, used * 6u, kBlock, GhostBox<N, P>::SMEM, st, f, \
                                          boundaries, used, substep, max_depth, copy_only_new, in_place, scratch); \
         if (e != cudaSuccess || in_place) return e;                                                         \
         k_ghost_commit<N, P><<<blocks_for((uint64_t)used * 3u * N * N), kBlock, 0, st>>>(                   \

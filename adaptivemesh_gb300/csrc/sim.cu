@@ -383,9 +383,9 @@ public:
         if (st) return st;
         FieldSet f;
         std::memset(&f, 0, sizeof(f));
-        f.old_f[0] = old_f; f.new_f[0] = new_f; f.ncomp = 1;
+        f.old_f[0] = old_f; f.new_f[0] = new_f; f.ncomp = 1; f.early = 1;
         return check(launch_copy_new_to_old(dims, f, d_positions, d_children, nullptr, tree.curr_used_slots(), tree.timer(),
-                                            (uint32_t)tree.read_max_depth(), stream, false, true));
+                                            (uint32_t)tree.read_max_depth(), stream));
     }
     // amr_criterion (SimpleWave.h:142-187) followed by the triage of modify_nodes (:228-248).
     int modify_nodes() override {
@@ -454,12 +454,12 @@ public:
         if (st) return st;
         FieldSet f;
         std::memset(&f, 0, sizeof(f));
-        f.old_f[0] = old_f; f.new_f[0] = new_f; f.ncomp = 1;
+        f.old_f[0] = old_f; f.new_f[0] = new_f; f.ncomp = 1; f.early = 1;
         // in place where the substep's restriction still holds: the predictor writes interiors alone, but new
         // domains' old and new fields are interpolated separately
         const bool restricted = in_timestep && !grown;
         st = check(launch_copy_boundaries(dims, f, d_boundaries, tree.curr_used_slots(), tree.timer(),
-                                          (uint32_t)tree.read_max_depth(), 1, ghost_stage, stream, restricted, true));
+                                          (uint32_t)tree.read_max_depth(), 1, ghost_stage, stream, restricted));
         if (!st && !restricted) launches++;
         return st;
     }
