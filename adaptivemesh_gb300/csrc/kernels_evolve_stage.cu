@@ -17,6 +17,10 @@
 // not unrolled: the unrolled kernel (80 KB of code) spent 41 % of its time waiting for instructions and
 // ran at 856 us a launch against 470.
 //
+// The values of the first and last three cells of a row are also written to the x ghost layers of the same-depth
+// neighbours that copy them (EvoArgs::feed): a fill of those layers by itself reads and writes 12-byte runs
+// and took 124 us a stage of the uniform depth-3 tree; here the stores alone are left (a root step 24.7 -> 21.4 ms).
+//
 // Measured on a GB300, 585 domains of 16^3 (2.40 M cells), one stage: 779 us for the two kernels it
 // replaces (317 + 462 on average over the stages), about 470 us now; a root step of the uniform
 // depth-3 tree 38.4 -> 28.2 ms.  What bounds it now: shared-memory reads (about 1 080 wavefronts per 32 cells,
@@ -294,12 +298,19 @@ __global__ void __launch_bounds__(StageShape<N, TY, TZ, R_, V::L>::CT, MINB)
     // the tile's padded and inner index of cell z (z + 1 lies a plane on); 32 bits are enough, as the 72
     // padded buffers of a simulation fit the device's memory
     uint32_t npi = 0, nii = 0;
+    // the cell of a neighbour's x ghost layer that holds this cell's value (~0: none)
+    uint32_t nxi = ~0u;
     int ndepth = 0;
     auto load_own = [&](uint32_t t) {   // of tile t, in domain nslot
         const uint32_t k = t % S::TILES, z = (k / (N / TY)) * TZ + zl, yy = (k % (N / TY)) * TY + y;
         npi = (nslot * T + z + 3) * T * T + (yy + 3) * T + x + 3;
         nii = (nslot * N + z) * N * N + yy * N + x;
         ndepth = pos_depth(a.positions[nslot]);
+        nxi = ~0u;
+        if (a.feed && (x < 3u || x >= N - 3u)) {
+            const int32_t to = a.feed[2u * nslot + (x < 3u ? 0u : 1u)];
+            if (to != -1) nxi = npi + ((uint32_t)to - nslot) * (T * T * T) + (x < 3u ? (uint32_t)N : 0u - (uint32_t)N);
+        }
 #pragma unroll
         for (int i = 0; i < 9; i++) {
             const float* q = a.fields[i < 6 ? F_GXX + i : F_BETAX + (i - 6)] + npi;
@@ -308,7 +319,7 @@ __global__ void __launch_bounds__(StageShape<N, TY, TZ, R_, V::L>::CT, MINB)
     };
     load_own(blockIdx.x);   // the grid has no more CTAs than tiles
     for (uint32_t t = blockIdx.x; t < tiles; t += gridDim.x) {
-        const uint32_t pi = npi, ii = nii, slot = nslot;
+        const uint32_t pi = npi, ii = nii, xi = nxi, slot = nslot;
         const int depth = ndepth;
         if (t + gridDim.x < tiles) nslot = a.items[(t + gridDim.x) / S::TILES];
         const float h = a.prm.outer_size / ((float)N * (float)(1u << depth));
@@ -676,6 +687,7 @@ __global__ void __launch_bounds__(StageShape<N, TY, TZ, R_, V::L>::CT, MINB)
                 }
                 if (f == F_CHI) o = at_least(o, a.prm.chi_floor - 1.f);   // chi (stored less 1) keeps its floor; a NaN stays
                 o.st(a.out[f] + pi, T * T);
+                if (xi != ~0u) o.st(a.out[f] + xi, T * T);
             }
         }
         if (!ok) {   // a wait of the update gave up
