@@ -111,8 +111,10 @@ struct EvoArgs {
     uint32_t n_items;
     uint32_t n_batch;             // domains of the whole substep (n_items, or more where each is launched alone)
     uint32_t n, p, t;             // size_domain, padding_domain, n + 2p
-    const int32_t* feed;          // per slot: the domains whose + and - x ghost layers are this domain's first and
-                                  // last three cells of a row, written with them (-1: none); nullptr: no feeding
+    // Six per slot, [2 axis + side]: the domain whose + (side 0) or - ghost layer along the axis is this domain's
+    // first or last three layers, written with them (-1: none).  A domain in a later axis's entry takes the
+    // ghosts along the earlier axes too (all of this domain's are fed).  nullptr: no feeding
+    const int32_t* feed;
     float dt0;                    // dt at depth 0
     int stage;                    // 1..4
     uint32_t deriv_zs;            // interior z-planes per CTA of the wave's stage and the constraints (0: the default)

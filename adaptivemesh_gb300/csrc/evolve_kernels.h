@@ -94,6 +94,7 @@ uint32_t evo_deriv_zs_candidates(uint32_t n, uint32_t* out);
 // One RK stage of the BSSN evolution (derivatives, right-hand side and stage update;
 // kernels_evolve_stage.cu), and the kernel's shared-memory limit, to be set outside a stream capture.
 cudaError_t prepare_evo_stage_bssn(uint32_t n);
+int evo_stage_feeds(uint32_t n, uint32_t n_batch);   // axes along which the launch writes neighbours' ghosts (EvoArgs::feed)
 cudaError_t launch_evo_stage_bssn(const EvoArgs& a, cudaStream_t st);
 cudaError_t launch_evo_stage_wave(const EvoArgs& a, cudaStream_t st);   // one RK stage of the wave
 cudaError_t launch_evo_ghost(const EvoGhostArgs& g, cudaStream_t st);

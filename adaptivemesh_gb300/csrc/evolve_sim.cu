@@ -63,7 +63,7 @@ public:
         if (e == cudaSuccess) e = dev_alloc(&deriv, std::max(inner * (size_t)nd, kind == AMR_SIM_BSSN_EVOLVE ? 0u : padded * WAVE_NF));
         for (int k = 0; k < 4 && e == cudaSuccess && kind == AMR_SIM_BSSN_EVOLVE; k++) e = dev_alloc(&cons.c[k], inner);
         if (e == cudaSuccess) e = dev_alloc(&d_evolved, s);
-        if (e == cudaSuccess && kind == AMR_SIM_BSSN_EVOLVE) e = dev_alloc(&d_feed, 2u * s);
+        if (e == cudaSuccess && kind == AMR_SIM_BSSN_EVOLVE) e = dev_alloc(&d_feed, 6u * s);
         if (e == cudaSuccess) e = dev_alloc(&d_lists, s * 2u * ((size_t)1u << kDepthLimit) + 2u * s);
         if (e == cudaSuccess) e = dev_alloc(&d_part, s * 5u * kEvoNormParts);
         if (e == cudaSuccess) e = dev_alloc(&d_norms, 8);
@@ -189,35 +189,47 @@ public:
                 face_copy[a][s] = (uint32_t)copies.size();
                 faces.insert(faces.end(), copies.begin(), copies.end());
             }
-        // The x faces whose source's RK stage writes them (BSSN): a same-depth domain exactly one domain along x,
-        // each side of a source to one face.  The fill after a stage takes the x faces but these, list 3.
-        std::vector<int32_t> feed(2u * tree.max_slots(), -1);
-        fed.assign(2u * tree.max_slots(), 0);
-        for (uint32_t i = 0; i < used && kind == AMR_SIM_BSSN_EVOLVE; i++)
-            for (uint32_t side = 0; side < 2 && evolved[i]; side++) {
-                if (face_class(i, 0, side) != 1) continue;
-                const uint64_t bd = tree.boundaries()[(size_t)i * 6u + 3u * side];
-                const uint32_t src = (uint32_t)bd & 0xFFFFFFu, w = (uint32_t)(bd >> 32);
-                if (src >= used || !evolved[src] || feed[2u * src + side] != -1) continue;
-                const int depth = pos_depth_host(tree.positions()[i]);
-                if (depth != (int)((uint32_t)bd >> 28) || depth != pos_depth_host(tree.positions()[src])) continue;
-                // the offset (tensors.h:335-348): (-1, 0, 0) for the + face, whose first source cell is the first
-                const float unit = std::ldexp(1.f, (int)(w >> 27) - 22), x = (float)(w & 255u) * unit;
-                if (x != 1.f || ((w >> 8) & 1u) != (side == 0u ? 1u : 0u) || ((w >> 9) & 255u) != 0u || ((w >> 18) & 255u) != 0u) continue;
-                feed[2u * src + side] = (int32_t)i;
-                fed[2u * i + side] = 1;
+        // The faces whose source's RK stage writes them (BSSN): a same-depth source exactly one domain along the
+        // axis, whose own ghosts along the earlier axes are all written so, each side of a source to one
+        // face.  The fill after a stage takes the other faces: lists 3, 4 and 5.
+        std::vector<int32_t> feed(6u * tree.max_slots(), -1);
+        fed.assign(6u * tree.max_slots(), 0);
+        for (uint32_t a = 0; a < 3; a++)
+            for (uint32_t i = 0; i < used && kind == AMR_SIM_BSSN_EVOLVE; i++)
+                for (uint32_t side = 0; side < 2 && evolved[i]; side++) {
+                    if (face_class(i, (int)a, side) != 1) continue;
+                    const uint64_t bd = tree.boundaries()[(size_t)i * 6u + a + 3u * side];
+                    const uint32_t src = (uint32_t)bd & 0xFFFFFFu, w = (uint32_t)(bd >> 32);
+                    if (src >= used || !evolved[src] || feed[6u * src + 2u * a + side] != -1) continue;
+                    const int depth = pos_depth_host(tree.positions()[i]);
+                    if (depth != (int)((uint32_t)bd >> 28) || depth != pos_depth_host(tree.positions()[src])) continue;
+                    // the offset (tensors.h:335-348): -1 along the axis for the + face, whose first source layer is the first
+                    bool along = true;
+                    for (uint32_t c = 0; c < 3; c++) {
+                        const float m = std::ldexp((float)((w >> (9u * c)) & 255u), (int)(w >> 27) - 22);
+                        const bool neg = ((w >> (9u * c + 8u)) & 1u) != 0u;
+                        along &= c == a ? m == 1.f && neg == (side == 0u) : m == 0.f;
+                    }
+                    for (uint32_t e = 0; e < 2u * a; e++) along &= fed[6u * src + e] != 0;
+                    if (!along) continue;
+                    feed[6u * src + 2u * a + side] = (int32_t)i;
+                    fed[6u * i + 2u * a + side] = 1;
+                }
+        for (int a = 0; a < 3; a++) {
+            face_off[3 + a] = face_off[a];
+            face_interp[3 + a] = face_interp[a];
+            face_copy[3 + a] = face_copy[a];
+            for (uint32_t s = 0; s < nsub; s++) {
+                copies.clear();
+                const uint32_t all_of = face_interp[a][s] + face_copy[a][s];
+                for (uint32_t k = 0; k < all_of; k++) {
+                    const uint32_t f = faces[face_off[a][s] + k];
+                    if (k < face_interp[a][s] || !fed[6u * (f >> 1) + 2u * (uint32_t)a + (f & 1u)]) copies.push_back(f);
+                }
+                face_off[3 + a][s] = (uint32_t)faces.size();
+                face_copy[3 + a][s] = (uint32_t)copies.size() - face_interp[a][s];
+                faces.insert(faces.end(), copies.begin(), copies.end());
             }
-        face_off[3] = face_off[0];
-        face_interp[3] = face_interp[0];
-        face_copy[3] = face_copy[0];
-        for (uint32_t s = 0; s < nsub; s++) {
-            copies.clear();
-            const std::vector<uint32_t> x(faces.begin() + face_off[0][s], faces.begin() + face_off[0][s] + face_interp[0][s] + face_copy[0][s]);
-            face_off[3][s] = (uint32_t)faces.size();
-            for (size_t k = 0; k < x.size(); k++)
-                if (k < face_interp[0][s] || !fed[x[k]]) copies.push_back(x[k]);
-            face_copy[3][s] = (uint32_t)copies.size() - face_interp[0][s];
-            faces.insert(faces.end(), copies.begin(), copies.end());
         }
         if (faces.size() > faces_cap) {
             cudaError_t e = cudaStreamSynchronize(stream);
@@ -287,7 +299,7 @@ public:
         for (int stage = 1; stage <= 4; stage++) {
             EvoArgs a = args(s, in[stage - 1], out[stage - 1], stage);
             // the last stage's ghosts belong to copy_bounds(), which a timestep calls next
-            const bool feeding = kind == AMR_SIM_BSSN_EVOLVE && (stage < 4 || in_timestep);
+            const int feeding = stage < 4 || in_timestep ? stage_feeds(s) : 0;
             if (feeding) a.feed = d_feed;
             if (mode == AMR_MODE_PLAIN) {
                 // the plain per-domain form: each domain's stage launched alone
@@ -309,7 +321,7 @@ public:
     int copy_bounds() override {
         int st = prepare();
         if (st) return st;
-        return fill(tree.timer(), new_f, 1.f, kind == AMR_SIM_BSSN_EVOLVE && in_timestep);
+        return fill(tree.timer(), new_f, 1.f, in_timestep ? stage_feeds(tree.timer()) : 0);
     }
     int corrector() override { return AMR_OK; }
 
@@ -577,7 +589,7 @@ public:
         }
         if (!add_p.empty()) {
             // the parents' ghost layers feed the new domains' interpolation stencils at their faces
-            if ((st = prepare()) || (st = fill(tree.timer(), new_f, 1.f, false))) return st;
+            if ((st = prepare()) || (st = fill(tree.timer(), new_f, 1.f, 0))) return st;
             tree.begin_batch();
             for (size_t i = 0; i < add_p.size(); i++) tree.add_node(add_p[i], add_o[i]);
             tree.end_batch();
@@ -587,7 +599,7 @@ public:
         graph_valid = false;
         if (!rem.empty() || !add_p.empty()) {
             // the ghost cells from the new neighbours, in both state buffers
-            if ((st = prepare()) || (st = fill(tree.timer(), new_f, 1.f, false)) || (st = sync_old())) return st;
+            if ((st = prepare()) || (st = fill(tree.timer(), new_f, 1.f, 0)) || (st = sync_old())) return st;
         }
         if (stats) {
             stats[0] = refined;
@@ -630,8 +642,9 @@ private:
         return check(kind == AMR_SIM_BSSN_EVOLVE ? launch_evo_stage_bssn(a, stream) : launch_evo_stage_wave(a, stream));
     }
     // ghost fill of `x` (the state at c_stage of the active domains' step), three axis passes
-    // stage_fed: the stage before wrote the fed x faces
-    int fill(uint32_t s, float* const* x, float c_stage, bool stage_fed) {
+    int stage_feeds(uint32_t s) const { return kind == AMR_SIM_BSSN_EVOLVE ? evo_stage_feeds(dims.n, evo_cnt[s]) : 0; }
+    // fed_axes: the stage before wrote the fed faces of so many axes
+    int fill(uint32_t s, float* const* x, float c_stage, int fed_axes) {
         if (evo_cnt[s] == 0) return AMR_OK;
         EvoGhostArgs g;
         std::memset(&g, 0, sizeof(g));
@@ -652,7 +665,7 @@ private:
                     g.n_interp = g.n_copy = 0;
                     for (int c = 2; c >= 1; c--)
                         for (uint32_t side = 0; side < 2; side++)
-                            if (face_class(i, axis, side) == c && !(axis == 0 && stage_fed && fed[2u * i + side])) {
+                            if (face_class(i, axis, side) == c && !(axis < fed_axes && fed[6u * i + 2u * (uint32_t)axis + side])) {
                                 g.face[g.n_interp + g.n_copy] = i << 1 | side;
                                 (c == 2 ? g.n_interp : g.n_copy)++;
                             }
@@ -662,7 +675,7 @@ private:
                 }
                 continue;
             }
-            const int list = axis == 0 && stage_fed ? 3 : axis;
+            const int list = axis < fed_axes ? 3 + axis : axis;
             g.faces = d_faces + face_off[list][s];
             g.n_interp = face_interp[list][s];
             g.n_copy = face_copy[list][s];
@@ -707,9 +720,9 @@ private:
     bool lists_valid = false;
     uint32_t* d_faces = nullptr;   // the ghost fill's face lists
     size_t faces_cap = 0;
-    std::vector<uint32_t> face_off[4], face_interp[4], face_copy[4];   // per axis (3: x without the fed faces) and substep
+    std::vector<uint32_t> face_off[6], face_interp[6], face_copy[6];   // per axis (3 ..: without the fed faces) and substep
     int32_t* d_feed = nullptr;     // EvoArgs::feed
-    std::vector<uint8_t> fed;      // per slot and side: the x face is written by its source's stage
+    std::vector<uint8_t> fed;      // per slot, axis and side: the face is written by its source's stage
     std::vector<uint32_t> act_off, act_cnt, act_leaves, evo_off, evo_cnt, leaves;
     uint32_t all_evolved_off = 0, all_evolved_cnt = 0, leaves_off = 0;
     uint32_t deriv_zs = 0;   // the derivative pass's slab depth (0: the default; amr_sim_autotune)

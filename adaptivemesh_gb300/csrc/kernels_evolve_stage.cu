@@ -17,13 +17,15 @@
 // not unrolled: the unrolled kernel (80 KB of code) spent 41 % of its time waiting for instructions and
 // ran at 856 us a launch against 470.
 //
-// The values of the first and last three cells of a row are also written to the x ghost layers of the same-depth
-// neighbours that copy them (EvoArgs::feed): a fill of those layers by itself reads and writes 12-byte runs
-// and took 124 us a stage of the uniform depth-3 tree; here the stores alone are left (a root step 24.7 -> 21.4 ms).
+// The values of the first and last three layers of cells along an axis are also written to the ghost layers of
+// the same-depth neighbours that copy them (EvoArgs::feed), edges and corners by way of two or three of them.
+// A fill of those layers by itself reads what was just written, along x in 12-byte runs: x 124, y 54 and z 47 us
+// a stage of the uniform depth-3 tree, a root step 24.7 ms; with x fed
+// 21.4, with x and y 20.5 (evo_stage_feeds has the rule).
 //
 // Measured on a GB300, 585 domains of 16^3 (2.40 M cells), one stage: 779 us for the two kernels it
 // replaces (317 + 462 on average over the stages), about 470 us now; a root step of the uniform
-// depth-3 tree 38.4 -> 28.2 ms.  What bounds it now: shared-memory reads (about 1 080 wavefronts per 32 cells,
+// depth-3 tree 38.4 -> 28.2 ms (20.5 now, with the other kernels' changes and the fed ghosts).  What bounds it now: shared-memory reads (about 1 080 wavefronts per 32 cells,
 // 52 % of the pipe) in the visits and, in the update, the memory traffic that all SMs issue at the same
 // time; the two do not overlap, as a CTA's registers and columns fill its SM.  One cell a thread and
 // twice the warps gave 30.0 ms.
@@ -48,14 +50,17 @@ struct V1 {
     static constexpr int L = 1;
     static __device__ __forceinline__ V1 splat(float x) { return V1{x}; }
     static __device__ __forceinline__ V1 ld(const float* q, int) { return V1{q[0]}; }   // q[i * stride] per cell i
-    __device__ __forceinline__ void st(float* q, int) const { q[0] = v; }
+    __device__ __forceinline__ void st(float* q, int, uint32_t cells = 1u) const { if (cells & 1u) q[0] = v; }
 };
 struct V2 {
     float2 v;
     static constexpr int L = 2;
     static __device__ __forceinline__ V2 splat(float x) { return V2{make_float2(x, x)}; }
     static __device__ __forceinline__ V2 ld(const float* q, int stride) { return V2{make_float2(q[0], q[stride])}; }
-    __device__ __forceinline__ void st(float* q, int stride) const { q[0] = v.x; q[stride] = v.y; }
+    __device__ __forceinline__ void st(float* q, int stride, uint32_t cells = 3u) const {   // bit i: cell i
+        if (cells & 1u) q[0] = v.x;
+        if (cells & 2u) q[stride] = v.y;
+    }
 };
 __device__ __forceinline__ V2 mk(float x, float y) { return V2{make_float2(x, y)}; }
 __device__ __forceinline__ V2 operator+(V2 a, V2 b) { return V2{__fadd2_rn(a.v, b.v)}; }
@@ -202,7 +207,7 @@ __device__ __forceinline__ V trace(const V* g, const V* m) {
     return fma(2.f, o, d);
 }
 
-template <int N, int TY, int TZ, int R_, class V, int MINB>
+template <int N, int TY, int TZ, int R_, class V, int MINB, int FEED>
 __global__ void __launch_bounds__(StageShape<N, TY, TZ, R_, V::L>::CT, MINB)
     k_evo_stage_bssn(const __grid_constant__ EvoArgs a) {
     using S = StageShape<N, TY, TZ, R_, V::L>;
@@ -298,19 +303,12 @@ __global__ void __launch_bounds__(StageShape<N, TY, TZ, R_, V::L>::CT, MINB)
     // the tile's padded and inner index of cell z (z + 1 lies a plane on); 32 bits are enough, as the 72
     // padded buffers of a simulation fit the device's memory
     uint32_t npi = 0, nii = 0;
-    // the cell of a neighbour's x ghost layer that holds this cell's value (~0: none)
-    uint32_t nxi = ~0u;
     int ndepth = 0;
     auto load_own = [&](uint32_t t) {   // of tile t, in domain nslot
         const uint32_t k = t % S::TILES, z = (k / (N / TY)) * TZ + zl, yy = (k % (N / TY)) * TY + y;
         npi = (nslot * T + z + 3) * T * T + (yy + 3) * T + x + 3;
         nii = (nslot * N + z) * N * N + yy * N + x;
         ndepth = pos_depth(a.positions[nslot]);
-        nxi = ~0u;
-        if (a.feed && (x < 3u || x >= N - 3u)) {
-            const int32_t to = a.feed[2u * nslot + (x < 3u ? 0u : 1u)];
-            if (to != -1) nxi = npi + ((uint32_t)to - nslot) * (T * T * T) + (x < 3u ? (uint32_t)N : 0u - (uint32_t)N);
-        }
 #pragma unroll
         for (int i = 0; i < 9; i++) {
             const float* q = a.fields[i < 6 ? F_GXX + i : F_BETAX + (i - 6)] + npi;
@@ -319,7 +317,7 @@ __global__ void __launch_bounds__(StageShape<N, TY, TZ, R_, V::L>::CT, MINB)
     };
     load_own(blockIdx.x);   // the grid has no more CTAs than tiles
     for (uint32_t t = blockIdx.x; t < tiles; t += gridDim.x) {
-        const uint32_t pi = npi, ii = nii, xi = nxi, slot = nslot;
+        const uint32_t pi = npi, ii = nii, slot = nslot;
         const int depth = ndepth;
         if (t + gridDim.x < tiles) nslot = a.items[(t + gridDim.x) / S::TILES];
         const float h = a.prm.outer_size / ((float)N * (float)(1u << depth));
@@ -599,6 +597,38 @@ __global__ void __launch_bounds__(StageShape<N, TY, TZ, R_, V::L>::CT, MINB)
             atomicExch(a.err, 1);
         }
         if (__any_sync(0xffffffffu, s_abort)) break;
+        // ---- the cells of neighbours' ghost layers that hold this cell's values (~0: none): along each axis, and
+        // at the edges and the corner by way of the neighbour along the earlier axis
+        uint32_t gx = ~0u, gy = ~0u, gz = ~0u, gxy = ~0u, gxz = ~0u, gyz = ~0u, gxyz = ~0u, zmask = 0u;
+        if (a.feed) {
+            const uint32_t k = t % S::TILES, z = (k / (N / TY)) * TZ + zl, yy = (k % (N / TY)) * TY + y;
+            auto side = [](uint32_t w) { return w < 3u ? 0 : (w >= N - 3u ? 1 : -1); };
+            const int sx = side(x), sy = side(yy);
+            int sz = -1;
+#pragma unroll
+            for (int i = 0; i < L; i++)
+                if (side(z + i) >= 0) { sz = side(z + i); zmask |= 1u << i; }
+            // from cell `at` of domain `in` to its image in the next domain along the axis
+            auto image = [&](uint32_t at, int32_t in, int axis, int s, int32_t& to) -> uint32_t {
+                to = -1;
+                if (in < 0 || s < 0) return ~0u;
+                to = a.feed[6 * in + 2 * axis + s];
+                const uint32_t n = axis == 0 ? N : (axis == 1 ? N * T : N * T * T);
+                return to < 0 ? ~0u : at + (uint32_t)(to - in) * (T * T * T) + (s == 0 ? n : 0u - n);
+            };
+            int32_t dx, dy, dz, dxy, dxz, dyz, dxyz;
+            gx = image(pi, (int32_t)slot, 0, sx, dx);
+            if constexpr (FEED > 1) {
+                gy = image(pi, (int32_t)slot, 1, sy, dy);
+                gxy = image(gx, dx, 1, sy, dxy);
+            }
+            if constexpr (FEED > 2) {
+                gz = image(pi, (int32_t)slot, 2, sz, dz);
+                gxz = image(gx, dx, 2, sz, dxz);
+                gyz = image(gy, dy, 2, sz, dyz);
+                gxyz = image(gxy, dxy, 2, sz, dxyz);
+            }
+        }
         // ---- right-hand sides, in the fields' order from P_T on
         {
             V rg[6], gc[3], ddb[3], Gam[3];
@@ -687,7 +717,15 @@ __global__ void __launch_bounds__(StageShape<N, TY, TZ, R_, V::L>::CT, MINB)
                 }
                 if (f == F_CHI) o = at_least(o, a.prm.chi_floor - 1.f);   // chi (stored less 1) keeps its floor; a NaN stays
                 o.st(a.out[f] + pi, T * T);
-                if (xi != ~0u) o.st(a.out[f] + xi, T * T);
+                if (gx != ~0u) o.st(a.out[f] + gx, T * T);
+                if (FEED > 1 && gy != ~0u) o.st(a.out[f] + gy, T * T);
+                if (FEED > 1 && gxy != ~0u) o.st(a.out[f] + gxy, T * T);
+                if (FEED > 2 && zmask) {   // uniform in the tile for one cell a thread, and in its z pairs
+                    if (gz != ~0u) o.st(a.out[f] + gz, T * T, zmask);
+                    if (gxz != ~0u) o.st(a.out[f] + gxz, T * T, zmask);
+                    if (gyz != ~0u) o.st(a.out[f] + gyz, T * T, zmask);
+                    if (gxyz != ~0u) o.st(a.out[f] + gxyz, T * T, zmask);
+                }
             }
         }
         if (!ok) {   // a wait of the update gave up
@@ -703,23 +741,38 @@ __global__ void __launch_bounds__(StageShape<N, TY, TZ, R_, V::L>::CT, MINB)
         for (uint32_t n = s_asked, q = n > (uint32_t)R ? n - R : 0u; q < n; q++) mbar_wait(&full[q % R], (q / R) & 1u);
 }
 
-template <int N, int TY, int TZ, int R_, class V, int MINB>
+template <int N, int TY, int TZ, int R_, class V, int MINB, int FEED>
 cudaError_t limit_t() {
     static std::atomic<uint64_t> configured{0};
-    return ensure_smem_limit(k_evo_stage_bssn<N, TY, TZ, R_, V, MINB>, StageShape<N, TY, TZ, R_, V::L>::SMEM, configured);
+    return ensure_smem_limit(k_evo_stage_bssn<N, TY, TZ, R_, V, MINB, FEED>, StageShape<N, TY, TZ, R_, V::L>::SMEM, configured);
 }
-template <int N, int TY, int TZ, int R_, class V, int MINB>
+template <int N, int TY, int TZ, int R_, class V, int MINB, int FEED>
 cudaError_t stage_t(const EvoArgs& a, int sms, cudaStream_t st) {
     using S = StageShape<N, TY, TZ, R_, V::L>;
-    const cudaError_t e = limit_t<N, TY, TZ, R_, V, MINB>();
+    const cudaError_t e = limit_t<N, TY, TZ, R_, V, MINB, FEED>();
     if (e != cudaSuccess) return e;
     const uint32_t tiles = a.n_items * (uint32_t)S::TILES, room = (uint32_t)(sms * MINB);
-    k_evo_stage_bssn<N, TY, TZ, R_, V, MINB><<<tiles < room ? tiles : room, S::CT, S::SMEM, st>>>(a);
+    k_evo_stage_bssn<N, TY, TZ, R_, V, MINB, FEED><<<tiles < room ? tiles : room, S::CT, S::SMEM, st>>>(a);
     return cudaGetLastError();
+}
+
+// a substep whose domains are too few to give every SM a large tile (launch_evo_stage_bssn)
+bool evo_stage_small(uint32_t n, uint32_t n_batch, int sms) {
+    return n == 8u ? n_batch <= (uint32_t)sms : n == 16u && n_batch * 8u <= (uint32_t)sms;
 }
 
 }  // namespace
 
+// Axes whose ghost layers a stage writes, for a substep of n_batch domains.  All three where launches count (the
+// small tiles) and at 32^3, whose surface is small beside its volume; along x and y elsewhere, where the z
+// layers' stores, 256 a plane and field all at once, cost more than the fill's pass: a root step of 585
+// domains of 16^3 22.0 ms with two axes and 24.3 with three, but of 9 domains 178 and 154 us; 9 domains of
+// 32^3 728 and 681 us.
+int evo_stage_feeds(uint32_t n, uint32_t n_batch) {
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
+    return n == 32u || evo_stage_small(n, n_batch, sms) ? 3 : 2;
+}
 cudaError_t launch_evo_stage_bssn(const EvoArgs& a, cudaStream_t st) {
     if (a.n_items == 0u) return cudaSuccess;
     if (a.stage < 1 || a.stage > 4) return cudaErrorInvalidValue;
@@ -734,18 +787,18 @@ cudaError_t launch_evo_stage_bssn(const EvoArgs& a, cudaStream_t st) {
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess) return e;
     switch (a.n) {
-        case 8: return a.n_batch <= (uint32_t)sms ? stage_t<8, 8, 2, 6, V1, 3>(a, sms, st) : stage_t<8, 8, 8, 6, V2, 1>(a, sms, st);
-        case 16: return a.n_batch * 8u <= (uint32_t)sms ? stage_t<16, 16, 1, 5, V1, 2>(a, sms, st)
-                                                         : stage_t<16, 16, 2, 6, V2, 1>(a, sms, st);
-        case 32: return stage_t<32, 8, 2, 6, V2, 1>(a, sms, st);
+        case 8: return evo_stage_small(8, a.n_batch, sms) ? stage_t<8, 8, 2, 6, V1, 3, 3>(a, sms, st) : stage_t<8, 8, 8, 6, V2, 1, 2>(a, sms, st);
+        case 16: return evo_stage_small(16, a.n_batch, sms) ? stage_t<16, 16, 1, 5, V1, 1, 3>(a, sms, st)
+                                                         : stage_t<16, 16, 2, 6, V2, 1, 2>(a, sms, st);
+        case 32: return stage_t<32, 8, 2, 6, V2, 1, 3>(a, sms, st);
         default: return cudaErrorInvalidValue;
     }
 }
 cudaError_t prepare_evo_stage_bssn(uint32_t n) {
     switch (n) {
-        case 8: { const cudaError_t e = limit_t<8, 8, 2, 6, V1, 3>(); return e == cudaSuccess ? limit_t<8, 8, 8, 6, V2, 1>() : e; }
-        case 16: { const cudaError_t e = limit_t<16, 16, 1, 5, V1, 2>(); return e == cudaSuccess ? limit_t<16, 16, 2, 6, V2, 1>() : e; }
-        case 32: return limit_t<32, 8, 2, 6, V2, 1>();
+        case 8: { const cudaError_t e = limit_t<8, 8, 2, 6, V1, 3, 3>(); return e == cudaSuccess ? limit_t<8, 8, 8, 6, V2, 1, 2>() : e; }
+        case 16: { const cudaError_t e = limit_t<16, 16, 1, 5, V1, 1, 3>(); return e == cudaSuccess ? limit_t<16, 16, 2, 6, V2, 1, 2>() : e; }
+        case 32: return limit_t<32, 8, 2, 6, V2, 1, 3>();
         default: return cudaErrorInvalidValue;
     }
 }
