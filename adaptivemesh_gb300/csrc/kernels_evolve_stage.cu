@@ -303,12 +303,24 @@ __global__ void __launch_bounds__(StageShape<N, TY, TZ, R_, V::L>::CT, MINB)
     // the tile's padded and inner index of cell z (z + 1 lies a plane on); 32 bits are enough, as the 72
     // padded buffers of a simulation fit the device's memory
     uint32_t npi = 0, nii = 0;
+    // Feeding: the side of the domain (0: its first layers, 1: its last, -1: neither) along an axis of this
+    // thread's cells, and the domains fed along each axis (-1: none), asked for with the tile's metric
+    auto side = [](uint32_t w) { return w < 3u ? 0 : (w >= N - 3u ? 1 : -1); };
+    auto side_z = [&](uint32_t z) { return L == 2 && side(z) < 0 ? side(z + 1u) : side(z); };
+    auto next_domain = [&](int32_t in, int axis, int s) { return in >= 0 && s >= 0 ? a.feed[6 * in + 2 * axis + s] : -1; };
+    const int sx = side(x);
+    int32_t ndx = -1, ndy = -1, ndz = -1;
     int ndepth = 0;
     auto load_own = [&](uint32_t t) {   // of tile t, in domain nslot
         const uint32_t k = t % S::TILES, z = (k / (N / TY)) * TZ + zl, yy = (k % (N / TY)) * TY + y;
         npi = (nslot * T + z + 3) * T * T + (yy + 3) * T + x + 3;
         nii = (nslot * N + z) * N * N + yy * N + x;
         ndepth = pos_depth(a.positions[nslot]);
+        if (a.feed) {
+            ndx = next_domain((int32_t)nslot, 0, sx);
+            if (FEED > 1) ndy = next_domain((int32_t)nslot, 1, side(yy));
+            if (FEED > 2) ndz = next_domain((int32_t)nslot, 2, side_z(z));
+        }
 #pragma unroll
         for (int i = 0; i < 9; i++) {
             const float* q = a.fields[i < 6 ? F_GXX + i : F_BETAX + (i - 6)] + npi;
@@ -319,6 +331,15 @@ __global__ void __launch_bounds__(StageShape<N, TY, TZ, R_, V::L>::CT, MINB)
     for (uint32_t t = blockIdx.x; t < tiles; t += gridDim.x) {
         const uint32_t pi = npi, ii = nii, slot = nslot;
         const int depth = ndepth;
+        // the domains at the edges and the corner, by way of the neighbours along the earlier axes
+        const uint32_t tk = t % S::TILES, cz = (tk / (N / TY)) * TZ + zl;
+        const int sy = side((tk % (N / TY)) * TY + y), sz = side_z(cz);
+        uint32_t zmask = 0u;   // bit i: cell i lies in the side's layers along z
+#pragma unroll
+        for (int i = 0; i < L; i++) zmask |= FEED > 2 && side(cz + i) >= 0 ? 1u << i : 0u;
+        const int32_t dx = ndx, dy = ndy, dz = ndz;
+        const int32_t dxy = FEED > 1 ? next_domain(dx, 1, sy) : -1;
+        const int32_t dxz = FEED > 2 ? next_domain(dx, 2, sz) : -1, dyz = FEED > 2 ? next_domain(dy, 2, sz) : -1;
         if (t + gridDim.x < tiles) nslot = a.items[(t + gridDim.x) / S::TILES];
         const float h = a.prm.outer_size / ((float)N * (float)(1u << depth));
         const float i12h = 1.f / (12.f * h), i12h2 = 1.f / (12.f * h * h), i144h2 = 1.f / (144.f * h * h);
@@ -443,6 +464,7 @@ __global__ void __launch_bounds__(StageShape<N, TY, TZ, R_, V::L>::CT, MINB)
                 }
             }
         }
+        const int32_t dxyz = FEED > 2 ? next_domain(dxy, 2, sz) : -1;
         // ---- the conformal factor and the lapse
 #pragma unroll 1
         for (int l = 0; l < 2; l++) {
@@ -597,26 +619,14 @@ __global__ void __launch_bounds__(StageShape<N, TY, TZ, R_, V::L>::CT, MINB)
             atomicExch(a.err, 1);
         }
         if (__any_sync(0xffffffffu, s_abort)) break;
-        // ---- the cells of neighbours' ghost layers that hold this cell's values (~0: none): along each axis, and
-        // at the edges and the corner by way of the neighbour along the earlier axis
-        uint32_t gx = ~0u, gy = ~0u, gz = ~0u, gxy = ~0u, gxz = ~0u, gyz = ~0u, gxyz = ~0u, zmask = 0u;
-        if (a.feed) {
-            const uint32_t k = t % S::TILES, z = (k / (N / TY)) * TZ + zl, yy = (k % (N / TY)) * TY + y;
-            auto side = [](uint32_t w) { return w < 3u ? 0 : (w >= N - 3u ? 1 : -1); };
-            const int sx = side(x), sy = side(yy);
-            int sz = -1;
-#pragma unroll
-            for (int i = 0; i < L; i++)
-                if (side(z + i) >= 0) { sz = side(z + i); zmask |= 1u << i; }
-            // from cell `at` of domain `in` to its image in the next domain along the axis
-            auto image = [&](uint32_t at, int32_t in, int axis, int s, int32_t& to) -> uint32_t {
-                to = -1;
-                if (in < 0 || s < 0) return ~0u;
-                to = a.feed[6 * in + 2 * axis + s];
+        // ---- the cells of neighbours' ghost layers that hold this cell's values (~0: none)
+        uint32_t gx = ~0u, gy = ~0u, gz = ~0u, gxy = ~0u, gxz = ~0u, gyz = ~0u, gxyz = ~0u;
+        {
+            // from cell `at` of domain `in` to its image in domain `to`, the next along the axis
+            auto image = [&](uint32_t at, int32_t in, int axis, int s, int32_t to) -> uint32_t {
                 const uint32_t n = axis == 0 ? N : (axis == 1 ? N * T : N * T * T);
                 return to < 0 ? ~0u : at + (uint32_t)(to - in) * (T * T * T) + (s == 0 ? n : 0u - n);
             };
-            int32_t dx, dy, dz, dxy, dxz, dyz, dxyz;
             gx = image(pi, (int32_t)slot, 0, sx, dx);
             if constexpr (FEED > 1) {
                 gy = image(pi, (int32_t)slot, 1, sy, dy);
