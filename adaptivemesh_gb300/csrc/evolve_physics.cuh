@@ -1,9 +1,9 @@
 // evolve_physics.cuh -- pointwise physics of the evolution kernels: analytic initial data and the
 // Hamiltonian and momentum constraints; and the BSSN equations (moving-puncture form: 1+log or harmonic
-// slicing, Gamma-driver shift) that the RK stage kernel (kernels_evolve_stage.cu) evaluates.  The reference has none of these (its BSSN module stops at
-// metric derivatives and Christoffel symbols, BSSN.h:38-102); the equations follow the standard
-// conformal formulation (Baumgarte & Shapiro; Campanelli et al. and Baker et al. 2006 for the
-// puncture gauge), with chi = det(gamma)^(-1/3):
+// slicing, Gamma-driver shift) that the RK stage kernel (kernels_evolve_stage.cu) evaluates.  The reference
+// has none of these (its BSSN module stops at metric derivatives and Christoffel symbols, BSSN.h:38-102); the
+// equations follow the standard conformal formulation (Baumgarte & Shapiro; Campanelli et al. and Baker et
+// al. 2006 for the puncture gauge), with chi = det(gamma)^(-1/3):
 //
 //   d_t chi     = beta.d chi + 2/3 chi (alpha K - d_k beta^k)
 //   d_t gt_ij   = beta.d gt_ij + gt_ik d_j beta^k + gt_jk d_i beta^k - 2/3 gt_ij d_k beta^k - 2 alpha At_ij

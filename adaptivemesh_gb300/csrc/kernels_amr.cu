@@ -23,14 +23,14 @@ inline uint32_t blocks_for(uint64_t n) { return (uint32_t)((n + kBlock - 1) / kB
 // child's 2x2x2 cells and the rest is copied.
 constexpr uint32_t kSlabs = 4;          // slabs per domain of a launch over all active domains (at least)
 constexpr uint32_t kParentSlabs = 16;   // ... of a launch over domains with children only (gathers)
-template <int N, int P>
+template <int N, int P, bool EARLY>
 __global__ void __launch_bounds__(kBlock) k_copy_new_to_old(const __grid_constant__ FieldSet f, const uint32_t* __restrict__ positions,
                                                         const int32_t* __restrict__ children,
                                                         const uint32_t* __restrict__ items, uint32_t substep,
                                                         uint32_t max_depth) {
     constexpr uint32_t T = N + 2 * P, CELLS = T * T * T, H = N / 2;
     static_assert(CELLS % 4 == 0, "padded domains are whole 16-byte vectors");
-    if (f.early) grid_dependency();
+    if constexpr (EARLY) grid_dependency();
     const uint32_t slot = items ? items[blockIdx.x] : blockIdx.x;
     const int depth = pos_depth(positions[slot]);
     if (depth == -1 || !active_depth(substep, (uint32_t)depth, max_depth)) return;
@@ -233,7 +233,7 @@ struct GhostBox {
 // arithmetic is the reference's per cell, so the values equal a fill of the pre-fill state.  A
 // box that would leave the domain's cube (only a root source can come near) or exceed the
 // shared-memory buffer is read from global memory instead.
-template <int N, int P>
+template <int N, int P, bool EARLY>
 __global__ void __launch_bounds__(kBlock, GhostBox<N, P>::MIN_CTAS) k_ghost_face(const __grid_constant__ FieldSet f, const uint64_t* __restrict__ bds, uint32_t used,
                                                       uint32_t substep, uint32_t max_depth, int copy_only_new,
                                                       int in_place, float* __restrict__ stage) {
@@ -242,7 +242,7 @@ __global__ void __launch_bounds__(kBlock, GhostBox<N, P>::MIN_CTAS) k_ghost_face
     extern __shared__ float sbox[];
     __shared__ uint32_t s_off[3][T];   // per axis and written coordinate: box-relative source index
     __shared__ float s_r[3][T];        // and offset from it
-    if (f.early) grid_dependency();
+    if constexpr (EARLY) grid_dependency();
     const uint32_t slot = blockIdx.x / 6u, face = blockIdx.x - slot * 6u;
     const uint64_t bd = bds[(size_t)slot * 6u + face];
     const GhostJob j = ghost_job(bd, substep, max_depth);
@@ -453,7 +453,7 @@ cudaError_t launch_copy_new_to_old(Dims d, const FieldSet& f, const uint32_t* po
                                    const uint32_t* items, uint32_t n_items, uint32_t substep, uint32_t max_depth,
                                    cudaStream_t st, bool parents_only) {
     if (n_items == 0 || f.ncomp == 0) return cudaSuccess;
-    // few domains: more slabs per domain, up to eight CTAs per SM in all, as many as an SM holds (a domain
+    // few domains: more slabs per domain, a cell per thread at least, up to eight CTAs per SM in all, as many as an SM holds (a domain
     // with children gathers 8 values a cell, 32 cells a thread in 4 slabs: 49 domains of 28^3, 8 of them
     // refined, took 23.6 us, and 9.2 in 16)
     int dev = 0, sms = 0;
@@ -461,10 +461,14 @@ cudaError_t launch_copy_new_to_old(Dims d, const FieldSet& f, const uint32_t* po
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     uint32_t slabs = parents_only ? kParentSlabs : kSlabs;
     const uint64_t per_slab = (uint64_t)n_items * (uint32_t)f.ncomp;
-    while (slabs < 64u && per_slab * slabs * 2u <= 8u * (uint64_t)(sms > 0 ? sms : 1)) slabs *= 2u;
+    while (slabs < 64u && d.t * d.t * d.t / (2u * slabs) >= (uint32_t)kBlock &&
+           per_slab * slabs * 2u <= 8u * (uint64_t)(sms > 0 ? sms : 1)) slabs *= 2u;
     const dim3 grid(n_items, (uint32_t)f.ncomp, slabs);
 #define AMR_RESTRICT(N, P) \
-    if (d.n == N && d.p == P) return launch_dependent(f.early != 0, k_copy_new_to_old<N, P>, grid, kBlock, 0, st, f, positions, children, items, substep, max_depth);
+    if (d.n == N && d.p == P) {                                                                                        \
+        const auto kernel = f.early ? k_copy_new_to_old<N, P, true> : k_copy_new_to_old<N, P, false>;                     \
+        return launch_dependent(f.early != 0, kernel, grid, kBlock, 0, st, f, positions, children, items, substep, max_depth); \
+    }
     AMR_FOR_EACH_CONFIG(AMR_RESTRICT)
 #undef AMR_RESTRICT
     return cudaErrorInvalidValue;
@@ -498,12 +502,13 @@ cudaError_t launch_copy_boundaries(Dims d, const FieldSet& f, const uint64_t* bo
     const int in_place = copy_only_new && sources_restricted ? 1 : 0;
 #define AMR_GHOST(N, P)                                                                                     \
     if (d.n == N && d.p == P) {                                                                             \
-        static std::atomic<uint64_t> configured{0};                                                         \
-        if (const cudaError_t e0 = ensure_smem_limit(k_ghost_face<N, P>, GhostBox<N, P>::SMEM, configured))   \
-            return e0;                                                                                      \
-        if (used == 0 || f.ncomp == 0) return cudaSuccess;                                                  \
-        cudaError_t e = launch_dependent(f.early != 0, k_ghost_face<N, P>, used * 6u, kBlock, GhostBox<N, P>::SMEM, st, f, \
-                                         boundaries, used, substep, max_depth, copy_only_new, in_place, scratch); \
+        static std::atomic<uint64_t> configured{0}, configured_early{0};                                    \
+        cudaError_t e = ensure_smem_limit(k_ghost_face<N, P, false>, GhostBox<N, P>::SMEM, configured);      \
+        if (e == cudaSuccess) e = ensure_smem_limit(k_ghost_face<N, P, true>, GhostBox<N, P>::SMEM, configured_early); \
+        if (e != cudaSuccess || used == 0 || f.ncomp == 0) return e;                                        \
+        const auto kernel = f.early ? k_ghost_face<N, P, true> : k_ghost_face<N, P, false>;                  \
+        e = launch_dependent(f.early != 0, kernel, used * 6u, kBlock, GhostBox<N, P>::SMEM, st, f, boundaries, used, \
+                             substep, max_depth, copy_only_new, in_place, scratch);                         \
         if (e != cudaSuccess || in_place) return e;                                                         \
         k_ghost_commit<N, P><<<blocks_for((uint64_t)used * 3u * N * N), kBlock, 0, st>>>(                   \
             f, boundaries, used, substep, max_depth, copy_only_new, scratch);                               \

@@ -20,15 +20,17 @@
 // The values of the first and last three layers of cells along an axis are also written to the ghost layers of
 // the same-depth neighbours that copy them (EvoArgs::feed), edges and corners by way of two or three of them.
 // A fill of those layers by itself reads what was just written, along x in 12-byte runs: x 124, y 54 and z 47 us
-// a stage of the uniform depth-3 tree, a root step 24.7 ms; with x fed
-// 21.4, with x and y 20.5 (evo_stage_feeds has the rule).
+// a stage of the uniform depth-3 tree, a root step 24.7 ms; with x fed 21.4, with x and y 20.2
+// (evo_stage_feeds has the rule).
 //
 // Measured on a GB300, 585 domains of 16^3 (2.40 M cells), one stage: 779 us for the two kernels it
-// replaces (317 + 462 on average over the stages), about 470 us now; a root step of the uniform
-// depth-3 tree 38.4 -> 28.2 ms (20.5 now, with the other kernels' changes and the fed ghosts).  What bounds it now: shared-memory reads (about 1 080 wavefronts per 32 cells,
-// 52 % of the pipe) in the visits and, in the update, the memory traffic that all SMs issue at the same
-// time; the two do not overlap, as a CTA's registers and columns fill its SM.  One cell a thread and
-// twice the warps gave 30.0 ms.
+// replaces (317 + 462 on average over the stages), 470 us now and 545 with the fed ghosts; a root step of the
+// uniform depth-3 tree 38.4 -> 28.2 ms (20.2 with the other kernels' changes and the fed ghosts).  What
+// bounds it: the latency of eight warps (38 % of the issue slots, 54 % of the shared-memory pipe, about 1 180
+// wavefronts per 32 cells) in the visits and, in the update, the memory traffic that all SMs issue at the
+// same time; the two do not overlap, as a CTA's registers and columns fill its SM.  One cell a thread and
+// twice the warps gave 30.0 ms; the update spread over the next tile's visits was 3 % faster with warm
+// caches and 3 to 5 % slower on small trees with cold ones.
 //
 // Compiled with contraction on, as kernels_evolve.cu (held to the FP64 oracle, no reference build to
 // reproduce).

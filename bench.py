@@ -388,7 +388,7 @@ def gauge_wave_report(am, cases, bmode: int, cpu: bool, plain: bool, depth: int 
         cases.tree_uniform(sim, depth)
         sim.set_evolution(am.Evolution(slicing=am.SLICING_1PLUSLOG, shift=0, ko_sigma=0.1, cfl=0.25, periodic=1))
         sim.initial_data(am.InitialData(kind=am.ID_GAUGE_WAVE, amplitude=1e-2, wavelength=1.0))
-        tuned = sim.autotune(3) if mode != am.MODE_PLAIN else None   # the derivative pass's slab depth
+        tuned = sim.autotune(3) if mode != am.MODE_PLAIN else None   # the constraint tiles' depth
         sim.timestep()                       # warm-up (graph capture)
         sim.synchronize()
         l0 = sim.kernel_launches
@@ -429,15 +429,14 @@ def gauge_wave_report(am, cases, bmode: int, cpu: bool, plain: bool, depth: int 
 
 def evolution_bytes_per_root_step(st, n: int, p: int = 3) -> float:
     """Algorithmic HBM bytes of one root step of the BSSN evolution: every evolved domain active at a
-    substep (covered parents included) does, per RK stage, a derivative pass (24 fields read once,
-    93 derivative planes written: 117 planes of n^3 floats) and an update (93 derivative planes and
-    the 24 fields read, plus the step-start values in stages 2-3 and the accumulator in stages 2-4;
-    the 24 fields written, plus the accumulator in stages 1-3: 165 + 213 + 213 + 165 planes over
-    the four stages), four ghost fills (every ghost cell of the 24 fields read once and written
-    once) and one restriction (the padded state of the 24 fields copied)."""
+    substep (covered parents included) does four RK stages, each one kernel that keeps its derivatives on
+    chip: the 24 fields read and written, plus the accumulator written in stages 1-3 and read in stages
+    2-4 and the step-start values in stages 2-3 (72 + 120 + 120 + 72 planes of n^3 floats), four ghost
+    fills (every ghost cell of the 24 fields read once and written once) and one restriction (the padded
+    state of the 24 fields copied)."""
     t = n + 2 * p
     used, pos, md = st["used_slots"], st["positions"], st["max_depth"]
-    per_domain = (4 * 117 + 165 + 213 + 213 + 165) * n ** 3 * 4 + 4 * (t ** 3 - n ** 3) * 24 * 8 + t ** 3 * 24 * 8
+    per_domain = (72 + 120 + 120 + 72) * n ** 3 * 4 + 4 * (t ** 3 - n ** 3) * 24 * 8 + t ** 3 * 24 * 8
     active = 0
     for k in range(used):
         q = int(pos[k])
@@ -461,7 +460,7 @@ def leaf_zone_cycles_of_substep(st, n: int, s: int) -> int:
 def single_puncture_report(am, E, bmode: int, plain: bool) -> dict:
     """A single Brill-Lindquist puncture (m = 1, seeded offset |d| < 0.05) on [-64, 64]^3, refined
     around it to depth 6 with shells of neighbours (2 121 domains of 16^3, 1 856 leaves), 1+log
-    slicing and the Gamma-driver (eta = 2).  Batched: the derivative pass's slab depth autotuned,
+    slicing and the Gamma-driver (eta = 2).  Batched: the constraint tiles' depth autotuned,
     one root step (64 finest substeps) replayed from a CUDA graph after a warm-up root step.  Both
     forms also run the first two substeps phase by phase (every domain active, then the finest
     level alone), the plain per-domain launches against the batched ones, which compute the same
@@ -563,7 +562,7 @@ def binary_run(am, E, punct, params, net, bmode: int, steps: int = 16) -> tuple[
         if step % 8 == 0:
             regrids.append(sim.regrid(params, net))
             if bmode != am.MODE_PLAIN:
-                sim.autotune(2)   # the derivative pass's slab depth for the new tree
+                sim.autotune(2)   # the constraint tiles' depth for the new tree
         zc += zone_cycles_per_root_step(sim.state(), 16)
         sim.timestep()
     sim.synchronize()
