@@ -209,7 +209,7 @@ cudaError_t gemm(const A& fa, const B& fb, const Epilogue& epi, int rows, int co
 // conv1's 64 tiles, 50 ns each, 102 us, whatever few of a 128 x 16 x 16 MMA's rows are used (ranges of K
 // summed afterwards took 12 us and changed the last bits of the gradients).
 //
-// One Adam step of 64 tiles, GB300: 2 730 -> 244 us, 27 -> 13 launches, every bit as before; forward
+// One Adam step of 64 tiles, GB300: 2 730 -> 234 us, 27 -> 13 launches, every bit as before; forward
 // pass of 256 tiles 330 -> 52 us.
 constexpr int kSlabRows = 8;
 constexpr int kSlabA = kSlabRows * kGemmK * 2, kSlabB = 16 * kGemmK * 2;   // bytes per K block
@@ -683,14 +683,20 @@ struct Estimator {
     float* part1 = nullptr;                                                 // db1's column sums, first half
     int step = 0;
     cudaStream_t stream = nullptr;
+    cudaStream_t side = nullptr;     // backward()'s work beside the chain of the convolutions' gradients
+    cudaEvent_t ev[3] = {};
 
     ~Estimator() {
         if (stream) cudaStreamSynchronize(stream);
+        if (side) cudaStreamSynchronize(side);
         for (void* p : {(void*)params, (void*)grads, (void*)adam_m, (void*)adam_v, (void*)wb, (void*)h1, (void*)h2,
                         (void*)h3, (void*)z1, (void*)z2, (void*)z3, (void*)out, (void*)dout, (void*)sq, (void*)dz3,
                         (void*)dz2, (void*)dz1, (void*)da2, (void*)loss, (void*)dz3b, (void*)dz2b, (void*)dz1b,
                         (void*)pa1, (void*)pb1, (void*)pa2, (void*)pb2, (void*)part1})
             cudaFree(p);
+        for (cudaEvent_t x : ev)
+            if (x) cudaEventDestroy(x);
+        if (side) cudaStreamDestroy(side);
         if (stream) cudaStreamDestroy(stream);
     }
     template <class T>
@@ -700,6 +706,9 @@ struct Estimator {
         max_batch = batch;
         const size_t B = batch;
         cudaError_t e = cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking);
+        if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking);
+        for (cudaEvent_t& x : ev)
+            if (e == cudaSuccess) e = cudaEventCreateWithFlags(&x, cudaEventDisableTiming);
         if (e == cudaSuccess) e = alloc(&params, kParams);
         if (e == cudaSuccess) e = alloc(&grads, kParams);
         if (e == cudaSuccess) e = alloc(&adam_m, kParams);
@@ -784,13 +793,27 @@ struct Estimator {
                                                            dz3b);
         return cudaGetLastError();
     }
-    // gradients of the mean squared error of the last forward pass (of x, with targets) into `grads`
+    // `to` goes on when what `from` holds so far is done
+    cudaError_t after(cudaStream_t from, cudaStream_t to, cudaEvent_t x) {
+        const cudaError_t e = cudaEventRecord(x, from);
+        return e == cudaSuccess ? cudaStreamWaitEvent(to, x, 0) : e;
+    }
+    // Gradients of the mean squared error of the last forward pass (of x, with targets) into `grads`.  What the
+    // convolutions' chain does not need, the dense layer's gradient and the small ones, runs beside it on a
+    // stream of its own: a step of 64 tiles, which waits for one chain of MMAs, 244 -> 234 us.
     cudaError_t backward(const float* x, int B) {
+        const cudaError_t e = backward_passes(x, B);
+        const cudaError_t joined = after(side, stream, ev[2]);   // in any case: nothing is left running beside the stream
+        return e == cudaSuccess ? joined : e;
+    }
+    cudaError_t backward_passes(const float* x, int B) {
         const bf16* W2 = wb + kK1 * kC1;
         const bf16* W3 = wb + kK1 * kC1 + kK2 * kC2;
         const int k1 = B * kP1, k2 = B * kP2;
         // dW3 = H2^T dZ3, dH2 = dZ3 W3^T through conv2's ReLU
-        cudaError_t e = gemm<32, 0, 1>(ColumnsT<kK3>{h2, B}, ColumnsT<kF>{dz3b, B}, Store<32, kF>{grads + kOffW3, kK3}, kK3, kF, B, stream);
+        cudaError_t e = after(stream, side, ev[0]);
+        if (e == cudaSuccess)
+            e = gemm<32, 0, 1>(ColumnsT<kK3>{h2, B}, ColumnsT<kF>{dz3b, B}, Store<32, kF>{grads + kOffW3, kK3}, kK3, kF, B, side);
         if (e == cudaSuccess)
             e = gemm<32, kF, 1>(RowsA<kF>{dz3b, B}, RowsA<kF>{W3, kK3}, ReluBack<32, kK3>{z2, dz2, dz2b, B}, B, kK3, kF, stream);
         // dA2 = dY2 W2^T, then col2im through conv1's ReLU
@@ -798,6 +821,9 @@ struct Estimator {
             e = gemm<32, kC2, 1>(RowsA<kC2>{dz2b, k2}, RowsA<kC2>{W2, kK2}, Store<32, kK2>{da2, k2}, k2, kK2, kC2, stream);
         if (e != cudaSuccess) return e;
         k_col2im2<<<blocks((int64_t)B * kP1 * kC1), 256, 0, stream>>>(da2, z1, B, dz1, dz1b);
+        if ((e = after(stream, side, ev[1])) != cudaSuccess) return e;
+        k_colsum1<<<16, 256, 0, side>>>(dz1, k1, part1);
+        k_small_grads<<<kSmallBlocks, 256, 0, side>>>(sq, dout, h3, dz3, dz2, part1, B, grads, loss);
         // dW1 = A1^T dY1 (rows 81..95 of A1 are zero, so their gradient is too) and dW2 = A2^T dY2
         const int64_t chunks = (int64_t)(kK1 + 16) * (k1 / kGemmK) * 8 + (int64_t)(kK2 + 16) * (k2 / kGemmK) * 8;
         k_pack<<<blocks(chunks), 256, 0, stream>>>(Conv1At{x}, ColumnsT<kC1>{dz1b, k1}, kK1, k1, pa1, pb1, Conv2At{h1},
@@ -808,8 +834,6 @@ struct Estimator {
         if ((e = ensure_smem_limit(k_stream_gemm, kStreamSmem, configured)) != cudaSuccess) return e;
         k_stream_gemm<<<(kK1 + kK2) / kSlabRows, 64, kStreamSmem, stream>>>(
             StreamGemm{pa1, pb1, grads + kOffW1, kK1, k1 / kGemmK}, StreamGemm{pa2, pb2, grads + kOffW2, kK2, k2 / kGemmK}, err);
-        k_colsum1<<<16, 256, 0, stream>>>(dz1, k1, part1);
-        k_small_grads<<<kSmallBlocks, 256, 0, stream>>>(sq, dout, h3, dz3, dz2, part1, B, grads, loss);
         return cudaGetLastError();
     }
     cudaError_t adam(float lr) {
