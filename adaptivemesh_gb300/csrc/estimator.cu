@@ -27,6 +27,7 @@
 #include <new>
 #include <vector>
 
+#include "amr_device.cuh"
 #include "capi_internal.h"
 #include "kernels.h"
 #include "tcgen05.cuh"
@@ -73,6 +74,7 @@ __device__ __forceinline__ Chunk zero_chunk() {
 
 template <int NT, int KC, int G, class A, class B, class Epilogue>
 __global__ void __launch_bounds__(128) k_gemm_bf16(const A fa, const B fb, const Epilogue epi, int k_runtime, int* err) {
+    grid_dependency();
     static_assert(NT == 16 || NT == 32, "M = 128 tiles take N in multiples of 16; 32 TMEM columns");
     constexpr int MT = kGemmM, KT = kGemmK, BC = NT * KT / 8 / 128;   // chunks of B per thread and block
     constexpr uint32_t LBO = 128u, SBO = (KT / 8) * 128u;   // bytes between core matrices along K / M
@@ -194,9 +196,9 @@ cudaError_t gemm(const A& fa, const B& fb, const Epilogue& epi, int rows, int co
     static std::atomic<uint64_t> configured{0};
     const cudaError_t e = ensure_smem_limit(k_gemm_bf16<NT, KC, G, A, B, Epilogue>, smem, configured);
     if (e != cudaSuccess) return e;
-    k_gemm_bf16<NT, KC, G><<<dim3((unsigned)((rows + kGemmM - 1) / kGemmM), (unsigned)((cols + NT - 1) / NT)), 128, smem, st>>>(
-        fa, fb, epi, K, err);
-    return cudaGetLastError();
+    return launch_dependent(true, k_gemm_bf16<NT, KC, G, A, B, Epilogue>,
+                            dim3((unsigned)((rows + kGemmM - 1) / kGemmM), (unsigned)((cols + NT - 1) / NT)), 128, smem, st, fa, fb,
+                            epi, K, err);
 }
 
 // ------------------------------------------------------------------ weight gradients of the convolutions
@@ -209,7 +211,7 @@ cudaError_t gemm(const A& fa, const B& fb, const Epilogue& epi, int rows, int co
 // conv1's 64 tiles, 50 ns each, 102 us, whatever few of a 128 x 16 x 16 MMA's rows are used (ranges of K
 // summed afterwards took 12 us and changed the last bits of the gradients).
 //
-// One Adam step of 64 tiles, GB300: 2 730 -> 234 us, 27 -> 13 launches, every bit as before; forward
+// One Adam step of 64 tiles, GB300: 2 730 -> 215 us, 27 -> 13 launches, every bit as before; forward
 // pass of 256 tiles 330 -> 52 us.
 constexpr int kSlabRows = 8;
 constexpr int kSlabA = kSlabRows * kGemmK * 2, kSlabB = 16 * kGemmK * 2;   // bytes per K block
@@ -230,6 +232,7 @@ __device__ __forceinline__ void pack_chunk(const A& fa, const B& fb, int rows, i
 template <class A1, class B1, class A2, class B2>
 __global__ void __launch_bounds__(256) k_pack(const A1 a1, const B1 b1, int rows1, int K1, Chunk* pa1, Chunk* pb1, const A2 a2,
                                               const B2 b2, int rows2, int K2, Chunk* pa2, Chunk* pb2) {
+    grid_dependency();
     const int n1 = (rows1 + 16) * (K1 / kGemmK) * 8, i = blockIdx.x * 256 + threadIdx.x;
     if (i < n1) pack_chunk(a1, b1, rows1, K1, i, pa1, pb1);
     else pack_chunk(a2, b2, rows2, K2, i - n1, pa2, pb2);
@@ -245,6 +248,7 @@ struct StreamGemm {
 constexpr int kStageBlocks = 4, kStages = 6;
 constexpr size_t kStreamSmem = (size_t)kStages * kStageBlocks * (kSlabA + kSlabB) + 16384u;
 __global__ void __launch_bounds__(64) k_stream_gemm(const StreamGemm g1, const StreamGemm g2, int* err) {
+    grid_dependency();
     extern __shared__ __align__(1024) unsigned char smem[];
     __shared__ __align__(8) uint64_t full[kStages], empty[kStages], done;
     __shared__ uint32_t s_tmem;
@@ -541,6 +545,7 @@ __global__ void __launch_bounds__(128) k_fc2(const bf16* __restrict__ h3, const 
                                              int B, float* __restrict__ out, const float* __restrict__ target,
                                              float* __restrict__ dout, float* __restrict__ sq, const float* __restrict__ z3,
                                              float* __restrict__ dz3, bf16* __restrict__ dz3b) {
+    grid_dependency();
     const int b = blockIdx.x * 4 + threadIdx.x / 32, k = threadIdx.x % 32;
     if (b >= B) return;
     const float h = __bfloat162float(h3[(int64_t)b * kF + k]), w = __bfloat162float(__float2bfloat16_rn(w4[k]));
@@ -563,6 +568,7 @@ __global__ void __launch_bounds__(128) k_fc2(const bf16* __restrict__ h3, const 
 // it, gathered in a fixed order (no atomics); dZ1 in FP32 and BF16
 __global__ void __launch_bounds__(256) k_col2im2(const float* __restrict__ da, const float* __restrict__ z1, int B,
                                                  float* __restrict__ dz1, bf16* __restrict__ dz1b) {
+    grid_dependency();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (int64_t)B * kP1 * kC1) return;
     const int c = (int)(i % kC1);
@@ -592,6 +598,7 @@ __global__ void __launch_bounds__(256) k_col2im2(const float* __restrict__ da, c
 // The first half of db1's column sums: part[t][c] = sum of rows t, t + 256, ... of column c, in that order.
 // 16 lanes read a row's 16 columns.
 __global__ void __launch_bounds__(256) k_colsum1(const float* __restrict__ x, int64_t rows, float* __restrict__ part) {
+    grid_dependency();
     const int t = blockIdx.x * 16 + threadIdx.x / kC1, c = threadIdx.x % kC1;
     float s = 0.f;
 #pragma unroll 16
@@ -605,6 +612,7 @@ __global__ void __launch_bounds__(256) k_small_grads(const float* __restrict__ s
                                                      const bf16* __restrict__ h3, const float* __restrict__ dz3,
                                                      const float* __restrict__ dz2, const float* __restrict__ part1, int B,
                                                      float* __restrict__ grads, float* __restrict__ loss) {
+    grid_dependency();
     const int k = blockIdx.x;
     float s = 0.f;
     if (k >= 1 && k < 2 + kF) {   // one chain over the tiles
@@ -644,6 +652,7 @@ __global__ void __launch_bounds__(256) k_small_grads(const float* __restrict__ s
 // Adam on the FP32 master parameters, and the BF16 copies of W1, W2, W3
 __global__ void k_adam(float* __restrict__ w, const float* __restrict__ g, float* __restrict__ m, float* __restrict__ v,
                        int64_t n, float lr, float b1, float b2, float eps, float c1, float c2, bf16* __restrict__ wb) {
+    grid_dependency();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float gi = g[i];
@@ -789,9 +798,8 @@ struct Estimator {
         if (e == cudaSuccess)
             e = gemm<32, kK3, 4>(RowsA<kK3>{h2, B}, WeightB<kF, kK3>{W3}, BiasRelu<32>{params + kOffB3, z3, h3, B}, B, kF, kK3, stream);
         if (e != cudaSuccess) return e;
-        k_fc2<<<(unsigned)((B + 3) / 4), 128, 0, stream>>>(h3, params + kOffW4, params + kOffB4, B, pred, target, dout, sq, z3, dz3,
-                                                           dz3b);
-        return cudaGetLastError();
+        return launch_dependent(true, k_fc2, (unsigned)((B + 3) / 4), 128, 0, stream, h3, params + kOffW4, params + kOffB4, B, pred,
+                                target, dout, sq, z3, dz3, dz3b);
     }
     // `to` goes on when what `from` holds so far is done
     cudaError_t after(cudaStream_t from, cudaStream_t to, cudaEvent_t x) {
@@ -801,6 +809,7 @@ struct Estimator {
     // Gradients of the mean squared error of the last forward pass (of x, with targets) into `grads`.  What the
     // convolutions' chain does not need, the dense layer's gradient and the small ones, runs beside it on a
     // stream of its own: a step of 64 tiles, which waits for one chain of MMAs, 244 -> 234 us.
+    // (The launches of both passes start while the kernel before drains: 234 -> 215 us.)
     cudaError_t backward(const float* x, int B) {
         const cudaError_t e = backward_passes(x, B);
         const cudaError_t joined = after(side, stream, ev[2]);   // in any case: nothing is left running beside the stream
@@ -820,10 +829,11 @@ struct Estimator {
         if (e == cudaSuccess)
             e = gemm<32, kC2, 1>(RowsA<kC2>{dz2b, k2}, RowsA<kC2>{W2, kK2}, Store<32, kK2>{da2, k2}, k2, kK2, kC2, stream);
         if (e != cudaSuccess) return e;
-        k_col2im2<<<blocks((int64_t)B * kP1 * kC1), 256, 0, stream>>>(da2, z1, B, dz1, dz1b);
-        if ((e = after(stream, side, ev[1])) != cudaSuccess) return e;
+        e = launch_dependent(true, k_col2im2, blocks((int64_t)B * kP1 * kC1), 256, 0, stream, da2, z1, B, dz1, dz1b);
+        if (e != cudaSuccess || (e = after(stream, side, ev[1])) != cudaSuccess) return e;
         k_colsum1<<<16, 256, 0, side>>>(dz1, k1, part1);
-        k_small_grads<<<kSmallBlocks, 256, 0, side>>>(sq, dout, h3, dz3, dz2, part1, B, grads, loss);
+        e = launch_dependent(true, k_small_grads, kSmallBlocks, 256, 0, side, sq, dout, h3, dz3, dz2, part1, B, grads, loss);
+        if (e != cudaSuccess) return e;
         // dW1 = A1^T dY1 (rows 81..95 of A1 are zero, so their gradient is too) and dW2 = A2^T dY2
         const int64_t chunks = (int64_t)(kK1 + 16) * (k1 / kGemmK) * 8 + (int64_t)(kK2 + 16) * (k2 / kGemmK) * 8;
         k_pack<<<blocks(chunks), 256, 0, stream>>>(Conv1At{x}, ColumnsT<kC1>{dz1b, k1}, kK1, k1, pa1, pb1, Conv2At{h1},
@@ -832,9 +842,9 @@ struct Estimator {
         if (!err) return cudaErrorMemoryAllocation;
         static std::atomic<uint64_t> configured{0};
         if ((e = ensure_smem_limit(k_stream_gemm, kStreamSmem, configured)) != cudaSuccess) return e;
-        k_stream_gemm<<<(kK1 + kK2) / kSlabRows, 64, kStreamSmem, stream>>>(
-            StreamGemm{pa1, pb1, grads + kOffW1, kK1, k1 / kGemmK}, StreamGemm{pa2, pb2, grads + kOffW2, kK2, k2 / kGemmK}, err);
-        return cudaGetLastError();
+        return launch_dependent(true, k_stream_gemm, (kK1 + kK2) / kSlabRows, 64, kStreamSmem, stream,
+                                StreamGemm{pa1, pb1, grads + kOffW1, kK1, k1 / kGemmK},
+                                StreamGemm{pa2, pb2, grads + kOffW2, kK2, k2 / kGemmK}, err);
     }
     cudaError_t adam(float lr) {
         step++;
