@@ -75,10 +75,6 @@ struct StencilArgs {
     uint32_t n_items;
     // single-operator kinds: 1 splits the items' planes evenly over the grid (fewer items than CTAs)
     uint32_t even;
-    uint32_t early;               // launched as launch_dependent's
-    // gradient and Hessian: also the SimpleWave predictor's new value into this padded field (nullptr: no)
-    float* step_out;
-    float outer_dt;
     uint32_t substep, max_depth;
     Geo geo;
     int* err;                     // set to 1 if a bounded wait gave up
@@ -93,6 +89,10 @@ struct StencilArgs {
     // Waits for copies already issued (the drain before a CTA leaves) always use kMaxSpins.
     uint32_t spin_limit;
     uint32_t withhold;
+    uint32_t early;               // launched as launch_dependent's
+    // gradient and Hessian: also the SimpleWave predictor's new value into this padded field (nullptr: no)
+    float* step_out;
+    float outer_dt;
 };
 
 template <int N, int P, int KIND>
