@@ -89,7 +89,8 @@ cudaError_t launch_evo_prolong(const EvoProlongArgs& g, cudaStream_t st);
 bool evo_config_supported(uint32_t n, uint32_t p);
 cudaError_t launch_evo_restrict(const EvoRestrictArgs& g, cudaStream_t st);
 cudaError_t launch_evo_init(const EvoInitArgs& a, cudaStream_t st);
-// The derivative pass's compiled slab depths for size_domain n (written to out, at most 4); their count.
+// The compiled depths of the wave's slabs and the constraints' tiles for size_domain n (written to out, at
+// most 4); their count.
 uint32_t evo_deriv_zs_candidates(uint32_t n, uint32_t* out);
 // One RK stage of the BSSN evolution (derivatives, right-hand side and stage update;
 // kernels_evolve_stage.cu), and the kernel's shared-memory limit, to be set outside a stream capture.

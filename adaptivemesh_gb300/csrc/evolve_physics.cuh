@@ -179,7 +179,7 @@ __device__ __forceinline__ void geometry(const float* u, const DV& dv, const Evo
         for (int j = i; j < 3; j++) {
             const int ij = sidx(i, j);
             float r = 0.f;
-            // -1/2 gt^lm d_l d_m gt_ij (contracted by the derivative pass)
+            // -1/2 gt^lm d_l d_m gt_ij (contracted where it was taken)
             r -= .5f * dv(D_GLAP + ij);
             // gt_k(i d_j) Gt^k
 #pragma unroll

@@ -318,7 +318,7 @@ __global__ void __launch_bounds__(StageShape<N, TY, TZ, R_, V::L>::CT, MINB)
         npi = (nslot * T + z + 3) * T * T + (yy + 3) * T + x + 3;
         nii = (nslot * N + z) * N * N + yy * N + x;
         ndepth = pos_depth(a.positions[nslot]);
-        if (a.feed) {
+        if (FEED > 0 && a.feed) {
             ndx = next_domain((int32_t)nslot, 0, sx);
             if (FEED > 1) ndy = next_domain((int32_t)nslot, 1, side(yy));
             if (FEED > 2) ndz = next_domain((int32_t)nslot, 2, side_z(z));
@@ -629,7 +629,7 @@ __global__ void __launch_bounds__(StageShape<N, TY, TZ, R_, V::L>::CT, MINB)
                 const uint32_t n = axis == 0 ? N : (axis == 1 ? N * T : N * T * T);
                 return to < 0 ? ~0u : at + (uint32_t)(to - in) * (T * T * T) + (s == 0 ? n : 0u - n);
             };
-            gx = image(pi, (int32_t)slot, 0, sx, dx);
+            if constexpr (FEED > 0) gx = image(pi, (int32_t)slot, 0, sx, dx);
             if constexpr (FEED > 1) {
                 gy = image(pi, (int32_t)slot, 1, sy, dy);
                 gxy = image(gx, dx, 1, sy, dxy);
@@ -641,6 +641,8 @@ __global__ void __launch_bounds__(StageShape<N, TY, TZ, R_, V::L>::CT, MINB)
                 gxyz = image(gxy, dxy, 2, sz, dxyz);
             }
         }
+        // tests per field are time where a warp has its scheduler alone (the small tiles): one for most warps
+        const bool feeds = (gx & gy & gz & gxy & gxz & gyz & gxyz) != ~0u;
         // ---- right-hand sides, in the fields' order from P_T on
         {
             V rg[6], gc[3], ddb[3], Gam[3];
@@ -729,14 +731,17 @@ __global__ void __launch_bounds__(StageShape<N, TY, TZ, R_, V::L>::CT, MINB)
                 }
                 if (f == F_CHI) o = at_least(o, a.prm.chi_floor - 1.f);   // chi (stored less 1) keeps its floor; a NaN stays
                 o.st(a.out[f] + pi, T * T);
-                if (gx != ~0u) o.st(a.out[f] + gx, T * T);
-                if (FEED > 1 && gy != ~0u) o.st(a.out[f] + gy, T * T);
-                if (FEED > 1 && gxy != ~0u) o.st(a.out[f] + gxy, T * T);
-                if (FEED > 2 && zmask) {   // uniform in the tile for one cell a thread, and in its z pairs
-                    if (gz != ~0u) o.st(a.out[f] + gz, T * T, zmask);
-                    if (gxz != ~0u) o.st(a.out[f] + gxz, T * T, zmask);
-                    if (gyz != ~0u) o.st(a.out[f] + gyz, T * T, zmask);
-                    if (gxyz != ~0u) o.st(a.out[f] + gxyz, T * T, zmask);
+                if (FEED > 0 && (L == 2 || feeds)) {
+                    float* const to = a.out[f];
+                    if (gx != ~0u) o.st(to + gx, T * T);
+                    if (FEED > 1 && gy != ~0u) o.st(to + gy, T * T);
+                    if (FEED > 1 && gxy != ~0u) o.st(to + gxy, T * T);
+                    if (FEED > 2 && zmask) {
+                        if (gz != ~0u) o.st(to + gz, T * T, zmask);
+                        if (gxz != ~0u) o.st(to + gxz, T * T, zmask);
+                        if (gyz != ~0u) o.st(to + gyz, T * T, zmask);
+                        if (gxyz != ~0u) o.st(to + gxyz, T * T, zmask);
+                    }
                 }
             }
         }
@@ -799,19 +804,31 @@ cudaError_t launch_evo_stage_bssn(const EvoArgs& a, cudaStream_t st) {
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess) return e;
     switch (a.n) {
-        case 8: return evo_stage_small(8, a.n_batch, sms) ? stage_t<8, 8, 2, 6, V1, 3, 3>(a, sms, st) : stage_t<8, 8, 8, 6, V2, 1, 2>(a, sms, st);
-        case 16: return evo_stage_small(16, a.n_batch, sms) ? stage_t<16, 16, 1, 5, V1, 1, 3>(a, sms, st)
-                                                         : stage_t<16, 16, 2, 6, V2, 1, 2>(a, sms, st);
+        case 8:
+            if (evo_stage_small(8, a.n_batch, sms))
+                return a.feed ? stage_t<8, 8, 2, 6, V1, 3, 3>(a, sms, st) : stage_t<8, 8, 2, 6, V1, 3, 0>(a, sms, st);
+            return stage_t<8, 8, 8, 6, V2, 1, 2>(a, sms, st);
+        case 16:
+            if (evo_stage_small(16, a.n_batch, sms))
+                return a.feed ? stage_t<16, 16, 1, 5, V1, 1, 3>(a, sms, st) : stage_t<16, 16, 1, 5, V1, 1, 0>(a, sms, st);
+            return stage_t<16, 16, 2, 6, V2, 1, 2>(a, sms, st);
         case 32: return stage_t<32, 8, 2, 6, V2, 1, 3>(a, sms, st);
         default: return cudaErrorInvalidValue;
     }
 }
 cudaError_t prepare_evo_stage_bssn(uint32_t n) {
+    cudaError_t e = cudaErrorInvalidValue;
     switch (n) {
-        case 8: { const cudaError_t e = limit_t<8, 8, 2, 6, V1, 3, 3>(); return e == cudaSuccess ? limit_t<8, 8, 8, 6, V2, 1, 2>() : e; }
-        case 16: { const cudaError_t e = limit_t<16, 16, 1, 5, V1, 1, 3>(); return e == cudaSuccess ? limit_t<16, 16, 2, 6, V2, 1, 2>() : e; }
+        case 8:
+            e = limit_t<8, 8, 2, 6, V1, 3, 3>();
+            if (e == cudaSuccess) e = limit_t<8, 8, 2, 6, V1, 3, 0>();
+            return e == cudaSuccess ? limit_t<8, 8, 8, 6, V2, 1, 2>() : e;
+        case 16:
+            e = limit_t<16, 16, 1, 5, V1, 1, 3>();
+            if (e == cudaSuccess) e = limit_t<16, 16, 1, 5, V1, 1, 0>();
+            return e == cudaSuccess ? limit_t<16, 16, 2, 6, V2, 1, 2>() : e;
         case 32: return limit_t<32, 8, 2, 6, V2, 1, 3>();
-        default: return cudaErrorInvalidValue;
+        default: return e;
     }
 }
 

@@ -338,8 +338,8 @@ int amr_sim_set_stencil_ctas(amr_sim* s, uint32_t ctas);
  *   amr_sim_set_stencil_ctas still wins).  The candidate launches write only scratch memory
  *   allocated for the call.
  *   AMR_SIM_BSSN_EVOLVE / AMR_SIM_WAVE_RK4: the depth (interior z-planes per CTA: 1, 2 or 4 at 16^3; 4 or
- *   8 at 8^3; 1 at 32^3) of the constraint pass's tiles (amr_sim_constraint_norms) or of the wave's
- *   derivative pass, timed over every evolved domain; only the derivative scratch is written.
+ *   8 at 8^3; 1 at 32^3) of the constraint pass's tiles (amr_sim_constraint_norms) or of the wave's RK
+ *   stage, timed over every evolved domain; only the derivative scratch is written.
  * The simulation's state is unchanged.  *n_tuned = shapes tuned.  AMR_SIM_WAVE: AMR_ERR_INVALID. */
 int amr_sim_autotune(amr_sim* s, uint32_t reps, uint32_t* n_tuned);
 /* The tuned pairs, up to capacity: (active domains, CTAs of the fused pass) for AMR_SIM_BSSN,
@@ -367,8 +367,7 @@ int amr_sim_kernel_timing(amr_sim* s, double* ms, uint64_t* launches);
 /* Buffers of these simulations (amr_sim_buffer, comp = field): which 0 the state at the start of
  * the current step (padded), 1 the latest state (padded), 2 the RK stage state (padded), 3 the RK
  * accumulator (inner layout), 4 the constraints H, M_x, M_y, M_z (inner layout, comp 0..3, written
- * by amr_sim_constraint_norms), 5 derivative scratch planes (inner layout; written by the wave's RK
- * stages and amr_sim_autotune).  The BSSN fields chi,
+ * by amr_sim_constraint_norms), 5 scratch planes (inner layout; written by amr_sim_autotune).  The BSSN fields chi,
  * gt_xx, gt_yy, gt_zz and alpha are stored less 1 (their deviation from flat space), which keeps
  * single-precision rounding relative to the deviation. */
 #define AMR_SLICING_1PLUSLOG 0  /* d_t alpha = beta.d alpha - 2 alpha K */
