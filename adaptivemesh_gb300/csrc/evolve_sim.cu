@@ -236,7 +236,7 @@ public:
             cudaFree(d_faces);
             d_faces = nullptr;
             faces_cap = 0;
-            if (e == cudaSuccess) e = dev_alloc(&d_faces, faces.size());
+            if (e == cudaSuccess) e = dev_alloc_unset(&d_faces, faces.size());
             if (e != cudaSuccess) return cuda_status(e);
             faces_cap = faces.size();
         }
@@ -497,9 +497,9 @@ public:
             cudaFree(d_feat); cudaFree(d_ind); cudaFree(d_pred);
             d_feat = d_ind = d_pred = nullptr;
             feat_cap = 0;
-            cudaError_t e = dev_alloc(&d_feat, need * 1536u);
-            if (e == cudaSuccess) e = dev_alloc(&d_ind, need);
-            if (e == cudaSuccess) e = dev_alloc(&d_pred, need);
+            cudaError_t e = dev_alloc_unset(&d_feat, need * 1536u);
+            if (e == cudaSuccess) e = dev_alloc_unset(&d_ind, need);
+            if (e == cudaSuccess) e = dev_alloc_unset(&d_pred, need);
             if (e != cudaSuccess) return cuda_status(e);
             feat_cap = need;
         }

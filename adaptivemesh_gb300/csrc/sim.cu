@@ -535,7 +535,8 @@ AMR_API int amr_sim_create(const amr_config* cfg, int kind, uint32_t node_slots,
     else return AMR_ERR_INVALID;
     if (!s) return AMR_ERR_CAPACITY;
     if (!evolution) s->kind_id = kind;
-    const int st = s->init();
+    int st = s->init();
+    if (!st) st = cuda_status(dev_alloc_done());
     if (st) { delete s; return st; }
     *out = new (std::nothrow) amr_sim{s};
     if (!*out) { delete s; return AMR_ERR_CAPACITY; }

@@ -28,14 +28,24 @@ inline int32_t host_prng_next(int32_t& s) {                       // fast_prng::
     return s;
 }
 
+// Device memory as it comes, for what is written whole before it is read.
 template <class T>
-inline cudaError_t dev_alloc(T** p, size_t count) {
+inline cudaError_t dev_alloc_unset(T** p, size_t count) {
     *p = nullptr;
     if (count == 0) return cudaSuccess;
-    cudaError_t e = cudaMalloc((void**)p, count * sizeof(T));
-    if (e != cudaSuccess) { *p = nullptr; return e; }
-    return cudaMemset(*p, 0, count * sizeof(T));
+    const cudaError_t e = cudaMalloc((void**)p, count * sizeof(T));
+    if (e != cudaSuccess) *p = nullptr;
+    return e;
 }
+// Device memory set to zero, on the legacy stream: a simulation's stream does not wait for that one, and beside other
+// work on the GPU the zeros may land late.  Whoever calls this waits with dev_alloc_done() before the
+// memory is used (amr_sim_create, after every allocation of init()).
+template <class T>
+inline cudaError_t dev_alloc(T** p, size_t count) {
+    const cudaError_t e = dev_alloc_unset(p, count);
+    return e == cudaSuccess && count ? cudaMemset(*p, 0, count * sizeof(T)) : e;
+}
+inline cudaError_t dev_alloc_done() { return cudaStreamSynchronize(nullptr); }
 
 class SimBase : public NodeHooks {
 public:
@@ -208,6 +218,7 @@ public:
         cudaFree(ghost_stage);
         ghost_stage_floats = 0;
         cudaError_t e = dev_alloc(&ghost_stage, need);
+        if (e == cudaSuccess) e = dev_alloc_done();
         if (e != cudaSuccess) return cuda_status(e);
         ghost_stage_floats = need;
         return AMR_OK;
