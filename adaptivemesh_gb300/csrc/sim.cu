@@ -536,7 +536,7 @@ AMR_API int amr_sim_create(const amr_config* cfg, int kind, uint32_t node_slots,
     if (!s) return AMR_ERR_CAPACITY;
     if (!evolution) s->kind_id = kind;
     int st = s->init();
-    if (!st) st = cuda_status(dev_alloc_done());
+    if (!st) st = cuda_status(legacy_done());
     if (st) { delete s; return st; }
     *out = new (std::nothrow) amr_sim{s};
     if (!*out) { delete s; return AMR_ERR_CAPACITY; }
@@ -971,6 +971,7 @@ AMR_API int amr_sim_load(amr_sim* s, const char* dir) {
     for (size_t i = 0; i < fields.size(); i++)
         if ((st = cuda_status(cudaMemcpy(targets[i], fields[i].data(), fields[i].size(), cudaMemcpyHostToDevice))))
             return st;
+    if ((st = cuda_status(legacy_done()))) return st;   // pageable copies may return before their last bytes arrive
     b->tree.restore(pos.data(), par.data(), ch.data(), bd.data(), life.data(), words[7], (int)words[8], words[9],
                     words[10]);
     b->rng = (int32_t)words[11];

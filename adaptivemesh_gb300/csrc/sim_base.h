@@ -38,14 +38,14 @@ inline cudaError_t dev_alloc_unset(T** p, size_t count) {
     return e;
 }
 // Device memory set to zero, on the legacy stream: a simulation's stream does not wait for that one, and beside other
-// work on the GPU the zeros may land late.  Whoever calls this waits with dev_alloc_done() before the
+// work on the GPU the zeros may land late.  Whoever calls this waits with legacy_done() before the
 // memory is used (amr_sim_create, after every allocation of init()).
 template <class T>
 inline cudaError_t dev_alloc(T** p, size_t count) {
     const cudaError_t e = dev_alloc_unset(p, count);
     return e == cudaSuccess && count ? cudaMemset(*p, 0, count * sizeof(T)) : e;
 }
-inline cudaError_t dev_alloc_done() { return cudaStreamSynchronize(nullptr); }
+inline cudaError_t legacy_done() { return cudaStreamSynchronize(nullptr); }
 
 class SimBase : public NodeHooks {
 public:
@@ -218,7 +218,7 @@ public:
         cudaFree(ghost_stage);
         ghost_stage_floats = 0;
         cudaError_t e = dev_alloc(&ghost_stage, need);
-        if (e == cudaSuccess) e = dev_alloc_done();
+        if (e == cudaSuccess) e = legacy_done();
         if (e != cudaSuccess) return cuda_status(e);
         ghost_stage_floats = need;
         return AMR_OK;

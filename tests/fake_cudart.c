@@ -20,10 +20,10 @@ static const void* kernel_stub[4096];
 static int kernels;
 static const char* launched[1 << 16];
 static struct { void* p; int v; size_t n; } zeroing[4096];   /* queued on the legacy stream */
-static int queued;
+static int queued, copying;   /* copying: the last pageable cudaMemcpy to the device may still be on its way */
 static void run_legacy_stream(void) {
     for (int i = 0; i < queued; i++) memset(zeroing[i].p, zeroing[i].v, zeroing[i].n);
-    queued = 0;
+    queued = copying = 0;
 }
 
 #define API __attribute__((visibility("default")))
@@ -43,7 +43,7 @@ API unsigned long long fake_uploaded(void) { return uploaded; }
 API int fake_copies(void) { return copies < 4096 ? copies : 4096; }
 API void* fake_copy_dst(int i) { return copy_dst[i]; }
 API unsigned long long fake_copy_bytes(int i) { return copy_bytes[i]; }
-API int fake_queued(void) { return queued; }   /* writes still queued on the legacy stream, which no other stream waits for */
+API int fake_queued(void) { return queued + copying; }   /* writes still queued on the legacy stream, which no other stream waits for */
 API const char* fake_kernel(long i) { return launched[i & 0xFFFF] ? launched[i & 0xFFFF] : ""; }
 
 /* ---- registration and launches */
@@ -94,7 +94,11 @@ static err_t copy(void* d, const void* s, size_t n, int kind) {
     }
     return 0;
 }
-API err_t cudaMemcpy(void* d, const void* s, size_t n, int kind) { run_legacy_stream(); return copy(d, s, n, kind); }
+API err_t cudaMemcpy(void* d, const void* s, size_t n, int kind) {
+    run_legacy_stream();
+    copying = kind == 1 && n != 0;   /* returns once the pageable source has been staged */
+    return copy(d, s, n, kind);
+}
 API err_t cudaMemcpyAsync(void* d, const void* s, size_t n, int kind, void* st) { return copy(d, s, n, kind); }
 API err_t cudaMemset(void* d, int v, size_t n) {   /* returns before the device has written */
     if (queued == 4096) run_legacy_stream();

@@ -28,3 +28,15 @@ def test_no_zeroing_is_queued_when_a_call_returns(am, tmp_path):
         print(json.dumps(out))
     """)
     assert out and all(v == 0 for v in out.values()), out
+
+
+def test_a_loaded_checkpoint_has_arrived(am, tmp_path):
+    """cudaMemcpy from pageable memory may return before the last bytes reach the device, on the legacy stream too."""
+    (tmp_path / "at").mkdir()
+    out = fake_cuda.run(tmp_path, f"""
+        sim = am.Sim(am.Config(8, 3, 1.0), am.SIM_BSSN_EVOLVE, slots=9, mode=am.MODE_BATCHED)
+        sim.save_checkpoint({str(tmp_path / "at")!r})
+        sim.load_checkpoint({str(tmp_path / "at")!r})
+        print(json.dumps(fake.fake_queued()))
+    """)
+    assert out == 0
