@@ -384,6 +384,8 @@ public:
         FieldSet f;
         std::memset(&f, 0, sizeof(f));
         f.old_f[0] = old_f; f.new_f[0] = new_f; f.ncomp = 1; f.early = 1;
+        restricted_timer = tree.timer();
+        restricted_depth = tree.read_max_depth();
         return check(launch_copy_new_to_old(dims, f, d_positions, d_children, nullptr, tree.curr_used_slots(), tree.timer(),
                                             (uint32_t)tree.read_max_depth(), stream));
     }
@@ -455,9 +457,11 @@ public:
         FieldSet f;
         std::memset(&f, 0, sizeof(f));
         f.old_f[0] = old_f; f.new_f[0] = new_f; f.ncomp = 1; f.early = 1;
-        // in place where the substep's restriction still holds: the predictor writes interiors alone, but new
-        // domains' old and new fields are interpolated separately
-        const bool restricted = in_timestep && !grown;
+        // In place where the substep's restriction covered every domain that is active now: the predictor writes
+        // interiors alone, but new domains' old and new fields are interpolated separately, and where the
+        // triage took the deepest levels away the counter is another, at which more domains are active.
+        const bool restricted = in_timestep && !grown && tree.timer() == restricted_timer &&
+                                tree.read_max_depth() == restricted_depth;
         st = check(launch_copy_boundaries(dims, f, d_boundaries, tree.curr_used_slots(), tree.timer(),
                                           (uint32_t)tree.read_max_depth(), 1, ghost_stage, stream, restricted));
         if (!st && !restricted) launches++;
@@ -512,6 +516,8 @@ private:
     float* crit = nullptr;
     float* crit_host = nullptr;
     bool grown = false;   // domains were added in this substep
+    uint32_t restricted_timer = 0;   // the counter and the depth that the substep's restriction ran at
+    int restricted_depth = 0;
 };
 
 }  // namespace amr
