@@ -120,6 +120,9 @@ struct EvoArgs {
     uint32_t deriv_zs;            // interior z-planes per CTA of the wave's stage and the constraints (0: the default)
     EvoParams prm;
     int* err;
+    // Failure-path test hooks of the BSSN stage, off when 0: polls before a data wait gives up in place of
+    // kMaxSpins, and q + 1 for the visit of each CTA whose data never comes whole
+    uint32_t spin_limit, withhold;
 };
 
 }  // namespace amr

@@ -636,6 +636,8 @@ private:
         a.deriv_zs = deriv_zs;
         a.prm = prm;
         a.err = err_flag;
+        a.spin_limit = fault_spin_limit;
+        a.withhold = fault_withhold;
         return a;
     }
     int stage_update(const EvoArgs& a) {   // one RK stage

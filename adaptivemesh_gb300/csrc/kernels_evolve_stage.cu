@@ -235,6 +235,7 @@ __global__ void __launch_bounds__(StageShape<N, TY, TZ, R_, V::L>::CT, MINB)
     const int visits = shift_on ? kVisits : kVisits - 3;   // a frozen shift's driver is not differentiated
     const int all_visits = visits + S::UPDATES;
     bool ok = true;
+    const uint32_t spins = a.spin_limit ? a.spin_limit : kMaxSpins;
 
     // Request visit i of tile t (of domain `slot`), the q-th of this CTA, by one whole warp, once every
     // warp has released the slot's previous contents.  Visits 0 .. visits - 1 bring a field's tile
@@ -243,15 +244,18 @@ __global__ void __launch_bounds__(StageShape<N, TY, TZ, R_, V::L>::CT, MINB)
     auto request = [&](uint32_t q, uint32_t t, uint32_t slot, int i) {
         if (t >= tiles) return;
         const uint32_t s = q % R;
-        if (q >= (uint32_t)R) ok = __all_sync(0xffffffffu, mbar_wait(&empty[s], ((q / R) - 1u) & 1u)) && ok;
+        // the whole warp or none of it: no lane's copy is issued without lane 0's announcement, as nothing would
+        // wait for it
+        ok = __all_sync(0xffffffffu, ok && (q < (uint32_t)R || mbar_wait(&empty[s], ((q / R) - 1u) & 1u, spins)));
         if (!ok) return;
         const uint32_t k = t % S::TILES, z0 = (k / (N / TY)) * TZ, y0 = (k % (N / TY)) * TY;
         float* dst = ring + (size_t)s * S::SLOT;
         const bool tile = i < visits;
         if (lane == 0) {
+            const uint32_t held = q + 1u == a.withhold;   // failure-path test: more announced than comes
             mbar_arrive_expect_tx(&full[s], 4u * (tile ? (uint32_t)(S::PLANES * S::CHUNK)
                                                    : (uint32_t)S::F * ((use_old ? (S::WHOLE ? S::OLD_F : TZ * (TY + 2) * T) : 0) +
-                                                                       (use_acc ? S::ACC_F : 0))));
+                                                                       (use_acc ? S::ACC_F : 0))) + held);
             atomicMax(&s_asked, q + 1u);   // the warps' requests may pass one another
         }
         __syncwarp();
@@ -353,7 +357,7 @@ __global__ void __launch_bounds__(StageShape<N, TY, TZ, R_, V::L>::CT, MINB)
         for (int i = 0; i < 6; i++) g[i] = own[i] + sp(i == 0 || i == 3 || i == 5 ? 1.f : 0.f);
         // The tile's next field: the warps take turns to request the field AHEAD visits on, then wait.
         int vi = 0;   // visits of this tile
-        auto wait = [&](uint32_t p) { ok = mbar_wait(&full[p % R], (p / R) & 1u) && ok; };
+        auto wait = [&](uint32_t p) { ok = mbar_wait(&full[p % R], (p / R) & 1u, spins) && ok; };
         auto visit = [&]() {
             if (warp == (uint32_t)vi % S::WARPS) {
                 const int j = vi + S::AHEAD;
@@ -717,6 +721,7 @@ __global__ void __launch_bounds__(StageShape<N, TY, TZ, R_, V::L>::CT, MINB)
                 ac[j] = V::ld(q + o_acc, TY * N);
             }
             release();
+            if (!ok) continue;   // what the slot holds is not this tile's
 #pragma unroll
             for (int j = 0; j < S::F; j++) {
                 const int f = u * S::F + j;
@@ -755,7 +760,8 @@ __global__ void __launch_bounds__(StageShape<N, TY, TZ, R_, V::L>::CT, MINB)
     // consumed, after an abort some may be in flight (bounded waits)
     __syncthreads();
     if (tid == 0 && s_abort)
-        for (uint32_t n = s_asked, q = n > (uint32_t)R ? n - R : 0u; q < n; q++) mbar_wait(&full[q % R], (q / R) & 1u);
+        for (uint32_t n = s_asked, q = n > (uint32_t)R ? n - R : 0u; q < n; q++)
+            mbar_wait(&full[q % R], (q / R) & 1u, q + 1u == a.withhold ? spins : kMaxSpins);
 }
 
 template <int N, int TY, int TZ, int R_, class V, int MINB, int FEED>

@@ -372,7 +372,8 @@ public:
     // CTAs of the fused BSSN pass: fixed by amr_sim_set_stencil_ctas (0: automatic), else the
     // autotuned choice for this domain count, else the library's rule (stencil_grid).
     uint32_t stencil_ctas = 0;
-    // failure-path test hooks of the fused pass (amr_sim_set_fault_injection; StencilArgs)
+    // failure-path test hooks of the fused pass and the BSSN evolution's stages (amr_sim_set_fault_injection;
+    // StencilArgs, EvoArgs)
     uint32_t fault_spin_limit = 0, fault_withhold = 0;
     std::vector<std::pair<uint32_t, uint32_t>> tuned_ctas;   // (active domains, CTAs)
     uint32_t fused_grid(uint32_t n_items) const {

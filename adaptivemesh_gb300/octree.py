@@ -308,7 +308,7 @@ class Sim:
         return {"refined": stats[0], "coarsened": stats[1], "overridden": stats[2], "leaves": stats[3]}
 
     def set_fault_injection(self, spin_limit: int = 0, withhold_plane: int = 0) -> None:
-        """Failure-path test hook of the fused pass (amr_sim_set_fault_injection); (0, 0) is off."""
+        """Failure-path test hook of the fused pass and the evolution's stages (amr_sim_set_fault_injection); (0, 0) is off."""
         check(load().amr_sim_set_fault_injection(self.h, spin_limit, withhold_plane), "amr_sim_set_fault_injection")
 
     def enable_kernel_timing(self, enable: bool = True) -> None:

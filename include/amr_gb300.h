@@ -318,10 +318,11 @@ int amr_sim_synchronize(amr_sim* s);
 /* Kernel launches the library issued for this simulation since creation (graph replays count
  * the kernels in the graph). */
 uint64_t amr_sim_kernel_launches(const amr_sim* s);
-/* Test hook of the failure path (no counterpart in the reference): with spin_limit != 0 the fused
- * BSSN pass's data waits give up after that many polls, and with withhold_plane = q + 1 each CTA's
- * producer skips its q-th plane request, so the waits on it run out.  The pass then leaves with
- * invalid results and amr_sim_synchronize returns AMR_ERR_TIMEOUT (once).  (0, 0) turns it off. */
+/* Test hook of the failure path (no counterpart in the reference): with spin_limit != 0 the data waits of the
+ * fused BSSN pass, or of the BSSN evolution's RK stages, give up after that many polls, and with
+ * withhold_plane = q + 1 each CTA's q-th request (of a plane, or of a field of the evolution) never
+ * completes, so the waits on it run out.  The pass then leaves with invalid results and amr_sim_synchronize returns
+ * AMR_ERR_TIMEOUT (once).  (0, 0) turns it off. */
 int amr_sim_set_fault_injection(amr_sim* s, uint32_t spin_limit, uint32_t withhold_plane);
 /* Number of CTAs of the fused BSSN derivative pass (AMR_MODE_BATCHED / AMR_MODE_GRAPH), in place
  * of the library's choice; 0 restores it.  Results do not depend on it (every CTA takes an equal
