@@ -831,13 +831,15 @@ struct Estimator {
         if (e != cudaSuccess) return e;
         e = launch_dependent(true, k_col2im2, blocks((int64_t)B * kP1 * kC1), 256, 0, stream, da2, z1, B, dz1, dz1b);
         if (e != cudaSuccess || (e = after(stream, side, ev[1])) != cudaSuccess) return e;
-        k_colsum1<<<16, 256, 0, side>>>(dz1, k1, part1);
-        e = launch_dependent(true, k_small_grads, kSmallBlocks, 256, 0, side, sq, dout, h3, dz3, dz2, part1, B, grads, loss);
+        e = launch_dependent(false, k_colsum1, 16, 256, 0, side, dz1, k1, part1);
+        if (e == cudaSuccess)
+            e = launch_dependent(true, k_small_grads, kSmallBlocks, 256, 0, side, sq, dout, h3, dz3, dz2, part1, B, grads, loss);
         if (e != cudaSuccess) return e;
         // dW1 = A1^T dY1 (rows 81..95 of A1 are zero, so their gradient is too) and dW2 = A2^T dY2
         const int64_t chunks = (int64_t)(kK1 + 16) * (k1 / kGemmK) * 8 + (int64_t)(kK2 + 16) * (k2 / kGemmK) * 8;
-        k_pack<<<blocks(chunks), 256, 0, stream>>>(Conv1At{x}, ColumnsT<kC1>{dz1b, k1}, kK1, k1, pa1, pb1, Conv2At{h1},
-                                                   ColumnsT<kC2>{dz2b, k2}, kK2, k2, pa2, pb2);
+        e = launch_dependent(false, k_pack<Conv1At, ColumnsT<kC1>, Conv2At, ColumnsT<kC2>>, blocks(chunks), 256, 0, stream, Conv1At{x},
+                             ColumnsT<kC1>{dz1b, k1}, kK1, k1, pa1, pb1, Conv2At{h1}, ColumnsT<kC2>{dz2b, k2}, kK2, k2, pa2, pb2);
+        if (e != cudaSuccess) return e;
         int* err = device_error_flag();
         if (!err) return cudaErrorMemoryAllocation;
         static std::atomic<uint64_t> configured{0};
