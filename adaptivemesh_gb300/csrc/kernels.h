@@ -52,7 +52,9 @@ cudaError_t launch_dependent(bool early, void (*kernel)(P...), dim3 grid, dim3 b
     c.stream = st;
     c.attrs = &at;
     c.numAttrs = early ? 1 : 0;
-    return cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);
+    const cudaError_t e = cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);
+    if (e != cudaSuccess) cudaGetLastError();   // the caller has it: the next launch must not find it again
+    return e;
 }
 
 enum StencilKind { SK_GRAD = 0, SK_GRAD_HESS = 1, SK_MIXED = 2, SK_BSSN = 3 };

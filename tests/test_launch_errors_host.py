@@ -64,3 +64,8 @@ def test_every_refused_launch_is_reported(scan):
     out = scan(False)
     assert all(n > 0 for n, _ in out.values())
     assert not any(bad for _, bad in out.values()), out
+
+
+def test_a_refused_launch_is_reported_once(scan):
+    out = scan(True)
+    assert not any(bad for _, bad in out.values()), out
