@@ -64,7 +64,7 @@ public:
         for (int k = 0; k < 4 && e == cudaSuccess && kind == AMR_SIM_BSSN_EVOLVE; k++) e = dev_alloc(&cons.c[k], inner);
         if (e == cudaSuccess) e = dev_alloc(&d_evolved, s);
         if (e == cudaSuccess && kind == AMR_SIM_BSSN_EVOLVE) e = dev_alloc(&d_feed, 6u * s);
-        if (e == cudaSuccess) e = dev_alloc(&d_lists, s * 2u * ((size_t)1u << kDepthLimit) + 2u * s);
+        if (e == cudaSuccess) e = dev_alloc(&d_lists, s * 2u * (kDepthLimit + 1u) + 2u * s);
         if (e == cudaSuccess) e = dev_alloc(&d_part, s * 5u * kEvoNormParts);
         if (e == cudaSuccess) e = dev_alloc(&d_norms, 8);
         if (e == cudaSuccess) {   // the stage kernels' shared-memory limits, outside any stream capture
@@ -129,12 +129,20 @@ public:
         }
     }
 
-    // ---- lists per substep: active domains (restriction) and active evolved domains
-    int build_lists() {
-        if (lists_valid) return AMR_OK;
+    // ---- lists: active domains (restriction) and active evolved domains.  The domains active at a substep depend on
+    // its trailing zeros alone, so that there are as many lists as depths.  (Host time of the constraint norms after
+    // a change of a tree of depth 6 and 1 569 domains, on an x86 core: 7.9 ms and 3.9 MB of uploads with a
+    // list and the faces per substep, 0.14 ms now; of a timestep's lists 7.7 and 1.3 ms.)
+    uint32_t set_of(uint32_t substep) const {
+        const uint32_t md = (uint32_t)tree.read_max_depth();
+        uint32_t k = 0;
+        while (k < md && !(substep >> k & 1u)) k++;
+        return k;
+    }
+    void list_domains(std::vector<uint32_t>& all, std::vector<uint8_t>& evolved) {
         const uint32_t md = (uint32_t)tree.read_max_depth(), used = tree.curr_used_slots();
-        const uint32_t nsub = 1u << md;
-        std::vector<uint8_t> evolved(tree.max_slots(), 0);
+        const uint32_t sets = md + 1u;   // set k: the domains at depth md - k and below
+        evolved.assign(tree.max_slots(), 0);
         leaves.clear();
         // Every live domain is evolved, covered parents included: a leaf beside a covered parent of
         // its own depth takes its ghost values from it at every stage (and the parent's values are
@@ -148,14 +156,14 @@ public:
         }
         std::vector<uint8_t> is_leaf(tree.max_slots(), 0);
         for (uint32_t i : leaves) is_leaf[i] = 1;
-        std::vector<uint32_t> all, sub;
-        act_off.assign(nsub, 0); act_cnt.assign(nsub, 0); act_leaves.assign(nsub, 0);
-        evo_off.assign(nsub, 0); evo_cnt.assign(nsub, 0);
-        for (uint32_t s = 0; s < nsub; s++) {
-            sub.clear();   // the substep's active domains in slot order
+        std::vector<uint32_t> sub;
+        act_off.assign(sets, 0); act_cnt.assign(sets, 0); act_leaves.assign(sets, 0);
+        evo_off.assign(sets, 0); evo_cnt.assign(sets, 0);
+        for (uint32_t s = 0; s < sets; s++) {
+            sub.clear();   // the set's domains in slot order
             for (uint32_t i = 0; i < used; i++) {
                 const int d = pos_depth_host(tree.positions()[i]);
-                if (d != -1 && (s & ((1u << (md - (uint32_t)d)) - 1u)) == 0u) sub.push_back(i);
+                if (d != -1 && md - (uint32_t)d <= s) sub.push_back(i);
             }
             // the restriction's list: the leaves (straight copies) first, then the domains with children
             act_off[s] = (uint32_t)all.size();
@@ -173,17 +181,22 @@ public:
         all_evolved_cnt = (uint32_t)all.size() - all_evolved_off;
         leaves_off = (uint32_t)all.size();
         all.insert(all.end(), leaves.begin(), leaves.end());
-        // the ghost fill's faces per substep and axis: interpolating ones first, then copies
-        std::vector<uint32_t> faces, copies;
-        for (int a = 0; a < 3; a++) { face_off[a].assign(nsub, 0); face_interp[a].assign(nsub, 0); face_copy[a].assign(nsub, 0); }
-        for (uint32_t s = 0; s < nsub; s++)
+    }
+    // ---- the ghost fill's face lists and the feed table, for the calls that step or fill
+    void list_faces(std::vector<uint32_t>& faces, std::vector<int32_t>& feed) {
+        const uint32_t md = (uint32_t)tree.read_max_depth(), used = tree.curr_used_slots(), sets = md + 1u;
+        auto depth_of = [&](uint32_t i) { return pos_depth_host(tree.positions()[i]); };   // -1: no domain
+        // the ghost fill's faces per set and axis: interpolating ones first, then copies
+        std::vector<uint32_t> copies;
+        for (int a = 0; a < 3; a++) { face_off[a].assign(sets, 0); face_interp[a].assign(sets, 0); face_copy[a].assign(sets, 0); }
+        for (uint32_t s = 0; s < sets; s++)
             for (int a = 0; a < 3; a++) {
                 copies.clear();
                 face_off[a][s] = (uint32_t)faces.size();
-                for (uint32_t k = evo_off[s]; k < evo_off[s] + evo_cnt[s]; k++)
-                    for (uint32_t side = 0; side < 2; side++) {
-                        const int c = face_class(all[k], a, side);
-                        if (c) (c == 2 ? faces : copies).push_back(all[k] << 1 | side);
+                for (uint32_t i = 0; i < used; i++)
+                    for (uint32_t side = 0; side < 2 && depth_of(i) != -1 && md - (uint32_t)depth_of(i) <= s; side++) {
+                        const int c = face_class(i, a, side);
+                        if (c) (c == 2 ? faces : copies).push_back(i << 1 | side);
                     }
                 face_interp[a][s] = (uint32_t)faces.size() - face_off[a][s];
                 face_copy[a][s] = (uint32_t)copies.size();
@@ -192,23 +205,22 @@ public:
         // The faces whose source's RK stage writes them (BSSN): a same-depth source exactly one domain along the
         // axis, whose own ghosts along the earlier axes are all written so, each side of a source to one
         // face.  The fill after a stage takes the other faces: lists 3, 4 and 5.
-        std::vector<int32_t> feed(6u * tree.max_slots(), -1);
+        feed.assign(6u * tree.max_slots(), -1);
         fed.assign(6u * tree.max_slots(), 0);
         for (uint32_t a = 0; a < 3; a++)
             for (uint32_t i = 0; i < used && kind == AMR_SIM_BSSN_EVOLVE; i++)
-                for (uint32_t side = 0; side < 2 && evolved[i]; side++) {
+                for (uint32_t side = 0; side < 2 && depth_of(i) != -1; side++) {
                     if (face_class(i, (int)a, side) != 1) continue;
                     const uint64_t bd = tree.boundaries()[(size_t)i * 6u + a + 3u * side];
                     const uint32_t src = (uint32_t)bd & 0xFFFFFFu, w = (uint32_t)(bd >> 32);
-                    if (src >= used || !evolved[src] || feed[6u * src + 2u * a + side] != -1) continue;
-                    const int depth = pos_depth_host(tree.positions()[i]);
-                    if (depth != (int)((uint32_t)bd >> 28) || depth != pos_depth_host(tree.positions()[src])) continue;
+                    if (src >= used || depth_of(src) == -1 || feed[6u * src + 2u * a + side] != -1) continue;
+                    if (depth_of(i) != (int)((uint32_t)bd >> 28) || depth_of(i) != depth_of(src)) continue;
                     // the offset (tensors.h:335-348): -1 along the axis for the + face, whose first source layer is the first
                     bool along = true;
                     for (uint32_t c = 0; c < 3; c++) {
-                        const float m = std::ldexp((float)((w >> (9u * c)) & 255u), (int)(w >> 27) - 22);
+                        const uint32_t m = (w >> (9u * c)) & 255u, e = w >> 27;   // m 2^(e - 22)
                         const bool neg = ((w >> (9u * c + 8u)) & 1u) != 0u;
-                        along &= c == a ? m == 1.f && neg == (side == 0u) : m == 0.f;
+                        along &= c == a ? e <= 22u && m == 1u << (22u - e) && neg == (side == 0u) : m == 0u;
                     }
                     for (uint32_t e = 0; e < 2u * a; e++) along &= fed[6u * src + e] != 0;
                     if (!along) continue;
@@ -219,7 +231,7 @@ public:
             face_off[3 + a] = face_off[a];
             face_interp[3 + a] = face_interp[a];
             face_copy[3 + a] = face_copy[a];
-            for (uint32_t s = 0; s < nsub; s++) {
+            for (uint32_t s = 0; s < sets; s++) {
                 copies.clear();
                 const uint32_t all_of = face_interp[a][s] + face_copy[a][s];
                 for (uint32_t k = 0; k < all_of; k++) {
@@ -231,8 +243,22 @@ public:
                 faces.insert(faces.end(), copies.begin(), copies.end());
             }
         }
+    }
+    int build_lists(bool with_faces) {
+        if (lists_valid && (faces_valid || !with_faces)) return AMR_OK;
+        std::vector<uint32_t> all, faces;
+        std::vector<uint8_t> evolved;
+        std::vector<int32_t> feed;
+        if (!lists_valid) {
+            list_domains(all, evolved);
+            faces_valid = false;
+        }
+        const size_t cap = (size_t)tree.max_slots() * 2u * (kDepthLimit + 1u) + 2u * tree.max_slots();
+        if (all.size() > cap) return AMR_ERR_CAPACITY;
+        if (with_faces && !faces_valid) list_faces(faces, feed);
+        cudaError_t e = cudaSuccess;
         if (faces.size() > faces_cap) {
-            cudaError_t e = cudaStreamSynchronize(stream);
+            e = cudaStreamSynchronize(stream);
             cudaFree(d_faces);
             d_faces = nullptr;
             faces_cap = 0;
@@ -240,31 +266,31 @@ public:
             if (e != cudaSuccess) return cuda_status(e);
             faces_cap = faces.size();
         }
-        const size_t cap = (size_t)tree.max_slots() * 2u * ((size_t)1u << kDepthLimit) + 2u * tree.max_slots();
-        if (all.size() > cap) return AMR_ERR_CAPACITY;
-        cudaError_t e = cudaMemcpyAsync(d_lists, all.data(), all.size() * 4u, cudaMemcpyHostToDevice, stream);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(d_evolved, evolved.data(), evolved.size(), cudaMemcpyHostToDevice, stream);
-        if (e == cudaSuccess && kind == AMR_SIM_BSSN_EVOLVE)
-            e = cudaMemcpyAsync(d_feed, feed.data(), feed.size() * 4u, cudaMemcpyHostToDevice, stream);
-        if (e == cudaSuccess && !faces.empty())
-            e = cudaMemcpyAsync(d_faces, faces.data(), faces.size() * 4u, cudaMemcpyHostToDevice, stream);
+        auto upload = [&](void* to, const void* from, size_t bytes) {
+            if (e == cudaSuccess && bytes) e = cudaMemcpyAsync(to, from, bytes, cudaMemcpyHostToDevice, stream);
+        };
+        upload(d_lists, all.data(), all.size() * 4u);
+        upload(d_evolved, evolved.data(), evolved.size());
+        if (kind == AMR_SIM_BSSN_EVOLVE) upload(d_feed, feed.data(), feed.size() * 4u);
+        upload(d_faces, faces.data(), faces.size() * 4u);
         if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
         if (e != cudaSuccess) return cuda_status(e);
         lists_valid = true;
+        faces_valid |= with_faces;
         return AMR_OK;
     }
-    int prepare() {
+    int prepare(bool faces = false) {
         int st = sync_octree();
         if (st) return st;
         if (!items_valid) { lists_valid = false; items_valid = true; }
-        return build_lists();
+        return build_lists(faces);
     }
 
     // ---- phases
     int copy_back() override {
-        int st = prepare();
+        int st = prepare(true);   // the predictor's lists too: one upload
         if (st) return st;
-        const uint32_t s = tree.timer();
+        const uint32_t s = set_of(tree.timer());
         if (act_cnt[s] == 0) return AMR_OK;
         EvoRestrictArgs g;
         std::memset(&g, 0, sizeof(g));
@@ -289,10 +315,10 @@ public:
     }
     int modify_nodes() override { return AMR_OK; }
     int predictor() override {
-        int st = prepare();
+        int st = prepare(true);
         if (st) return st;
-        const uint32_t s = tree.timer();
-        if (evo_cnt[s] == 0) return AMR_OK;
+        const uint32_t s = tree.timer(), set = set_of(s);
+        if (evo_cnt[set] == 0) return AMR_OK;
         float* const* in[4] = {old_f, stage_f, new_f, stage_f};
         float* const* out[4] = {stage_f, new_f, stage_f, new_f};
         const float c_next[3] = {.5f, .5f, 1.f};
@@ -304,7 +330,7 @@ public:
             if (mode == AMR_MODE_PLAIN) {
                 // the plain per-domain form: each domain's stage launched alone
                 const uint32_t* base = a.items;
-                for (uint32_t i = 0; i < evo_cnt[s]; i++) {
+                for (uint32_t i = 0; i < evo_cnt[set]; i++) {
                     a.items = base + i;
                     a.n_items = 1;
                     if ((st = stage_update(a))) return st;
@@ -319,7 +345,7 @@ public:
         return AMR_OK;
     }
     int copy_bounds() override {
-        int st = prepare();
+        int st = prepare(true);
         if (st) return st;
         return fill(tree.timer(), new_f, 1.f, in_timestep ? stage_feeds(tree.timer()) : 0);
     }
@@ -327,7 +353,7 @@ public:
 
     int timestep() override {
         if (mode != AMR_MODE_GRAPH) return SimBase::timestep();
-        int st = prepare();
+        int st = prepare(true);
         if (st) return st;
         if (tree.timer() != 0u) return SimBase::timestep();
         const uint32_t nsub = 1u << tree.read_max_depth();
@@ -589,7 +615,7 @@ public:
         }
         if (!add_p.empty()) {
             // the parents' ghost layers feed the new domains' interpolation stencils at their faces
-            if ((st = prepare()) || (st = fill(tree.timer(), new_f, 1.f, 0))) return st;
+            if ((st = prepare(true)) || (st = fill(tree.timer(), new_f, 1.f, 0))) return st;
             tree.begin_batch();
             for (size_t i = 0; i < add_p.size(); i++) tree.add_node(add_p[i], add_o[i]);
             tree.end_batch();
@@ -599,7 +625,7 @@ public:
         graph_valid = false;
         if (!rem.empty() || !add_p.empty()) {
             // the ghost cells from the new neighbours, in both state buffers
-            if ((st = prepare()) || (st = fill(tree.timer(), new_f, 1.f, 0)) || (st = sync_old())) return st;
+            if ((st = prepare(true)) || (st = fill(tree.timer(), new_f, 1.f, 0)) || (st = sync_old())) return st;
         }
         if (stats) {
             stats[0] = refined;
@@ -626,8 +652,9 @@ private:
             a.acc[f] = acc[f];
         }
         a.positions = d_positions;
-        a.items = d_lists + (evo_off.empty() ? 0u : evo_off[s]);
-        a.n_items = a.n_batch = evo_cnt.empty() ? 0u : evo_cnt[s];
+        const uint32_t set = set_of(s);
+        a.items = d_lists + (evo_off.empty() ? 0u : evo_off[set]);
+        a.n_items = a.n_batch = evo_cnt.empty() ? 0u : evo_cnt[set];
         a.n = dims.n;
         a.p = dims.p;
         a.t = dims.t;
@@ -648,14 +675,16 @@ private:
     // least two of the fill's launches fall away: 9 domains of 8^3 in a periodic box 131 -> 97 us a root step,
     // but without periodic faces, where the outer domains' y and z faces stay in the fill, 83 -> 91.
     int stage_feeds(uint32_t s) const {
-        const int axes = kind == AMR_SIM_BSSN_EVOLVE ? evo_stage_feeds(dims.n, evo_cnt[s]) : 0;
+        const uint32_t set = set_of(s);
+        const int axes = kind == AMR_SIM_BSSN_EVOLVE ? evo_stage_feeds(dims.n, evo_cnt[set]) : 0;
         int gone = 0;
-        for (int a = 0; a < 3; a++) gone += face_interp[3 + a][s] + face_copy[3 + a][s] == 0u;
+        for (int a = 0; a < 3; a++) gone += face_interp[3 + a][set] + face_copy[3 + a][set] == 0u;
         return axes == 3 && dims.n != 32u && gone < 2 ? 0 : axes;
     }
     // fed_axes: the stage before wrote the fed faces of so many axes
     int fill(uint32_t s, float* const* x, float c_stage, int fed_axes) {
-        if (evo_cnt[s] == 0) return AMR_OK;
+        const uint32_t set = set_of(s);
+        if (evo_cnt[set] == 0) return AMR_OK;
         EvoGhostArgs g;
         std::memset(&g, 0, sizeof(g));
         for (int f = 0; f < nf; f++) { g.X[f] = x[f]; g.old_f[f] = old_f[f]; g.new_f[f] = new_f[f]; }
@@ -686,9 +715,9 @@ private:
                 continue;
             }
             const int list = axis < fed_axes ? 3 + axis : axis;
-            g.faces = d_faces + face_off[list][s];
-            g.n_interp = face_interp[list][s];
-            g.n_copy = face_copy[list][s];
+            g.faces = d_faces + face_off[list][set];
+            g.n_interp = face_interp[list][set];
+            g.n_copy = face_copy[list][set];
             if (g.n_interp + g.n_copy == 0u) continue;
             const int st = check(launch_evo_ghost(g, stream));
             if (st) return st;
@@ -727,10 +756,10 @@ private:
     uint32_t* d_lists = nullptr;
     double* d_part = nullptr;
     double* d_norms = nullptr;
-    bool lists_valid = false;
+    bool lists_valid = false, faces_valid = false;
     uint32_t* d_faces = nullptr;   // the ghost fill's face lists
     size_t faces_cap = 0;
-    std::vector<uint32_t> face_off[6], face_interp[6], face_copy[6];   // per axis (3 ..: without the fed faces) and substep
+    std::vector<uint32_t> face_off[6], face_interp[6], face_copy[6];   // per axis (3 ..: without the fed faces) and set
     int32_t* d_feed = nullptr;     // EvoArgs::feed
     std::vector<uint8_t> fed;      // per slot, axis and side: the face is written by its source's stage
     std::vector<uint32_t> act_off, act_cnt, act_leaves, evo_off, evo_cnt, leaves;
