@@ -475,7 +475,7 @@ public:
         if ((st = take_device_error(err_flag))) return st;
         deriv_zs = best;
         tuned_ctas.assign(1, {all_evolved_cnt, best});
-        graph_valid = false;
+        if (!bssn) graph_valid = false;   // a timestep launches no constraints: its capture holds
         if (n_tuned) *n_tuned = 1;
         return AMR_OK;
     }
