@@ -74,8 +74,10 @@ enum BssnDeriv : int {
     D_AT1 = 45,                   // d_k A_ij at D_AT1 + 3 c + k (6 components)
     BSSN_ND = 63
 };
-// Planes of the derivative scratch (amr_sim_buffer 5), which the tuning call writes.
-constexpr int kBssnScratch = 111, kWaveScratch = 3;
+// Planes of the scratch (amr_sim_buffer 5), which the tuning call alone writes: the four constraints, or the wave's
+// two padded fields.  (Derivatives are stored nowhere: their 111 planes were a third of a 16^3 simulation's
+// memory.)
+constexpr int kBssnScratch = 4, kWaveScratch = 3;
 
 // Physics and gauge choices (the C ABI's amr_evolution, resolved).
 struct EvoParams {

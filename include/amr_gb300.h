@@ -368,7 +368,8 @@ int amr_sim_kernel_timing(amr_sim* s, double* ms, uint64_t* launches);
 /* Buffers of these simulations (amr_sim_buffer, comp = field): which 0 the state at the start of
  * the current step (padded), 1 the latest state (padded), 2 the RK stage state (padded), 3 the RK
  * accumulator (inner layout), 4 the constraints H, M_x, M_y, M_z (inner layout, comp 0..3, written
- * by amr_sim_constraint_norms), 5 scratch planes (inner layout; written by amr_sim_autotune).  The BSSN fields chi,
+ * by amr_sim_constraint_norms), 5 scratch planes (inner layout, comp 0..3, of the wave 0..2; written by
+ * amr_sim_autotune).  The BSSN fields chi,
  * gt_xx, gt_yy, gt_zz and alpha are stored less 1 (their deviation from flat space), which keeps
  * single-precision rounding relative to the deviation. */
 #define AMR_SLICING_1PLUSLOG 0  /* d_t alpha = beta.d alpha - 2 alpha K */
