@@ -117,6 +117,7 @@ struct EvoArgs {
     // first or last three layers, written with them (-1: none).  A domain in a later axis's entry takes the
     // ghosts along the earlier axes too (all of this domain's are fed).  nullptr: no feeding
     const int32_t* feed;
+    int feed_axes;                // axes along which the feed table is followed: 0, 2 or 3
     float dt0;                    // dt at depth 0
     int stage;                    // 1..4
     uint32_t deriv_zs;            // interior z-planes per CTA of the wave's stage and the constraints (0: the default)

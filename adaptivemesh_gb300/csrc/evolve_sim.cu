@@ -327,6 +327,7 @@ public:
             // the last stage's ghosts belong to copy_bounds(), which a timestep calls next
             const int feeding = stage < 4 || in_timestep ? stage_feeds(s) : 0;
             if (feeding) a.feed = d_feed;
+            a.feed_axes = feeding;
             if (mode == AMR_MODE_PLAIN) {
                 // the plain per-domain form: each domain's stage launched alone
                 const uint32_t* base = a.items;
@@ -670,17 +671,19 @@ private:
     int stage_update(const EvoArgs& a) {   // one RK stage
         return check(kind == AMR_SIM_BSSN_EVOLVE ? launch_evo_stage_bssn(a, stream) : launch_evo_stage_wave(a, stream));
     }
-    // ghost fill of `x` (the state at c_stage of the active domains' step), three axis passes
-    // Axes whose fed faces substep s's stages write.  The small tiles (8^3 and 16^3, three axes) feed where at
-    // least two of the fill's launches fall away: 9 domains of 8^3 in a periodic box 131 -> 97 us a root step,
-    // but without periodic faces, where the outer domains' y and z faces stay in the fill, 83 -> 91.
+    // Axes whose fed faces substep s's stages write.  Where fewer than two of the fill's launches fall away (trees
+    // with faces on an open boundary or beside coarser domains), three axes lose to the other choices: a root step
+    // of 9 domains of 8^3 in an open box 208 us without feeding and 234 with, of 16^3 271 and 280; the
+    // small tiles then feed nothing.  At 32^3 (940 us with three axes, 913 with two, 1 095 without; an uneven
+    // tree of 16 domains 3.13, 3.02, 3.20 ms) x and y are fed in any case.
     int stage_feeds(uint32_t s) const {
         const uint32_t set = set_of(s);
         const int axes = kind == AMR_SIM_BSSN_EVOLVE ? evo_stage_feeds(dims.n, evo_cnt[set]) : 0;
         int gone = 0;
         for (int a = 0; a < 3; a++) gone += face_interp[3 + a][set] + face_copy[3 + a][set] == 0u;
-        return axes == 3 && dims.n != 32u && gone < 2 ? 0 : axes;
+        return axes == 3 && gone < 2 ? (dims.n == 32u ? 2 : 0) : axes;
     }
+    // Ghost fill of `x` (the state at c_stage of the active domains' step), three axis passes.
     // fed_axes: the stage before wrote the fed faces of so many axes
     int fill(uint32_t s, float* const* x, float c_stage, int fed_axes) {
         const uint32_t set = set_of(s);

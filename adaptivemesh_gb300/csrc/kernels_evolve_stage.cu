@@ -787,14 +787,15 @@ bool evo_stage_small(uint32_t n, uint32_t n_batch, int sms) {
 }  // namespace
 
 // Axes whose ghost layers a stage writes, for a substep of n_batch domains.  All three where launches count (the
-// small tiles) and at 32^3, whose surface is small beside its volume; along x and y elsewhere, where the z
-// layers' stores, 256 a plane and field all at once, cost more than the fill's pass: a root step of 585
-// domains of 16^3 22.0 ms with two axes and 24.3 with three, but of 9 domains 178 and 154 us; 9 domains of
-// 32^3 728 and 681 us.
+// small tiles, and at 32^3 up to as many domains as at 16^3); along x and y elsewhere, where the z layers'
+// stores, N^2 a plane and field all at once, cost more than the fill's pass.  A root step (GB300, cold caches,
+// periodic, so that every face is fed) with 0, 1, 2 and 3 axes: 9 domains of 8^3 188, 165, 152, 142 us, 73 492,
+// 422, 384, 363, 585 5.14, 4.61, 4.56, 5.49 ms; 9 of 16^3 244, 199, 173, 150 us, 73 1.75, 1.58, 1.53, 1.59 ms,
+// 585 24.8, 21.4, 20.7, 22.8; 9 of 32^3 930, 771, 681, 646 us, 73 10.56, 8.99, 8.73, 8.99 ms, 585 164, 137, 134, 140.
 int evo_stage_feeds(uint32_t n, uint32_t n_batch) {
     int dev = 0, sms = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
-    return n == 32u || evo_stage_small(n, n_batch, sms) ? 3 : 2;
+    return evo_stage_small(n == 32u ? 16u : n, n_batch, sms) ? 3 : 2;
 }
 cudaError_t launch_evo_stage_bssn(const EvoArgs& a, cudaStream_t st) {
     if (a.n_items == 0u) return cudaSuccess;
@@ -818,7 +819,7 @@ cudaError_t launch_evo_stage_bssn(const EvoArgs& a, cudaStream_t st) {
             if (evo_stage_small(16, a.n_batch, sms))
                 return a.feed ? stage_t<16, 16, 1, 5, V1, 1, 3>(a, sms, st) : stage_t<16, 16, 1, 5, V1, 1, 0>(a, sms, st);
             return stage_t<16, 16, 2, 6, V2, 1, 2>(a, sms, st);
-        case 32: return stage_t<32, 8, 2, 6, V2, 1, 3>(a, sms, st);
+        case 32: return a.feed_axes == 3 ? stage_t<32, 8, 2, 6, V2, 1, 3>(a, sms, st) : stage_t<32, 8, 2, 6, V2, 1, 2>(a, sms, st);
         default: return cudaErrorInvalidValue;
     }
 }
@@ -833,7 +834,9 @@ cudaError_t prepare_evo_stage_bssn(uint32_t n) {
             e = limit_t<16, 16, 1, 5, V1, 1, 3>();
             if (e == cudaSuccess) e = limit_t<16, 16, 1, 5, V1, 1, 0>();
             return e == cudaSuccess ? limit_t<16, 16, 2, 6, V2, 1, 2>() : e;
-        case 32: return limit_t<32, 8, 2, 6, V2, 1, 3>();
+        case 32:
+            e = limit_t<32, 8, 2, 6, V2, 1, 3>();
+            return e == cudaSuccess ? limit_t<32, 8, 2, 6, V2, 1, 2>() : e;
         default: return e;
     }
 }
