@@ -436,7 +436,7 @@ public:
         if (n_tuned) *n_tuned = 0;
         if (capturing || reps == 0u || reps > 100u) return AMR_ERR_INVALID;
         int st = wait_side(-1, 0);
-        if (!st) st = prepare();
+        if (!st) st = prepare(true);   // also the lists of the timesteps that follow
         if (st) return st;
         if (all_evolved_cnt == 0u) return AMR_OK;
         uint32_t cand[4];

@@ -26,3 +26,19 @@ def test_uploads_after_a_tree_change(am, tmp_path):
     sets = out["depth"] + 1
     most = out["slots"] * (4 + 32 + 48 + 1 + 24) + 4 * out["used"] * (2 * sets + 2 + 2 * 6 * sets)
     assert out["norms"] <= most and out["timestep"] <= most, (out, most)
+
+
+def test_nothing_is_listed_after_tuning(am, tmp_path):
+    """amr_sim_autotune lists what the timesteps that follow need: the first of them uploads nothing."""
+    out = fake_cuda.run(tmp_path, """
+        out = []
+        for kind in (am.SIM_BSSN_EVOLVE, am.SIM_WAVE_RK4):
+            sim = am.Sim(am.Config(16, 3, 1.0), kind, slots=64, mode=am.MODE_GRAPH)
+            cases.tree_uneven(sim)
+            sim.autotune(2)
+            fake.fake_reset(0)
+            sim.timestep()
+            out.append(fake.fake_uploaded())
+        print(json.dumps(out))
+    """)
+    assert out == [0, 0]
