@@ -18,6 +18,7 @@
 // stage (stages 2 and 4), all padded; the RK accumulator (inner layout).
 #include <algorithm>
 #include <cmath>
+#include <numeric>
 
 #include "evolve_kernels.h"
 #include "sim_base.h"
@@ -130,9 +131,9 @@ public:
     }
 
     // ---- lists: active domains (restriction) and active evolved domains.  The domains active at a substep depend on
-    // its trailing zeros alone, so that there are as many lists as depths.  (Host time of the constraint norms after
-    // a change of a tree of depth 6 and 1 569 domains, on an x86 core: 7.9 ms and 3.9 MB of uploads with a
-    // list and the faces per substep, 0.14 ms now; of a timestep's lists 7.7 and 1.3 ms.)
+    // its trailing zeros alone, so that there are as many lists as depths.  (Host time after a change of a tree of
+    // depth 6 and 1 569 domains, on an x86 core: 7.9 ms and 3.9 MB of uploads with lists per substep, 0.4 ms
+    // now; 585 domains of depth 3 0.24 and 0.13 ms.)
     uint32_t set_of(uint32_t substep) const {
         const uint32_t md = (uint32_t)tree.read_max_depth();
         uint32_t k = 0;
@@ -182,20 +183,27 @@ public:
         leaves_off = (uint32_t)all.size();
         all.insert(all.end(), leaves.begin(), leaves.end());
     }
-    // ---- the ghost fill's face lists and the feed table, for the calls that step or fill
+    // ---- the ghost fill's face lists and the feed table
     void list_faces(std::vector<uint32_t>& faces, std::vector<int32_t>& feed) {
         const uint32_t md = (uint32_t)tree.read_max_depth(), used = tree.curr_used_slots(), sets = md + 1u;
-        auto depth_of = [&](uint32_t i) { return pos_depth_host(tree.positions()[i]); };   // -1: no domain
+        std::vector<int8_t> depth(used);      // -1: no domain
+        std::vector<uint8_t> cls(6u * used);  // face_class, [2 axis + side]
+        for (uint32_t i = 0; i < used; i++) {
+            depth[i] = (int8_t)pos_depth_host(tree.positions()[i]);
+            for (uint32_t f = 0; f < 6u && depth[i] != -1; f++) cls[6u * i + f] = (uint8_t)face_class(i, (int)(f / 2u), f & 1u);
+        }
         // the ghost fill's faces per set and axis: interpolating ones first, then copies
         std::vector<uint32_t> copies;
+        copies.reserve(2u * used);
+        faces.reserve(12u * std::accumulate(evo_cnt.begin(), evo_cnt.end(), (size_t)0));
         for (int a = 0; a < 3; a++) { face_off[a].assign(sets, 0); face_interp[a].assign(sets, 0); face_copy[a].assign(sets, 0); }
         for (uint32_t s = 0; s < sets; s++)
             for (int a = 0; a < 3; a++) {
                 copies.clear();
                 face_off[a][s] = (uint32_t)faces.size();
                 for (uint32_t i = 0; i < used; i++)
-                    for (uint32_t side = 0; side < 2 && depth_of(i) != -1 && md - (uint32_t)depth_of(i) <= s; side++) {
-                        const int c = face_class(i, a, side);
+                    for (uint32_t side = 0; side < 2 && md - (uint32_t)depth[i] <= s; side++) {   // (no domain has class 0)
+                        const int c = cls[6u * i + 2u * (uint32_t)a + side];
                         if (c) (c == 2 ? faces : copies).push_back(i << 1 | side);
                     }
                 face_interp[a][s] = (uint32_t)faces.size() - face_off[a][s];
@@ -209,12 +217,12 @@ public:
         fed.assign(6u * tree.max_slots(), 0);
         for (uint32_t a = 0; a < 3; a++)
             for (uint32_t i = 0; i < used && kind == AMR_SIM_BSSN_EVOLVE; i++)
-                for (uint32_t side = 0; side < 2 && depth_of(i) != -1; side++) {
-                    if (face_class(i, (int)a, side) != 1) continue;
+                for (uint32_t side = 0; side < 2; side++) {
+                    if (cls[6u * i + 2u * a + side] != 1) continue;
                     const uint64_t bd = tree.boundaries()[(size_t)i * 6u + a + 3u * side];
                     const uint32_t src = (uint32_t)bd & 0xFFFFFFu, w = (uint32_t)(bd >> 32);
-                    if (src >= used || depth_of(src) == -1 || feed[6u * src + 2u * a + side] != -1) continue;
-                    if (depth_of(i) != (int)((uint32_t)bd >> 28) || depth_of(i) != depth_of(src)) continue;
+                    if (src >= used || depth[src] == -1 || feed[6u * src + 2u * a + side] != -1) continue;
+                    if (depth[i] != (int)((uint32_t)bd >> 28) || depth[i] != depth[src]) continue;
                     // the offset (tensors.h:335-348): -1 along the axis for the + face, whose first source layer is the first
                     bool along = true;
                     for (uint32_t c = 0; c < 3; c++) {
@@ -244,18 +252,15 @@ public:
             }
         }
     }
-    int build_lists(bool with_faces) {
-        if (lists_valid && (faces_valid || !with_faces)) return AMR_OK;
+    int build_lists() {
+        if (lists_valid) return AMR_OK;
         std::vector<uint32_t> all, faces;
         std::vector<uint8_t> evolved;
         std::vector<int32_t> feed;
-        if (!lists_valid) {
-            list_domains(all, evolved);
-            faces_valid = false;
-        }
+        list_domains(all, evolved);
+        list_faces(faces, feed);
         const size_t cap = (size_t)tree.max_slots() * 2u * (kDepthLimit + 1u) + 2u * tree.max_slots();
         if (all.size() > cap) return AMR_ERR_CAPACITY;
-        if (with_faces && !faces_valid) list_faces(faces, feed);
         cudaError_t e = cudaSuccess;
         if (faces.size() > faces_cap) {
             e = cudaStreamSynchronize(stream);
@@ -276,19 +281,18 @@ public:
         if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
         if (e != cudaSuccess) return cuda_status(e);
         lists_valid = true;
-        faces_valid |= with_faces;
         return AMR_OK;
     }
-    int prepare(bool faces = false) {
+    int prepare() {
         int st = sync_octree();
         if (st) return st;
         if (!items_valid) { lists_valid = false; items_valid = true; }
-        return build_lists(faces);
+        return build_lists();
     }
 
     // ---- phases
     int copy_back() override {
-        int st = prepare(true);   // the predictor's lists too: one upload
+        int st = prepare();
         if (st) return st;
         const uint32_t s = set_of(tree.timer());
         if (act_cnt[s] == 0) return AMR_OK;
@@ -315,7 +319,7 @@ public:
     }
     int modify_nodes() override { return AMR_OK; }
     int predictor() override {
-        int st = prepare(true);
+        int st = prepare();
         if (st) return st;
         const uint32_t s = tree.timer(), set = set_of(s);
         if (evo_cnt[set] == 0) return AMR_OK;
@@ -346,7 +350,7 @@ public:
         return AMR_OK;
     }
     int copy_bounds() override {
-        int st = prepare(true);
+        int st = prepare();
         if (st) return st;
         return fill(tree.timer(), new_f, 1.f, in_timestep ? stage_feeds(tree.timer()) : 0);
     }
@@ -354,7 +358,7 @@ public:
 
     int timestep() override {
         if (mode != AMR_MODE_GRAPH) return SimBase::timestep();
-        int st = prepare(true);
+        int st = prepare();
         if (st) return st;
         if (tree.timer() != 0u) return SimBase::timestep();
         const uint32_t nsub = 1u << tree.read_max_depth();
@@ -436,7 +440,7 @@ public:
         if (n_tuned) *n_tuned = 0;
         if (capturing || reps == 0u || reps > 100u) return AMR_ERR_INVALID;
         int st = wait_side(-1, 0);
-        if (!st) st = prepare(true);   // also the lists of the timesteps that follow
+        if (!st) st = prepare();
         if (st) return st;
         if (all_evolved_cnt == 0u) return AMR_OK;
         uint32_t cand[4];
@@ -616,7 +620,7 @@ public:
         }
         if (!add_p.empty()) {
             // the parents' ghost layers feed the new domains' interpolation stencils at their faces
-            if ((st = prepare(true)) || (st = fill(tree.timer(), new_f, 1.f, 0))) return st;
+            if ((st = prepare()) || (st = fill(tree.timer(), new_f, 1.f, 0))) return st;
             tree.begin_batch();
             for (size_t i = 0; i < add_p.size(); i++) tree.add_node(add_p[i], add_o[i]);
             tree.end_batch();
@@ -626,7 +630,7 @@ public:
         graph_valid = false;
         if (!rem.empty() || !add_p.empty()) {
             // the ghost cells from the new neighbours, in both state buffers
-            if ((st = prepare(true)) || (st = fill(tree.timer(), new_f, 1.f, 0)) || (st = sync_old())) return st;
+            if ((st = prepare()) || (st = fill(tree.timer(), new_f, 1.f, 0)) || (st = sync_old())) return st;
         }
         if (stats) {
             stats[0] = refined;
@@ -759,7 +763,7 @@ private:
     uint32_t* d_lists = nullptr;
     double* d_part = nullptr;
     double* d_norms = nullptr;
-    bool lists_valid = false, faces_valid = false;
+    bool lists_valid = false;
     uint32_t* d_faces = nullptr;   // the ghost fill's face lists
     size_t faces_cap = 0;
     std::vector<uint32_t> face_off[6], face_interp[6], face_copy[6];   // per axis (3 ..: without the fed faces) and set
