@@ -424,8 +424,6 @@ __global__ void __launch_bounds__(StageShape<N, TY, TZ, R_, V::L>::CT, MINB)
                         cl[i][si(j, l)] = w;
                     }
 #pragma unroll
-            for (int c = 0; c < 6; c++) Rc[c] = -.5f * back(P_T + 18 + c);
-#pragma unroll
             for (int i = 0; i < 3; i++)
 #pragma unroll
                 for (int c = 0; c < 6; c++)
@@ -439,8 +437,10 @@ __global__ void __launch_bounds__(StageShape<N, TY, TZ, R_, V::L>::CT, MINB)
 #pragma unroll
                 for (int j = i; j < 3; j++)
 #pragma unroll
-                    for (int l = 0; l < 3; l++)
-                        Rc[si(i, j)] = fma(gd[l], cl[i][si(j, l)] + cl[j][si(i, l)], Rc[si(i, j)]);
+                    for (int l = 0; l < 3; l++) {
+                        const V w = cl[i][si(j, l)] + cl[j][si(i, l)];
+                        Rc[si(i, j)] = l == 0 ? gd[l] * w : fma(gd[l], w, Rc[si(i, j)]);
+                    }
             // gt^lm (Gt^k_li Gt_jkm + Gt^k_lj Gt_ikm + Gt^k_im Gt_klj): with Q_i^km = gt^ml Gt^k_li the
             // three terms are Q_i^km Gt_jkm, Q_j^km Gt_ikm and Q_i^km Gt_kmj
 #pragma unroll
@@ -469,6 +469,10 @@ __global__ void __launch_bounds__(StageShape<N, TY, TZ, R_, V::L>::CT, MINB)
                     Rc[si(i, j)] = r;
                 }
             }
+            // the second derivatives' part last: the terms above are small beside it, and would each be
+            // rounded at its size
+#pragma unroll
+            for (int c = 0; c < 6; c++) Rc[c] = fma(-.5f, back(P_T + 18 + c), Rc[c]);
         }
         const int32_t dxyz = FEED > 2 ? next_domain(dxy, 2, sz) : -1;
         // ---- the conformal factor and the lapse
@@ -539,16 +543,22 @@ __global__ void __launch_bounds__(StageShape<N, TY, TZ, R_, V::L>::CT, MINB)
             const V s = (-4.f / 3.f) * alpha, k0 = back(P_T + 9), k1 = back(P_T + 10), k2 = back(P_T + 11);
             const V ha = .5f * alpha;
 #pragma unroll
+            V t[6];   // summed by themselves and unscaled: one rounding at the size of the whole
+#pragma unroll
             for (int l = 0; l < 3; l++) {
                 V e[3];
 #pragma unroll
-                for (int j = 0; j < 3; j++) e[j] = ha * back(P_T + 3 * l + j);
+                for (int j = 0; j < 3; j++) e[j] = back(P_T + 3 * l + j);
 #pragma unroll
                 for (int i = 0; i < 3; i++)
 #pragma unroll
-                    for (int j = i; j < 3; j++)
-                        Rc[si(i, j)] = fma(g[si(l, i)], e[j], fma(g[si(l, j)], e[i], Rc[si(i, j)]));
+                    for (int j = i; j < 3; j++) {
+                        const V w = g[si(l, j)] * e[i];
+                        t[si(i, j)] = fma(g[si(l, i)], e[j], l == 0 ? w : fma(g[si(l, j)], e[i], t[si(i, j)]));
+                    }
             }
+#pragma unroll
+            for (int c = 0; c < 6; c++) Rc[c] = fma(ha, t[c], Rc[c]);
 #pragma unroll
             for (int c = 0; c < 6; c++) keep(P_X + c, Rc[c]);
 #pragma unroll
