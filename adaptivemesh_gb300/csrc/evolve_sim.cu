@@ -434,8 +434,8 @@ public:
     }
     // Launch-shape tuning (amr_sim_autotune): the depth (interior z-planes per CTA) of the wave's stage
     // kernel, or of the BSSN constraints' tiles, timed at every compiled depth over all evolved domains, reps
-    // launches each with CUDA events; the fastest is kept.  Only the derivative scratch is written, so
-    // the state is unchanged.
+    // launches each with CUDA events; the fastest is kept.  Only the scratch is written, so the state is
+    // unchanged.
     int autotune(uint32_t reps, uint32_t* n_tuned) override {
         if (n_tuned) *n_tuned = 0;
         if (capturing || reps == 0u || reps > 100u) return AMR_ERR_INVALID;
@@ -448,7 +448,7 @@ public:
         const size_t inner = (size_t)tree.max_slots() * dims.n * dims.n * dims.n;
         const size_t padded = (size_t)tree.max_slots() * dims.t * dims.t * dims.t;
         const bool bssn = kind == AMR_SIM_BSSN_EVOLVE;
-        // the results go to the derivative scratch: the constraints' four planes, or the wave's two
+        // the results go to the scratch: the constraints' four planes, or the wave's two
         // fields (stage 4, which writes nothing else)
         float* to[kMaxFields] = {};
         ConsPtrs cons_to = {};

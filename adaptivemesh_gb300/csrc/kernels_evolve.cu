@@ -52,8 +52,8 @@ __global__ void k_evo_init(EvoInitArgs a) {
 // ------------------------------------------------------------------ one RK4 stage of the wave
 // A CTA per (domain, slab of ZS interior z-planes): the padded planes (ZS + 6) of u and v, one bulk copy
 // each, then per cell the Laplacian, the Kreiss-Oliger terms, the right-hand side and the stage update.
-// A derivative pass and an update kernel took 9 us a stage on 15 domains of 16^3, most of it their two
-// launches.  ZS is a launch-shape choice (amr_sim_autotune times the compiled ones); the default takes
+// (With a derivative pass and an update kernel, a root step of a root and one child of 16^3 took 62.3 us a pass,
+// with this 54.8, most of it launches that depend on one another.)  ZS is a launch-shape choice (amr_sim_autotune times the compiled ones); the default takes
 // two cells per thread at 16^3, one at 8^3, four at 32^3.
 constexpr int wave_default_zs(int n) { return n == 8 ? 4 : (n == 16 ? 2 : 1); }
 template <int N, int ZS>

@@ -20,13 +20,12 @@
 // The values of the first and last three layers of cells along an axis are also written to the ghost layers of
 // the same-depth neighbours that copy them (EvoArgs::feed), edges and corners by way of two or three of them.
 // A fill of those layers by itself reads what was just written, along x in 12-byte runs: x 124, y 54 and z 47 us
-// a stage of the uniform depth-3 tree, a root step 24.7 ms; with x fed 21.4, with x and y 20.2
-// (evo_stage_feeds has the rule).
+// a stage of the uniform depth-3 tree (evo_stage_feeds has the rule and a root step's times).
 //
 // Measured on a GB300, 585 domains of 16^3 (2.40 M cells), one stage: 779 us for the two kernels it
-// replaces (317 + 462 on average over the stages), 470 us now and 545 with the fed ghosts; a root step of the
-// uniform depth-3 tree 38.4 -> 28.2 ms (20.2 with the other kernels' changes and the fed ghosts).  What
-// bounds it: the latency of eight warps (38 % of the issue slots, 54 % of the shared-memory pipe, about 1 180
+// replaces (317 + 462 on average over the stages), 470 us by itself and 545 with x and y fed; a root step of the
+// uniform depth-3 tree 38.4 -> 28.2 ms with this kernel alone, 20.1 now with the fed ghosts and the other
+// kernels' changes.  What bounds it: the latency of eight warps (38 % of the issue slots, 54 % of the shared-memory pipe, about 1 180
 // wavefronts per 32 cells) in the visits and, in the update, the memory traffic that all SMs issue at the
 // same time; the two do not overlap, as a CTA's registers and columns fill its SM.  One cell a thread and
 // twice the warps gave 30.0 ms; the update spread over the next tile's visits was 3 % faster with warm
@@ -812,10 +811,11 @@ cudaError_t launch_evo_stage_bssn(const EvoArgs& a, cudaStream_t st) {
     if (a.stage < 1 || a.stage > 4) return cudaErrorInvalidValue;
     // The tile: 512 cells of whole planes at 16^3 and 8^3 (one copy a field; 8 rows of two planes at 32^3,
     // where whole planes would be 1024 threads), except where the domains are too few to give every SM
-    // such a tile.  Then smaller tiles of one cell a thread, with more CTAs: at 8^3, 9 domains, a root
-    // step of 248 -> 201 us, 73 domains 669 -> 622, but 585 domains 6.98 -> 7.33 ms; at 16^3, 9 domains
-    // 285 -> 250 us, 73 domains 2.00 -> 2.33 ms.  A domain of 32^3 has 64 tiles.  The rule reads the
-    // substep's domains, not this launch's, so that a domain launched alone rounds as in a batch.
+    // such a tile.  Then smaller tiles of one cell a thread, with more CTAs.  A root step (periodic, cold caches, the
+    // better number of fed axes on either side), large and small tiles: at 8^3, 9 domains 204 and 142 us,
+    // 73 domains 445 and 363, 585 domains 4.57 and 4.75 ms; at 16^3, 9 domains 200 and 150 us, 73 domains
+    // 1.53 and 1.85 ms.  A domain of 32^3 has 64 tiles.  The rule reads the substep's domains, not this
+    // launch's, so that a domain launched alone rounds as in a batch.
     int dev = 0, sms = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);

@@ -340,15 +340,15 @@ int amr_sim_set_stencil_ctas(amr_sim* s, uint32_t ctas);
  *   allocated for the call.
  *   AMR_SIM_BSSN_EVOLVE / AMR_SIM_WAVE_RK4: the depth (interior z-planes per CTA: 1, 2 or 4 at 16^3; 4 or
  *   8 at 8^3; 1 at 32^3) of the constraint pass's tiles (amr_sim_constraint_norms) or of the wave's RK
- *   stage, timed over every evolved domain; only the derivative scratch is written.
+ *   stage, timed over every evolved domain; only the scratch planes (buffer 5) are written.
  * The simulation's state is unchanged.  *n_tuned = shapes tuned.  AMR_SIM_WAVE: AMR_ERR_INVALID. */
 int amr_sim_autotune(amr_sim* s, uint32_t reps, uint32_t* n_tuned);
 /* The tuned pairs, up to capacity: (active domains, CTAs of the fused pass) for AMR_SIM_BSSN,
- * (evolved domains, z-planes per derivative slab) for the evolution kinds; *count = how many
+ * (evolved domains, z-planes per tile of the constraints or slab of the wave's stage) for the evolution kinds; *count = how many
  * there are (AMR_ERR_CAPACITY if more than capacity). */
 int amr_sim_tuned_shapes(const amr_sim* s, uint32_t capacity, uint32_t* domains, uint32_t* ctas, uint32_t* count);
-/* Optional timing of the dominant kernel (the derivative stencil) with CUDA events on the
- * simulation's stream.  amr_sim_kernel_timing returns the summed milliseconds and launch count
+/* Optional timing of the dominant kernel (the plugins' derivative stencil, the evolutions' whole RK stage) with
+ * CUDA events on the simulation's stream.  amr_sim_kernel_timing returns the summed milliseconds and launch count
  * since the last reset. */
 int amr_sim_enable_kernel_timing(amr_sim* s, int enable);
 int amr_sim_kernel_timing(amr_sim* s, double* ms, uint64_t* launches);
