@@ -468,8 +468,10 @@ __global__ void __launch_bounds__(StageShape<N, TY, TZ, R_, V::L>::CT, MINB)
                     Rc[si(i, j)] = r;
                 }
             }
-            // the second derivatives' part last: the terms above are small beside it, and would each be
-            // rounded at its size
+            // The second derivatives' part last: the terms above are small beside it, and would each be rounded at
+            // its size.  (With it first, and the connection functions' products added one by one, the errors against
+            // 64 bits were 0.8 % above those of the two kernels before after one step of 9 domains of 8^3, 0.1 %
+            // after eight; now 0.5 % above and 0.04 % below, means over 24 states and 18 fields.)
 #pragma unroll
             for (int c = 0; c < 6; c++) Rc[c] = fma(-.5f, back(P_T + 18 + c), Rc[c]);
         }
@@ -541,7 +543,6 @@ __global__ void __launch_bounds__(StageShape<N, TY, TZ, R_, V::L>::CT, MINB)
         {
             const V s = (-4.f / 3.f) * alpha, k0 = back(P_T + 9), k1 = back(P_T + 10), k2 = back(P_T + 11);
             const V ha = .5f * alpha;
-#pragma unroll
             V t[6];   // summed by themselves and unscaled: one rounding at the size of the whole
 #pragma unroll
             for (int l = 0; l < 3; l++) {
