@@ -459,9 +459,10 @@ public:
         f.old_f[0] = old_f; f.new_f[0] = new_f; f.ncomp = 1; f.early = 1;
         // In place where the substep's restriction covered every domain that is active now: the predictor writes
         // interiors alone, but new domains' old and new fields are interpolated separately, and where the
-        // triage took the deepest levels away the counter is another, at which more domains are active.
-        const bool restricted = in_timestep && !grown && tree.timer() == restricted_timer &&
-                                tree.read_max_depth() == restricted_depth;
+        // triage took the deepest levels away the counter is another, at which more domains are active.  Used slots
+        // without a domain keep their boundary records, which the fill follows, and are never restricted.
+        bool restricted = in_timestep && !grown && tree.timer() == restricted_timer && tree.read_max_depth() == restricted_depth;
+        for (uint32_t i = 0; i < tree.curr_used_slots() && restricted; i++) restricted = pos_depth_host(tree.positions()[i]) != -1;
         st = check(launch_copy_boundaries(dims, f, d_boundaries, tree.curr_used_slots(), tree.timer(),
                                           (uint32_t)tree.read_max_depth(), 1, ghost_stage, stream, restricted));
         if (!st && !restricted) launches++;

@@ -117,7 +117,8 @@ public:
     }
     // Set while timestep() runs its substeps: each copy_bounds then follows the substep's copy_back, so every
     // domain that was active there has old == new outside the cells its children cover.  Domains that
-    // modify_nodes() adds have not, nor those that become active as it removes the deepest levels.
+    // modify_nodes() adds have not, nor those that become active as it removes the deepest levels, nor
+    // used slots that hold no domain.
     bool in_timestep = false;
     virtual int buffer(int which, int comp, void** ptr, uint64_t* count) = 0;
     // Launch-shape autotuning (amr_sim_autotune): only the BSSN plugin has a tunable pass.

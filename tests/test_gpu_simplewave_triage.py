@@ -80,3 +80,48 @@ def test_fill_after_the_deepest_levels_are_removed(am, cuda):
         assert np.count_nonzero(x != y) == 0, f"buffer {which}: {np.count_nonzero(x != y)} of {cells} words differ"
     whole.close()
     phased.close()
+
+
+def test_fill_with_slots_that_hold_no_domain(am, cuda):
+    """Slots whose domain was removed keep their boundary records, and the fill follows them though no restriction covered
+    their sources: one timestep against the phases called one by one, every word of the used slots bit for bit."""
+    import torch
+    cfg = am.Config(28, 2, 100.0)
+    t = cfg.total
+    sims = []
+    for _ in range(2):
+        sim = am.Sim(cfg, am.SIM_WAVE, slots=64, mode=am.MODE_BATCHED)
+        for c in range(8):
+            sim.add_node(0, c)
+        first = int(sim.state()["children"][0])
+        for c in range(8):
+            sim.add_node(first, c)
+        gone = [int(v) for v in sim.state()["children"][first * 8: first * 8 + 4]]
+        sim.remove_nodes(gone)
+        sim.synchronize()
+        st = sim.state()
+        used = st["used_slots"]
+        assert used == 17 and np.count_nonzero(st["positions"][:used] == 0xFFFFFFFF) == 4
+        rng = np.random.default_rng(3)
+        for which, far in ((am.Sim.OLD, 1e6), (am.Sim.NEW, 0.)):   # the live domains nearly flat: the tree stays
+            f = (.5 + 1e-4 * rng.random((used, t ** 3))).astype(np.float32)
+            f[gone] += np.float32(far)
+            sim.tensor(which)[: used * t ** 3].copy_(torch.from_numpy(f.reshape(-1)))
+        torch.cuda.synchronize()
+        sims.append(sim)
+    whole, phased = sims
+    whole.timestep()
+    while True:
+        for ph in PHASES:
+            phased.phase(getattr(am, "PHASE_" + ph))
+        if phased.state()["timer"] == 0:
+            break
+    whole.synchronize()
+    phased.synchronize()
+    a, b = whole.state(), phased.state()
+    assert all(np.array_equal(a[k], b[k]) for k in a) and a["used_slots"] == used
+    for which in (am.Sim.NEW, am.Sim.OLD):
+        x, y = (s.tensor(which)[: used * t ** 3].cpu().numpy().view(np.uint32) for s in sims)
+        assert np.count_nonzero(x != y) == 0, f"buffer {which}: {np.count_nonzero(x != y)} words differ"
+    whole.close()
+    phased.close()
