@@ -438,6 +438,8 @@ public:
         }
         for (uint32_t i = 0, s = used * 8u; i < s; i++) {
             const float weight = ay * 3.f / (1.f - urgency);
+            // a domain that went with its parent above keeps its values, but nothing can be added to it
+            if (pos_depth_host(tree.positions()[i >> 3u]) == -1) continue;
             if (c[i] > weight && tree.children()[i] == -1) {
                 tree.add_node((int32_t)(i >> 3u), (int32_t)(i & 7u));
                 grown = true;
